@@ -327,7 +327,7 @@ def run(st):
         s.recompute_positional_data()
         s.solve(case["steps"])
         s.get_field(pcg.LAYOUT_PLANAR, np.float64, out=st.image)
-        return [st.image, s.get_internalized(), s.get_counts().astype(np.int64)]
+        return [st.image, s.get_internalized(), s.get_counts().view(np.int32)]
     if case["kind"] == "moved":
         s.recompute_positional_data()
     s.solve(case["steps"])

@@ -9,11 +9,11 @@
 // agents) and runs every phase as ONE launch over all domains:
 //
 //  * sweeps: one persistent launch per axis.  The tiles of all domains form one
-//    list (domains ordered by decreasing tile cost); CTAs take tiles from an
-//    atomic counter, find the tile's domain by binary search over the list's
-//    prefix sums, and solve it with the domain's own line mapping and tile shape.
-//    y/z tiles move through the domain's TMA tensor map (kept in global memory),
-//    one mbarrier per chunk, so solving starts when the first chunk lands.
+//    list (domains ordered by decreasing tile cost); CTAs (a warp, or in FP64 one
+//    for each half of the lines, sweep_solvers.cuh) take tiles from an atomic counter,
+//    find the tile's domain from a hint table, and solve it with the domain's own
+//    line mapping and tile shape.  y/z tiles move through the domain's TMA tensor
+//    map (kept in global memory).
 //  * Dirichlet faces/interior, bulk and the cell phases: one launch each over the
 //    concatenated items of all domains (face voxels, interior nodes, rows, agents).
 //  * the whole step is captured once in a CUDA graph and replayed.
@@ -26,9 +26,9 @@
 // Autotuner: per sweep axis and size bucket (line length rounded up to 16, and
 // for x the substrate count) candidate mappings are timed on the batch's own
 // domains (fields saved and restored) and the fastest is kept for the process.
-//   x:   row-per-thread (one thread carries all S recurrences of a row, walking it
-//        as 16-byte chunks) or substrate-per-thread (S lanes share a row, one
-//        recurrence each), times rows per tile;
+//   x:   row-per-thread (a lane owns a row and solves its substrates one after
+//        another) or substrate-per-thread (S lanes share a row, one line each), times
+//        rows per tile;
 //   y/z: points per TMA chunk (how early a line's solve can start vs. how many
 //        copies a tile takes).
 #include <algorithm>
@@ -60,7 +60,6 @@ enum : uint32_t
 
 constexpr uint32_t kMaxChunks = 64;        // y/z boxes per line (TMA operations per tile)
 constexpr uint64_t kClearChunk = 4096;     // voxels of the ballot counts cleared per warp item
-constexpr uint64_t kXSmemDefault = 32768;  // default shared-memory budget of an x tile
 constexpr double kTuneShare = 0.01;        // buckets below this share of an axis keep the defaults
 constexpr uint64_t kGroupBytes = 16 * 1024; // y/z: tiles of a domain taken together up to this many bytes,
 											 // or up to the batch's largest tile when that is larger
@@ -78,11 +77,11 @@ struct BatchDomain
 	uint32_t box_rows[3], boxes[3];
 	uint64_t yz_xblocks;       // y/z: tiles across a row (32 elements each)
 	uint32_t yz_group[3];      // y/z: consecutive tiles per work unit (short lines share a CTA's buffer)
-	const void* coef[3];
-	uint64_t coef_len[3];
-	uint64_t coef_comp_off[3]; // compressed tables (elements into coef)
-	uint64_t coef_blo_off[3];  // FP32: full tables of the multipliers' lo parts (elements into coef)
-	uint32_t coef_head[3];     // head points of the compressed tables
+	const void* tab[3];        // coefficient tables (capi.cu) and their head points
+	uint32_t head[3];
+	const void* sc[3];         // FP64: scale factors of each axis
+	uint32_t scaled[3];        // FP64: the axis's sweep applies its factors
+	const void *gx, *gy;       // FP64: per-point factors of axes 0 and 1 for the last sweep (null: none)
 	FaceArgs faces;
 	const uint64_t* dir_offsets;
 	const void* dir_values;
@@ -161,309 +160,203 @@ __device__ __forceinline__ void fence_tensormap_acquire(const void* map)
 
 // ------------------------------------------------------------------ sweeps
 
-// Row-per-thread x solver of the batch: one thread carries the ST recurrences of
-// a row, walking it in groups of lcm(ST, VN) elements (whole 16-byte chunks, so
-// each element's substrate is a compile-time index).  A group's chunks and
-// coefficients are loaded together; there is no cross-group prefetch, which keeps
-// every substrate variant light enough to share one kernel (batched tiles are
-// small, so many CTAs per SM hide the latency instead).
-// MC adds substrate s's inputs / outputs to acc_in[s] / acc_out[s].
-template <typename T, int ST, int MC = 0>
-__device__ __forceinline__ void solve_row_lite(T* row, const T* __restrict__ cB, const T* __restrict__ cE,
-											   const T* __restrict__ cC, const T* __restrict__ cBl, uint32_t n,
-											   MassAcc<T>* acc_in = nullptr, MassAcc<T>* acc_out = nullptr)
+// The units of a persistent batched sweep, in ticket order.  A unit's work-list entry
+// and domain are resolved by the first warp while the previous unit's tiles load,
+// and a new domain's descriptor is prefetched into L1 then; the CTA's other warp
+// reads them from shared memory.
+struct Unit
 {
-	constexpr bool kLo = sizeof(T) == 4;
-	using V = typename Vec16<T>::type;
-	constexpr int VN = Vec16<T>::N;
-	constexpr int GE = group_elems(ST, VN);
-	constexpr int U = GE / VN;
-	const uint32_t total = n * ST;
-	const uint32_t groups = (total + GE - 1) / GE;
-	V* __restrict__ vrow = reinterpret_cast<V*>(row);
-	const V* vE = reinterpret_cast<const V*>(cE);
-	const V* vB = reinterpret_cast<const V*>(cB);
-	T d[ST], c[ST];
-#pragma unroll
-	for (int s = 0; s < ST; s++)
-	{
-		d[s] = T(0);
-		c[s] = __ldg(cC + s);
-	}
-	for (uint32_t g = 0; g < groups; g++)
-	{
-		V x[U], e[U];
-#pragma unroll
-		for (int q = 0; q < U; q++)
-		{
-			x[q] = vrow[g * U + q];
-			e[q] = __ldg(vE + g * U + q);
-		}
-#pragma unroll
-		for (int q = 0; q < U; q++)
-#pragma unroll
-			for (int u = 0; u < VN; u++)
-			{
-				const int s = (q * VN + u) % ST;
-				if (g * GE + q * VN + u < total)
-				{
-					if constexpr ((MC & kMcIn) != 0)
-						acc_in[s].add(vget<V, T>(x[q], u));
-					d[s] = dev::fmadd(vget<V, T>(e[q], u), d[s], vget<V, T>(x[q], u));
-					vset<V, T>(x[q], u, d[s]);
-				}
-			}
-#pragma unroll
-		for (int q = 0; q < U; q++)
-			vrow[g * U + q] = x[q];
-	}
-#pragma unroll
-	for (int s = 0; s < ST; s++)
-		d[s] = T(0);
-	for (int g = (int)groups - 1; g >= 0; g--)
-	{
-		V x[U], bb[U], bl[U];
-#pragma unroll
-		for (int q = 0; q < U; q++)
-		{
-			x[q] = vrow[g * U + q];
-			bb[q] = __ldg(vB + g * U + q);
-			if constexpr (kLo)
-				bl[q] = __ldg(reinterpret_cast<const V*>(cBl) + g * U + q);
-		}
-#pragma unroll
-		for (int q = U - 1; q >= 0; q--)
-#pragma unroll
-			for (int u = VN - 1; u >= 0; u--)
-			{
-				const int s = (q * VN + u) % ST;
-				if ((uint32_t)g * GE + q * VN + u < total)
-				{
-					d[s] = bwd_step(c[s], d[s], vget<V, T>(x[q], u), vget<V, T>(bb[q], u),
-									kLo ? vget<V, T>(bl[q], u) : T(0));
-					vset<V, T>(x[q], u, d[s]);
-					if constexpr ((MC & kMcOut) != 0)
-						acc_out[s].add(d[s]);
-				}
-			}
-#pragma unroll
-		for (int q = 0; q < U; q++)
-			vrow[g * U + q] = x[q];
-	}
+	uint32_t t, k; // ticket and work-list entry (a launch has fewer than 2^32 units)
+};
+
+__device__ __forceinline__ Unit resolve_unit(const WorkList& l, uint32_t t)
+{
+	return { t, t < l.total ? find_entry(l, t) : 0u };
 }
 
-// One row per thread; `active` threads hold a row.  With MC every thread of the
-// warp calls it (the mass totals are summed across the warp): the rows' input
-// totals go to mc_in[s] and, when mc_out is given (x is the domain's last
-// sweep), their output totals to mc_out[s].
-template <typename T, int ST, int MC>
-__device__ __forceinline__ void solve_x_row_st(T* row, const T* cB, const T* cE, const T* cC, const T* cBl, uint32_t n,
-											   bool active, double* mc_in, double* mc_out)
-{
-	MassAcc<T> ai[ST], ao[ST];
-#pragma unroll
-	for (int s = 0; s < ST; s++)
-	{
-		ai[s].zero();
-		ao[s].zero();
-	}
-	if (active)
-		solve_row_lite<T, ST, MC>(row, cB, cE, cC, cBl, n, ai, ao);
-	if constexpr (MC != 0)
-	{
-#pragma unroll
-		for (int s = 0; s < ST; s++)
-		{
-			if (mc_in)
-				flush_classes(ai[s].value(), 1, kLanes, mc_in + s);
-			if (mc_out)
-				flush_classes(ao[s].value(), 1, kLanes, mc_out + s);
-		}
-	}
-}
+// The domain of a unit inside the list.
+__device__ __forceinline__ uint32_t unit_domain(const WorkList& l, const Unit& u) { return __ldg(l.dom + u.k); }
 
-template <typename T, int MC>
-__device__ __forceinline__ void solve_x_row(T* row, const T* cB, const T* cE, const T* cC, const T* cBl, uint32_t n,
-											uint32_t S, bool active, double* mc_in, double* mc_out)
+// Draws the next unit (warp 0; all its lanes call it) and leaves it in *slot; `di` is
+// the current unit's domain.
+__device__ __forceinline__ void draw_unit(const BatchArgs& b, uint32_t drawn, uint32_t di, Unit* slot)
 {
-	switch (S)
-	{
-	case 1: solve_x_row_st<T, 1, MC>(row, cB, cE, cC, cBl, n, active, mc_in, mc_out); break;
-	case 2: solve_x_row_st<T, 2, MC>(row, cB, cE, cC, cBl, n, active, mc_in, mc_out); break;
-	case 3: solve_x_row_st<T, 3, MC>(row, cB, cE, cC, cBl, n, active, mc_in, mc_out); break;
-	case 4: solve_x_row_st<T, 4, MC>(row, cB, cE, cC, cBl, n, active, mc_in, mc_out); break;
-	case 5: solve_x_row_st<T, 5, MC>(row, cB, cE, cC, cBl, n, active, mc_in, mc_out); break;
-	case 6: solve_x_row_st<T, 6, MC>(row, cB, cE, cC, cBl, n, active, mc_in, mc_out); break;
-	case 7: solve_x_row_st<T, 7, MC>(row, cB, cE, cC, cBl, n, active, mc_in, mc_out); break;
-	case 8: solve_x_row_st<T, 8, MC>(row, cB, cE, cC, cBl, n, active, mc_in, mc_out); break;
-	default:
-		if (active)
-			solve_row_generic<T, MC>(row, cB, cE, cC, cBl, n, S, mc_in, mc_out);
-		break;
-	}
+	const uint32_t lane = threadIdx.x & 31;
+	const Unit u = resolve_unit(b.list, __shfl_sync(0xffffffffu, drawn, 0));
+	const uint32_t dn = unit_domain(b.list, u);
+	if (dn != di && lane * 128 < sizeof(BatchDomain))
+		asm volatile("prefetch.global.L1 [%0];" ::"l"(reinterpret_cast<const char*>(b.doms + dn) + lane * 128));
+	if (lane == 0)
+		*slot = u;
 }
 
 // x: a tile is x_rows whole rows of one domain, bulk-copied into shared memory.
-// MC (mass check in this batch): for domains with the check on, the tile's input
-// totals (and output totals when x is the domain's last sweep) go to its mc_tot.
-template <typename T, int MC>
-__global__ void __launch_bounds__(kLanes) batch_sweep_x_kernel(BatchArgs b)
+// Substrate mapping: lane (r, s) solves substrate s of row r (above 32 substrates,
+// lanes take a row's substrates 32 at a time); row mapping: a lane owns a row, its
+// substrates one after another.
+// MULTI: some domain takes several passes over a tile (row mapping, or more than 32
+// substrates).  SCALED (FP64): some domain's x sweep applies its scale factors (1-D,
+// or factors not deferred).  MC (mass check in this batch): for domains with the check on, the
+// tile's input totals (and output totals when x is the domain's last sweep) go to
+// its mc_tot.
+//
+// Registers are capped so that shared memory and not the register file sets how many
+// CTAs an SM holds (FP32 otherwise took 222 a thread: 149 -> 181 us on 48 domains).
+template <typename T, int MC, bool SCALED, bool MULTI>
+__global__ void __launch_bounds__(sweep_threads<T>(), sizeof(T) == 4 ? 16 : 5) batch_sweep_x_kernel(BatchArgs b)
 {
 	extern __shared__ __align__(128) unsigned char smem[];
 	uint64_t* bar = reinterpret_cast<uint64_t*>(smem);
+	Unit& next = *reinterpret_cast<Unit*>(smem + 8);
 	T* tile = reinterpret_cast<T*>(smem + 16);
-	const uint32_t tid = threadIdx.x;
-	if (tid == 0)
+	const uint32_t lane = threadIdx.x & 31, half = threadIdx.x >> 5;
+	if (threadIdx.x == 0)
 	{
 		dev::mbar_init(bar, 1);
 		dev::fence_mbar_init();
 	}
 	__syncthreads();
 	uint32_t phase = 0;
-	uint32_t next = 0;
-	if (tid == 0)
-		next = atomicAdd(b.counter, 1u);
-	// A unit's work-list entry and domain are resolved while the previous unit's
-	// rows load, and a new domain's descriptor is prefetched into L1 then (the CTA
-	// is one warp).
-	auto resolve = [&](uint64_t u, uint32_t& k, uint32_t& di) {
-		k = di = 0;
-		if (u < b.list.total)
-		{
-			k = find_entry(b.list, u);
-			di = __ldg(b.list.dom + k);
-		}
-	};
-	uint64_t t = __shfl_sync(0xffffffffu, next, 0);
-	uint32_t k, di;
-	resolve(t, k, di);
-	for (;;)
+	Unit cur = resolve_unit(b.list, blockIdx.x);
+	while (cur.t < b.list.total)
 	{
-		if (t >= b.list.total)
-			break;
-		if (tid == 0)
-			next = atomicAdd(b.counter, 1u); // the following tile's ticket, in flight meanwhile
+		uint32_t drawn = 0;
+		if (threadIdx.x == 0)
+			drawn = gridDim.x + atomicAdd(b.counter, 1u); // the following tile's ticket, in flight meanwhile
+		const uint32_t di = unit_domain(b.list, cur);
 		if (b.steps_left[di] == 0)
 		{
-			t = __shfl_sync(0xffffffffu, next, 0);
-			resolve(t, k, di);
+			if (half == 0)
+				draw_unit(b, drawn, di, &next);
+			__syncthreads();
+			cur = next;
+			__syncthreads();
 			continue;
 		}
 		const BatchDomain& D = b.doms[di];
-		const uint32_t R = D.x_rows, S = D.S, n = D.n[0];
-		const uint64_t r0 = (t - __ldg(b.list.base + k)) * R;
+		const uint32_t R = D.x_rows, S = D.S, n = D.n[0], m = line_split<T>(n);
+		const uint64_t r0 = (cur.t - __ldg(b.list.base + cur.k)) * R;
 		const uint32_t nrows = (uint32_t)min((uint64_t)R, D.rows - r0);
 		const uint32_t row_bytes = (uint32_t)round_up(D.row_len * sizeof(T), 16);
-		const uint64_t spitch = D.x_smem_pitch;
+		const uint32_t spitch = (uint32_t)D.x_smem_pitch;
 		T* g = static_cast<T*>(D.field) + r0 * D.pitch;
-		if (tid == 0)
-			dev::mbar_arrive_expect_tx(bar, nrows * row_bytes);
-		__syncthreads();
-		if (tid < nrows)
-			dev::bulk_g2s(tile + tid * spitch, g + tid * D.pitch, row_bytes, bar);
-		const uint64_t tn = __shfl_sync(0xffffffffu, next, 0);
-		uint32_t kn, dn;
-		resolve(tn, kn, dn);
-		if (dn != di && tid * 128 < sizeof(BatchDomain))
-			asm volatile("prefetch.global.L1 [%0];" ::"l"(reinterpret_cast<const char*>(b.doms + dn) + tid * 128));
-		const T* cB = static_cast<const T*>(D.coef[0]);
-		const T* cE = cB + D.coef_len[0];
-		const T* cC = cE + D.coef_len[0];
-		const T* cBl = sizeof(T) == 4 ? cB + D.coef_blo_off[0] : nullptr;
-		const uint32_t rl = tid / S, s = tid % S;
-		LineCoef<T> L {};
-		if (D.x_mode != kMapRow) // coefficient loads overlap the tile's arrival
-			L = line_coef<T>(static_cast<const T*>(D.coef[0]) + D.coef_comp_off[0], S, D.coef_head[0], n, s);
-		const bool ok = __all_sync(0xffffffffu, dev::mbar_wait(bar, phase));
-		if (!ok)
+		if (half == 0)
 		{
-			if (tid == 0)
-				report(b, DEV_ERR_WAIT_TIMEOUT, di);
-			return;
+			if (lane == 0)
+				dev::mbar_arrive_expect_tx(bar, nrows * row_bytes);
+			__syncwarp();
+			if (lane < nrows)
+				dev::bulk_g2s(tile + lane * spitch, g + lane * D.pitch, row_bytes, bar);
+			draw_unit(b, drawn, di, &next);
 		}
-		double* mc_in = MC != 0 ? D.mc_tot : nullptr;
-		double* mc_out = MC != 0 && D.mc_tot && D.dims == 1 ? D.mc_tot + S : nullptr;
-		if (D.x_mode == kMapRow)
-			solve_x_row<T, MC>(tile + tid * spitch, cB, cE, cC, cBl, n, S, tid < nrows, mc_in, mc_out);
-		else
+		const T* tab = static_cast<const T*>(D.tab[0]);
+		const uint32_t head = D.head[0];
+		const bool by_row = MULTI && D.x_mode == kMapRow, wide = MULTI && S > kLanes;
+		const uint32_t r_local = by_row ? lane : (wide ? 0 : lane / S);
+		const uint32_t s0 = by_row ? 0 : (wide ? lane : lane % S), s_step = by_row ? 1 : kLanes;
+		// the first lines' coefficient loads overlap the tile's arrival
+		LineCoef<T> L = line_coef(tab, S, head, n, MULTI ? min(s0, S - 1) : s0, half);
+		if (!__syncthreads_and(dev::mbar_wait(bar, phase)))
 		{
+			if (threadIdx.x == 0)
+				report(b, DEV_ERR_WAIT_TIMEOUT, di);
+			break;
+		}
+		double* mc = MC != 0 ? D.mc_tot : nullptr;
+		const uint32_t passes = !MULTI ? 1 : (by_row ? S : (S + kLanes - 1) / kLanes);
+		for (uint32_t ps = 0; ps < passes; ps++)
+		{
+			const uint32_t s = s0 + ps * s_step, sc = MULTI ? min(s, S - 1) : s;
+			if (MULTI && ps)
+				L = line_coef(tab, S, head, n, sc, half);
+			const bool on = r_local < nrows && (!MULTI || s < S);
+			T* row = tile + r_local * spitch + s;
 			MassAcc<T> ai, ao;
 			ai.zero();
 			ao.zero();
-			if (rl < nrows)
-				solve_line<T, 0, MC>(tile + rl * spitch + s, n, S, L, &ai, &ao);
-			if constexpr (MC != 0)
+			const Strided<T, 0, 1> left { row, S };
+			const Strided<T, 0, -1> right { row + (n - 1) * S, S };
+			if (SCALED && D.scaled[0])
 			{
-				// lanes rl * S + s share substrate s (S <= 32 on this mapping)
-				if (mc_in)
-					flush_classes(ai.value(), S, kLanes, mc_in + s % S);
-				if (mc_out)
-					flush_classes(ao.value(), S, kLanes, mc_out + s % S);
+				const T* scale = static_cast<const T*>(D.sc[0]) + sc;
+				if constexpr (SCALED)
+					solve_tile<T, Strided<T, 0, 1>, Strided<T, 0, -1>, MC, 1>(
+						left, right, n, half, on, L, line_scale(T(1), __ldg(scale), scale + S, (int)S, n, half), &ai, &ao);
 			}
+			else
+				solve_tile<T, Strided<T, 0, 1>, Strided<T, 0, -1>, MC, 0>(left, right, n, half, on, L, {}, &ai, &ao);
+			if constexpr (MC != 0)
+				if (mc)
+				{
+					// lanes of one substrate: all (row mapping), S apart, or each its own
+					const uint32_t stride = by_row ? 1 : (wide ? kLanes : S);
+					flush_classes(ai.value(), stride, kLanes, mc + s);
+					if (D.dims == 1)
+						flush_classes(ao.value(), stride, kLanes, mc + S + s);
+				}
 		}
+		cur = next;
 		dev::fence_proxy_async_smem();
 		__syncthreads();
-		if (tid < nrows)
-			dev::bulk_s2g(g + tid * D.pitch, tile + tid * spitch, row_bytes);
-		dev::bulk_commit();
-		dev::bulk_wait_read();
-		__syncthreads();
+		if (half == 0)
+		{
+			if (lane < nrows)
+				dev::bulk_s2g(g + lane * D.pitch, tile + lane * spitch, row_bytes);
+			dev::bulk_commit();
+			dev::bulk_wait_read();
+			__syncwarp();
+		}
 		phase ^= 1;
-		t = tn;
-		k = kn;
-		di = dn;
 	}
-	dev::bulk_wait_all();
+	if (half == 0)
+		dev::bulk_wait_all();
 }
+
+struct FaceRef
+{
+	const void* face_values;
+	const uint8_t* face_conds;
+	uint32_t face_mask, S, nx, ny, nz;
+};
 
 // y/z: a tile is 32 consecutive (x,s) columns at every point of one line
 // set of one domain; its boxes arrive through the domain's tensor map on one
-// mbarrier, the warp solves it in place, and the boxes are stored back before the
-// next tile is requested (several single-warp CTAs per SM overlap these phases).
-// MC (mass check in this batch): on the domain's last sweep, each tile's solved
-// totals (before its faces are written) go to the domain's mc_tot.
-template <typename T, int AXIS, int MC>
-__global__ void __launch_bounds__(kLanes) batch_sweep_yz_kernel(BatchArgs b)
+// mbarrier, the warps solve their halves of it in place, and the boxes are stored
+// back before the next tile is requested (several CTAs per SM overlap these phases).
+// SCALED (FP64): some domain's sweep of this axis applies the scale factors (its last
+// sweep, or factors not deferred).  MC (mass check in this batch): on the domain's last
+// sweep, each tile's solved totals (before its faces are written) go to the domain's
+// mc_tot.
+template <typename T, int AXIS, int MC, bool SCALED>
+__global__ void __launch_bounds__(sweep_threads<T>()) batch_sweep_yz_kernel(BatchArgs b)
 {
 	extern __shared__ __align__(128) unsigned char smem[];
 	uint64_t* full = reinterpret_cast<uint64_t*>(smem);
+	Unit& next = *reinterpret_cast<Unit*>(smem + 8);
 	T* base = reinterpret_cast<T*>(smem + 128);
-	const uint32_t lane = threadIdx.x;
-	if (lane == 0)
+	const uint32_t lane = threadIdx.x & 31, half = threadIdx.x >> 5;
+	if (threadIdx.x == 0)
 	{
 		dev::mbar_init(full, 1);
 		dev::fence_mbar_init();
 	}
-	__syncwarp();
+	__syncthreads();
 	uint32_t phase = 0, prev = 0xffffffffu, bad = 0;
 	bool ok = true;
-	uint32_t next = 0;
-	if (lane == 0)
-		next = atomicAdd(b.counter, 1u);
-	// A unit's work-list entry and domain are resolved while the previous unit's
-	// tiles load, and a new domain's descriptor is prefetched into L1 then.
-	auto resolve = [&](uint64_t u, uint32_t& k, uint32_t& di) {
-		k = di = 0;
-		if (u < b.list.total)
-		{
-			k = find_entry(b.list, u);
-			di = __ldg(b.list.dom + k);
-		}
-	};
-	uint64_t t = __shfl_sync(0xffffffffu, next, 0);
-	uint32_t k, di;
-	resolve(t, k, di);
-	for (;; phase ^= 1)
+	Unit cur = resolve_unit(b.list, blockIdx.x);
+	while (cur.t < b.list.total)
 	{
-		if (t >= b.list.total)
-			break;
-		if (lane == 0)
-			next = atomicAdd(b.counter, 1u); // the following tile's ticket, in flight meanwhile
+		uint32_t drawn = 0;
+		if (threadIdx.x == 0)
+			drawn = gridDim.x + atomicAdd(b.counter, 1u); // the following unit's ticket, in flight meanwhile
+		const uint32_t di = unit_domain(b.list, cur);
 		if (b.steps_left[di] == 0)
 		{
-			phase ^= 1; // no tile was loaded: keep the barrier's parity
-			t = __shfl_sync(0xffffffffu, next, 0);
-			resolve(t, k, di);
+			if (half == 0)
+				draw_unit(b, drawn, di, &next);
+			__syncthreads();
+			cur = next;
+			__syncthreads();
 			continue;
 		}
 		const BatchDomain& D = b.doms[di];
@@ -471,9 +364,9 @@ __global__ void __launch_bounds__(kLanes) batch_sweep_yz_kernel(BatchArgs b)
 		// tiles share the buffer, so one ticket, lookup and wait serve them all)
 		const uint32_t group = D.yz_group[AXIS];
 		const uint64_t tiles = D.yz_xblocks * (AXIS == 1 ? D.n[2] : D.n[1]);
-		const uint64_t lt0 = (t - __ldg(b.list.base + k)) * group;
+		const uint64_t lt0 = (cur.t - __ldg(b.list.base + cur.k)) * group;
 		const uint32_t gcount = (uint32_t)min((uint64_t)group, tiles - lt0);
-		const uint32_t R = D.box_rows[AXIS], nc = D.boxes[AXIS], n = D.n[AXIS], S = D.S;
+		const uint32_t R = D.box_rows[AXIS], nc = D.boxes[AXIS], n = D.n[AXIS], S = D.S, m = line_split<T>(n);
 		const uint32_t chunk_elems = R * kLanes, tile_elems = nc * chunk_elems;
 		const CUtensorMap* map = b.tmaps + 2 * di + (AXIS - 1);
 		// the unit's first tile (x block, outer index) by one 32-bit division per unit
@@ -488,7 +381,7 @@ __global__ void __launch_bounds__(kLanes) batch_sweep_yz_kernel(BatchArgs b)
 				ob++;
 			}
 		};
-		if (lane == 0)
+		if (threadIdx.x == 0)
 		{
 			if (di != prev)
 				fence_tensormap_acquire(map);
@@ -508,48 +401,76 @@ __global__ void __launch_bounds__(kLanes) batch_sweep_yz_kernel(BatchArgs b)
 			}
 		}
 		prev = di;
-		const uint64_t tn = __shfl_sync(0xffffffffu, next, 0);
-		uint32_t kn, dn;
-		resolve(tn, kn, dn);
-		if (dn != di && lane * 128 < sizeof(BatchDomain))
-			asm volatile("prefetch.global.L1 [%0];" ::"l"(reinterpret_cast<const char*>(b.doms + dn) + lane * 128));
-		const T* comp = static_cast<const T*>(D.coef[AXIS]) + D.coef_comp_off[AXIS];
+		if (half == 0)
+		{
+			__syncwarp();
+			draw_unit(b, drawn, di, &next);
+		}
+		const T* tab = static_cast<const T*>(D.tab[AXIS]);
+		const uint32_t head = D.head[AXIS], row_len = (uint32_t)D.row_len;
 		// the first tile's coefficient loads overlap the group's arrival
-		uint32_t xb = xb0, ob = ob0;
-		int x0 = (int)(xb * kLanes), o = (int)ob;
-		LineCoef<T> L = line_coef<T>(comp, S, D.coef_head[AXIS], n,
-									 (uint64_t)(x0 + lane) < D.row_len ? (uint32_t)((x0 + lane) % S) : 0);
-		ok = __all_sync(0xffffffffu, dev::mbar_wait(full, phase));
+		uint32_t xb = xb0, o = ob0;
+		uint32_t col = xb * kLanes + lane;
+		LineCoef<T> L = line_coef(tab, S, head, n, col < row_len ? col % S : 0, half);
+		ok = __syncthreads_and(dev::mbar_wait(full, phase));
 		if (!ok)
 		{
 			bad = di;
 			break;
 		}
+		phase ^= 1;
+		cur = next;
 		for (uint32_t j = 0; j < gcount; j++)
 		{
 			if (j)
 			{
-				step_tile(xb, ob);
-				x0 = (int)(xb * kLanes), o = (int)ob;
-				L = line_coef<T>(comp, S, D.coef_head[AXIS], n,
-								 (uint64_t)(x0 + lane) < D.row_len ? (uint32_t)((x0 + lane) % S) : 0);
+				step_tile(xb, o);
+				col = xb * kLanes + lane;
+				L = line_coef(tab, S, head, n, col < row_len ? col % S : 0, half);
 			}
+			const bool in_row = col < row_len;
+			const uint32_t s = in_row ? col % S : 0;
+			T* tile = base + j * tile_elems;
 			MassAcc<T> acc;
 			acc.zero();
-			solve_line<T, kLanes, MC>(base + j * tile_elems + lane, n, 0, L, nullptr, &acc);
-			if constexpr (MC != 0)
-				if (D.mc_tot && D.dims == AXIS + 1)
-					flush_classes(acc.value(), S < kLanes ? S : kLanes, kLanes,
-								  D.mc_tot + S + ((uint32_t)x0 + lane) % S);
-			// the last sweep of the domain writes its boundary faces (the batch's
-			// Dirichlet launch then covers interior nodes and 1-D domains only)
+			const Strided<T, kLanes, 1> left { tile + lane, 0 };
+			const Strided<T, kLanes, -1> right { tile + (n - 1) * kLanes + lane, 0 };
+			if (SCALED && D.scaled[AXIS])
+			{
+				if constexpr (SCALED)
+				{
+					T g = T(1);
+					if (D.gx && D.dims == AXIS + 1)
+						g = __ldg(static_cast<const T*>(D.gx) + (in_row ? col : 0));
+					if (AXIS == 2 && D.gy)
+						g *= __ldg(static_cast<const T*>(D.gy) + (uint64_t)s * D.n[1] + o);
+					const T* scale = static_cast<const T*>(D.sc[AXIS]);
+					solve_tile<T, Strided<T, kLanes, 1>, Strided<T, kLanes, -1>, MC, 1>(
+						left, right, n, half, true, L, line_scale(g, __ldg(scale + s), scale + S + (uint64_t)s * n, 1, n, half),
+						nullptr, &acc);
+				}
+			}
+			else
+				solve_tile<T, Strided<T, kLanes, 1>, Strided<T, kLanes, -1>, MC, 0>(left, right, n, half, true, L, {}, nullptr,
+																					&acc);
 			if (D.dims == AXIS + 1)
-				fielddev::faces_on_column<T, AXIS>(D.faces, base + j * tile_elems + lane, n, kLanes,
-												   (uint64_t)x0 + lane, (uint64_t)o);
+			{
+				if constexpr (MC != 0)
+					if (D.mc_tot)
+						flush_classes(acc.value(), S < kLanes ? S : kLanes, kLanes, D.mc_tot + S + col % S);
+				// the last sweep of the domain writes its boundary faces (the batch's
+				// Dirichlet launch then covers interior nodes and 1-D domains only)
+				if (D.faces.face_mask && in_row)
+				{
+					const FaceRef f { D.faces.values, D.faces.conds, D.faces.face_mask, S, D.n[0], D.n[1], D.n[2] };
+					fielddev::faces_on_half<T, AXIS>(f, col / S, s, o, half == 0 ? tile + lane : tile + m * kLanes + lane,
+													 half == 0 ? m : n - m, kLanes, half == 0, half == 0 ? n == m : n > m);
+				}
+			}
 		}
 		dev::fence_proxy_async_smem();
-		__syncwarp();
-		if (lane == 0)
+		__syncthreads();
+		if (threadIdx.x == 0)
 		{
 			uint32_t xs_b = xb0, os_b = ob0;
 			for (uint32_t j = 0; j < gcount; j++, step_tile(xs_b, os_b))
@@ -567,14 +488,10 @@ __global__ void __launch_bounds__(kLanes) batch_sweep_yz_kernel(BatchArgs b)
 			dev::bulk_commit();
 			dev::bulk_wait_read();
 		}
-		__syncwarp();
-		t = tn;
-		k = kn;
-		di = dn;
 	}
-	if (!ok && lane == 0)
+	if (!ok && threadIdx.x == 0)
 		report(b, DEV_ERR_WAIT_TIMEOUT, bad);
-	if (lane == 0)
+	if (threadIdx.x == 0)
 		dev::bulk_wait_all();
 }
 
@@ -875,31 +792,17 @@ uint64_t bucket_key(int axis, size_t w, uint64_t S, uint64_t n)
 	return (uint64_t)axis | (w == 8 ? 4ull : 0ull) | ((axis == 0 ? S : 0ull) << 3) | (bucket_of(n) << 16);
 }
 
-// Shared-memory pitch (elements) of a batched x row: whole vector groups, and an
-// odd number of 16-byte chunks mod 8 (1), so the 8 lanes of a quarter-warp reading
-// one chunk of 8 consecutive rows hit distinct bank groups.
-uint64_t batch_x_pitch(const Context* c)
+// Shared-memory pitch (elements) of a batched x row: with a lane per row, the pitch
+// of one substrate alone.
+uint64_t batch_x_pitch(const Context* c, uint32_t mode)
 {
-	const uint64_t vn = 16 / c->wsize;
-	const uint64_t ge = (uint64_t)group_elems((int)std::min<uint64_t>(c->S, 9), (int)vn);
-	uint64_t chunks = round_up(c->row_len, c->S <= 8 ? ge : vn) / vn;
-	chunks += (1 + 8 - chunks % 8) % 8;
-	return chunks * vn;
-}
-
-uint64_t x_row_stage_bytes(const Context* c, uint32_t mode)
-{
-	return (mode == kMapSubstrate ? sweep_x_sub_pitch(c->row_len, c->S, c->wsize) : batch_x_pitch(c)) * c->wsize;
+	return sweep_x_pitch(c->row_len, mode == kMapSubstrate ? c->S : 1, c->wsize);
 }
 
 // Largest valid rows-per-tile of a mapping under a shared-memory budget.
 uint32_t x_rows_cap(const Context* c, uint32_t mode, uint64_t smem_budget)
 {
-	const uint64_t lanes_per_row = mode == kMapRow ? 1 : c->S;
-	uint64_t r = smem_budget / x_row_stage_bytes(c, mode);
-	const uint64_t cap = kLanes / lanes_per_row;
-	r = std::min(r, cap);
-	return (uint32_t)std::max<uint64_t>(r, 1);
+	return (uint32_t)x_tile_rows(c->row_len, mode == kMapSubstrate ? c->S : 1, c->wsize, smem_budget);
 }
 
 AxisConfig default_config(const Context* c, int axis)
@@ -907,9 +810,8 @@ AxisConfig default_config(const Context* c, int axis)
 	AxisConfig a;
 	if (axis == 0)
 	{
-		// measured on uneven batches: substrate-per-thread beats row-per-thread for every S
-		a.mode = c->S <= kLanes ? kMapSubstrate : kMapRow;
-		a.rows = x_rows_cap(c, a.mode, kXSmemDefault);
+		a.mode = kMapSubstrate;
+		a.rows = x_rows_cap(c, a.mode, x_tile_budget(c->wsize));
 		return a;
 	}
 	uint32_t R, nc;
@@ -960,6 +862,8 @@ struct pcg_batch
 	int max_dims = 0;
 	bool built = false;
 	bool any_mass_check = false; // some domain has the per-step mass check on
+	bool any_multi = false;      // some domain's x tiles take several passes
+	bool any_scaled[3] = { false, false, false }; // some domain's sweep of the axis applies its factors
 
 	std::vector<uint8_t> h_recompute, dev_recompute;
 	bool dev_recompute_valid = false;
@@ -1055,13 +959,11 @@ BatchDomain describe_domain(pcg_batch* b, size_t d)
 	for (int a = 0; a < 3; a++)
 	{
 		D.n[a] = (uint32_t)c->n[a];
-		D.coef[a] = c->coef[a].ptr;
-		D.coef_len[a] = c->coef_len[a];
 	}
 	const AxisConfig& x = b->cfg[0][d];
 	D.x_rows = x.rows;
 	D.x_mode = x.mode;
-	D.x_smem_pitch = x.mode == kMapSubstrate ? sweep_x_sub_pitch(c->row_len, c->S, c->wsize) : batch_x_pitch(c);
+	D.x_smem_pitch = batch_x_pitch(c, x.mode);
 	for (int a = 1; a < c->dims; a++)
 	{
 		D.box_rows[a] = b->cfg[a][d].rows;
@@ -1072,10 +974,18 @@ BatchDomain describe_domain(pcg_batch* b, size_t d)
 	D.yz_xblocks = (c->row_len + kLanes - 1) / kLanes;
 	for (int a = 0; a < c->dims; a++)
 	{
-		D.coef_comp_off[a] = c->coef_comp_off[a];
-		D.coef_blo_off[a] = c->coef_blo_off[a];
-		D.coef_head[a] = c->coef_head[a];
+		D.tab[a] = c->coef[a].ptr;
+		D.head[a] = c->coef_head[a];
+		if (c->wsize == 8)
+		{
+			D.sc[a] = c->scale_table(a);
+			D.scaled[a] = a == c->dims - 1 || !c->defer_scale;
+		}
 	}
+	if (c->defer_scale && c->dims > 1) // FP64
+		D.gx = c->scale_table(0) + c->S;
+	if (c->defer_scale && c->dims > 2)
+		D.gy = c->scale_table(1) + c->S;
 	D.faces = make_face_args(c);
 	D.dir_offsets = static_cast<const uint64_t*>(c->dir_offsets.ptr);
 	D.dir_values = c->dir_values.ptr;
@@ -1235,10 +1145,15 @@ int upload_domains(pcg_batch* b)
 {
 	const size_t N = b->ctx.size();
 	b->any_mass_check = false;
+	b->any_multi = false;
+	std::fill(b->any_scaled, b->any_scaled + 3, false);
 	for (size_t d = 0; d < N; d++)
 	{
 		b->h_doms[d] = describe_domain(b, d);
 		b->any_mass_check |= b->h_doms[d].mc_tot != nullptr;
+		b->any_multi |= b->h_doms[d].x_mode == kMapRow || b->h_doms[d].S > kLanes;
+		for (int a = 0; a < C(b, d)->dims; a++)
+			b->any_scaled[a] |= b->h_doms[d].scaled[a] != 0;
 	}
 	// y/z: every CTA's buffer holds the batch's largest tile, so a short-line
 	// domain groups its tiles up to that size (at least kGroupBytes) instead of
@@ -1301,17 +1216,27 @@ uint64_t sweep_smem(pcg_batch* b, int axis, const std::vector<size_t>& subset)
 	return best;
 }
 
-template <typename T>
-const void* sweep_kernel(int axis, bool mass_check)
+// The kernel of a sweep axis for the domains of the batch: with or without the mass
+// check and, in FP64, domains that apply their scale factors there; x also with or
+// without domains that take several passes over a tile.
+using SweepFn = void (*)(BatchArgs);
+template <typename T, bool SCALED, bool MULTI>
+SweepFn sweep_kernel_of(int axis, bool mass_check)
 {
 	if (axis == 0)
-		return mass_check ? reinterpret_cast<const void*>(batch_sweep_x_kernel<T, kMcIn | kMcOut>)
-						  : reinterpret_cast<const void*>(batch_sweep_x_kernel<T, 0>);
+		return mass_check ? batch_sweep_x_kernel<T, kMcIn | kMcOut, SCALED, MULTI> : batch_sweep_x_kernel<T, 0, SCALED, MULTI>;
 	if (axis == 1)
-		return mass_check ? reinterpret_cast<const void*>(batch_sweep_yz_kernel<T, 1, kMcOut>)
-						  : reinterpret_cast<const void*>(batch_sweep_yz_kernel<T, 1, 0>);
-	return mass_check ? reinterpret_cast<const void*>(batch_sweep_yz_kernel<T, 2, kMcOut>)
-					  : reinterpret_cast<const void*>(batch_sweep_yz_kernel<T, 2, 0>);
+		return mass_check ? batch_sweep_yz_kernel<T, 1, kMcOut, SCALED> : batch_sweep_yz_kernel<T, 1, 0, SCALED>;
+	return mass_check ? batch_sweep_yz_kernel<T, 2, kMcOut, SCALED> : batch_sweep_yz_kernel<T, 2, 0, SCALED>;
+}
+
+template <typename T>
+SweepFn sweep_kernel(const pcg_batch* b, int axis, bool mass_check)
+{
+	if constexpr (sizeof(T) == 8)
+		if (b->any_scaled[axis])
+			return b->any_multi ? sweep_kernel_of<T, true, true>(axis, mass_check) : sweep_kernel_of<T, true, false>(axis, mass_check);
+	return b->any_multi ? sweep_kernel_of<T, false, true>(axis, mass_check) : sweep_kernel_of<T, false, false>(axis, mass_check);
 }
 
 // The dynamic shared-memory limit of a batched sweep kernel only ever grows, so
@@ -1334,15 +1259,16 @@ int raise_smem_limit(const void* k, int device, uint64_t smem)
 template <typename T>
 int sweep_grid(pcg_batch* b, int axis, uint64_t smem, uint64_t tiles, unsigned* grid)
 {
-	const void* k = sweep_kernel<T>(axis, b->any_mass_check);
+	const void* k = reinterpret_cast<const void*>(sweep_kernel<T>(b, axis, b->any_mass_check));
 	if (smem > kMaxSmemBytes)
 		return fail(PCG_ERR_UNSUPPORTED, "a batched sweep tile exceeds shared memory");
 	int rc;
 	for (int mc = 0; mc < 2; mc++) // both variants: a later call may switch the check
-		if ((rc = raise_smem_limit(sweep_kernel<T>(axis, mc != 0), b->device, smem)))
+		if ((rc = raise_smem_limit(reinterpret_cast<const void*>(sweep_kernel<T>(b, axis, mc != 0)),
+								   b->device, smem)))
 			return rc;
 	int per_sm = 0;
-	PCG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kLanes, smem));
+	PCG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, sweep_threads<T>(), smem));
 	if (per_sm < 1)
 		return fail(PCG_ERR_UNSUPPORTED, "a batched sweep tile does not fit on an SM");
 	uint64_t g = (uint64_t)per_sm * (uint64_t)b->sm_count;
@@ -1514,15 +1440,7 @@ template <typename T>
 int launch_sweep(pcg_batch* b, int axis, const BatchArgs& a, unsigned grid, uint64_t smem, double bytes)
 {
 	LaunchScope s(b, axis == 0 ? K_SWEEP_X : axis == 1 ? K_SWEEP_Y : K_SWEEP_Z, bytes);
-	const bool mc = b->any_mass_check;
-	if (axis == 0)
-		(mc ? batch_sweep_x_kernel<T, kMcIn | kMcOut> : batch_sweep_x_kernel<T, 0>)<<<grid, kLanes, smem, b->stream>>>(a);
-	else if (axis == 1)
-		(mc ? batch_sweep_yz_kernel<T, 1, kMcOut>
-			: batch_sweep_yz_kernel<T, 1, 0>)<<<grid, kLanes, smem, b->stream>>>(a);
-	else
-		(mc ? batch_sweep_yz_kernel<T, 2, kMcOut>
-			: batch_sweep_yz_kernel<T, 2, 0>)<<<grid, kLanes, smem, b->stream>>>(a);
+	sweep_kernel<T>(b, axis, b->any_mass_check)<<<grid, sweep_threads<T>(), smem, b->stream>>>(a);
 	PCG_CUDA_TRY(cudaGetLastError());
 	return PCG_OK;
 }
@@ -1703,7 +1621,7 @@ int refresh(pcg_batch* b)
 				if (a == 0 && (cfg.mode != kMapSubstrate || c->S > kLanes))
 					cfg.mode = kMapRow;
 				if (cfg.rows == 0)
-					cfg.rows = a == 0 ? x_rows_cap(c, cfg.mode, kXSmemDefault) : dflt.rows;
+					cfg.rows = a == 0 ? x_rows_cap(c, cfg.mode, x_tile_budget(c->wsize)) : dflt.rows;
 			}
 			if (a == 0)
 				cfg.rows = std::min(cfg.rows, x_rows_cap(c, cfg.mode, kMaxSmemBytes - 16));
@@ -1857,11 +1775,8 @@ std::vector<AxisConfig> candidates(const Context* c, int axis)
 	};
 	if (axis == 0)
 	{
-		if (c->S <= kLanes)
-			for (uint64_t budget : { (uint64_t)16384, (uint64_t)32768, (uint64_t)57344 })
-				add({ kMapSubstrate, x_rows_cap(c, kMapSubstrate, budget) });
-		for (uint64_t budget : { (uint64_t)32768, (uint64_t)57344 })
-			add({ kMapRow, x_rows_cap(c, kMapRow, budget) });
+		for (uint64_t budget : { (uint64_t)16384, (uint64_t)32768, (uint64_t)57344 })
+			add({ kMapSubstrate, x_rows_cap(c, kMapSubstrate, budget) });
 		return out;
 	}
 	const uint64_t n = c->n[axis];

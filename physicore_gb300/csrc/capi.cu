@@ -14,6 +14,7 @@
 #include <mutex>
 
 #include "pcg_internal.cuh"
+#include "sweep_solvers.cuh"
 
 namespace pcg {
 
@@ -419,123 +420,157 @@ static void colsum_multipliers(uint64_t n, uint64_t S, uint64_t shape, uint64_t 
 	}
 }
 
-// Device coefficient table of one axis: [B | E | C], C[s] = c.  For x, B and E are
-// flat in the field's (i, s) order, B[i*S+s] = b'_i, E[i*S+s] = e_{i-1} (0 at i = 0),
-// so a 16-byte chunk of coefficients matches a chunk of a row.  For y and z they are
-// per-substrate rows, B[s*cp + i], padded to cp = a multiple of the solver block.
-// FP32 tables hold the column-sum-exact multipliers as hi + lo (colsum_multipliers):
-// B is the hi part and a B_lo table of the same layout follows C.
+// FP32 table of one axis (line_coef in sweep_solvers.cuh).  b'_i and e_i converge to a
+// constant within a few points, so a line needs only a head of H points (the first
+// index from which every stored value up to n-2 equals the value at n-2, rounded up
+// to the solver block and taken over all substrates), that middle constant and the
+// values of the last point.  The multipliers are the column-sum-exact ones as hi +
+// lo (colsum_multipliers).
+static uint64_t coefficient_table_fp32(const Context* c, int axis, std::vector<float>& tab)
+{
+	const uint64_t S = c->S, n = c->n[axis];
+	std::vector<double> b, e, cc, B;
+	std::vector<float> Bhi;
+	precompute_axis(n, S, c->voxel[axis], (uint64_t)c->dims, c->dt, c->D.data(), c->decay.data(), b, e, cc);
+	colsum_multipliers(n, S, c->voxel[axis], (uint64_t)c->dims, c->dt, c->D.data(), c->decay.data(), e, cc, B, Bhi);
+	// by point and substrate: the multiplier's hi part, lo = B - hi, and e_{i-1}
+	auto hi = [&](uint64_t i, uint64_t s) { return Bhi[i * S + s]; };
+	auto lo = [&](uint64_t i, uint64_t s) { return (float)(B[i * S + s] - (double)Bhi[i * S + s]); };
+	auto ee = [&](uint64_t i, uint64_t s) { return i == 0 ? 0.0f : (float)e[(i - 1) * S + s]; };
+	uint64_t H = 1;
+	for (uint64_t s = 0; s < S; s++)
+	{
+		uint64_t h = n;
+		if (n >= 2)
+		{
+			const uint64_t m = n - 2;
+			h = m;
+			while (h > 0 && hi(h - 1, s) == hi(m, s) && ee(h - 1, s) == ee(m, s) && lo(h - 1, s) == lo(m, s))
+				h--;
+		}
+		H = std::max(H, h);
+	}
+	H = round_up(H, kBlockPoints);
+	if (H >= n)
+		H = round_up(n, kBlockPoints); // the whole line lives in the head
+	const uint64_t kS = round_up(S, 4);
+	tab.assign(3 * S * H + 7 * kS, 0.0f);
+	float* hB = tab.data();
+	float* hE = hB + S * H;
+	float* k = hE + S * H;
+	float* hBl = k + 5 * kS;
+	float* kl = hBl + S * H;
+	for (uint64_t s = 0; s < S; s++)
+	{
+		for (uint64_t i = 0; i < std::min(H, n); i++)
+		{
+			hB[s * H + i] = hi(i, s);
+			hE[s * H + i] = ee(i, s);
+			hBl[s * H + i] = lo(i, s);
+		}
+		const uint64_t m = n >= 2 ? n - 2 : 0;
+		k[s] = hi(m, s);
+		k[kS + s] = ee(m, s);
+		k[2 * kS + s] = hi(n - 1, s);
+		k[3 * kS + s] = n == 1 ? 0.0f : ee(n - 1, s);
+		k[4 * kS + s] = (float)cc[s];
+		kl[s] = lo(m, s);
+		kl[kS + s] = lo(n - 1, s);
+	}
+	return H;
+}
+
+// FP64 table of one axis for the two-sided solve (sweep_solvers.cuh), in doubles:
+//   [E rows S x H | G rows S x H | e | ws | wl | wr, S each | converged factor S |
+//    factors: axis 0 at [i*S + s], the others at [s*n + i]]
+// E[j] = e_{j-1} (0 for j = 0) and G[j] = e_{j+1} for the H head points counted from a
+// line's end, e the value they converge to, b' the factors (mirrored about the
+// meeting point), and at the meeting point, with tl = e and tr = e of the two halves'
+// last points, ws = 1 / (1 - tl tr), wl = ws tr, wr = ws tl.  *shrink: the smallest
+// factor.
+static uint64_t coefficient_table_fp64(const Context* c, int axis, std::vector<double>& tab, uint64_t* scale_off,
+									   double* shrink)
+{
+	const uint64_t S = c->S, n = c->n[axis];
+	const uint64_t m = solvers::line_split<double>((uint32_t)n), lr = n - m, L = std::max(m, lr);
+	// the elimination from a line's end (diffusion_solver.cpp:29-86): b' and e to the
+	// meeting point; an end point has r subtracted, once when n = 1
+	std::vector<double> b(L * S), e(L * S);
+	const double h2 = (double)(c->voxel[axis] * c->voxel[axis]);
+	uint64_t H = 1;
+	for (uint64_t s = 0; s < S; s++)
+	{
+		const double r = -1 * -c->dt * c->D[s] / h2;
+		for (uint64_t j = 0; j < L; j++)
+		{
+			double v = 1 + c->decay[s] * c->dt / (double)c->dims + 2 * c->dt * c->D[s] / h2;
+			if (j == 0 || j == n - 1)
+				v -= c->dt * c->D[s] / h2;
+			b[j * S + s] = 1 / (j ? v - r * r * b[(j - 1) * S + s] : v);
+			e[j * S + s] = r * b[j * S + s];
+		}
+		// head: the points before which something still changes, and one on for the
+		// inward coefficients, which lag by a point
+		uint64_t h = L - 1;
+		while (h > 0 && b[(h - 1) * S + s] == b[(L - 1) * S + s])
+			h--;
+		H = std::max(H, h + 1);
+	}
+	H = round_up(H, kBlockPoints);
+	const uint64_t head = S * H, k = 2 * head;
+	*scale_off = k + 4 * S;
+	tab.assign(*scale_off + S + n * S, 0.0);
+	double* sc = tab.data() + *scale_off;
+	for (uint64_t s = 0; s < S; s++)
+	{
+		for (uint64_t j = 0; j < std::min(H, L); j++)
+		{
+			tab[s * H + j] = j ? e[(j - 1) * S + s] : 0.0;
+			tab[head + s * H + j] = e[std::min(j + 1, L - 1) * S + s];
+		}
+		const double tl = e[(m - 1) * S + s], tr = lr ? e[(lr - 1) * S + s] : 0.0;
+		const double ws = lr ? 1 / (1 - tl * tr) : 1.0;
+		tab[k + s] = e[(L - 1) * S + s];
+		tab[k + S + s] = ws;
+		tab[k + 2 * S + s] = ws * tr;
+		tab[k + 3 * S + s] = ws * tl;
+		sc[s] = b[(L - 1) * S + s];
+		for (uint64_t i = 0; i < n; i++)
+		{
+			const double f = b[(i < m ? i : n - 1 - i) * S + s];
+			sc[S + (axis == 0 ? i * S + s : s * n + i)] = f;
+			*shrink = std::min(*shrink, f);
+		}
+	}
+	return H;
+}
+
 template <typename T>
 static int upload_coefficients(Context* c)
 {
-	const uint64_t S = c->S;
-	constexpr bool kLo = sizeof(T) == 4;
+	// FP64: how far the values between the sweeps may exceed the field's when the
+	// factors are left to the last sweep
+	double growth = 1.0;
 	for (int axis = 0; axis < c->dims; axis++)
 	{
-		const uint64_t n = c->n[axis];
-		std::vector<double> b, e, cc, B;
-		std::vector<float> Bhi;
-		precompute_axis(n, S, c->voxel[axis], (uint64_t)c->dims, c->dt, c->D.data(), c->decay.data(), b, e, cc);
-		if (kLo)
+		std::vector<T> tab;
+		if constexpr (sizeof(T) == 4)
+			c->coef_head[axis] = (uint32_t)coefficient_table_fp32(c, axis, tab);
+		else
 		{
-			colsum_multipliers(n, S, c->voxel[axis], (uint64_t)c->dims, c->dt, c->D.data(), c->decay.data(), e, cc,
-							   B, Bhi);
-			b = B;
+			double shrink = 1.0;
+			c->coef_head[axis] = (uint32_t)coefficient_table_fp64(c, axis, tab, &c->coef_scale_off[axis], &shrink);
+			if (axis < c->dims - 1)
+				growth /= shrink;
 		}
-		// FP32: the multiplier's hi part (chosen by colsum_multipliers) and lo = B - hi
-		auto hi = [&](uint64_t k) { return kLo ? (T)Bhi[k] : (T)b[k]; };
-		auto lo = [&](uint64_t k) { return kLo ? (T)(b[k] - (double)Bhi[k]) : T(0); };
-		const uint64_t cp = coef_row_pitch(n);
-		const uint64_t len = axis == 0 ? coef_table_len(n, S, sizeof(T)) : S * cp;
-		const uint64_t blo_off = 2 * len + round_up(S, 16 / sizeof(T));
-		const uint64_t total = blo_off + (kLo ? len : 0);
-		// Compressed tables.  b'_i and e_i converge to a constant within a few
-		// points, so a line needs only a head of H points (the first index from which
-		// every stored value up to n-2 equals the value at n-2, rounded up to the solver
-		// block and taken over all substrates), that middle constant and the values of
-		// the last point.  Stored values are the same rounded numbers as the full table.
-		const uint64_t vn = 16 / sizeof(T);
-		uint64_t H = 0;
-		{
-			for (uint64_t sub = 0; sub < S; sub++)
-			{
-				uint64_t h = n;
-				if (n >= 2)
-				{
-					const T bm = hi((n - 2) * S + sub);
-					const T em = n >= 3 ? (T)e[(n - 3) * S + sub] : T(0);
-					h = n - 2;
-					const T blm = lo((n - 2) * S + sub);
-					while (h > 0)
-					{
-						const uint64_t i = h - 1;
-						const T bi = hi(i * S + sub);
-						const T ei = i == 0 ? T(0) : (T)e[(i - 1) * S + sub];
-						if (bi != bm || ei != em || lo(i * S + sub) != blm)
-							break;
-						h = i;
-					}
-				}
-				H = std::max(H, h);
-			}
-			H = round_up(std::max<uint64_t>(H, 1), kBlockPoints);
-			if (H >= n)
-				H = round_up(n, kBlockPoints); // the whole line lives in the head
-		}
-		const uint64_t kS = round_up(S, vn);
-		const uint64_t comp_total = 2 * S * H + 5 * kS + (kLo ? S * H + 2 * kS : 0);
-		c->coef_len[axis] = len;
-		c->coef_elems[axis] = total;
-		c->coef_comp_off[axis] = total;
-		c->coef_blo_off[axis] = kLo ? blo_off : 0;
-		c->coef_head[axis] = (uint32_t)H;
-		std::vector<T> tab(total + comp_total, T(0));
-		for (uint64_t i = 0; i < n; i++)
-			for (uint64_t s = 0; s < S; s++)
-			{
-				const uint64_t at = axis == 0 ? i * S + s : s * cp + i;
-				tab[at] = hi(i * S + s);
-				tab[len + at] = i == 0 ? T(0) : (T)e[(i - 1) * S + s];
-				if (kLo)
-					tab[blo_off + at] = lo(i * S + s);
-			}
-		for (uint64_t s = 0; s < S; s++)
-			tab[2 * len + s] = (T)cc[s];
-		{
-			T* hB = tab.data() + total;
-			T* hE = hB + S * H;
-			T* k = hE + S * H; // [mid b' | mid e | last b' | last e | c], each kS long
-			T* hBl = k + 5 * kS; // FP32: [head b' lo | mid b' lo | last b' lo]
-			T* kl = hBl + S * H;
-			for (uint64_t sub = 0; sub < S; sub++)
-			{
-				for (uint64_t i = 0; i < std::min(H, n); i++)
-				{
-					hB[sub * H + i] = hi(i * S + sub);
-					hE[sub * H + i] = i == 0 ? T(0) : (T)e[(i - 1) * S + sub];
-					if (kLo)
-						hBl[sub * H + i] = lo(i * S + sub);
-				}
-				const uint64_t m = n >= 2 ? n - 2 : 0;
-				k[sub] = hi(m * S + sub);
-				k[kS + sub] = m == 0 ? T(0) : (T)e[(m - 1) * S + sub];
-				k[2 * kS + sub] = hi((n - 1) * S + sub);
-				k[3 * kS + sub] = n == 1 ? T(0) : (T)e[(n - 2) * S + sub];
-				k[4 * kS + sub] = (T)cc[sub];
-				if (kLo)
-				{
-					kl[sub] = lo(m * S + sub);
-					kl[kS + sub] = lo((n - 1) * S + sub);
-				}
-			}
-		}
-		int rc = dalloc(c, c->coef[axis], tab.size() * sizeof(T));
+		const int rc = dalloc(c, c->coef[axis], tab.size() * sizeof(T));
 		if (rc)
 			return rc;
 		PCG_CUDA_TRY(cudaMemcpyAsync(c->coef[axis].ptr, tab.data(), tab.size() * sizeof(T), cudaMemcpyHostToDevice,
 									 c->stream));
 		PCG_CUDA_TRY(stream_wait(c)); // the host table dies at scope exit
 	}
+	c->defer_scale = sizeof(T) == 8 && growth <= 1048576.0; // 2^20; false for NaN too
 	return PCG_OK;
 }
 

@@ -72,12 +72,14 @@ const char* kernel_name(int id);
 
 // ------------------------------------------------------------------ launch geometry
 
-constexpr int kLanes = 32;           // lines per y/z tile, rows per x tile (one warp per CTA)
-constexpr int kStages = 2;           // shared-memory ring depth of the persistent sweeps
+constexpr int kLanes = 32;           // lines per y/z tile, rows per x tile
 constexpr uint64_t kMaxSmemBytes = 227 * 1024;
-constexpr uint64_t kCoefSmemLimit = 64 * 1024; // larger coefficient tables stay in global memory
 constexpr uint64_t kBlockPoints = 8;           // line points per pipelined solver block
-constexpr uint64_t kXTileBytes = 32 * 1024;    // shared memory of a substrate-mapped x tile
+
+// Shared memory of an x tile.  FP32: more CTAs per SM beat fuller warps.  FP64: an
+// instruction costs the FP64 pipe the same however few of the warp's lanes hold a
+// line, so tiles grow until the lanes are full, with 4 CTAs (8 warps) left per SM.
+__host__ __device__ constexpr uint64_t x_tile_budget(uint64_t wsize) { return (wsize == 4 ? 32 : 56) * 1024; }
 
 __host__ __device__ constexpr uint64_t round_up(uint64_t v, uint64_t m) { return (v + m - 1) / m * m; }
 
@@ -85,53 +87,48 @@ __host__ __device__ constexpr uint64_t round_up(uint64_t v, uint64_t m) { return
 // side, cells_device.cuh): 3 S values of w bytes in whole 16-byte units, so that a
 // gather of one agent's terms touches one short run of memory, not three rows.
 __host__ __device__ constexpr uint64_t term_stride(uint64_t S, uint64_t w) { return round_up(3 * S * w, 16) / w; }
-__host__ __device__ constexpr int gcd_i(int a, int b) { return b == 0 ? a : gcd_i(b, a % b); }
-// Elements per x-sweep vector group: the smallest multiple of both S and a 16-byte chunk.
-__host__ __device__ constexpr int group_elems(int S, int vn) { return S <= 8 ? S / gcd_i(S, vn) * vn : vn; }
 
 // ------------------------------------------------------------------ argument block
 
-// A Thomas sweep over one axis.  The coefficient table of the axis is
-// [B | E | C]: B[i*S+s] = b'_i, E[i*S+s] = e_{i-1} (E = 0 for i = 0), each
-// padded to coef_len elements, then C[s] = c padded to a 16-byte multiple.
+// A sweep over one axis.  `tab` is the axis's coefficient table (capi.cu): head rows
+// and per-substrate constants; FP64: and the scale factors.
 struct SweepArgs
 {
 	void* field;
-	const void* coef;
-	uint64_t coef_len;    // elements of one padded B or E table
-	uint64_t coef_elems;  // elements of the whole [B | E | C] table
+	const void* tab;
+	uint32_t head;        // head points H of the table
 	uint32_t S;
 	uint32_t n;           // line length
 	uint64_t row_len;     // nx*S: elements of one row
 	uint64_t pitch;       // row pitch of the field (elements)
 	uint64_t tiles;
 	// y/z sweeps: a tile is 32 consecutive (x,s) elements of all n points of a line set
-	uint64_t line_stride; // elements between consecutive points of a line
-	uint64_t outer_stride;
 	uint64_t xblocks;
 	uint32_t box_rows;    // line points per TMA box (<= 256)
 	uint32_t boxes;       // boxes per tile (boxes * box_rows >= n)
-	uint64_t comp_off;    // compressed coefficient tables (elements into coef)
-	uint64_t blo_off;     // FP32: full table of the multipliers' lo parts (elements into coef)
-	uint32_t head;        // head points of the compressed tables
 	// x sweep: a tile is rows_per_tile whole rows
 	uint64_t rows;        // ny*nz
-	uint64_t smem_pitch;  // shared-memory row pitch (elements); in 16-byte chunks == threads per row (mod 8)
+	uint64_t smem_pitch;  // shared-memory row pitch (elements)
 	uint32_t rows_per_tile;
 	uint32_t* err;
-	uint32_t* ticket; // tile counter of the launch (zeroed before it), tiles handed out in order
+	uint32_t* ticket; // tile counter of the launch, tiles handed out in order
+	// FP64 sweeps that scale their results: this axis's factors ([S] converged, then
+	// per point: axis 0 at [x*S + s], the others at [s*n + i]) and, at the last sweep
+	// of a step, the per-point factors of axis 0 and axis 1 (null when there are none)
+	const void* sc;
+	const void* gx;
+	const void* gy;
 	// y/z, last sweep of a step that also applies Dirichlet: the boundary faces
-	// are written into each solved tile before it is stored (FaceArgs in
-	// field_device.cuh); face_mask 0 when not fused
+	// are written into each solved tile before it is stored (field_device.cuh);
+	// face_mask 0 when not fused
 	const void* face_values;
 	const uint8_t* face_conds;
 	uint32_t face_mask;
-	uint64_t nx, ny, nz;
+	uint32_t nx, ny, nz;
 	// mass check (kernels instantiated with it): FP64 totals [before S | after S];
 	// the x sweep adds its inputs, the last sweep its outputs (x as well when the
 	// mesh is 1-D)
 	double* mc_tot;
-	uint32_t mc_x_out;
 };
 
 // ------------------------------------------------------------------ context
@@ -216,11 +213,10 @@ struct Context
 	CUtensorMap tmap[3];
 	uint32_t tmap_box_rows[3] = { 0, 0, 0 };
 	uint32_t tmap_boxes[3] = { 0, 0, 0 };
-	uint64_t coef_len[3] = { 0, 0, 0 };
-	uint64_t coef_elems[3] = { 0, 0, 0 };
-	uint64_t coef_comp_off[3] = { 0, 0, 0 }; // compressed tables (head rows, constants)
-	uint64_t coef_blo_off[3] = { 0, 0, 0 };  // FP32: the full table of the multipliers' lo parts
-	uint32_t coef_head[3] = { 0, 0, 0 };     // head points per substrate of the compressed tables
+	uint32_t coef_head[3] = { 0, 0, 0 };      // head points per substrate of the tables
+	uint64_t coef_scale_off[3] = { 0, 0, 0 }; // FP64: the scale factors (elements into coef)
+	bool defer_scale = false; // FP64: the last sweep applies every axis's factors (sweep_solvers.cuh)
+	const double* scale_table(int axis) const { return static_cast<const double*>(coef[axis].ptr) + coef_scale_off[axis]; }
 	// One allocation at initialisation sized by estimate_device_bytes, from which
 	// the context's buffers are carved in turn (dozens of pool allocations per
 	// context cost milliseconds once many contexts come and go, as under a server)
@@ -406,13 +402,11 @@ struct DeviceGuard
 };
 
 // geometry helpers shared by the launchers and the feasibility checks
-uint64_t coef_table_len(uint64_t n, uint64_t S, size_t wsize);
-uint64_t coef_row_pitch(uint64_t n);
-uint64_t sweep_x_smem_pitch(uint64_t row_len, uint64_t S, size_t wsize);
-// x mapping of the single-domain sweep: substrate-per-thread (true) or row-per-thread
+// x tiles: shared-memory row pitch and rows per tile
+uint64_t sweep_x_pitch(uint64_t row_len, uint64_t S, size_t wsize);
+uint64_t x_tile_rows(uint64_t row_len, uint64_t S, size_t wsize, uint64_t budget);
+// substrate counts of the fused x + y sweep
 bool x_substrate_mapping(uint64_t S);
-uint64_t sweep_x_sub_pitch(uint64_t row_len, uint64_t S, size_t wsize);
-uint64_t x_threads_per_row(uint64_t S, size_t wsize);
 uint64_t sweep_smem_bytes(const Context* c, int axis);
 int prepare_sweep_maps(Context* c);
 // y/z chunk geometry: points per TMA box and boxes per line

@@ -1,8 +1,29 @@
-// sweep_solvers.cuh -- per-line Thomas solvers shared by the single-domain and
-// batched sweeps.  Arithmetic per line follows the reference
-// (openmp_solver/src/diffusion_solver.cpp:116-202 and 390-794): forward
-// d_i = d_i + e_{i-1} d_{i-1}, then d_i = (d_i + c d_{i+1}) b'_i downwards, both
-// started from a zero carry (e_{-1} = 0; c*0 = 0 gives d_{n-1} b'_{n-1}).
+// sweep_solvers.cuh -- per-line tridiagonal solvers shared by the single-domain and
+// batched sweeps (the reference: openmp_solver/src/diffusion_solver.cpp:116-202 and
+// 390-794).
+//
+// FP32: forward elimination and back substitution over the whole line by one lane,
+//   d_i = x_i + e_{i-1} d_{i-1}, then d_i = (b'_i c) d_{i+1} + b'_i d_i downwards
+// (both from a zero carry; b' as a pair hi + lo).  These sweeps move their bytes at
+// the copy bandwidth; what a shorter chain would save they do not wait for.
+//
+// FP64: the FP64 pipe sets the pace (one warp instruction per 16 cycles of an SM, with
+// a latency of several of those), so the line is solved with the fewest
+// operations and in two halves side by side.  It is eliminated from both ends
+// towards a meeting point and solved outwards from there (a twisted factorisation of
+// the same matrix); the halves belong to the CTA's two warps.  With r = dt D / h^2,
+// b'_j and e_j = r b'_j the reference's own values (the matrix reads the same from
+// either end, so both halves use one table), each half runs
+//   inward    d_j = x_j + e_{j-1} d_{j-1}                j = 0 .. L-1
+//   meeting   y   = w d + w' d'                          (d' the other half's last d)
+//   outward   y_j = d_j + e_{j+1} y_{j+1}                j = L-2 .. 0
+// and the line's solution is b'_j y_j.  That factor depends on the substrate and the
+// position along the swept axis only, so it commutes with the sweeps of the other
+// axes: a step's sweeps leave it out and the last one multiplies by the product
+// (SC = 1): 7 FP64 operations per point and 3-D step instead of 9, and 1 in the
+// dependent chain of a point instead of 3.  A mesh whose factors would let the values
+// between the sweeps grow past 2^20 of the field's applies them in every sweep.
+// 160x144x128, 3 substrates: x 96.5 -> 56.3, y 84.5 -> 56.7, z 80.4 -> 79.7 us.
 #pragma once
 
 #include "pcg_internal.cuh"
@@ -10,39 +31,21 @@
 namespace pcg {
 namespace solvers {
 
-constexpr int kBlock = 8;      // recurrence steps per pipelined block (y/z, one point per step)
-constexpr int kChunkBlock = 4; // 16-byte chunks per pipelined block (x, several points per chunk)
+constexpr int kBlock = 8; // recurrence steps per pipelined block
 
+// Threads of a sweep CTA: a warp per tile (FP32), or one for each half of its lines.
 template <typename T>
-struct Vec16;
-template <>
-struct Vec16<float>
+constexpr int sweep_threads()
 {
-	using type = float4;
-	static constexpr int N = 4;
-};
-template <>
-struct Vec16<double>
-{
-	using type = double2;
-	static constexpr int N = 2;
-};
-
-template <typename V, typename T>
-__device__ __forceinline__ T vget(const V& v, int u)
-{
-	return reinterpret_cast<const T*>(&v)[u];
-}
-template <typename V, typename T>
-__device__ __forceinline__ void vset(V& v, int u, T x)
-{
-	reinterpret_cast<T*>(&v)[u] = x;
+	return sizeof(T) == 4 ? 32 : 64;
 }
 
-template <typename V>
-__device__ __forceinline__ V ldg_vec(const V* p)
+// Points of a line that the first warp solves: all (FP32), or a whole number of
+// blocks near the middle; lines of at most one block have no second half.
+template <typename T>
+__host__ __device__ constexpr uint32_t line_split(uint32_t n)
 {
-	return __ldg(p);
+	return sizeof(T) == 4 || n <= 8 ? n : (n + 8) / 16 * 8;
 }
 
 // Mass-check accumulators: a lane's running total of the values a sweep reads
@@ -116,52 +119,98 @@ __device__ __forceinline__ void flush_classes(double v, uint32_t stride, uint32_
 		atomicAdd(dst, v);
 }
 
-// One lane's coefficients along a line, from the compressed tables of an axis:
-// points j < H read the substrate's head rows, points H <= j < n-1 share the middle
-// constants, and point n-1 has its own (when H >= n the head holds the whole line).
-// H is a multiple of kBlock, so a block of points is either all head or all
-// middle/last.  The stored values are the full table's (the host picks H so that
-// every point from H to n-2 holds exactly the middle value).
-template <typename T>
-struct LineCoef
+// Points of one line in shared memory, counted from the end where a warp starts:
+// point j at p[DIR * j * stride].  STRIDE 0: the run-time stride.
+template <typename T, int STRIDE, int DIR>
+struct Strided
 {
-	const T* hB;
-	const T* hE;
-	const T* hBl; // FP32: lo parts of the multipliers (head rows), null for FP64
-	uint32_t H, n;
-	T mB, mE, lB, lE, c;
-	T mBl, lBl; // FP32: lo parts of the middle and last multipliers
+	T* p;
+	uint32_t st;
+	__device__ __forceinline__ int stride() const { return DIR * (STRIDE ? STRIDE : (int)st); }
+	__device__ __forceinline__ T& at(uint32_t j) const { return p[(int)j * stride()]; }
+	__device__ __forceinline__ void load(uint32_t j, T (&x)[kBlock]) const
+	{
+		const T* b = p + (int)j * stride();
+#pragma unroll
+		for (int k = 0; k < kBlock; k++)
+			x[k] = b[k * stride()];
+	}
+	__device__ __forceinline__ void store(uint32_t j, const T (&x)[kBlock]) const
+	{
+		T* b = p + (int)j * stride();
+#pragma unroll
+		for (int k = 0; k < kBlock; k++)
+			b[k * stride()] = x[k];
+	}
 };
 
-// One backward step d = (x + c d) b'.  FP32: evaluated as d = (b' c) d + b' x, with
-// the FP32 coupling b' c = RN(bh * c) and the product b' x taken with the
-// multiplier's pair bh + lo (the host's column-sum-exact multipliers account for
-// the coupling's rounding), so the chain from one point to the next is a single
-// fma (b' x does not depend on the chain).  FP64 tables hold b' itself (lo
-// unused) and keep the reference's form.
-__device__ __forceinline__ float bwd_step(float c, float d, float x, float bh, float bl)
+// FP32 points side by side (one substrate, a lane per row): blocks move as two
+// 16-byte accesses, so the rows of a warp, an odd number of 16-byte chunks apart, meet
+// no bank conflict.  Rows start on 16-byte boundaries and blocks at multiples of 8.
+struct RowLine
 {
-	const float bc = bh * c;
-	const float xb = dev::fmadd(x, bh, x * bl);
-	return dev::fmadd(bc, d, xb);
-}
-__device__ __forceinline__ double bwd_step(double c, double d, double x, double bh, double)
-{
-	return dev::fmadd(c, d, x) * bh;
-}
+	float* p;
+	__device__ __forceinline__ float& at(uint32_t j) const { return p[j]; }
+	__device__ __forceinline__ void load(uint32_t j, float (&x)[kBlock]) const
+	{
+#pragma unroll
+		for (int c = 0; c < 2; c++)
+		{
+			const float4 v = *reinterpret_cast<const float4*>(p + j + 4 * c);
+			x[4 * c] = v.x, x[4 * c + 1] = v.y, x[4 * c + 2] = v.z, x[4 * c + 3] = v.w;
+		}
+	}
+	__device__ __forceinline__ void store(uint32_t j, const float (&x)[kBlock]) const
+	{
+#pragma unroll
+		for (int c = 0; c < 2; c++)
+			*reinterpret_cast<float4*>(p + j + 4 * c) = make_float4(x[4 * c], x[4 * c + 1], x[4 * c + 2], x[4 * c + 3]);
+	}
+};
 
-// Compressed table of an axis: [head b' (S x H) | head e (S x H) | mid b' | mid e |
-// last b' | last e | c], the five constant arrays kS = S rounded up to 16 bytes long;
-// FP32 tables continue with [head b' lo (S x H) | mid b' lo | last b' lo].
 template <typename T>
-__device__ __forceinline__ LineCoef<T> line_coef(const T* comp, uint32_t S, uint32_t H, uint32_t n, uint32_t s)
+struct LineCoef;
+
+// The scale factors of one lane's half line at the last FP64 sweep: g the column's
+// factor from the other axes, mid = g times the converged factor, and the line's own
+// factors in memory (point j of the half at row[j * step]) for the head points.
+template <typename T>
+struct LineScale
 {
-	constexpr uint32_t VN = 16 / sizeof(T);
-	const uint32_t kS = (S + VN - 1) / VN * VN;
-	const T* k = comp + 2ull * S * H;
-	LineCoef<T> L;
-	L.hB = comp + (uint64_t)s * H;
-	L.hE = comp + (uint64_t)S * H + (uint64_t)s * H;
+	double g, mid;
+	const double* row;
+	int step;
+};
+
+// ------------------------------------------------------------------ FP32
+
+// One lane's coefficients along a line, from the axis's table: points j < H read the
+// substrate's head rows, points H <= j < n-1 share the middle constants, and point
+// n-1 has its own (when H >= n the head holds the whole line).  H is a multiple of
+// kBlock, so a block of points is either all head or all middle/last.
+template <>
+struct LineCoef<float>
+{
+	const float* hB;
+	const float* hE;
+	const float* hBl; // lo parts of the multipliers (head rows)
+	uint32_t H, n;
+	float mB, mE, lB, lE, c;
+	float mBl, lBl; // lo parts of the middle and last multipliers
+};
+
+// FP32 table of an axis: [head b' (S x H) | head e (S x H) | mid b' | mid e |
+// last b' | last e | c], the five constant arrays kS = S rounded up to 16 bytes long,
+// then [head b' lo (S x H) | mid b' lo | last b' lo].
+__device__ __forceinline__ LineCoef<float> line_coef(const float* tab, uint32_t S, uint32_t H, uint32_t n, uint32_t s,
+													 uint32_t)
+{
+	const uint32_t kS = (S + 3) / 4 * 4;
+	const float* k = tab + 2ull * S * H;
+	const float* lo = k + 5 * kS;
+	LineCoef<float> L;
+	L.hB = tab + (uint64_t)s * H;
+	L.hE = tab + (uint64_t)S * H + (uint64_t)s * H;
 	L.H = H;
 	L.n = n;
 	L.mB = __ldg(k + s);
@@ -169,29 +218,29 @@ __device__ __forceinline__ LineCoef<T> line_coef(const T* comp, uint32_t S, uint
 	L.lB = __ldg(k + 2 * kS + s);
 	L.lE = __ldg(k + 3 * kS + s);
 	L.c = __ldg(k + 4 * kS + s);
-	if constexpr (sizeof(T) == 4)
-	{
-		const T* lo = k + 5 * kS;
-		L.hBl = lo + (uint64_t)s * H;
-		L.mBl = __ldg(lo + (uint64_t)S * H + s);
-		L.lBl = __ldg(lo + (uint64_t)S * H + kS + s);
-	}
-	else
-	{
-		L.hBl = nullptr;
-		L.mBl = L.lBl = T(0);
-	}
+	L.hBl = lo + (uint64_t)s * H;
+	L.mBl = __ldg(lo + (uint64_t)S * H + s);
+	L.lBl = __ldg(lo + (uint64_t)S * H + kS + s);
 	return L;
 }
 
-template <typename T>
-__device__ __forceinline__ T coef_at(const T* head, uint32_t H, T mid, T last, uint32_t n, uint32_t j)
+// One backward step d = (x + c d) b', evaluated as (b' c) d + b' x with the coupling
+// b' c = RN(bh * c) and the product b' x taken with the multiplier's pair bh + bl
+// (the host's column-sum-exact multipliers account for the coupling's rounding), so
+// the chain from one point to the next is a single fma.
+__device__ __forceinline__ float bwd_step(float c, float d, float x, float bh, float bl)
+{
+	const float bc = bh * c;
+	const float xb = dev::fmadd(x, bh, x * bl);
+	return dev::fmadd(bc, d, xb);
+}
+
+__device__ __forceinline__ float coef_at(const float* head, uint32_t H, float mid, float last, uint32_t n, uint32_t j)
 {
 	return j < H ? __ldg(head + j) : (j == n - 1 ? last : mid);
 }
 
-// One line of n points at col[j * stride] in shared memory (stride = STRIDE, or the
-// run-time value when STRIDE is 0) with the lane's coefficients L.  The line is
+// One line of n points in shared memory with the lane's coefficients L.  The line is
 // three runs: head blocks of kBlock points [0, hb) (coefficients from the head
 // rows), middle blocks [hb, q) (the middle constants, held in registers) and the
 // points from q * kBlock on, which hold point n-1 (coefficients chosen per point;
@@ -203,91 +252,78 @@ __device__ __forceinline__ T coef_at(const T* head, uint32_t H, T mid, T last, u
 //
 // MC (kMcIn / kMcOut bits) adds the line's input values to *acc_in and its
 // solved values to *acc_out.
-template <typename T, int STRIDE, int MC = 0>
-__device__ __forceinline__ void solve_line(T* __restrict__ col, uint32_t n, uint32_t rt_stride, const LineCoef<T>& L,
-										   MassAcc<T>* acc_in = nullptr, MassAcc<T>* acc_out = nullptr)
+template <class AC, int MC>
+__device__ __forceinline__ void solve_line(const AC& ac, uint32_t n, const LineCoef<float>& L, MassAcc<float>* acc_in,
+										   MassAcc<float>* acc_out)
 {
-	using V = typename Vec16<T>::type;
-	constexpr int P = kBlock, VN = Vec16<T>::N, NV = P / VN;
-	constexpr bool kLo = sizeof(T) == 4;
-	const uint32_t st = STRIDE ? (uint32_t)STRIDE : rt_stride;
+	constexpr int P = kBlock, NV = P / 4;
 	const uint32_t nb = n / P;
 	const uint32_t hb = min(L.H / P, nb);
 	const uint32_t q = max((n - 1) / P, hb); // blocks [hb, q) have j0 >= H and j0 + P <= n - 1
-	const T c = L.c;
+	const float c = L.c;
 	// the middle coupling of the backward step, as bwd_step forms it per point
-	const T mbc = kLo ? L.mB * c : T(0);
-	// offsets within the tile stay far below 2^32
-	auto load = [&](uint32_t b, T(&x)[P]) {
-		const T* blk = col + b * (uint32_t)P * st;
-#pragma unroll
-		for (int k = 0; k < P; k++)
-			x[k] = blk[k * st];
-	};
-	auto fetch_head = [&](const T* head, uint32_t b, V(&out)[NV]) {
+	const float mbc = L.mB * c;
+	auto fetch_head = [&](const float* head, uint32_t b, float(&out)[P]) {
 #pragma unroll
 		for (int v = 0; v < NV; v++)
-			out[v] = __ldg(reinterpret_cast<const V*>(head + b * P) + v);
+		{
+			const float4 q = __ldg(reinterpret_cast<const float4*>(head + b * P) + v);
+			out[4 * v] = q.x, out[4 * v + 1] = q.y, out[4 * v + 2] = q.z, out[4 * v + 3] = q.w;
+		}
 	};
-	T d = T(0);
+	float d = 0.f;
 
 	// ---- forward elimination
-	auto fwd_mid = [&](uint32_t b, const T(&x)[P]) {
-		T* blk = col + b * (uint32_t)P * st;
+	auto fwd_mid = [&](uint32_t b, float(&x)[P]) {
 		if constexpr ((MC & kMcIn) != 0)
 			acc_in->add_block(x);
 #pragma unroll
 		for (int k = 0; k < P; k++)
-		{
-			d = dev::fmadd(L.mE, d, x[k]);
-			blk[k * st] = d;
-		}
+			x[k] = d = dev::fmadd(L.mE, d, x[k]);
+		ac.store(b * P, x);
 	};
 	if (hb)
 	{
-		T x[P], xn[P];
-		V e[NV], en[NV];
-		load(0, x);
+		float x[P], xn[P];
+		float e[P], en[P];
+		ac.load((0) * P, x);
 		fetch_head(L.hE, 0, e);
 		for (uint32_t b = 0; b < hb; b++)
 		{
 			if (b + 1 < hb)
 			{
-				load(b + 1, xn);
+				ac.load((b + 1) * P, xn);
 				fetch_head(L.hE, b + 1, en);
 			}
 			if constexpr ((MC & kMcIn) != 0)
 				acc_in->add_block(x);
-			T* blk = col + b * (uint32_t)P * st;
+#pragma unroll
+			for (int k = 0; k < P; k++)
+				x[k] = d = dev::fmadd(e[k], d, x[k]);
+			ac.store(b * P, x);
 #pragma unroll
 			for (int k = 0; k < P; k++)
 			{
-				d = dev::fmadd(vget<V, T>(e[k / VN], k % VN), d, x[k]);
-				blk[k * st] = d;
-			}
-#pragma unroll
-			for (int k = 0; k < P; k++)
 				x[k] = xn[k];
-#pragma unroll
-			for (int v = 0; v < NV; v++)
-				e[v] = en[v];
+				e[k] = en[k];
+			}
 		}
 	}
 	if (hb < q)
 	{
-		T xa[P], xb[P];
+		float xa[P], xb[P];
 		uint32_t b = hb;
-		load(b, xa);
+		ac.load((b) * P, xa);
 		for (; b + 2 < q; b += 2)
 		{
-			load(b + 1, xb);
+			ac.load((b + 1) * P, xb);
 			fwd_mid(b, xa);
-			load(b + 2, xa);
+			ac.load((b + 2) * P, xa);
 			fwd_mid(b + 1, xb);
 		}
 		if (b + 1 < q)
 		{
-			load(b + 1, xb);
+			ac.load((b + 1) * P, xb);
 			fwd_mid(b, xa);
 			fwd_mid(b + 1, xb);
 		}
@@ -296,54 +332,46 @@ __device__ __forceinline__ void solve_line(T* __restrict__ col, uint32_t n, uint
 	}
 	for (uint32_t j = q * P; j < n; j++)
 	{
-		const T xj = col[j * st];
+		const float xj = ac.at(j);
 		if constexpr ((MC & kMcIn) != 0)
 			acc_in->add(xj);
 		d = dev::fmadd(coef_at(L.hE, L.H, L.mE, L.lE, n, j), d, xj);
-		col[j * st] = d;
+		ac.at(j) = d;
 	}
 
 	// ---- back substitution
-	d = T(0);
+	d = 0.f;
 	for (int j = (int)n - 1; j >= (int)(q * P); j--)
 	{
-		const T bl = kLo ? coef_at(L.hBl, L.H, L.mBl, L.lBl, n, (uint32_t)j) : T(0);
-		d = bwd_step(c, d, col[(uint32_t)j * st], coef_at(L.hB, L.H, L.mB, L.lB, n, (uint32_t)j), bl);
-		col[(uint32_t)j * st] = d;
+		const float bl = coef_at(L.hBl, L.H, L.mBl, L.lBl, n, (uint32_t)j);
+		d = bwd_step(c, d, ac.at((uint32_t)j), coef_at(L.hB, L.H, L.mB, L.lB, n, (uint32_t)j), bl);
+		ac.at((uint32_t)j) = d;
 		if constexpr ((MC & kMcOut) != 0)
 			acc_out->add(d);
 	}
-	auto bwd_mid = [&](uint32_t b, const T(&x)[P]) {
-		T* blk = col + b * (uint32_t)P * st;
-		T y[P];
+	auto bwd_mid = [&](uint32_t b, float(&x)[P]) {
 #pragma unroll
 		for (int k = P - 1; k >= 0; k--)
-		{
-			if constexpr (kLo)
-				d = dev::fmadd(mbc, d, dev::fmadd(x[k], L.mB, x[k] * L.mBl));
-			else
-				d = dev::fmadd(c, d, x[k]) * L.mB;
-			blk[k * st] = d;
-			y[k] = d;
-		}
+			x[k] = d = dev::fmadd(mbc, d, dev::fmadd(x[k], L.mB, x[k] * L.mBl));
 		if constexpr ((MC & kMcOut) != 0)
-			acc_out->add_block(y);
+			acc_out->add_block(x);
+		ac.store(b * P, x);
 	};
 	if (hb < q)
 	{
-		T xa[P], xb[P];
+		float xa[P], xb[P];
 		uint32_t b = q - 1;
-		load(b, xa);
+		ac.load((b) * P, xa);
 		for (; b >= hb + 2; b -= 2)
 		{
-			load(b - 1, xb);
+			ac.load((b - 1) * P, xb);
 			bwd_mid(b, xa);
-			load(b - 2, xa);
+			ac.load((b - 2) * P, xa);
 			bwd_mid(b - 1, xb);
 		}
 		if (b >= hb + 1)
 		{
-			load(b - 1, xb);
+			ac.load((b - 1) * P, xb);
 			bwd_mid(b, xa);
 			bwd_mid(b - 1, xb);
 		}
@@ -352,413 +380,279 @@ __device__ __forceinline__ void solve_line(T* __restrict__ col, uint32_t n, uint
 	}
 	if (hb)
 	{
-		T x[P], xn[P];
-		V bb[NV], bn[NV], bl[NV], bln[NV];
-		load(hb - 1, x);
+		float x[P], xn[P];
+		float bb[P], bn[P], bl[P], bln[P];
+		ac.load((hb - 1) * P, x);
 		fetch_head(L.hB, hb - 1, bb);
-		if constexpr (kLo)
-			fetch_head(L.hBl, hb - 1, bl);
+		fetch_head(L.hBl, hb - 1, bl);
 		for (int b = (int)hb - 1; b >= 0; b--)
 		{
 			if (b > 0)
 			{
-				load((uint32_t)b - 1, xn);
+				ac.load(((uint32_t)b - 1) * P, xn);
 				fetch_head(L.hB, (uint32_t)b - 1, bn);
-				if constexpr (kLo)
-					fetch_head(L.hBl, (uint32_t)b - 1, bln);
+				fetch_head(L.hBl, (uint32_t)b - 1, bln);
 			}
-			T* blk = col + (uint32_t)b * (uint32_t)P * st;
-			T y[P];
 #pragma unroll
 			for (int k = P - 1; k >= 0; k--)
-			{
-				d = bwd_step(c, d, x[k], vget<V, T>(bb[k / VN], k % VN), kLo ? vget<V, T>(bl[k / VN], k % VN) : T(0));
-				blk[k * st] = d;
-				y[k] = d;
-			}
+				x[k] = d = bwd_step(c, d, x[k], bb[k], bl[k]);
 			if constexpr ((MC & kMcOut) != 0)
-				acc_out->add_block(y);
+				acc_out->add_block(x);
+			ac.store((uint32_t)b * P, x);
 #pragma unroll
 			for (int k = 0; k < P; k++)
+			{
 				x[k] = xn[k];
-#pragma unroll
-			for (int v = 0; v < NV; v++)
-			{
-				bb[v] = bn[v];
-				if constexpr (kLo)
-					bl[v] = bln[v];
+				bb[k] = bn[k];
+				bl[k] = bln[k];
 			}
 		}
 	}
 }
 
-// S*sizeof(T) a multiple of 16 bytes: thread h of a row's TPR threads owns chunk
-// slot h of every x position (VN substrates, VN independent recurrences).
-// MC adds element u's inputs / outputs to acc_in[u] / acc_out[u] (substrate h*VN + u).
-// cBl: the FP32 multipliers' lo parts (same layout as cB), null for FP64.
-template <typename T, int TPR, int MC = 0>
-__device__ __forceinline__ void solve_row_chunks(T* row, const T* __restrict__ cB, const T* __restrict__ cE,
-												 const T* __restrict__ cC, const T* __restrict__ cBl, uint32_t n, int h,
-												 MassAcc<T>* acc_in = nullptr, MassAcc<T>* acc_out = nullptr)
+// ------------------------------------------------------------------ FP64
+
+// One lane's coefficients for its half of a line, from the axis's table (capi.cu):
+// points j < H take theirs from the substrate's head rows, the others share e.
+template <>
+struct LineCoef<double>
 {
-	using V = typename Vec16<T>::type;
-	constexpr int VN = Vec16<T>::N, P = kChunkBlock;
-	constexpr bool kLo = sizeof(T) == 4;
-	V* __restrict__ vrow = reinterpret_cast<V*>(row) + h;
-	const V* vE = reinterpret_cast<const V*>(cE) + h;
-	const V* vB = reinterpret_cast<const V*>(cB) + h;
-	const V* vBl = kLo ? reinterpret_cast<const V*>(cBl) + h : nullptr;
-	const uint32_t nb = n / P;
-	T d[VN], c[VN];
+	const double* hE; // inward coefficients of the head points
+	const double* hG; // outward
+	uint32_t H;
+	double e;
+	double ws, wo; // meeting point: weights of the half's own and the other half's value
+};
+
+__device__ __forceinline__ LineCoef<double> line_coef(const double* tab, uint32_t S, uint32_t H, uint32_t, uint32_t s,
+													  uint32_t half)
+{
+	const double* k = tab + 2 * S * H + s;
+	LineCoef<double> L;
+	L.hE = tab + s * H;
+	L.hG = tab + (S + s) * H;
+	L.H = H;
+	L.e = __ldg(k);
+	L.ws = __ldg(k + S);
+	L.wo = __ldg(k + (2 + half) * S);
+	return L;
+}
+
+// The scale factors of a lane's half line from the axis's table: `sc` points at the
+// factor of the line's point 0, `step` separates its points', `mid` is the converged
+// one.
+__device__ __forceinline__ LineScale<double> line_scale(double g, double mid, const double* sc, int step, uint32_t n,
+														uint32_t half)
+{
+	return { g, g * mid, half == 0 ? sc : sc + (int64_t)(n - 1) * step, half == 0 ? step : -step };
+}
+
+// The 8 head coefficients from point j on.
+__device__ __forceinline__ void head_block(const double* row, uint32_t j, double (&c)[kBlock])
+{
 #pragma unroll
-	for (int u = 0; u < VN; u++)
+	for (int v = 0; v < kBlock / 2; v++)
 	{
-		d[u] = T(0);
-		c[u] = __ldg(cC + h * VN + u);
-	}
-	auto step_fwd = [&](V& v, const V& e) {
-#pragma unroll
-		for (int u = 0; u < VN; u++)
-		{
-			if constexpr ((MC & kMcIn) != 0)
-				acc_in[u].add(vget<V, T>(v, u));
-			d[u] = dev::fmadd(vget<V, T>(e, u), d[u], vget<V, T>(v, u));
-			vset<V, T>(v, u, d[u]);
-		}
-	};
-	auto step_bwd = [&](V& v, const V& b, const V& bl) {
-#pragma unroll
-		for (int u = 0; u < VN; u++)
-		{
-			d[u] = bwd_step(c[u], d[u], vget<V, T>(v, u), vget<V, T>(b, u), kLo ? vget<V, T>(bl, u) : T(0));
-			vset<V, T>(v, u, d[u]);
-			if constexpr ((MC & kMcOut) != 0)
-				acc_out[u].add(d[u]);
-		}
-	};
-	auto ldg_lo = [&](uint32_t k) {
-		V z {};
-		if constexpr (kLo)
-			z = ldg_vec(vBl + k);
-		return z;
-	};
-	{
-		V x[P], xn[P], e[P], en[P];
-		if (nb)
-#pragma unroll
-			for (int q = 0; q < P; q++)
-			{
-				x[q] = vrow[q * TPR];
-				e[q] = ldg_vec(vE + q * TPR);
-			}
-		for (uint32_t b = 0; b < nb; b++)
-		{
-			const uint32_t i0 = b * P;
-			if (b + 1 < nb)
-#pragma unroll
-				for (int q = 0; q < P; q++)
-				{
-					xn[q] = vrow[(i0 + P + q) * TPR];
-					en[q] = ldg_vec(vE + (i0 + P + q) * TPR);
-				}
-#pragma unroll
-			for (int q = 0; q < P; q++)
-			{
-				step_fwd(x[q], e[q]);
-				vrow[(i0 + q) * TPR] = x[q];
-			}
-#pragma unroll
-			for (int q = 0; q < P; q++)
-			{
-				x[q] = xn[q];
-				e[q] = en[q];
-			}
-		}
-		for (uint32_t i = nb * P; i < n; i++)
-		{
-			V v = vrow[i * TPR];
-			step_fwd(v, ldg_vec(vE + i * TPR));
-			vrow[i * TPR] = v;
-		}
-	}
-#pragma unroll
-	for (int u = 0; u < VN; u++)
-		d[u] = T(0);
-	for (int i = (int)n - 1; i >= (int)(nb * P); i--)
-	{
-		V v = vrow[i * TPR];
-		step_bwd(v, ldg_vec(vB + i * TPR), ldg_lo(i * TPR));
-		vrow[i * TPR] = v;
-	}
-	{
-		V x[P], xn[P], bb[P], bn[P], bl[P], bln[P];
-		if (nb)
-#pragma unroll
-			for (int q = 0; q < P; q++)
-			{
-				x[q] = vrow[((nb - 1) * P + q) * TPR];
-				bb[q] = ldg_vec(vB + ((nb - 1) * P + q) * TPR);
-				bl[q] = ldg_lo(((nb - 1) * P + q) * TPR);
-			}
-		for (int b = (int)nb - 1; b >= 0; b--)
-		{
-			const uint32_t i0 = (uint32_t)b * P;
-			if (b > 0)
-#pragma unroll
-				for (int q = 0; q < P; q++)
-				{
-					xn[q] = vrow[(i0 - P + q) * TPR];
-					bn[q] = ldg_vec(vB + (i0 - P + q) * TPR);
-					bln[q] = ldg_lo((i0 - P + q) * TPR);
-				}
-#pragma unroll
-			for (int q = P - 1; q >= 0; q--)
-			{
-				step_bwd(x[q], bb[q], bl[q]);
-				vrow[(i0 + q) * TPR] = x[q];
-			}
-#pragma unroll
-			for (int q = 0; q < P; q++)
-			{
-				x[q] = xn[q];
-				bb[q] = bn[q];
-				bl[q] = bln[q];
-			}
-		}
+		const double2 a = __ldg(reinterpret_cast<const double2*>(row + j) + v);
+		c[2 * v] = a.x, c[2 * v + 1] = a.y;
 	}
 }
 
-// ST substrates (1..8) not filling whole chunks: the row is a stream of chunks,
-// element k of substrate k % ST.  Blocks of NB chunks hold whole groups of
-// lcm(ST, VN) elements, so each element's substrate is a compile-time index.  The
-// blocks that lie wholly inside the row run without per-element tests, two
-// register sets in turn (the next block's chunks and coefficients load while the
-// current block's chain runs, and no block is copied from one set to the other);
-// the chunks after them, at most NB + U - 1, test each element against the row's
-// end.  MC adds substrate s's inputs / outputs to acc_in[s] / acc_out[s].
-template <typename T, int ST, int MC = 0>
-__device__ __forceinline__ void solve_row_vec(T* row, const T* __restrict__ cB, const T* __restrict__ cE,
-											  const T* __restrict__ cC, const T* __restrict__ cBl, uint32_t n,
-											  MassAcc<T>* acc_in = nullptr, MassAcc<T>* acc_out = nullptr)
+// Inward elimination of a half line of len points; returns the last value (also
+// left in the tile).  The blocks of 8 that hold head points take their
+// coefficients from the head rows; the others alternate two register sets, the
+// next block's points requested before the current block's dependent chain.  All
+// counts are the same for every lane of a warp.
+template <class AC, int MC>
+__device__ __forceinline__ double solve_inward(const AC& ac, uint32_t len, const LineCoef<double>& L, MassAcc<double>* acc)
 {
-	using V = typename Vec16<T>::type;
-	constexpr int VN = Vec16<T>::N;
-	constexpr int GE = group_elems(ST, VN);
-	constexpr int U = GE / VN;
-	constexpr int NB = U * ((kChunkBlock + U - 1) / U); // chunks per block
-	const uint32_t total = n * ST;
-	const uint32_t nchunks = (total + GE - 1) / GE * U; // whole groups (tail elements tested)
-	const uint32_t nfull = total / (NB * VN);           // blocks wholly inside the row
-	constexpr bool kLo = sizeof(T) == 4;
-	V* __restrict__ vrow = reinterpret_cast<V*>(row);
-	const V* vE = reinterpret_cast<const V*>(cE);
-	const V* vB = reinterpret_cast<const V*>(cB);
-	const V* vBl = reinterpret_cast<const V*>(cBl);
-	auto ldg_lo = [&](uint32_t k) {
-		V z {};
-		if constexpr (kLo)
-			z = ldg_vec(vBl + k);
-		return z;
-	};
-	T d[ST], c[ST];
-#pragma unroll
-	for (int s = 0; s < ST; s++)
-	{
-		d[s] = T(0);
-		c[s] = __ldg(cC + s);
-	}
-	// In a block or group starting at chunk k0 (k0*VN a multiple of ST), element
-	// k0*VN + q*VN + u has substrate (q*VN + u) % ST.  TEST: check the element
-	// against the row's end.
-	auto fwd_chunk = [&](V& v, const V& e, int q, uint32_t k, bool test) {
-#pragma unroll
-		for (int u = 0; u < VN; u++)
-		{
-			const int s = (q * VN + u) % ST;
-			if (!test || k * VN + u < total)
-			{
-				if constexpr ((MC & kMcIn) != 0)
-					acc_in[s].add(vget<V, T>(v, u));
-				d[s] = dev::fmadd(vget<V, T>(e, u), d[s], vget<V, T>(v, u));
-				vset<V, T>(v, u, d[s]);
-			}
-		}
-	};
-	auto bwd_chunk = [&](V& v, const V& b, const V& bl, int q, uint32_t k, bool test) {
-#pragma unroll
-		for (int u = VN - 1; u >= 0; u--)
-		{
-			const int s = (q * VN + u) % ST;
-			if (!test || k * VN + u < total)
-			{
-				d[s] = bwd_step(c[s], d[s], vget<V, T>(v, u), vget<V, T>(b, u), kLo ? vget<V, T>(bl, u) : T(0));
-				vset<V, T>(v, u, d[s]);
-				if constexpr ((MC & kMcOut) != 0)
-					acc_out[s].add(d[s]);
-			}
-		}
-	};
-
-	// ---- forward elimination
-	auto fwd_load = [&](uint32_t b, V(&x)[NB], V(&e)[NB]) {
-#pragma unroll
-		for (int q = 0; q < NB; q++)
-		{
-			x[q] = vrow[b * NB + q];
-			e[q] = ldg_vec(vE + b * NB + q);
-		}
-	};
-	auto fwd_block = [&](uint32_t b, V(&x)[NB], const V(&e)[NB]) {
-#pragma unroll
-		for (int q = 0; q < NB; q++)
-		{
-			fwd_chunk(x[q], e[q], q, b * NB + q, false);
-			vrow[b * NB + q] = x[q];
-		}
-	};
-	if (nfull)
-	{
-		V xa[NB], ea[NB], xb[NB], eb[NB];
-		uint32_t b = 0;
-		fwd_load(0, xa, ea);
-		for (; b + 2 < nfull; b += 2)
-		{
-			fwd_load(b + 1, xb, eb);
-			fwd_block(b, xa, ea);
-			fwd_load(b + 2, xa, ea);
-			fwd_block(b + 1, xb, eb);
-		}
-		if (b + 1 < nfull)
-		{
-			fwd_load(b + 1, xb, eb);
-			fwd_block(b, xa, ea);
-			fwd_block(b + 1, xb, eb);
-		}
-		else
-			fwd_block(b, xa, ea);
-	}
-	for (uint32_t k0 = nfull * NB; k0 < nchunks; k0 += U)
-	{
-#pragma unroll
-		for (int q = 0; q < U; q++)
-		{
-			V v = vrow[k0 + q];
-			fwd_chunk(v, ldg_vec(vE + k0 + q), q, k0 + q, true);
-			vrow[k0 + q] = v;
-		}
-	}
-
-	// ---- back substitution
-#pragma unroll
-	for (int s = 0; s < ST; s++)
-		d[s] = T(0);
-	for (int k0 = (int)nchunks - U; k0 >= (int)(nfull * NB); k0 -= U)
-	{
-#pragma unroll
-		for (int q = U - 1; q >= 0; q--)
-		{
-			V v = vrow[k0 + q];
-			bwd_chunk(v, ldg_vec(vB + k0 + q), ldg_lo(k0 + q), q, (uint32_t)(k0 + q), true);
-			vrow[k0 + q] = v;
-		}
-	}
-	auto bwd_load = [&](uint32_t b, V(&x)[NB], V(&bb)[NB], V(&bl)[NB]) {
-#pragma unroll
-		for (int q = 0; q < NB; q++)
-		{
-			x[q] = vrow[b * NB + q];
-			bb[q] = ldg_vec(vB + b * NB + q);
-			bl[q] = ldg_lo(b * NB + q);
-		}
-	};
-	auto bwd_block = [&](uint32_t b, V(&x)[NB], const V(&bb)[NB], const V(&bl)[NB]) {
-#pragma unroll
-		for (int q = NB - 1; q >= 0; q--)
-		{
-			bwd_chunk(x[q], bb[q], bl[q], q, b * NB + q, false);
-			vrow[b * NB + q] = x[q];
-		}
-	};
-	if (nfull)
-	{
-		V xa[NB], ba[NB], la[NB], xb[NB], bbb[NB], lb[NB];
-		uint32_t b = nfull - 1;
-		bwd_load(b, xa, ba, la);
-		for (; b >= 2; b -= 2)
-		{
-			bwd_load(b - 1, xb, bbb, lb);
-			bwd_block(b, xa, ba, la);
-			bwd_load(b - 2, xa, ba, la);
-			bwd_block(b - 1, xb, bbb, lb);
-		}
-		if (b >= 1)
-		{
-			bwd_load(b - 1, xb, bbb, lb);
-			bwd_block(b, xa, ba, la);
-			bwd_block(b - 1, xb, bbb, lb);
-		}
-		else
-			bwd_block(b, xa, ba, la);
-	}
-}
-
-// Any S: one recurrence at a time, scalar shared-memory accesses.  MC adds
-// substrate s's input / output total of the row to mc_in[s] / mc_out[s] (FP64
-// atomics per row; a path for rare substrate counts).
-template <typename T, int MC = 0>
-__device__ __forceinline__ void solve_row_generic(T* row, const T* cB, const T* cE, const T* cC, const T* cBl,
-												  uint32_t n, uint32_t S, double* mc_in = nullptr,
-												  double* mc_out = nullptr)
-{
-	for (uint32_t s = 0; s < S; s++)
-	{
-		MassAcc<T> ai, ao;
-		ai.zero();
-		ao.zero();
-		T d = T(0);
-		for (uint32_t i = 0; i < n; i++)
-		{
-			if constexpr ((MC & kMcIn) != 0)
-				ai.add(row[i * S + s]);
-			d = dev::fmadd(__ldg(cE + i * S + s), d, row[i * S + s]);
-			row[i * S + s] = d;
-		}
-		const T c = __ldg(cC + s);
-		d = T(0);
-		for (int i = (int)n - 1; i >= 0; i--)
-		{
-			d = bwd_step(c, d, row[i * S + s], __ldg(cB + i * S + s), sizeof(T) == 4 ? __ldg(cBl + i * S + s) : T(0));
-			row[i * S + s] = d;
-			if constexpr ((MC & kMcOut) != 0)
-				ao.add(d);
-		}
+	constexpr int P = kBlock;
+	const uint32_t nb = len / P, hb = min(L.H / P, nb);
+	double d = 0.0;
+	auto mid = [&](uint32_t b, double(&x)[P]) {
 		if constexpr ((MC & kMcIn) != 0)
-			if (mc_in)
-				atomicAdd(mc_in + s, ai.value());
+			acc->add_block(x);
+#pragma unroll
+		for (int k = 0; k < P; k++)
+			x[k] = d = dev::fmadd(L.e, d, x[k]);
+		ac.store(b * P, x);
+	};
+	if (hb)
+	{
+		double x[P], xn[P], c[P], cn[P];
+		ac.load(0, x);
+		head_block(L.hE, 0, c);
+		for (uint32_t b = 0; b < hb; b++)
+		{
+			if (b + 1 < hb)
+			{
+				ac.load((b + 1) * P, xn);
+				head_block(L.hE, (b + 1) * P, cn);
+			}
+			if constexpr ((MC & kMcIn) != 0)
+				acc->add_block(x);
+#pragma unroll
+			for (int k = 0; k < P; k++)
+				x[k] = d = dev::fmadd(c[k], d, x[k]);
+			ac.store(b * P, x);
+#pragma unroll
+			for (int k = 0; k < P; k++)
+			{
+				x[k] = xn[k];
+				c[k] = cn[k];
+			}
+		}
+	}
+	if (hb < nb)
+	{
+		double xa[P], xb[P];
+		uint32_t b = hb;
+		ac.load(b * P, xa);
+		for (; b + 2 < nb; b += 2)
+		{
+			ac.load((b + 1) * P, xb);
+			mid(b, xa);
+			ac.load((b + 2) * P, xa);
+			mid(b + 1, xb);
+		}
+		if (b + 1 < nb)
+		{
+			ac.load((b + 1) * P, xb);
+			mid(b, xa);
+			mid(b + 1, xb);
+		}
+		else
+			mid(b, xa);
+	}
+	for (uint32_t j = nb * P; j < len; j++)
+	{
+		const double x = ac.at(j);
+		if constexpr ((MC & kMcIn) != 0)
+			acc->add(x);
+		d = dev::fmadd(j < L.H ? __ldg(L.hE + j) : L.e, d, x);
+		ac.at(j) = d;
+	}
+	return d;
+}
+
+// Outward substitution from the meeting point's value y.  SC: the stored values
+// are the solution (times the column's factor), else the solution over the line's
+// factors.
+template <class AC, int MC, int SC>
+__device__ __forceinline__ void solve_outward(const AC& ac, uint32_t len, const LineCoef<double>& L, double ymeet,
+											  const LineScale<double>& F, MassAcc<double>* acc)
+{
+	constexpr int P = kBlock;
+	const uint32_t nb = len / P, hb = min(L.H / P, nb);
+	ac.at(len - 1) = ymeet; // the recurrence then starts from a zero carry
+	double y = 0.0;
+	auto factor = [&](uint32_t j) { return F.g * __ldg(F.row + (int64_t)((int)j * F.step)); };
+	auto mid = [&](uint32_t b, double(&x)[P]) {
+#pragma unroll
+		for (int k = P - 1; k >= 0; k--)
+		{
+			y = dev::fmadd(L.e, y, x[k]);
+			x[k] = SC ? y * F.mid : y;
+		}
 		if constexpr ((MC & kMcOut) != 0)
-			if (mc_out)
-				atomicAdd(mc_out + s, ao.value());
+			acc->add_block(x);
+		ac.store(b * P, x);
+	};
+	for (int j = (int)len - 1; j >= (int)(nb * P); j--)
+	{
+		y = dev::fmadd((uint32_t)j < L.H ? __ldg(L.hG + j) : L.e, y, ac.at(j));
+		const double o = SC ? y * ((uint32_t)j < L.H ? factor(j) : F.mid) : y;
+		ac.at(j) = o;
+		if constexpr ((MC & kMcOut) != 0)
+			acc->add(o);
+	}
+	if (hb < nb)
+	{
+		double xa[P], xb[P];
+		uint32_t b = nb - 1;
+		ac.load(b * P, xa);
+		for (; b >= hb + 2; b -= 2)
+		{
+			ac.load((b - 1) * P, xb);
+			mid(b, xa);
+			ac.load((b - 2) * P, xa);
+			mid(b - 1, xb);
+		}
+		if (b >= hb + 1)
+		{
+			ac.load((b - 1) * P, xb);
+			mid(b, xa);
+			mid(b - 1, xb);
+		}
+		else
+			mid(b, xa);
+	}
+	for (int b = (int)hb - 1; b >= 0; b--)
+	{
+		double x[P], c[P], f[P];
+		ac.load((uint32_t)b * P, x);
+		head_block(L.hG, (uint32_t)b * P, c);
+		if constexpr (SC != 0)
+#pragma unroll
+			for (int k = 0; k < P; k++)
+				f[k] = factor((uint32_t)(b * P + k));
+#pragma unroll
+		for (int k = P - 1; k >= 0; k--)
+		{
+			y = dev::fmadd(c[k], y, x[k]);
+			x[k] = SC ? y * f[k] : y;
+		}
+		if constexpr ((MC & kMcOut) != 0)
+			acc->add_block(x);
+		ac.store((uint32_t)b * P, x);
 	}
 }
 
-template <typename T, int ST>
-constexpr int x_tpr()
-{
-	return (ST > 0 && ST <= 8 && (ST * (int)sizeof(T)) % 16 == 0) ? ST * (int)sizeof(T) / 16 : 1;
-}
+// ------------------------------------------------------------------ tiles
 
-
-// Solves one x row of substrate count S at compile time when S <= 8.
-template <typename T, int ST>
-__device__ __forceinline__ void solve_row(T* row, const T* cB, const T* cE, const T* cC, const T* cBl, uint32_t n,
-										  uint32_t S, int h)
+// The lines of one tile, one per lane: `left` reaches a lane's line from point 0,
+// `right` from point n-1.  Lanes without a line (on == false) only take part in the
+// barriers.  FP32: the CTA's one warp solves whole lines.  FP64: warp `half` solves
+// its half of them; two barriers separate the reads of the other half's meeting
+// value from the writes around them (a line without a second half needs none).
+template <typename T, class ACL, class ACR, int MC, int SC>
+__device__ __forceinline__ void solve_tile(const ACL& left, const ACR& right, uint32_t n, uint32_t half, bool on,
+										   const LineCoef<T>& L, const LineScale<T>& F, MassAcc<T>* acc_in = nullptr,
+										   MassAcc<T>* acc_out = nullptr)
 {
-	if constexpr (ST == 0)
-		solve_row_generic<T>(row, cB, cE, cC, cBl, n, S);
-	else if constexpr ((ST * (int)sizeof(T)) % 16 == 0)
-		solve_row_chunks<T, x_tpr<T, ST>()>(row, cB, cE, cC, cBl, n, h);
+	if constexpr (sizeof(T) == 4)
+	{
+		if (on)
+			solve_line<ACL, MC>(left, n, L, acc_in, acc_out);
+	}
 	else
-		solve_row_vec<T, ST>(row, cB, cE, cC, cBl, n);
+	{
+		const uint32_t m = line_split<T>(n);
+		T own = T(0), other = T(0);
+		if (on)
+		{
+			if (half == 0)
+				own = solve_inward<ACL, MC>(left, m, L, acc_in);
+			else if (n > m)
+				own = solve_inward<ACR, MC>(right, n - m, L, acc_in);
+		}
+		if (n > m)
+		{
+			__syncthreads();
+			if (on)
+				other = half == 0 ? right.at(n - m - 1) : left.at(m - 1);
+			__syncthreads();
+		}
+		if (on)
+		{
+			// the solution at the half's inner end, over its scale factor
+			const T y = dev::fmadd(L.ws, own, L.wo * other);
+			if (half == 0)
+				solve_outward<ACL, MC, SC>(left, m, L, y, F, acc_out);
+			else if (n > m)
+				solve_outward<ACR, MC, SC>(right, n - m, L, y, F, acc_out);
+		}
+	}
 }
 
 } // namespace solvers

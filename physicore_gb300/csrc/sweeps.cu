@@ -1,35 +1,31 @@
-// sweeps.cu -- ADI/LOD Thomas sweeps along x, y and z on sm_103a.
+// sweeps.cu -- ADI/LOD tridiagonal sweeps along x, y and z on sm_103a.
 //
-// Arithmetic per line follows the reference (openmp_solver/src/diffusion_solver.cpp:
-// 116-202 for x, 390-794 for y/z; coefficients of diffusion_solver.cpp:29-86):
-//   forward   d_i  = d_i + e_{i-1} d_{i-1}            i = 1..n-1
-//             d_{n-1} = d_{n-1} b'_{n-1}
-//   backward  d_i  = (d_i + c d_{i+1}) b'_i            i = n-2..0
-// with each line using the coefficients of its own substrate.  Both passes start
-// from a zero carry: e_{-1} = 0 makes the first forward step d_0 = d_0, and c*0 = 0
-// makes the first backward step d_{n-1} b'_{n-1}, so every step has one form.
+// Each line solves the reference's matrix of its substrate (openmp_solver/src/
+// diffusion_solver.cpp:116-202 for x, 390-794 for y/z; coefficients of
+// diffusion_solver.cpp:29-86); the solvers are in sweep_solvers.cuh.
 //
 // GB300 mapping (our own design):
-//  * A line must stay on chip between its forward and backward pass, so shared
-//    memory bounds how many lines an SM can hold (~160 lines of 320 FP32 points).
-//    Every byte of it therefore holds line data: tiles are single-stage, the
-//    coefficient tables are read through L1 (__ldg, 16-byte vectors), and tile
-//    sizes are chosen so that several CTAs share an SM and all four schedulers
-//    have warps to issue.
-//  * Persistent CTAs (one warp) walk their tiles: TMA loads complete on an
-//    mbarrier, the warp solves the tile in place, and TMA stores write it back; the
-//    next load is issued as soon as the stores have read shared memory.  Several
-//    such CTAs per SM overlap one another's loads, compute and stores.
-//  * Solvers run in blocks of P steps without per-step predicates; the next block's
-//    points and coefficients are requested before the current block's dependent
-//    chain, so load latency overlaps the chain.
+//  * A line must stay on chip between its two passes, so shared memory bounds how
+//    many lines an SM can hold (~160 lines of 320 FP32 points).  Every byte of it
+//    therefore holds line data: tiles are single-stage, the coefficient tables are
+//    read through L1 (__ldg, 16-byte vectors), and tile sizes are chosen so that
+//    several CTAs share an SM.
+//  * FP32: a CTA is one warp on one tile.  FP64, which the FP64 pipe's latency and
+//    rate bound, not memory: two warps, one for each half of the tile's lines.
+//  * Persistent CTAs walk their tiles (the first is the CTA's index, the next ones
+//    come from an atomic counter drawn while the current tile is solved): TMA loads
+//    complete on an mbarrier, the tile is solved in place, and TMA stores
+//    write it back; the next load is issued as soon as the stores have read shared
+//    memory.  Several such CTAs per SM overlap one another's loads, compute and
+//    stores.
+//  * Solvers run in blocks of 8 steps without per-step predicates; the next block's
+//    points are requested before the current block's dependent chain, so load
+//    latency overlaps the chain.
 //  * y/z: a tile is 32 consecutive (x,s) elements of a row at every point of the
-//    lines; lane t solves column t of the [n][32] tile (bank-conflict free) with
-//    the coefficient row of its substrate ([s][j] table).
-//  * x: a tile is R whole rows; a row is walked as a stream of 16-byte chunks,
-//    element k belonging to substrate k % S, with one carry per substrate.  When a
-//    voxel's substrates fill whole chunks, TPR threads share a row, one chunk slot
-//    each; rows are TPR (mod 8) chunks apart so quarter-warps hit distinct banks.
+//    lines; lane t of a warp solves column t of the [n][32] tile (bank-conflict
+//    free).
+//  * x: a tile is R whole rows and lane (r, s) solves substrate s of row r; one
+//    FP32 substrate alone takes a thread per row and 16-byte accesses.
 //  * Every wait is bounded; a timeout sets a device error bit instead of trapping.
 #include "field_device.cuh"
 #include "pcg_internal.cuh"
@@ -46,278 +42,233 @@ using namespace solvers;
 // The y/z sweep.  A tile is 32 consecutive (x,s) elements at all n points of the
 // lines of one outer index; it arrives as nc TMA tensor boxes (32, R) of the field
 // described as the 3-D tensor (x*S+s, y, z), all completing on one mbarrier.  The
-// warp solves the tile in place and stores it back with nc box stores; the next
-// tile's loads start once the stores have read shared memory.  Loads and compute
-// overlap across the several single-warp CTAs an SM holds; within a CTA the solver
-// runs without per-chunk bookkeeping.  Coefficients come from the compressed
-// tables (head rows, then per-substrate constants), so most points need no
-// coefficient load at all.
+// CTA solves its lines in place and one thread stores it back with nc box stores; the next tile's loads start once the stores have read
+// shared memory.  Loads and compute overlap across the CTAs an SM holds.
+// Coefficients come from the axis's table (head rows, then per-substrate
+// constants), so most points need no coefficient load at all.
 //
+// SC = 1 (FP64: the step's last sweep, or every sweep of a mesh whose factors are not
+// deferred): the stored values are multiplied by the scale factors.
 // MC = kMcOut (the step's last sweep with the mass check on): the lanes also sum
 // their solved values before the faces are written, into a.mc_tot[S + s].  A
 // lane's substrate is the same in every tile when S divides 32 (it then keeps one
 // running total and adds it once at the end), else it adds its total per tile.
-template <typename T, int AXIS, int MC>
-__global__ void __launch_bounds__(kLanes) sweep_yz_kernel(SweepArgs a, const __grid_constant__ CUtensorMap tmap)
+template <typename T, int AXIS, int MC, int SC>
+__global__ void __launch_bounds__(sweep_threads<T>()) sweep_yz_kernel(SweepArgs a, const __grid_constant__ CUtensorMap tmap)
 {
 	extern __shared__ __align__(128) unsigned char smem[];
 	uint64_t* full = reinterpret_cast<uint64_t*>(smem);
+	uint32_t& next = *reinterpret_cast<uint32_t*>(smem + 8);
 	T* base = reinterpret_cast<T*>(smem + 128);
-	const uint32_t lane = threadIdx.x;
-	const uint32_t n = a.n, S = a.S, R = a.box_rows, nc = a.boxes;
+	const uint32_t lane = threadIdx.x & 31, half = threadIdx.x >> 5;
+	const uint32_t n = a.n, m = line_split<T>(n), S = a.S, R = a.box_rows, nc = a.boxes;
 	const uint32_t chunk_elems = R * kLanes;
-	const T* comp = static_cast<const T*>(a.coef) + a.comp_off;
-	if (lane == 0)
+	if (threadIdx.x == 0)
 	{
 		dev::mbar_init(full, 1);
 		dev::fence_mbar_init();
 	}
-	__syncwarp();
+	__syncthreads();
 	bool ok = true;
 	MassAcc<T> acc;
 	acc.zero();
 	const bool per_tile = (kLanes % S) != 0;
 	const uint32_t classes = S < kLanes ? S : kLanes;
 	// 32-bit tile arithmetic: a launch has fewer than 2^32 tiles
-	const uint32_t xblocks = (uint32_t)a.xblocks, nouter = (uint32_t)(a.tiles / a.xblocks);
-	for (uint32_t phase = 0;; phase ^= 1)
+	const uint32_t xblocks = (uint32_t)a.xblocks, tiles = (uint32_t)a.tiles, nouter = tiles / xblocks;
+	uint32_t t = blockIdx.x;
+	for (uint32_t phase = 0; t < tiles; phase ^= 1)
 	{
-		uint32_t t32 = 0;
-		if (lane == 0)
-			t32 = atomicAdd(a.ticket, 1u);
-		const uint32_t t = __shfl_sync(0xffffffffu, t32, 0);
-		if (t >= a.tiles)
-			break;
-		const int x0 = (int)((t % xblocks) * kLanes);
+		const uint32_t x0 = (t % xblocks) * kLanes;
 		// y takes its z-planes from the last down: the x sweep that ran just before
 		// wrote the highest planes last, and their lines are still in L2
-		const int o = AXIS == 1 ? (int)(nouter - 1 - t / xblocks) : (int)(t / xblocks);
-		if (lane == 0)
+		const uint32_t o = AXIS == 1 ? nouter - 1 - t / xblocks : t / xblocks;
+		uint32_t drawn = 0;
+		if (threadIdx.x == 0)
 		{
 			dev::mbar_arrive_expect_tx(full, nc * chunk_elems * (uint32_t)sizeof(T));
 			for (uint32_t c = 0; c < nc; c++)
 			{
 				if (AXIS == 1)
-					dev::tma_load_3d(base + c * chunk_elems, &tmap, x0, (int)(c * R), o, full);
+					dev::tma_load_3d(base + c * chunk_elems, &tmap, (int)x0, (int)(c * R), (int)o, full);
 				else
-					dev::tma_load_3d(base + c * chunk_elems, &tmap, x0, o, (int)(c * R), full);
+					dev::tma_load_3d(base + c * chunk_elems, &tmap, (int)x0, (int)o, (int)(c * R), full);
 			}
+			drawn = gridDim.x + atomicAdd(a.ticket, 1u);
 		}
 		// lanes past the row hold zero-filled columns that are never stored
-		const uint32_t s = (uint64_t)(x0 + lane) < a.row_len ? (uint32_t)((x0 + lane) % S) : 0;
-		const LineCoef<T> L = line_coef<T>(comp, S, a.head, n, s);
-		ok = __all_sync(0xffffffffu, dev::mbar_wait(full, phase));
+		const uint32_t col = x0 + lane;
+		const bool in_row = col < a.row_len;
+		const uint32_t s = in_row ? col % S : 0;
+		const LineCoef<T> L = line_coef(static_cast<const T*>(a.tab), S, a.head, n, s, half);
+		LineScale<T> F {};
+		if constexpr (SC != 0)
+		{
+			T g = T(1);
+			if (a.gx)
+				g = __ldg(static_cast<const T*>(a.gx) + (in_row ? col : 0));
+			if (AXIS == 2 && a.gy)
+				g *= __ldg(static_cast<const T*>(a.gy) + (uint64_t)s * a.ny + o);
+			const T* sc = static_cast<const T*>(a.sc);
+			F = line_scale(g, __ldg(sc + s), sc + S + (uint64_t)s * n, 1, n, half);
+		}
+		ok = __syncthreads_and(dev::mbar_wait(full, phase));
 		if (!ok)
 			break;
-		solve_line<T, kLanes, MC>(base + lane, n, 0, L, nullptr, &acc);
+		solve_tile<T, Strided<T, kLanes, 1>, Strided<T, kLanes, -1>, MC, SC>(
+			{ base + lane, 0 }, { base + (n - 1) * kLanes + lane, 0 }, n, half, true, L, F, nullptr, &acc);
 		if constexpr ((MC & kMcOut) != 0)
 			if (per_tile)
 			{
-				flush_classes(acc.value(), classes, kLanes, a.mc_tot + S + ((uint64_t)x0 + lane) % S);
+				flush_classes(acc.value(), classes, kLanes, a.mc_tot + S + col % S);
 				acc.zero();
 			}
-		if (a.face_mask)
+		if (a.face_mask && in_row)
 		{
-			FaceArgs f {};
-			f.values = a.face_values;
-			f.conds = a.face_conds;
-			f.face_mask = a.face_mask;
-			f.S = S;
-			f.nx = a.nx, f.ny = a.ny, f.nz = a.nz;
-			fielddev::faces_on_column<T, AXIS>(f, base + lane, n, kLanes, (uint64_t)x0 + lane, (uint64_t)o);
+			const uint32_t len = half == 0 ? m : n - m;
+			fielddev::faces_on_half<T, AXIS>(a, col / S, s, o, half == 0 ? base + lane : base + m * kLanes + lane, len,
+											 kLanes, half == 0, half == 0 ? n == m : n > m);
 		}
+		if (threadIdx.x == 0)
+			next = drawn;
 		dev::fence_proxy_async_smem();
-		__syncwarp();
-		if (lane == 0)
+		__syncthreads();
+		t = next;
+		if (threadIdx.x == 0)
 		{
 			for (uint32_t c = 0; c < nc; c++)
 			{
 				if (AXIS == 1)
-					dev::tma_store_3d(&tmap, x0, (int)(c * R), o, base + c * chunk_elems);
+					dev::tma_store_3d(&tmap, (int)x0, (int)(c * R), (int)o, base + c * chunk_elems);
 				else
-					dev::tma_store_3d(&tmap, x0, o, (int)(c * R), base + c * chunk_elems);
+					dev::tma_store_3d(&tmap, (int)x0, (int)o, (int)(c * R), base + c * chunk_elems);
 			}
 			dev::bulk_commit();
 			dev::bulk_wait_read();
 		}
-		__syncwarp();
 	}
 	if constexpr ((MC & kMcOut) != 0)
 		if (!per_tile)
 			flush_classes(acc.value(), classes, kLanes, a.mc_tot + S + lane % S);
-	if (!ok && lane == 0)
+	if (!ok && threadIdx.x == 0)
 		atomicOr(a.err, DEV_ERR_WAIT_TIMEOUT);
-	if (lane == 0)
+	if (threadIdx.x == 0)
 		dev::bulk_wait_all();
 }
 
 // ------------------------------------------------------------------ x
 
-// Row-per-thread mapping: a tile is rows_per_tile consecutive rows and the CTA has
-// rows_per_tile * TPR threads (<= 32); TPR threads share a row when its substrates
-// fill whole 16-byte chunks.
-// MC (the mass check on): the threads also sum their rows' inputs (kMcIn) and, on
-// a 1-D mesh where x is the last sweep, their outputs (kMcOut) per substrate.
-template <typename T, int ST, int MC>
-__global__ void __launch_bounds__(kLanes) sweep_x_kernel(SweepArgs a)
+// The x sweep: a tile is rows_per_tile whole rows.  Lane (r, s) of a warp
+// solves substrate s of row r, points S elements apart in shared
+// memory; row pitches are chosen so that the lanes of a warp touch distinct banks.
+// ST = S when it is a compile-time constant (accesses with immediate offsets), 0
+// for the run-time path, -1 above 32 substrates, where a lane takes several lines
+// of the tile's one row in turn.  VEC (one FP32 substrate): a lane per row, 16-byte
+// accesses.  MC (the mass check on): the lanes also sum their lines' inputs (kMcIn)
+// and, on a 1-D mesh, outputs (kMcOut), added once at the end (per line when S is
+// above 32).
+template <typename T, int ST, int MC, int SC, bool VEC>
+__global__ void __launch_bounds__(sweep_threads<T>()) sweep_x_kernel(SweepArgs a)
 {
-	constexpr int TPR = x_tpr<T, ST>();
-	constexpr bool kChunks = ST > 0 && (ST * (int)sizeof(T)) % 16 == 0;
-	constexpr int NA = kChunks ? Vec16<T>::N : (ST > 0 ? ST : 1);
-	MassAcc<T> ai[NA], ao[NA];
-#pragma unroll
-	for (int u = 0; u < NA; u++)
-	{
-		ai[u].zero();
-		ao[u].zero();
-	}
+	constexpr bool kWide = ST < 0;
+	constexpr int STRIDE = ST > 0 ? ST : 0;
 	extern __shared__ __align__(128) unsigned char smem[];
 	uint64_t* bar = reinterpret_cast<uint64_t*>(smem);
-	uint32_t& ticket = *reinterpret_cast<uint32_t*>(smem + 8);
+	uint32_t& next = *reinterpret_cast<uint32_t*>(smem + 8);
 	T* tile = reinterpret_cast<T*>(smem + 16);
-	const int tid = threadIdx.x;
-	const uint32_t R = a.rows_per_tile;
-	const int r_local = tid / TPR, h = tid % TPR;
-	const uint32_t n = a.n;
+	const uint32_t lane = threadIdx.x & 31, half = threadIdx.x >> 5;
+	const uint32_t R = a.rows_per_tile, S = STRIDE ? (uint32_t)STRIDE : a.S, n = a.n;
+	const uint32_t r_local = kWide ? 0 : lane / S, s0 = kWide ? lane : lane % S;
+	const uint32_t pitch = (uint32_t)a.smem_pitch;
 	const uint32_t row_bytes = (uint32_t)round_up(a.row_len * sizeof(T), 16);
-	const T* cB = static_cast<const T*>(a.coef);
-	const T* cE = cB + a.coef_len;
-	const T* cC = cE + a.coef_len;
-	const T* cBl = sizeof(T) == 4 ? cB + a.blo_off : nullptr;
-	if (tid == 0)
+	if (threadIdx.x == 0)
 	{
 		dev::mbar_init(bar, 1);
 		dev::fence_mbar_init();
 	}
 	__syncthreads();
-
-	for (uint32_t phase = 0;; phase ^= 1)
-	{
-		if (tid == 0)
-			ticket = atomicAdd(a.ticket, 1u);
-		__syncthreads();
-		const uint64_t t = ticket;
-		if (t >= a.tiles)
-			break;
-		const uint64_t r0 = t * R;
-		const uint32_t nrows = (uint32_t)(a.rows - r0 < (uint64_t)R ? a.rows - r0 : (uint64_t)R);
-		T* g = static_cast<T*>(a.field) + r0 * a.pitch;
-		if (tid == 0)
-			dev::mbar_arrive_expect_tx(bar, nrows * row_bytes);
-		__syncthreads();
-		if ((uint32_t)tid < nrows)
-			dev::bulk_g2s(tile + tid * a.smem_pitch, g + tid * a.pitch, row_bytes, bar);
-		if (!__syncthreads_and(dev::mbar_wait(bar, phase)))
-		{
-			if (tid == 0)
-				atomicOr(a.err, DEV_ERR_WAIT_TIMEOUT);
-			break;
-		}
-		if ((uint32_t)r_local < nrows)
-		{
-			T* row = tile + r_local * a.smem_pitch;
-			if constexpr (ST == 0)
-				solve_row_generic<T, MC>(row, cB, cE, cC, cBl, n, a.S, a.mc_tot, a.mc_tot + a.S);
-			else if constexpr (kChunks)
-				solve_row_chunks<T, TPR, MC>(row, cB, cE, cC, cBl, n, h, ai, ao);
-			else
-				solve_row_vec<T, ST, MC>(row, cB, cE, cC, cBl, n, ai, ao);
-		}
-		dev::fence_proxy_async_smem();
-		__syncthreads();
-		if ((uint32_t)tid < nrows)
-			dev::bulk_s2g(g + tid * a.pitch, tile + tid * a.smem_pitch, row_bytes);
-		dev::bulk_commit();
-		dev::bulk_wait_read();
-		__syncthreads();
-	}
-	if constexpr (MC != 0 && ST > 0)
-	{
-		// thread r * TPR + h holds substrates h * VN + u (chunks) or u (one thread per row)
-#pragma unroll
-		for (int u = 0; u < NA; u++)
-		{
-			const uint32_t sub = kChunks ? (uint32_t)(h * Vec16<T>::N + u) : (uint32_t)u;
-			flush_classes(ai[u].value(), TPR, blockDim.x, a.mc_tot + sub);
-			if constexpr ((MC & kMcOut) != 0)
-				flush_classes(ao[u].value(), TPR, blockDim.x, a.mc_tot + a.S + sub);
-		}
-	}
-	dev::bulk_wait_all();
-}
-
-// Substrate-per-thread mapping: a tile is rows_per_tile rows and thread
-// (r, s) = (tid / S, tid % S) solves substrate s of row r, a line of n points
-// S elements apart in shared memory, with the compressed coefficients of s (most
-// points need no coefficient load).  Row pitches are chosen so that the lanes of
-// a warp touch distinct banks.
-// ST = S when it is a compile-time constant (stride-S shared-memory accesses with
-// immediate offsets), 0 for the run-time path.  MC (the mass check on): lane
-// (r, s) also sums its lines' inputs (kMcIn) and, on a 1-D mesh, outputs (kMcOut)
-// over all its tiles, added once at the end.
-template <typename T, int ST, int MC>
-__global__ void __launch_bounds__(kLanes) sweep_x_sub_kernel(SweepArgs a)
-{
-	extern __shared__ __align__(128) unsigned char smem[];
-	uint64_t* bar = reinterpret_cast<uint64_t*>(smem);
-	uint32_t& ticket = *reinterpret_cast<uint32_t*>(smem + 8);
-	T* tile = reinterpret_cast<T*>(smem + 16);
-	const uint32_t tid = threadIdx.x;
-	const uint32_t R = a.rows_per_tile, S = ST ? (uint32_t)ST : a.S, n = a.n;
-	const uint32_t r_local = tid / S, s = tid % S;
-	const uint32_t row_bytes = (uint32_t)round_up(a.row_len * sizeof(T), 16);
-	const LineCoef<T> L = line_coef<T>(static_cast<const T*>(a.coef) + a.comp_off, S, a.head, n, s);
+	LineCoef<T> L = line_coef(static_cast<const T*>(a.tab), S, a.head, n, kWide ? min(s0, S - 1) : s0, half);
 	MassAcc<T> ai, ao;
 	ai.zero();
 	ao.zero();
-	if (tid == 0)
+	const uint32_t tiles = (uint32_t)a.tiles;
+	uint32_t t = blockIdx.x;
+	bool ok = true;
+	for (uint32_t phase = 0; t < tiles; phase ^= 1)
 	{
-		dev::mbar_init(bar, 1);
-		dev::fence_mbar_init();
-	}
-	__syncthreads();
-	for (uint32_t phase = 0;; phase ^= 1)
-	{
-		if (tid == 0)
-			ticket = atomicAdd(a.ticket, 1u);
-		__syncthreads();
-		const uint64_t t = ticket;
-		if (t >= a.tiles)
-			break;
-		const uint64_t r0 = t * R;
+		const uint64_t r0 = (uint64_t)t * R;
 		const uint32_t nrows = (uint32_t)(a.rows - r0 < (uint64_t)R ? a.rows - r0 : (uint64_t)R);
 		T* g = static_cast<T*>(a.field) + r0 * a.pitch;
-		if (tid == 0)
-			dev::mbar_arrive_expect_tx(bar, nrows * row_bytes);
-		__syncthreads();
-		if (tid < nrows)
-			dev::bulk_g2s(tile + tid * a.smem_pitch, g + tid * a.pitch, row_bytes, bar);
-		if (!__syncthreads_and(dev::mbar_wait(bar, phase)))
+		uint32_t drawn = 0;
+		if (half == 0)
 		{
-			if (tid == 0)
-				atomicOr(a.err, DEV_ERR_WAIT_TIMEOUT);
-			break;
+			if (lane == 0)
+				dev::mbar_arrive_expect_tx(bar, nrows * row_bytes);
+			__syncwarp();
+			if (lane < nrows)
+				dev::bulk_g2s(tile + lane * pitch, g + lane * a.pitch, row_bytes, bar);
+			if (lane == 0)
+				drawn = gridDim.x + atomicAdd(a.ticket, 1u);
 		}
-		if (r_local < nrows)
-			solve_line<T, ST, MC>(tile + r_local * a.smem_pitch + s, n, S, L, &ai, &ao);
+		ok = __syncthreads_and(dev::mbar_wait(bar, phase));
+		if (!ok)
+			break;
+		T* row = tile + r_local * pitch;
+		if constexpr (VEC)
+			solve_tile<T, RowLine, RowLine, MC, 0>({ row }, { row }, n, half, r_local < nrows, L, LineScale<T> {}, &ai, &ao);
+		else
+			for (uint32_t sb = 0; sb < (kWide ? S : 1u); sb += kLanes)
+			{
+				const uint32_t s = s0 + sb;
+				const bool on = r_local < nrows && (!kWide || s < S);
+				if (kWide && sb)
+					L = line_coef(static_cast<const T*>(a.tab), S, a.head, n, min(s, S - 1), half);
+				LineScale<T> F {};
+				if constexpr (SC != 0)
+				{
+					const T* sc = static_cast<const T*>(a.sc) + min(s, S - 1);
+					F = line_scale(T(1), __ldg(sc), sc + S, (int)S, n, half);
+				}
+				solve_tile<T, Strided<T, STRIDE, 1>, Strided<T, STRIDE, -1>, MC, SC>(
+					{ row + s, S }, { row + (n - 1) * S + s, S }, n, half, on, L, F, &ai, &ao);
+				if constexpr (MC != 0 && kWide)
+					if (on)
+					{
+						atomicAdd(a.mc_tot + s, ai.value());
+						if ((MC & kMcOut) != 0)
+							atomicAdd(a.mc_tot + S + s, ao.value());
+						ai.zero();
+						ao.zero();
+					}
+			}
+		if (kWide)
+			L = line_coef(static_cast<const T*>(a.tab), S, a.head, n, s0, half);
+		if (threadIdx.x == 0)
+			next = drawn;
 		dev::fence_proxy_async_smem();
 		__syncthreads();
-		if (tid < nrows)
-			dev::bulk_s2g(g + tid * a.pitch, tile + tid * a.smem_pitch, row_bytes);
-		dev::bulk_commit();
-		dev::bulk_wait_read();
-		__syncthreads();
+		t = next;
+		if (half == 0)
+		{
+			if (lane < nrows)
+				dev::bulk_s2g(g + lane * a.pitch, tile + lane * pitch, row_bytes);
+			dev::bulk_commit();
+			dev::bulk_wait_read();
+			__syncwarp();
+		}
 	}
-	if constexpr (MC != 0)
+	if constexpr (MC != 0 && !kWide)
 	{
-		// lanes r * S + s share substrate s (S <= 32 on this mapping)
-		flush_classes(ai.value(), S, kLanes, a.mc_tot + s);
+		// lanes r * S + s share substrate s
+		flush_classes(ai.value(), S, kLanes, a.mc_tot + s0);
 		if constexpr ((MC & kMcOut) != 0)
-			flush_classes(ao.value(), S, kLanes, a.mc_tot + S + s);
+			flush_classes(ao.value(), S, kLanes, a.mc_tot + S + s0);
 	}
-	dev::bulk_wait_all();
+	if (!ok && threadIdx.x == 0)
+		atomicOr(a.err, DEV_ERR_WAIT_TIMEOUT);
+	if (half == 0)
+		dev::bulk_wait_all();
 }
-
 // ------------------------------------------------------------------ fused x + y
 
 // The x and y sweeps of a 3-D mesh in one persistent launch, z-slab by z-slab.
@@ -373,7 +324,7 @@ __device__ __forceinline__ bool wait_at_least(const uint32_t* p, uint32_t target
 }
 
 template <typename T, int ST, int MC>
-__global__ void __launch_bounds__(kLanes)
+__global__ void __launch_bounds__(sweep_threads<T>())
 	sweep_xy_kernel(SweepArgs ax, SweepArgs ay, const __grid_constant__ CUtensorMap tmap, XYArgs f)
 {
 	extern __shared__ __align__(128) unsigned char smem[];
@@ -381,18 +332,16 @@ __global__ void __launch_bounds__(kLanes)
 	uint64_t* bar_y = reinterpret_cast<uint64_t*>(smem + 8);
 	uint32_t* s_ticket = reinterpret_cast<uint32_t*>(smem + 16);
 	T* buf = reinterpret_cast<T*>(smem + 128);
-	const uint32_t tid = threadIdx.x;
-	// x: lane (r, s) solves substrate s of row r of the tile
+	const uint32_t tid = threadIdx.x, lane = tid & 31, half = tid >> 5;
+	// x: lane (r, s) of either warp solves its half of substrate s of row r of the tile
 	const uint32_t S = ST ? (uint32_t)ST : ax.S, nx_pts = ax.n, R = ax.rows_per_tile;
-	const uint32_t r_local = tid / S, s = tid % S;
+	const uint32_t r_local = lane / S, s = lane % S;
 	const uint32_t row_bytes = (uint32_t)round_up(ax.row_len * sizeof(T), 16);
-	const LineCoef<T> Lx = line_coef<T>(static_cast<const T*>(ax.coef) + ax.comp_off, S, ax.head, nx_pts, s);
-	MassAcc<T> ai, ao;
+	const LineCoef<T> Lx = line_coef(static_cast<const T*>(ax.tab), S, ax.head, nx_pts, s, half);
+	MassAcc<T> ai;
 	ai.zero();
-	ao.zero();
 	// y
 	const uint32_t ny_pts = ay.n, Ry = ay.box_rows, nc = ay.boxes, chunk_elems = Ry * kLanes;
-	const T* ycomp = static_cast<const T*>(ay.coef) + ay.comp_off;
 	if (tid == 0)
 	{
 		dev::mbar_init(bar_x, 1);
@@ -407,8 +356,11 @@ __global__ void __launch_bounds__(kLanes)
 	auto signal = [&]() {
 		if (pending < 0)
 			return;
-		dev::bulk_wait_all();
-		fence_proxy_async_global();
+		if (half == 0)
+		{
+			dev::bulk_wait_all();
+			fence_proxy_async_global();
+		}
 		__syncthreads();
 		if (tid == 0)
 		{
@@ -446,11 +398,14 @@ __global__ void __launch_bounds__(kLanes)
 			const uint64_t r0 = slab_r0 + (uint64_t)u * R;
 			const uint32_t nrows = (uint32_t)min((uint64_t)R, slab_r1 - r0);
 			T* g = static_cast<T*>(ax.field) + r0 * ax.pitch;
-			if (tid == 0)
-				dev::mbar_arrive_expect_tx(bar_x, nrows * row_bytes);
-			__syncthreads();
-			if (tid < nrows)
-				dev::bulk_g2s(buf + tid * ax.smem_pitch, g + tid * ax.pitch, row_bytes, bar_x);
+			if (half == 0)
+			{
+				if (lane == 0)
+					dev::mbar_arrive_expect_tx(bar_x, nrows * row_bytes);
+				__syncwarp();
+				if (lane < nrows)
+					dev::bulk_g2s(buf + lane * ax.smem_pitch, g + lane * ax.pitch, row_bytes, bar_x);
+			}
 			signal(); // the previous x tile's stores had this long to complete
 			if (!__syncthreads_and(dev::mbar_wait(bar_x, phase_x)))
 			{
@@ -458,14 +413,18 @@ __global__ void __launch_bounds__(kLanes)
 				break;
 			}
 			phase_x ^= 1;
-			if (r_local < nrows)
-				solve_line<T, ST, MC>(buf + r_local * ax.smem_pitch + s, nx_pts, S, Lx, &ai, &ao);
+			T* row = buf + r_local * ax.smem_pitch + s;
+			solve_tile<T, Strided<T, ST, 1>, Strided<T, ST, -1>, MC, 0>(
+				{ row, S }, { row + (nx_pts - 1) * S, S }, nx_pts, half, r_local < nrows, Lx, LineScale<T> {}, &ai);
 			dev::fence_proxy_async_smem();
 			__syncthreads();
-			if (tid < nrows)
-				dev::bulk_s2g(g + tid * ax.pitch, buf + tid * ax.smem_pitch, row_bytes);
-			dev::bulk_commit();
-			dev::bulk_wait_read();
+			if (half == 0)
+			{
+				if (lane < nrows)
+					dev::bulk_s2g(g + lane * ax.pitch, buf + lane * ax.smem_pitch, row_bytes);
+				dev::bulk_commit();
+				dev::bulk_wait_read();
+			}
 			__syncthreads();
 			pending = (int)slab;
 		}
@@ -493,17 +452,18 @@ __global__ void __launch_bounds__(kLanes)
 				for (uint32_t c = 0; c < nc; c++)
 					dev::tma_load_3d(buf + c * chunk_elems, &tmap, x0, (int)(c * Ry), o, bar_y);
 			}
-			const uint32_t sy = (uint64_t)(x0 + tid) < ay.row_len ? (uint32_t)((x0 + tid) % ay.S) : 0;
-			const LineCoef<T> Ly = line_coef<T>(ycomp, ay.S, ay.head, ny_pts, sy);
-			if (!__all_sync(0xffffffffu, dev::mbar_wait(bar_y, phase_y)))
+			const uint32_t sy = (uint64_t)(x0 + lane) < ay.row_len ? (uint32_t)((x0 + lane) % ay.S) : 0;
+			const LineCoef<T> Ly = line_coef(static_cast<const T*>(ay.tab), ay.S, ay.head, ny_pts, sy, half);
+			if (!__syncthreads_and(dev::mbar_wait(bar_y, phase_y)))
 			{
 				ok = false;
 				break;
 			}
 			phase_y ^= 1;
-			solve_line<T, kLanes>(buf + tid, ny_pts, 0, Ly);
+			solve_tile<T, Strided<T, kLanes, 1>, Strided<T, kLanes, -1>, 0, 0>(
+				{ buf + lane, 0 }, { buf + (ny_pts - 1) * kLanes + lane, 0 }, ny_pts, half, true, Ly, LineScale<T> {});
 			dev::fence_proxy_async_smem();
-			__syncwarp();
+			__syncthreads();
 			if (tid == 0)
 			{
 				for (uint32_t c = 0; c < nc; c++)
@@ -519,68 +479,44 @@ __global__ void __launch_bounds__(kLanes)
 		atomicOr(ax.err, DEV_ERR_WAIT_TIMEOUT);
 	if constexpr (MC != 0)
 		flush_classes(ai.value(), S, kLanes, ax.mc_tot + s);
-	dev::bulk_wait_all();
+	if (half == 0)
+		dev::bulk_wait_all();
 }
 
 struct Plan
 {
 	uint64_t smem;
-	int threads;
 	uint64_t rows_per_tile;
+	uint64_t pitch; // x: shared-memory row pitch (elements)
 };
 
 template <typename T>
 Plan plan(const Context* c, int axis)
 {
 	Plan p {};
-	if (axis == 0 && x_substrate_mapping(c->S))
-	{
-		const uint64_t row_stage = sweep_x_sub_pitch(c->row_len, c->S, sizeof(T)) * sizeof(T);
-		// ~32 KB tiles: more CTAs (warps) per SM beat fuller warps here
-		uint64_t rows = std::min<uint64_t>(kXTileBytes / row_stage, kLanes / c->S);
-		rows = std::max<uint64_t>(rows, 1);
-		p.rows_per_tile = rows;
-		p.smem = 16 + rows * row_stage;
-		p.threads = kLanes; // lanes past rows * S idle
-		return p;
-	}
 	if (axis == 0)
 	{
-		const uint64_t row_stage = sweep_x_smem_pitch(c->row_len, c->S, sizeof(T)) * sizeof(T);
-		const uint64_t tpr = x_threads_per_row(c->S, sizeof(T));
-		// aim for >= 4 CTAs per SM so that every scheduler has a warp
-		uint64_t rows = (kMaxSmemBytes / 4) / row_stage;
-		const uint64_t cap = kLanes / tpr;
-		rows = rows < 1 ? 1 : (rows > cap ? cap : rows);
-		p.rows_per_tile = rows;
-		p.smem = 16 + rows * row_stage;
-		p.threads = (int)(rows * tpr);
+		p.pitch = sweep_x_pitch(c->row_len, c->S, sizeof(T));
+		p.rows_per_tile = x_tile_rows(c->row_len, c->S, sizeof(T), x_tile_budget(sizeof(T)));
+		p.smem = 16 + p.rows_per_tile * p.pitch * sizeof(T);
 		return p;
 	}
 	uint32_t box_rows, boxes;
 	box_geometry(c->n[axis], box_rows, boxes);
 	p.smem = 128 + (uint64_t)boxes * box_rows * kLanes * sizeof(T);
-	p.threads = kLanes;
 	return p;
 }
 
-template <typename KernelT>
-int launch_persistent(Context* c, KernelT kernel, const SweepArgs& a, const Plan& p, int kid, double bytes)
+// CTAs of a persistent sweep launch: every one the device holds at once, at most
+// one per tile.
+int persistent_grid(Context* c, const void* kernel, int threads, uint64_t smem, uint64_t tiles, uint64_t* grid)
 {
-	PCG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem));
+	PCG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
 	int per_sm = 0;
-	PCG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, p.threads, p.smem));
+	PCG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
 	if (per_sm < 1)
 		return fail(PCG_ERR_UNSUPPORTED, "sweep tile does not fit in shared memory");
-	uint64_t grid = (uint64_t)per_sm * (uint64_t)c->sm_count;
-	if (grid > a.tiles)
-		grid = a.tiles;
-	PCG_CUDA_TRY(cudaMemsetAsync(a.ticket, 0, sizeof(uint32_t), c->stream));
-	cudaEvent_t ev;
-	launch_begin(c, kid, bytes, &ev);
-	kernel<<<(unsigned)grid, p.threads, p.smem, c->stream>>>(a);
-	launch_end(c, kid, ev);
-	PCG_CUDA_TRY(cudaGetLastError());
+	*grid = std::min<uint64_t>((uint64_t)per_sm * (uint64_t)c->sm_count, tiles);
 	return PCG_OK;
 }
 
@@ -588,9 +524,8 @@ SweepArgs base_args(const Context* c, int axis)
 {
 	SweepArgs a {};
 	a.field = c->field.ptr;
-	a.coef = c->coef[axis].ptr;
-	a.coef_len = c->coef_len[axis];
-	a.coef_elems = c->coef_elems[axis];
+	a.tab = c->coef[axis].ptr;
+	a.head = c->coef_head[axis];
 	a.S = (uint32_t)c->S;
 	a.n = (uint32_t)c->n[axis];
 	a.row_len = c->row_len;
@@ -598,58 +533,82 @@ SweepArgs base_args(const Context* c, int axis)
 	a.rows = c->rows;
 	a.err = static_cast<uint32_t*>(c->err.ptr);
 	a.ticket = static_cast<uint32_t*>(c->tickets.ptr) + axis;
-	a.blo_off = c->coef_blo_off[axis];
+	a.nx = (uint32_t)c->n[0], a.ny = (uint32_t)c->n[1], a.nz = (uint32_t)c->n[2];
+	if (c->wsize == 8)
+		a.sc = c->scale_table(axis);
+	if (c->wsize == 8 && axis == c->dims - 1 && c->defer_scale)
+	{
+		// the last sweep applies the earlier axes' factors (their per-point tables
+		// follow the S converged ones)
+		if (axis > 0)
+			a.gx = c->scale_table(0) + c->S;
+		if (axis > 1)
+			a.gy = c->scale_table(1) + c->S;
+	}
 	return a;
 }
 
+using XKernel = void (*)(SweepArgs);
+
+// The x kernel: S at compile time up to 8, a vector kernel for one FP32 substrate.
 template <typename T, int MC>
-int dispatch_sweep_x(Context* c, const SweepArgs& a, const Plan& p, bool sub)
+XKernel x_kernel_by_s(uint64_t S)
 {
-	const double bytes = 2.0 * (double)(c->V * c->S) * (double)sizeof(T);
-	if (sub)
-		switch (c->S)
-		{
-		case 3: return launch_persistent(c, sweep_x_sub_kernel<T, 3, MC>, a, p, K_SWEEP_X, bytes);
-		case 4: return launch_persistent(c, sweep_x_sub_kernel<T, 4, MC>, a, p, K_SWEEP_X, bytes);
-		case 5: return launch_persistent(c, sweep_x_sub_kernel<T, 5, MC>, a, p, K_SWEEP_X, bytes);
-		case 6: return launch_persistent(c, sweep_x_sub_kernel<T, 6, MC>, a, p, K_SWEEP_X, bytes);
-		case 7: return launch_persistent(c, sweep_x_sub_kernel<T, 7, MC>, a, p, K_SWEEP_X, bytes);
-		case 8: return launch_persistent(c, sweep_x_sub_kernel<T, 8, MC>, a, p, K_SWEEP_X, bytes);
-		default: return launch_persistent(c, sweep_x_sub_kernel<T, 0, MC>, a, p, K_SWEEP_X, bytes);
-		}
-	switch (c->S)
+	switch (S)
 	{
-	case 1: return launch_persistent(c, sweep_x_kernel<T, 1, MC>, a, p, K_SWEEP_X, bytes);
-	case 2: return launch_persistent(c, sweep_x_kernel<T, 2, MC>, a, p, K_SWEEP_X, bytes);
-	case 3: return launch_persistent(c, sweep_x_kernel<T, 3, MC>, a, p, K_SWEEP_X, bytes);
-	case 4: return launch_persistent(c, sweep_x_kernel<T, 4, MC>, a, p, K_SWEEP_X, bytes);
-	case 5: return launch_persistent(c, sweep_x_kernel<T, 5, MC>, a, p, K_SWEEP_X, bytes);
-	case 6: return launch_persistent(c, sweep_x_kernel<T, 6, MC>, a, p, K_SWEEP_X, bytes);
-	case 7: return launch_persistent(c, sweep_x_kernel<T, 7, MC>, a, p, K_SWEEP_X, bytes);
-	case 8: return launch_persistent(c, sweep_x_kernel<T, 8, MC>, a, p, K_SWEEP_X, bytes);
-	default: return launch_persistent(c, sweep_x_kernel<T, 0, MC>, a, p, K_SWEEP_X, bytes);
+	case 1: return sweep_x_kernel<T, 1, MC, 0, sizeof(T) == 4>;
+	case 2: return sweep_x_kernel<T, 2, MC, 0, false>;
+	case 3: return sweep_x_kernel<T, 3, MC, 0, false>;
+	case 4: return sweep_x_kernel<T, 4, MC, 0, false>;
+	case 5: return sweep_x_kernel<T, 5, MC, 0, false>;
+	case 6: return sweep_x_kernel<T, 6, MC, 0, false>;
+	case 7: return sweep_x_kernel<T, 7, MC, 0, false>;
+	case 8: return sweep_x_kernel<T, 8, MC, 0, false>;
+	default: return S <= kLanes ? sweep_x_kernel<T, 0, MC, 0, false> : sweep_x_kernel<T, -1, MC, 0, false>;
 	}
+}
+
+// On a 1-D mesh x is also the last sweep: it sums its outputs as well, and an FP64
+// sweep that applies its factors itself (1-D, or factors not deferred) takes the
+// run-time kernel.
+template <typename T>
+XKernel x_kernel(const Context* c, bool mass_check)
+{
+	constexpr int SC = sizeof(T) == 8;
+	const bool wide = c->S > kLanes;
+	if (c->dims == 1 && mass_check)
+		return wide ? sweep_x_kernel<T, -1, kMcIn | kMcOut, SC, false> : sweep_x_kernel<T, 0, kMcIn | kMcOut, SC, false>;
+	if (SC && !c->defer_scale && mass_check)
+		return wide ? sweep_x_kernel<T, -1, kMcIn, SC, false> : sweep_x_kernel<T, 0, kMcIn, SC, false>;
+	if (c->dims == 1 || (SC && !c->defer_scale))
+		return wide ? sweep_x_kernel<T, -1, 0, SC, false> : sweep_x_kernel<T, 0, 0, SC, false>;
+	return mass_check ? x_kernel_by_s<T, kMcIn>(c->S) : x_kernel_by_s<T, 0>(c->S);
 }
 
 template <typename T>
 int run_sweep_x(Context* c, bool mass_check)
 {
 	SweepArgs a = base_args(c, 0);
-	const bool sub = x_substrate_mapping(c->S);
-	a.smem_pitch = sub ? sweep_x_sub_pitch(c->row_len, c->S, sizeof(T)) : sweep_x_smem_pitch(c->row_len, c->S, sizeof(T));
-	a.comp_off = c->coef_comp_off[0];
-	a.head = c->coef_head[0];
 	const Plan p = plan<T>(c, 0);
 	if (p.smem > kMaxSmemBytes)
 		return fail(PCG_ERR_UNSUPPORTED, "x rows too long for the shared-memory x sweep");
+	a.smem_pitch = p.pitch;
 	a.rows_per_tile = (uint32_t)p.rows_per_tile;
 	a.tiles = (c->rows + p.rows_per_tile - 1) / p.rows_per_tile;
-	if (!mass_check)
-		return dispatch_sweep_x<T, 0>(c, a, p, sub);
-	a.mc_tot = static_cast<double*>(c->mc_tot.ptr);
-	a.mc_x_out = c->dims == 1 ? 1u : 0u;
-	// on a 1-D mesh x is also the last sweep: it sums its outputs as well
-	return c->dims == 1 ? dispatch_sweep_x<T, kMcIn | kMcOut>(c, a, p, sub) : dispatch_sweep_x<T, kMcIn>(c, a, p, sub);
+	if (mass_check)
+		a.mc_tot = static_cast<double*>(c->mc_tot.ptr);
+	const XKernel kernel = x_kernel<T>(c, mass_check);
+	uint64_t grid;
+	int rc;
+	if ((rc = persistent_grid(c, reinterpret_cast<const void*>(kernel), sweep_threads<T>(), p.smem, a.tiles, &grid)))
+		return rc;
+	PCG_CUDA_TRY(cudaMemsetAsync(a.ticket, 0, sizeof(uint32_t), c->stream));
+	cudaEvent_t ev;
+	launch_begin(c, K_SWEEP_X, 2.0 * (double)(c->V * c->S) * (double)sizeof(T), &ev);
+	kernel<<<(unsigned)grid, sweep_threads<T>(), p.smem, c->stream>>>(a);
+	launch_end(c, K_SWEEP_X, ev);
+	PCG_CUDA_TRY(cudaGetLastError());
+	return PCG_OK;
 }
 
 // The fused x + y launch (sweep_xy_kernel): slabs of about c->xy_slab_bytes of
@@ -660,10 +619,8 @@ template <typename T>
 int run_sweep_xy(Context* c, bool mass_check)
 {
 	SweepArgs ax = base_args(c, 0);
-	ax.smem_pitch = sweep_x_sub_pitch(c->row_len, c->S, sizeof(T));
-	ax.comp_off = c->coef_comp_off[0];
-	ax.head = c->coef_head[0];
 	const Plan px = plan<T>(c, 0);
+	ax.smem_pitch = px.pitch;
 	ax.rows_per_tile = (uint32_t)px.rows_per_tile;
 	if (mass_check)
 		ax.mc_tot = static_cast<double*>(c->mc_tot.ptr);
@@ -671,8 +628,6 @@ int run_sweep_xy(Context* c, bool mass_check)
 	ay.xblocks = (c->row_len + kLanes - 1) / kLanes;
 	ay.box_rows = c->tmap_box_rows[1];
 	ay.boxes = c->tmap_boxes[1];
-	ay.comp_off = c->coef_comp_off[1];
-	ay.head = c->coef_head[1];
 	const Plan py = plan<T>(c, 1);
 	const uint64_t R = px.rows_per_tile, ny = c->n[1], nz = c->n[2];
 	const uint64_t plane_bytes = ny * c->pitch * sizeof(T);
@@ -695,12 +650,10 @@ int run_sweep_xy(Context* c, bool mass_check)
 		default: return mc ? sweep_xy_kernel<T, 0, kMcIn> : sweep_xy_kernel<T, 0, 0>;
 		}
 	}();
-	PCG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-	int per_sm = 0;
-	PCG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kLanes, smem));
-	if (per_sm < 1)
-		return fail(PCG_ERR_UNSUPPORTED, "fused x/y tile does not fit in shared memory");
-	const uint64_t resident = (uint64_t)per_sm * (uint64_t)c->sm_count;
+	uint64_t resident;
+	int rc;
+	if ((rc = persistent_grid(c, reinterpret_cast<const void*>(kernel), sweep_threads<T>(), smem, ~0ull, &resident)))
+		return rc;
 	// the lag must exceed the tiles in flight (about one per resident CTA), else y
 	// tiles are handed out while their slab's x tiles are still being solved
 	const uint64_t slab_tiles = (P * ny + R - 1) / R + P * ay.xblocks;
@@ -731,7 +684,6 @@ int run_sweep_xy(Context* c, bool mass_check)
 		}
 		if (first >= 0xffffffffull)
 			return fail(PCG_ERR_UNSUPPORTED, "too many tiles for the fused x/y sweep");
-		int rc;
 		if ((rc = dalloc(c, c->xy_segs, segs.size() * sizeof(uint4))) ||
 			(rc = dalloc(c, c->xy_done, nslab * sizeof(uint32_t))))
 			return rc;
@@ -759,10 +711,20 @@ int run_sweep_xy(Context* c, bool mass_check)
 	const double bytes = 2.0 * (double)(c->V * c->S) * (double)sizeof(T);
 	cudaEvent_t ev;
 	launch_begin(c, K_SWEEP_XY, bytes, &ev);
-	kernel<<<(unsigned)grid, kLanes, smem, c->stream>>>(ax, ay, c->tmap[1], f);
+	kernel<<<(unsigned)grid, sweep_threads<T>(), smem, c->stream>>>(ax, ay, c->tmap[1], f);
 	launch_end(c, K_SWEEP_XY, ev);
 	PCG_CUDA_TRY(cudaGetLastError());
 	return PCG_OK;
+}
+
+// FP64: `scale` when the sweep applies the scale factors (the last one always does).
+template <typename T, int AXIS>
+auto yz_kernel(bool scale, bool mass_check) -> void (*)(SweepArgs, const CUtensorMap)
+{
+	constexpr int SC = sizeof(T) == 8;
+	if (mass_check)
+		return sweep_yz_kernel<T, AXIS, kMcOut, SC>;
+	return scale ? sweep_yz_kernel<T, AXIS, 0, SC> : sweep_yz_kernel<T, AXIS, 0, 0>;
 }
 
 template <typename T>
@@ -777,26 +739,11 @@ int run_sweep_yz(Context* c, int axis, bool fuse_faces, bool mass_check)
 		a.face_values = f.values;
 		a.face_conds = f.conds;
 		a.face_mask = f.face_mask;
-		a.nx = c->n[0], a.ny = c->n[1], a.nz = c->n[2];
-	}
-	if (axis == 1)
-	{
-		a.line_stride = c->pitch;
-		a.outer_stride = c->n[1] * c->pitch;
-		a.tiles = c->n[2];
-	}
-	else
-	{
-		a.line_stride = c->n[1] * c->pitch;
-		a.outer_stride = c->pitch;
-		a.tiles = c->n[1];
 	}
 	a.xblocks = (c->row_len + kLanes - 1) / kLanes;
-	a.tiles *= a.xblocks;
+	a.tiles = a.xblocks * (axis == 1 ? c->n[2] : c->n[1]);
 	a.box_rows = c->tmap_box_rows[axis];
 	a.boxes = c->tmap_boxes[axis];
-	a.comp_off = c->coef_comp_off[axis];
-	a.head = c->coef_head[axis];
 	const Plan p = plan<T>(c, axis);
 	if (p.smem > kMaxSmemBytes)
 		return fail(PCG_ERR_UNSUPPORTED, "lines too long for the shared-memory y/z sweep");
@@ -804,20 +751,16 @@ int run_sweep_yz(Context* c, int axis, bool fuse_faces, bool mass_check)
 		return fail(PCG_ERR_INVALID, "tensor maps of the field were not prepared");
 	const int kid = axis == 1 ? K_SWEEP_Y : K_SWEEP_Z;
 	const double bytes = 2.0 * (double)(c->V * c->S) * (double)sizeof(T);
-	auto kernel = mass_check ? (axis == 1 ? sweep_yz_kernel<T, 1, kMcOut> : sweep_yz_kernel<T, 2, kMcOut>)
-							 : (axis == 1 ? sweep_yz_kernel<T, 1, 0> : sweep_yz_kernel<T, 2, 0>);
-	PCG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem));
-	int per_sm = 0;
-	PCG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, p.threads, p.smem));
-	if (per_sm < 1)
-		return fail(PCG_ERR_UNSUPPORTED, "sweep tile does not fit in shared memory");
-	uint64_t grid = (uint64_t)per_sm * (uint64_t)c->sm_count;
-	if (grid > a.tiles)
-		grid = a.tiles;
+	const bool scale = axis == c->dims - 1 || !c->defer_scale;
+	auto kernel = axis == 1 ? yz_kernel<T, 1>(scale, mass_check) : yz_kernel<T, 2>(scale, mass_check);
+	uint64_t grid;
+	int rc;
+	if ((rc = persistent_grid(c, reinterpret_cast<const void*>(kernel), sweep_threads<T>(), p.smem, a.tiles, &grid)))
+		return rc;
 	PCG_CUDA_TRY(cudaMemsetAsync(a.ticket, 0, sizeof(uint32_t), c->stream));
 	cudaEvent_t ev;
 	launch_begin(c, kid, bytes, &ev);
-	kernel<<<(unsigned)grid, p.threads, p.smem, c->stream>>>(a, c->tmap[axis]);
+	kernel<<<(unsigned)grid, sweep_threads<T>(), p.smem, c->stream>>>(a, c->tmap[axis]);
 	launch_end(c, kid, ev);
 	PCG_CUDA_TRY(cudaGetLastError());
 	return PCG_OK;
@@ -856,46 +799,30 @@ void box_geometry(uint64_t n, uint32_t& box_rows, uint32_t& boxes)
 	box_rows = (uint32_t)round_up((n + nc - 1) / nc, 8);
 }
 
-uint64_t coef_table_len(uint64_t n, uint64_t S, size_t wsize)
-{
-	const int vn = (int)(16 / wsize);
-	return round_up(n * S, (uint64_t)group_elems((int)S, vn));
-}
-
-uint64_t coef_row_pitch(uint64_t n) { return round_up(n, kBlock); }
-
-uint64_t x_threads_per_row(uint64_t S, size_t wsize)
-{
-	return (S <= 8 && (S * wsize) % 16 == 0) ? S * wsize / 16 : 1;
-}
-
 bool x_substrate_mapping(uint64_t S) { return S >= 3 && S <= kLanes; }
 
-// Shared-memory row pitch (elements) of the substrate-per-thread x mapping: whole
-// 16-byte chunks, and rows S elements (rounded up to a chunk) apart modulo the 32
-// banks, so that lane (r, s) of a warp reads bank r*S + s (mod 32) for FP32.
-uint64_t sweep_x_sub_pitch(uint64_t row_len, uint64_t S, size_t wsize)
+// Shared-memory row pitch (elements) of an x tile: whole 16-byte chunks, and rows
+// S elements (rounded up to a chunk) apart modulo the 32 banks, so that lane (r, s)
+// of a warp reads bank r*S + s (mod 32) for FP32 (two lanes of a bank for S = 2);
+// one FP32 substrate alone moves in 16-byte chunks, whose rows lie an odd number of
+// chunks apart.  A row that only fits without the padding goes without it.
+uint64_t sweep_x_pitch(uint64_t row_len, uint64_t S, size_t wsize)
 {
 	const uint64_t vn = 16 / wsize;
 	const uint64_t mod = 128 / wsize; // elements spanning the 32 banks
 	const uint64_t want = round_up(S, vn) % mod;
 	uint64_t p = round_up(row_len, vn);
-	while (p % mod != want)
+	while (S <= kLanes && p % mod != want)
 		p += vn;
-	return p;
+	return 16 + p * wsize <= kMaxSmemBytes ? p : round_up(row_len, vn);
 }
 
-uint64_t sweep_x_smem_pitch(uint64_t row_len, uint64_t S, size_t wsize)
+// Rows of an x tile: one per S lanes of a warp, while the tile stays within
+// `budget` bytes.
+uint64_t x_tile_rows(uint64_t row_len, uint64_t S, size_t wsize, uint64_t budget)
 {
-	const uint64_t vn = 16 / wsize;
-	const uint64_t ge = (uint64_t)group_elems((int)S, (int)vn);
-	const uint64_t tpr = x_threads_per_row(S, wsize);
-	uint64_t chunks = round_up(row_len, ge) / vn;
-	// rows tpr (mod 8) chunks apart: the 8 lanes of a quarter-warp (8/tpr rows x tpr
-	// chunk slots) read 8 distinct 16-byte bank groups
-	const uint64_t want = tpr % 8;
-	chunks += (want + 8 - chunks % 8) % 8;
-	return chunks * vn;
+	const uint64_t row_stage = sweep_x_pitch(row_len, S, wsize) * wsize;
+	return std::max<uint64_t>(1, std::min<uint64_t>(budget / row_stage, kLanes / S));
 }
 
 int encode_field_map(const Context* c, int axis, uint32_t box_rows, CUtensorMap* out, uint32_t box_cols)
@@ -941,7 +868,10 @@ int launch_sweep_x(Context* c, bool mass_check)
 	return c->wsize == 4 ? run_sweep_x<float>(c, mass_check) : run_sweep_x<double>(c, mass_check);
 }
 
-bool xy_fusable(const Context* c) { return c->fuse_xy && c->dims == 3 && x_substrate_mapping(c->S) && c->n[2] > 1; }
+bool xy_fusable(const Context* c)
+{
+	return c->fuse_xy && c->dims == 3 && x_substrate_mapping(c->S) && c->n[2] > 1 && (c->wsize == 4 || c->defer_scale);
+}
 
 int launch_sweep_xy(Context* c, bool mass_check)
 {

@@ -545,15 +545,16 @@ __global__ void batch_bulk_kernel(BatchArgs b)
 			continue;
 		const BatchDomain& D = b.doms[__ldg(b.list.dom + k)];
 		const uint64_t r = u - __ldg(b.list.base + k);
+		T* field = static_cast<T*>(D.field);
 		const T* sp = static_cast<const T*>(D.bulk[0]);
 		const T* up = static_cast<const T*>(D.bulk[1]);
 		const T* tp = static_cast<const T*>(D.bulk[2]);
-		if (D.bulk_mode == PCG_BULK_PER_VOXEL)
-			fielddev::bulk_row<T, true>(static_cast<T*>(D.field), sp, up, tp, D.row_len, D.pitch, r, D.S, (T)D.dt,
-										lane);
-		else
-			fielddev::bulk_row<T, false>(static_cast<T*>(D.field), sp, up, tp, D.row_len, D.pitch, r, D.S, (T)D.dt,
-										 lane);
+		const uint32_t row_len = (uint32_t)D.row_len, row_chunks = (uint32_t)(round_up(row_len * sizeof(T), 16) / 16);
+		for (uint32_t c = lane; c < row_chunks; c += 32)
+			if (D.bulk_mode == PCG_BULK_PER_VOXEL)
+				fielddev::bulk_chunk<T, true>(field, sp, up, tp, row_len, D.pitch, r, c, D.S, (T)D.dt);
+			else
+				fielddev::bulk_chunk<T, false>(field, sp, up, tp, row_len, D.pitch, r, c, D.S, (T)D.dt);
 	}
 }
 

@@ -101,45 +101,66 @@ __device__ __forceinline__ void face_item(const FaceArgs& a, uint64_t idx)
 	}
 }
 
-// One row of the bulk update by the 32 lanes of a warp; a lane walks the row's
-// (x,s) run with its substrate index advanced incrementally.
-template <typename T, bool PER_VOXEL>
-__device__ __forceinline__ void bulk_row(T* field, const T* supply, const T* uptake, const T* target,
-										 uint64_t row_len, uint64_t pitch, uint64_t r, uint32_t S, T dt, int lane)
+// The bulk update of one voxel-substrate (bulk_solver.cpp:12-49): D' = (D + dt S T) /
+// (1 + dt (U + S)); FP32 as D + (dt S T - D dt (U + S)) / (1 + dt (U + S)), so that a
+// small dt (U + S) keeps its precision (its sum with 1 only scales the correction).
+template <typename T>
+__device__ __forceinline__ T bulk_value(T D, T Sr, T U, T Tt, T dt)
 {
-	const uint32_t s_step = 32 % S;
-	T* row = field + r * pitch;
-	uint32_t s = (uint32_t)lane % S;
-	for (uint64_t k = lane; k < row_len; k += 32)
+	if constexpr (sizeof(T) == 4)
 	{
-		T Sr, U, Tt;
-		if (PER_VOXEL)
-		{
-			const uint64_t o = r * pitch + k;
-			Sr = supply[o];
-			U = uptake[o];
-			Tt = target[o];
-		}
-		else
-		{
-			Sr = supply[s];
-			U = uptake[s];
-			Tt = target[s];
-		}
-		// bulk_solver.cpp:12-49: D' = (D + dt S T) / (1 + dt (U + S)); FP32 as
-		// D + (dt S T - D dt (U + S)) / (1 + dt (U + S)), so that a small dt (U + S)
-		// keeps its precision (its sum with 1 only scales the correction)
-		if constexpr (sizeof(T) == 4)
-		{
-			const T a = dt * Sr * Tt, b = dt * (U + Sr);
-			row[k] = row[k] + fmaf(-row[k], b, a) / (T(1) + b);
-		}
-		else
-			row[k] = (row[k] + dt * Sr * Tt) / (T(1) + dt * (U + Sr));
-		s += s_step;
-		if (s >= S)
-			s -= S;
+		const T a = dt * Sr * Tt, b = dt * (U + Sr);
+		return D + fmaf(-D, b, a) / (T(1) + b);
 	}
+	else
+		return (D + dt * Sr * Tt) / (T(1) + dt * (U + Sr));
+}
+
+// The 16-byte chunk c of row r (fields and per-voxel tables have the same layout, and
+// rows start on 32-byte boundaries; the row's last chunk may hold fewer of its
+// elements).  Memory sets the pace only with whole chunks in flight per thread: one
+// element per thread and turn, a warp walking a row, ran at 0.5 TB/s.
+template <typename T, bool PER_VOXEL>
+__device__ __forceinline__ void bulk_chunk(T* field, const T* supply, const T* uptake, const T* target, uint32_t row_len,
+										   uint64_t pitch, uint64_t r, uint32_t c, uint32_t S, T dt)
+{
+	constexpr uint32_t VN = 16 / sizeof(T);
+	union Chunk
+	{
+		uint4 u;
+		T t[VN];
+	};
+	const uint64_t off = r * pitch + (uint64_t)c * VN;
+	const uint32_t left = row_len - c * VN;
+	Chunk d, sp, up, tp;
+	d.u = *reinterpret_cast<const uint4*>(field + off);
+	if constexpr (PER_VOXEL)
+	{
+		sp.u = __ldg(reinterpret_cast<const uint4*>(supply + off));
+		up.u = __ldg(reinterpret_cast<const uint4*>(uptake + off));
+		tp.u = __ldg(reinterpret_cast<const uint4*>(target + off));
+	}
+	else
+	{
+		uint32_t s = c * VN % S;
+#pragma unroll
+		for (uint32_t q = 0; q < VN; q++)
+		{
+			sp.t[q] = __ldg(supply + s);
+			up.t[q] = __ldg(uptake + s);
+			tp.t[q] = __ldg(target + s);
+			if (++s == S)
+				s = 0;
+		}
+	}
+#pragma unroll
+	for (uint32_t q = 0; q < VN; q++)
+		d.t[q] = bulk_value(d.t[q], sp.t[q], up.t[q], tp.t[q], dt);
+	if (left >= VN)
+		*reinterpret_cast<uint4*>(field + off) = d.u;
+	else // the padding after the row keeps its zeros
+		for (uint32_t q = 0; q < left; q++)
+			field[off + q] = d.t[q];
 }
 
 // The boundary faces of the voxels of one half of a solved y/z column in shared

@@ -29,16 +29,18 @@ __global__ void dirichlet_interior_kernel(T* field, const uint64_t* offsets, con
 	}
 }
 
-// A warp per row.
+// A thread per 16-byte chunk (chunks of a row side by side, so few long rows fill the
+// device as well as many short ones): 97x131x61 x 5, uniform rates, 65.7 -> 9.3 us (cold);
+// 1000x800 x 3, per voxel, 92.4 -> 8.5 us.
 template <typename T, bool PER_VOXEL>
-__global__ void bulk_kernel(T* field, const T* supply, const T* uptake, const T* target, uint64_t row_len,
-							uint64_t pitch, uint64_t rows, uint32_t S, T dt)
+__global__ void bulk_kernel(T* field, const T* supply, const T* uptake, const T* target, uint32_t row_len,
+							uint64_t pitch, uint32_t chunks, uint32_t row_chunks, uint32_t S, T dt)
 {
-	const int lane = threadIdx.x & 31;
-	const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-	const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-	for (uint64_t r = warp; r < rows; r += nwarps)
-		fielddev::bulk_row<T, PER_VOXEL>(field, supply, uptake, target, row_len, pitch, r, S, dt, lane);
+	const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; // fewer than 2^32 field elements, so chunks too
+	if (k >= chunks)
+		return;
+	const uint32_t r = k / row_chunks, c = k % row_chunks;
+	fielddev::bulk_chunk<T, PER_VOXEL>(field, supply, uptake, target, row_len, pitch, r, c, S, dt);
 }
 
 // FP64 mass per substrate: a warp per row, one substrate at a time.
@@ -191,19 +193,16 @@ static int run_bulk(Context* c)
 	if (c->bulk_mode == PCG_BULK_NONE)
 		return PCG_OK;
 	const bool pv = c->bulk_mode == PCG_BULK_PER_VOXEL;
-	const unsigned grid = grid_for(c, c->rows * 32, 256);
+	const uint64_t row_chunks = round_up(c->row_len * sizeof(T), 16) / 16, chunks = c->rows * row_chunks;
+	const unsigned grid = (unsigned)((chunks + 255) / 256);
 	cudaEvent_t ev;
 	const double bytes = (double)(c->V * c->S * sizeof(T)) * (pv ? 5.0 : 2.0);
 	launch_begin(c, K_BULK, bytes, &ev);
-	const T* sp = static_cast<const T*>(c->bulk[0].ptr);
-	const T* up = static_cast<const T*>(c->bulk[1].ptr);
-	const T* tp = static_cast<const T*>(c->bulk[2].ptr);
-	if (pv)
-		bulk_kernel<T, true><<<grid, 256, 0, c->stream>>>(static_cast<T*>(c->field.ptr), sp, up, tp, c->row_len,
-														  c->pitch, c->rows, (uint32_t)c->S, (T)c->dt);
-	else
-		bulk_kernel<T, false><<<grid, 256, 0, c->stream>>>(static_cast<T*>(c->field.ptr), sp, up, tp, c->row_len,
-														   c->pitch, c->rows, (uint32_t)c->S, (T)c->dt);
+	auto kernel = pv ? bulk_kernel<T, true> : bulk_kernel<T, false>;
+	kernel<<<grid, 256, 0, c->stream>>>(static_cast<T*>(c->field.ptr), static_cast<const T*>(c->bulk[0].ptr),
+										static_cast<const T*>(c->bulk[1].ptr), static_cast<const T*>(c->bulk[2].ptr),
+										(uint32_t)c->row_len, c->pitch, (uint32_t)chunks, (uint32_t)row_chunks,
+										(uint32_t)c->S, (T)c->dt);
 	launch_end(c, K_BULK, ev);
 	PCG_CUDA_TRY(cudaGetLastError());
 	return PCG_OK;

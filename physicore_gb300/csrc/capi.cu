@@ -214,6 +214,20 @@ void dfree(DeviceBuffer& b)
 	b.carved = false;
 }
 
+static std::mutex g_smem_mu;
+static std::map<std::pair<const void*, int>, bool> g_smem_allowed;
+
+int allow_smem(const void* kernel, int device)
+{
+	std::lock_guard<std::mutex> lk(g_smem_mu);
+	bool& done = g_smem_allowed[{ kernel, device }];
+	if (done)
+		return PCG_OK;
+	PCG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmemBytes));
+	done = true;
+	return PCG_OK;
+}
+
 static cudaEvent_t get_event(Context* c)
 {
 	if (!c->event_pool.empty())
@@ -740,7 +754,7 @@ int ensure_device_state(Context* c, bool defer_clear = false)
 		if (!rc)
 			rc = dalloc(c, c->flags, sizeof(uint32_t) * 8);
 		if (!rc)
-			rc = dalloc(c, c->tickets, sizeof(uint32_t) * 4);
+			rc = dalloc(c, c->tickets, sizeof(uint32_t) * 8);
 		if (rc)
 			return rc;
 		c->words_cleared = false;
@@ -749,6 +763,7 @@ int ensure_device_state(Context* c, bool defer_clear = false)
 	{
 		PCG_CUDA_TRY(cudaMemsetAsync(c->err.ptr, 0, sizeof(uint32_t) * 4, c->stream));
 		PCG_CUDA_TRY(cudaMemsetAsync(c->flags.ptr, 0, sizeof(uint32_t) * 8, c->stream));
+		PCG_CUDA_TRY(cudaMemsetAsync(c->tickets.ptr, 0, sizeof(uint32_t) * 8, c->stream));
 		c->words_cleared = true;
 	}
 	return PCG_OK;

@@ -43,6 +43,7 @@ using namespace cellsdev;
 template <typename T>
 __global__ void cells_place_kernel(CellArgs a)
 {
+	dev::pdl_wait();
 	const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
 	if (i == 0)
 	{
@@ -77,6 +78,7 @@ constexpr unsigned kClassifyChunks = 4; // 32-agent chunks per warp
 template <typename T>
 __global__ void __launch_bounds__(kClassifyBlock, 2) cells_classify_kernel(CellArgs a)
 {
+	dev::pdl_wait();
 	constexpr int K = kClassifyChunks;
 	__shared__ uint32_t part[3][kClassifyBlock / 32];
 	__shared__ uint32_t base[3];
@@ -196,6 +198,7 @@ __global__ void __launch_bounds__(kClassifyBlock, 2) cells_classify_kernel(CellA
 // flight hide.
 __global__ void cells_group_kernel(CellArgs a)
 {
+	dev::pdl_wait();
 	const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
 	if (i >= a.A)
 		return;
@@ -216,6 +219,7 @@ __global__ void cells_group_kernel(CellArgs a)
 template <typename T, int SC>
 __global__ void cells_group_sum_kernel(CellArgs a)
 {
+	dev::pdl_wait();
 	const uint32_t count = __ldg(a.flags + a.list_word);
 	const uint32_t lane = threadIdx.x & 31;
 	const uint64_t gw = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
@@ -316,6 +320,7 @@ __global__ void cells_group_sum_kernel(CellArgs a)
 template <typename T>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 1) cells_apply_kernel(CellArgs a)
 {
+	dev::pdl_wait();
 	const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
 	if (i < a.A)
 		agent_apply<T>(a, i);
@@ -330,6 +335,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 1) cells_apply_kerne
 template <typename T, int SC>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 1) cells_apply_writers_kernel(CellArgs a)
 {
+	dev::pdl_wait();
 	const uint32_t count = __ldg(a.flags + 4);
 	const bool list = 2ull * count < a.A;
 	const uint64_t n = list ? count : a.A;
@@ -341,25 +347,20 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 1) cells_apply_write
 template <typename T, int SC>
 __global__ void cells_internalize_kernel(CellArgs a)
 {
+	dev::pdl_wait();
 	const uint32_t count = __ldg(a.flags + a.list_word);
 	for (uint64_t j = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; j < count; j += (uint64_t)gridDim.x * blockDim.x)
 		agent_internalize<T, SC>(a, __ldg(a.shared + j));
 }
 
-// Launches KERNEL<T, S> for S = 1..8, KERNEL<T, 0> otherwise.
+// launch_chained of KERNEL<T, S> for S = 1..8, KERNEL<T, 0> otherwise.
 #define PCG_LAUNCH_BY_S(KERNEL, T, S, GRID, BLOCK, STREAM, ARGS)                                                       \
-	switch (S)                                                                                                         \
+	do                                                                                                                 \
 	{                                                                                                                  \
-	case 1: KERNEL<T, 1><<<GRID, BLOCK, 0, STREAM>>>(ARGS); break;                                                   \
-	case 2: KERNEL<T, 2><<<GRID, BLOCK, 0, STREAM>>>(ARGS); break;                                                   \
-	case 3: KERNEL<T, 3><<<GRID, BLOCK, 0, STREAM>>>(ARGS); break;                                                   \
-	case 4: KERNEL<T, 4><<<GRID, BLOCK, 0, STREAM>>>(ARGS); break;                                                   \
-	case 5: KERNEL<T, 5><<<GRID, BLOCK, 0, STREAM>>>(ARGS); break;                                                   \
-	case 6: KERNEL<T, 6><<<GRID, BLOCK, 0, STREAM>>>(ARGS); break;                                                   \
-	case 7: KERNEL<T, 7><<<GRID, BLOCK, 0, STREAM>>>(ARGS); break;                                                   \
-	case 8: KERNEL<T, 8><<<GRID, BLOCK, 0, STREAM>>>(ARGS); break;                                                   \
-	default: KERNEL<T, 0><<<GRID, BLOCK, 0, STREAM>>>(ARGS);                                                         \
-	}
+		void (*by_s__[9])(CellArgs) = { KERNEL<T, 0>, KERNEL<T, 1>, KERNEL<T, 2>, KERNEL<T, 3>, KERNEL<T, 4>,          \
+										KERNEL<T, 5>, KERNEL<T, 6>, KERNEL<T, 7>, KERNEL<T, 8> };                      \
+		PCG_CUDA_TRY(launch_chained(by_s__[(S) <= 8 ? (S) : 0], GRID, BLOCK, 0, STREAM, ARGS));                        \
+	} while (0)
 
 // release_internal (cell_solver.cpp:274-289) for one agent
 template <typename T>
@@ -457,13 +458,13 @@ static int run_ballot(Context* c, const CellArgs& a, cudaStream_t stream, int sm
 	if (c)
 		launch_begin(c, K_CELLS_LOCATE,
 					 A * (8.0 * a.dims + 1 + 4 + 4 + 4 + 4) + (a.terms ? A * (5 * S * 8 + 8 + 3 * S * w) : 0), &ev);
-	cells_place_kernel<T><<<grid, block, 0, stream>>>(a);
+	PCG_CUDA_TRY(launch_chained(cells_place_kernel<T>, grid, block, 0, stream, a));
 	if (c)
 		launch_end(c, K_CELLS_LOCATE, ev);
 	PCG_CUDA_TRY(cudaGetLastError());
 	if (c)
 		launch_begin(c, K_CELLS_BALLOT, A * (4 + 4 + 4 + 1), &ev);
-	cells_classify_kernel<T><<<cgrid, kClassifyBlock, 0, stream>>>(a);
+	PCG_CUDA_TRY(launch_chained(cells_classify_kernel<T>, cgrid, kClassifyBlock, 0, stream, a));
 	if (c && c->timing && c->h_words) // list lengths for the per-agent byte counts
 	{
 		PCG_CUDA_TRY(
@@ -478,7 +479,7 @@ static int run_ballot(Context* c, const CellArgs& a, cudaStream_t stream, int sm
 	// slot, and the pair written
 	if (c)
 		launch_begin(c, K_CELLS_GROUP, A, &ev);
-	cells_group_kernel<<<grid, block, 0, stream>>>(a);
+	PCG_CUDA_TRY(launch_chained(cells_group_kernel, grid, block, 0, stream, a));
 	if (c)
 		launch_end(c, K_CELLS_GROUP, ev, 20.0);
 	PCG_CUDA_TRY(cudaGetLastError());
@@ -486,24 +487,7 @@ static int run_ballot(Context* c, const CellArgs& a, cudaStream_t stream, int sm
 	// context)
 	if (c)
 		launch_begin(c, K_CELLS_REDUCE, 0.0, &ev);
-	switch (a.S)
-	{
-#define PCG_GROUP_SUM(SV)                                                                                              \
-	case SV:                                                                                                           \
-		cells_group_sum_kernel<T, SV><<<lgrid, block, 0, stream>>>(a);                                                 \
-		break;
-		PCG_GROUP_SUM(1)
-		PCG_GROUP_SUM(2)
-		PCG_GROUP_SUM(3)
-		PCG_GROUP_SUM(4)
-		PCG_GROUP_SUM(5)
-		PCG_GROUP_SUM(6)
-		PCG_GROUP_SUM(7)
-		PCG_GROUP_SUM(8)
-#undef PCG_GROUP_SUM
-	default:
-		cells_group_sum_kernel<T, 0><<<lgrid, block, 0, stream>>>(a);
-	}
+	PCG_LAUNCH_BY_S(cells_group_sum_kernel, T, a.S, lgrid, block, stream, a);
 	if (c)
 		launch_end(c, K_CELLS_REDUCE, ev, 8.0 + 3 * S * w);
 	PCG_CUDA_TRY(cudaGetLastError());
@@ -625,9 +609,9 @@ int launch_cells_fp32_buffers(const CellStepBuffers& b, cudaStream_t stream)
 	int rc = run_ballot<float>(nullptr, a, stream, sm_count);
 	if (rc)
 		return rc;
-	cells_apply_kernel<float><<<grid, block, 0, stream>>>(a);
+	PCG_CUDA_TRY(launch_chained(cells_apply_kernel<float>, grid, block, 0, stream, a));
 	if (b.internalized)
-		cells_internalize_kernel<float, 0><<<grid, block, 0, stream>>>(a);
+		PCG_CUDA_TRY(launch_chained(cells_internalize_kernel<float, 0>, grid, block, 0, stream, a));
 	PCG_CUDA_TRY(cudaGetLastError());
 	return PCG_OK;
 }

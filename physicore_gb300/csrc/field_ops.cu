@@ -12,6 +12,7 @@ namespace {
 template <typename T>
 __global__ void dirichlet_faces_kernel(FaceArgs a)
 {
+	dev::pdl_wait();
 	for (uint64_t idx = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; idx < a.total * a.S;
 		 idx += (uint64_t)gridDim.x * blockDim.x)
 		fielddev::face_item<T>(a, idx);
@@ -21,6 +22,7 @@ template <typename T>
 __global__ void dirichlet_interior_kernel(T* field, const uint64_t* offsets, const T* values, const uint8_t* conds,
 										  uint64_t K, uint64_t S)
 {
+	dev::pdl_wait();
 	for (uint64_t idx = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; idx < K * S;
 		 idx += (uint64_t)gridDim.x * blockDim.x)
 	{
@@ -36,6 +38,7 @@ template <typename T, bool PER_VOXEL>
 __global__ void bulk_kernel(T* field, const T* supply, const T* uptake, const T* target, uint32_t row_len,
 							uint64_t pitch, uint32_t chunks, uint32_t row_chunks, uint32_t S, T dt)
 {
+	dev::pdl_wait();
 	const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; // fewer than 2^32 field elements, so chunks too
 	if (k >= chunks)
 		return;
@@ -72,6 +75,7 @@ __global__ void mass_kernel(const T* field, double* out, uint64_t nx, uint64_t p
 // out = [before S | after S | worst S | factor S].
 __global__ void mass_check_finish_kernel(double* tot, uint32_t S, double* out)
 {
+	dev::pdl_wait();
 	for (uint32_t s = threadIdx.x; s < S; s += blockDim.x)
 	{
 		const double b = tot[s], a = tot[S + s];
@@ -165,7 +169,7 @@ static int run_dirichlet(Context* c, bool faces_done)
 	{
 		cudaEvent_t ev;
 		launch_begin(c, K_DIRICHLET_FACES, (double)(a.total * c->S * sizeof(T)), &ev);
-		dirichlet_faces_kernel<T><<<grid_for(c, a.total * c->S, 256), 256, 0, c->stream>>>(a);
+		PCG_CUDA_TRY(launch_chained(dirichlet_faces_kernel<T>, grid_for(c, a.total * c->S, 256), 256, 0, c->stream, a));
 		launch_end(c, K_DIRICHLET_FACES, ev);
 		PCG_CUDA_TRY(cudaGetLastError());
 	}
@@ -173,9 +177,10 @@ static int run_dirichlet(Context* c, bool faces_done)
 	{
 		cudaEvent_t ev;
 		launch_begin(c, K_DIRICHLET_INTERIOR, (double)(c->K * (8 + c->S * (2 * sizeof(T) + 1))), &ev);
-		dirichlet_interior_kernel<T><<<grid_for(c, c->K * c->S, 256), 256, 0, c->stream>>>(
-			static_cast<T*>(c->field.ptr), static_cast<const uint64_t*>(c->dir_offsets.ptr),
-			static_cast<const T*>(c->dir_values.ptr), static_cast<const uint8_t*>(c->dir_conds.ptr), c->K, c->S);
+		PCG_CUDA_TRY(launch_chained(dirichlet_interior_kernel<T>, grid_for(c, c->K * c->S, 256), 256, 0, c->stream,
+									static_cast<T*>(c->field.ptr), static_cast<const uint64_t*>(c->dir_offsets.ptr),
+									static_cast<const T*>(c->dir_values.ptr),
+									static_cast<const uint8_t*>(c->dir_conds.ptr), c->K, c->S));
 		launch_end(c, K_DIRICHLET_INTERIOR, ev);
 		PCG_CUDA_TRY(cudaGetLastError());
 	}
@@ -199,10 +204,10 @@ static int run_bulk(Context* c)
 	const double bytes = (double)(c->V * c->S * sizeof(T)) * (pv ? 5.0 : 2.0);
 	launch_begin(c, K_BULK, bytes, &ev);
 	auto kernel = pv ? bulk_kernel<T, true> : bulk_kernel<T, false>;
-	kernel<<<grid, 256, 0, c->stream>>>(static_cast<T*>(c->field.ptr), static_cast<const T*>(c->bulk[0].ptr),
-										static_cast<const T*>(c->bulk[1].ptr), static_cast<const T*>(c->bulk[2].ptr),
-										(uint32_t)c->row_len, c->pitch, (uint32_t)chunks, (uint32_t)row_chunks,
-										(uint32_t)c->S, (T)c->dt);
+	PCG_CUDA_TRY(launch_chained(kernel, grid, 256, 0, c->stream, static_cast<T*>(c->field.ptr),
+								static_cast<const T*>(c->bulk[0].ptr), static_cast<const T*>(c->bulk[1].ptr),
+								static_cast<const T*>(c->bulk[2].ptr), (uint32_t)c->row_len, c->pitch, (uint32_t)chunks,
+								(uint32_t)row_chunks, (uint32_t)c->S, (T)c->dt));
 	launch_end(c, K_BULK, ev);
 	PCG_CUDA_TRY(cudaGetLastError());
 	return PCG_OK;
@@ -230,8 +235,8 @@ int launch_mass_check_finish(Context* c)
 {
 	cudaEvent_t ev;
 	launch_begin(c, K_MASS_CHECK, (double)(c->S * 6 * sizeof(double)), &ev);
-	mass_check_finish_kernel<<<1, 64, 0, c->stream>>>(static_cast<double*>(c->mc_tot.ptr), (uint32_t)c->S,
-													  static_cast<double*>(c->mc_out.ptr));
+	PCG_CUDA_TRY(launch_chained(mass_check_finish_kernel, 1, 64, 0, c->stream, static_cast<double*>(c->mc_tot.ptr),
+								(uint32_t)c->S, static_cast<double*>(c->mc_out.ptr)));
 	launch_end(c, K_MASS_CHECK, ev);
 	PCG_CUDA_TRY(cudaGetLastError());
 	return PCG_OK;

@@ -17,7 +17,7 @@
 //    complete on an mbarrier, the tile is solved in place, and TMA stores
 //    write it back; the next load is issued as soon as the stores have read shared
 //    memory.  Several such CTAs per SM overlap one another's loads, compute and
-//    stores.
+//    stores.  The last CTA to leave clears the counter for the next launch.
 //  * Solvers run in blocks of 8 steps without per-step predicates; the next block's
 //    points are requested before the current block's dependent chain, so load
 //    latency overlaps the chain.
@@ -69,6 +69,7 @@ __global__ void __launch_bounds__(sweep_threads<T>()) sweep_yz_kernel(SweepArgs 
 		dev::fence_mbar_init();
 	}
 	__syncthreads();
+	dev::pdl_wait();
 	bool ok = true;
 	MassAcc<T> acc;
 	acc.zero();
@@ -154,6 +155,7 @@ __global__ void __launch_bounds__(sweep_threads<T>()) sweep_yz_kernel(SweepArgs 
 		atomicOr(a.err, DEV_ERR_WAIT_TIMEOUT);
 	if (threadIdx.x == 0)
 		dev::bulk_wait_all();
+	dev::leave(a.ticket);
 }
 
 // ------------------------------------------------------------------ x
@@ -187,6 +189,7 @@ __global__ void __launch_bounds__(sweep_threads<T>()) sweep_x_kernel(SweepArgs a
 		dev::fence_mbar_init();
 	}
 	__syncthreads();
+	dev::pdl_wait();
 	LineCoef<T> L = line_coef(static_cast<const T*>(a.tab), S, a.head, n, kWide ? min(s0, S - 1) : s0, half);
 	MassAcc<T> ai, ao;
 	ai.zero();
@@ -268,7 +271,9 @@ __global__ void __launch_bounds__(sweep_threads<T>()) sweep_x_kernel(SweepArgs a
 		atomicOr(a.err, DEV_ERR_WAIT_TIMEOUT);
 	if (half == 0)
 		dev::bulk_wait_all();
+	dev::leave(a.ticket);
 }
+
 // ------------------------------------------------------------------ fused x + y
 
 // The x and y sweeps of a 3-D mesh in one persistent launch, z-slab by z-slab.
@@ -336,6 +341,7 @@ __global__ void __launch_bounds__(sweep_threads<T>())
 	// x: lane (r, s) of either warp solves its half of substrate s of row r of the tile
 	const uint32_t S = ST ? (uint32_t)ST : ax.S, nx_pts = ax.n, R = ax.rows_per_tile;
 	const uint32_t r_local = lane / S, s = lane % S;
+	dev::pdl_wait();
 	const uint32_t row_bytes = (uint32_t)round_up(ax.row_len * sizeof(T), 16);
 	const LineCoef<T> Lx = line_coef(static_cast<const T*>(ax.tab), S, ax.head, nx_pts, s, half);
 	MassAcc<T> ai;
@@ -481,6 +487,7 @@ __global__ void __launch_bounds__(sweep_threads<T>())
 		flush_classes(ai.value(), S, kLanes, ax.mc_tot + s);
 	if (half == 0)
 		dev::bulk_wait_all();
+	dev::leave(f.ticket);
 }
 
 struct Plan
@@ -509,14 +516,21 @@ Plan plan(const Context* c, int axis)
 
 // CTAs of a persistent sweep launch: every one the device holds at once, at most
 // one per tile.
-int persistent_grid(Context* c, const void* kernel, int threads, uint64_t smem, uint64_t tiles, uint64_t* grid)
+int persistent_grid(Context* c, int slot, const void* kernel, int threads, uint64_t smem, uint64_t tiles, uint64_t* grid)
 {
-	PCG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-	int per_sm = 0;
-	PCG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
-	if (per_sm < 1)
-		return fail(PCG_ERR_UNSUPPORTED, "sweep tile does not fit in shared memory");
-	*grid = std::min<uint64_t>((uint64_t)per_sm * (uint64_t)c->sm_count, tiles);
+	Context::Resident& r = c->resident[slot];
+	if (r.kernel != kernel || r.smem != smem)
+	{
+		const int rc = allow_smem(kernel, c->device);
+		if (rc)
+			return rc;
+		int per_sm = 0;
+		PCG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
+		if (per_sm < 1)
+			return fail(PCG_ERR_UNSUPPORTED, "sweep tile does not fit in shared memory");
+		r = { kernel, smem, per_sm };
+	}
+	*grid = std::min<uint64_t>((uint64_t)r.per_sm * (uint64_t)c->sm_count, tiles);
 	return PCG_OK;
 }
 
@@ -532,7 +546,7 @@ SweepArgs base_args(const Context* c, int axis)
 	a.pitch = c->pitch;
 	a.rows = c->rows;
 	a.err = static_cast<uint32_t*>(c->err.ptr);
-	a.ticket = static_cast<uint32_t*>(c->tickets.ptr) + axis;
+	a.ticket = static_cast<uint32_t*>(c->tickets.ptr) + 2 * axis;
 	a.nx = (uint32_t)c->n[0], a.ny = (uint32_t)c->n[1], a.nz = (uint32_t)c->n[2];
 	if (c->wsize == 8)
 		a.sc = c->scale_table(axis);
@@ -600,12 +614,11 @@ int run_sweep_x(Context* c, bool mass_check)
 	const XKernel kernel = x_kernel<T>(c, mass_check);
 	uint64_t grid;
 	int rc;
-	if ((rc = persistent_grid(c, reinterpret_cast<const void*>(kernel), sweep_threads<T>(), p.smem, a.tiles, &grid)))
+	if ((rc = persistent_grid(c, 0, reinterpret_cast<const void*>(kernel), sweep_threads<T>(), p.smem, a.tiles, &grid)))
 		return rc;
-	PCG_CUDA_TRY(cudaMemsetAsync(a.ticket, 0, sizeof(uint32_t), c->stream));
 	cudaEvent_t ev;
 	launch_begin(c, K_SWEEP_X, 2.0 * (double)(c->V * c->S) * (double)sizeof(T), &ev);
-	kernel<<<(unsigned)grid, sweep_threads<T>(), p.smem, c->stream>>>(a);
+	PCG_CUDA_TRY(launch_chained(kernel, (unsigned)grid, sweep_threads<T>(), p.smem, c->stream, a));
 	launch_end(c, K_SWEEP_X, ev);
 	PCG_CUDA_TRY(cudaGetLastError());
 	return PCG_OK;
@@ -652,7 +665,7 @@ int run_sweep_xy(Context* c, bool mass_check)
 	}();
 	uint64_t resident;
 	int rc;
-	if ((rc = persistent_grid(c, reinterpret_cast<const void*>(kernel), sweep_threads<T>(), smem, ~0ull, &resident)))
+	if ((rc = persistent_grid(c, 3, reinterpret_cast<const void*>(kernel), sweep_threads<T>(), smem, ~0ull, &resident)))
 		return rc;
 	// the lag must exceed the tiles in flight (about one per resident CTA), else y
 	// tiles are handed out while their slab's x tiles are still being solved
@@ -701,17 +714,16 @@ int run_sweep_xy(Context* c, bool mass_check)
 	f.total = c->xy_total;
 	f.planes = (uint32_t)P;
 	f.done = static_cast<uint32_t*>(c->xy_done.ptr);
-	f.ticket = static_cast<uint32_t*>(c->tickets.ptr) + 3;
+	f.ticket = static_cast<uint32_t*>(c->tickets.ptr) + 6;
 	f.ny = ny;
 	f.nz = nz;
 	const uint64_t grid = std::min<uint64_t>(resident, c->xy_total);
-	PCG_CUDA_TRY(cudaMemsetAsync(f.ticket, 0, sizeof(uint32_t), c->stream));
 	PCG_CUDA_TRY(cudaMemsetAsync(f.done, 0, c->xy_nslab * sizeof(uint32_t), c->stream));
 	// minimal traffic of the two sweeps: the field read once and written once
 	const double bytes = 2.0 * (double)(c->V * c->S) * (double)sizeof(T);
 	cudaEvent_t ev;
 	launch_begin(c, K_SWEEP_XY, bytes, &ev);
-	kernel<<<(unsigned)grid, sweep_threads<T>(), smem, c->stream>>>(ax, ay, c->tmap[1], f);
+	PCG_CUDA_TRY(launch_chained(kernel, (unsigned)grid, sweep_threads<T>(), smem, c->stream, ax, ay, c->tmap[1], f));
 	launch_end(c, K_SWEEP_XY, ev);
 	PCG_CUDA_TRY(cudaGetLastError());
 	return PCG_OK;
@@ -755,12 +767,11 @@ int run_sweep_yz(Context* c, int axis, bool fuse_faces, bool mass_check)
 	auto kernel = axis == 1 ? yz_kernel<T, 1>(scale, mass_check) : yz_kernel<T, 2>(scale, mass_check);
 	uint64_t grid;
 	int rc;
-	if ((rc = persistent_grid(c, reinterpret_cast<const void*>(kernel), sweep_threads<T>(), p.smem, a.tiles, &grid)))
+	if ((rc = persistent_grid(c, axis, reinterpret_cast<const void*>(kernel), sweep_threads<T>(), p.smem, a.tiles, &grid)))
 		return rc;
-	PCG_CUDA_TRY(cudaMemsetAsync(a.ticket, 0, sizeof(uint32_t), c->stream));
 	cudaEvent_t ev;
 	launch_begin(c, kid, bytes, &ev);
-	kernel<<<(unsigned)grid, sweep_threads<T>(), p.smem, c->stream>>>(a, c->tmap[axis]);
+	PCG_CUDA_TRY(launch_chained(kernel, (unsigned)grid, sweep_threads<T>(), p.smem, c->stream, a, c->tmap[axis]));
 	launch_end(c, kid, ev);
 	PCG_CUDA_TRY(cudaGetLastError());
 	return PCG_OK;

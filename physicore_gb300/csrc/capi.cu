@@ -875,11 +875,9 @@ static int alloc_agents(Context* c, uint64_t A)
 		return rc;
 	if ((rc = dalloc(c, c->a_shared, std::max<uint64_t>(A, 1) * sizeof(uint32_t))))
 		return rc;
-	if ((rc = dalloc(c, c->a_rank, std::max<uint64_t>(A, 1) * sizeof(uint32_t))))
+	if ((rc = dalloc(c, c->a_sums, std::max<uint64_t>(A, 1) * sizeof(uint32_t))))
 		return rc;
 	if ((rc = dalloc(c, c->a_writers, std::max<uint64_t>(A, 1) * sizeof(uint32_t))))
-		return rc;
-	if ((rc = dalloc(c, c->a_sorted, std::max<uint64_t>(A, 1) * 2 * sizeof(uint32_t))))
 		return rc;
 	c->term_stride = term_stride(S, w);
 	for (DeviceBuffer* b : { &c->a_terms, &c->a_reduced })
@@ -960,6 +958,7 @@ int upload_agents(Context* c, uint64_t A, const double* positions, const double*
 	}
 	c->recompute_cells = true;
 	c->terms_dirty = true;
+	c->counts_follow_vox = false; // the new agents' voxels are not known yet
 	return PCG_OK;
 }
 
@@ -1071,7 +1070,7 @@ int pcg_destroy(pcg_context* c)
 								 &c->a_active,	 &c->a_internal, &c->a_frac,	&c->a_foff,		 &c->a_terms,
 								 &c->a_reduced,
 								 &c->owner,		 &c->counts,	&c->a_role,		&c->a_shared,	 &c->rb_staging[0],
-								 &c->rb_staging[1], &c->a_rank,	&c->a_sorted,	&c->a_writers,	 &c->xy_segs,
+								 &c->rb_staging[1], &c->a_sums,	&c->a_writers,	 &c->xy_segs,
 								 &c->xy_done };
 	for (auto* b : all)
 		pcg::dfree(*b);
@@ -1767,7 +1766,7 @@ int pcg_set_kernel_timing(pcg_context* c, int enable)
 		PCG_CUDA_TRY(stream_wait(c));
 		PCG_CUDA_TRY(cudaMemcpy(c->h_words + 2, static_cast<uint32_t*>(c->flags.ptr) + 2, sizeof(uint32_t),
 								cudaMemcpyDeviceToHost));
-		PCG_CUDA_TRY(cudaMemcpy(c->h_words + 3, static_cast<uint32_t*>(c->flags.ptr) + 4, sizeof(uint32_t),
+		PCG_CUDA_TRY(cudaMemcpy(c->h_words + 3, static_cast<uint32_t*>(c->flags.ptr) + 3, sizeof(uint32_t),
 								cudaMemcpyDeviceToHost));
 		c->shared_agents = c->h_words[2];
 		c->writer_agents = c->h_words[3];

@@ -9,17 +9,16 @@
 //   release      (274-289)  D += I F / Vv, I = 0
 //
 // GB300 design:
-//  * place: one thread per agent computes its voxel index exactly as
+//  * locate: one thread per agent computes its voxel index exactly as
 //    cartesian_mesh::voxel_position does (mesh.cpp:37-61; locate in
 //    cells_device.cuh: an FP32 estimate decides unless it lies within its error
 //    bound of a voxel boundary, where the FP64 division decides), so the
-//    agent->voxel maps and the per-voxel counts are bit-exact with the reference;
-//    a run of lanes in one voxel counts with one atomic, whose returned offset
-//    ranks the agents of the voxel.
-//  * ballot: rank 0 wins the voxel (the reference's first compare-and-swap wins,
-//    cell_solver.cpp:79-101); the agents of shared voxels are grouped by voxel and
-//    each group is summed by a segmented warp reduction instead of every agent
-//    adding its terms to the winner's row with contended atomics
+//    agent->voxel maps and the per-voxel counts are bit-exact with the reference.
+//  * ballot: a run of lanes in one voxel counts with one atomic, whose returned
+//    offset ranks the agents of the voxel; rank 0 wins (the reference's first
+//    compare-and-swap wins, cell_solver.cpp:79-101).
+//  * group lists the agents of shared voxels and those that write a voxel; reduce
+//    adds the terms of the shared ones to a row per voxel with four-value atomics
 //    (cell_solver.cpp:102-127); the conflict flag stays on the device, so the step
 //    never waits on the host (the Thrust backend copies it back every step,
 //    thrust_solver/src/cell_solver.cpp:251-252).
@@ -36,281 +35,249 @@ namespace {
 
 using namespace cellsdev;
 
-// place: terms (after new agent data), voxel, count and rank; the step's words
-// (conflict flag, list length, reserved group slots) start at zero.  One agent
-// per thread: two per thread (both chunks' loads and atomics in flight together)
-// measured slower on the dense workload, 78 -> 107 us.
+// clear: the counts of the last ballot, before the voxels that it recorded are
+// overwritten.  With BY_AGENT only the voxels that held an agent are written: the
+// counts are zero everywhere else.  One scattered word per agent (a 32-byte sector
+// each) against the whole array: the launcher takes the agents when they are fewer
+// than one per 16 voxels (320x320x256, 200,000 agents: 5.9 us, against 16 for the
+// array's 105 MB at the copy bandwidth; 200^3, 4M agents: the array, 7 us).
+template <bool BY_AGENT>
+__global__ void cells_clear_kernel(uint32_t* counts, const uint32_t* vox, uint64_t n)
+{
+	dev::pdl_wait();
+	const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+	if constexpr (BY_AGENT)
+	{
+		if (i < n && vox[i] != kNoAgent)
+			counts[vox[i]] = 0;
+	}
+	else // n counts, four to a thread (the array starts on a 16-byte boundary)
+	{
+		const uint64_t k = 4 * i;
+		if (k + 4 <= n)
+			*reinterpret_cast<uint4*>(counts + k) = make_uint4(0, 0, 0, 0);
+		else
+			for (uint64_t q = k; q < n; q++)
+				counts[q] = 0;
+	}
+}
+
+// locate: terms (after new agent data) and voxel; the step's words (conflict flag,
+// list lengths) start at zero.
 template <typename T>
-__global__ void cells_place_kernel(CellArgs a)
+__global__ void cells_locate_kernel(CellArgs a)
 {
 	dev::pdl_wait();
 	const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
 	if (i == 0)
 	{
 		a.flags[0] = a.flags[1] = a.flags[2] = a.flags[3] = 0;
-		if (a.writers)
-			a.flags[4] = 0;
 	}
-	uint32_t v[1] = { kNoAgent };
-	if (i < a.A)
-	{
-		if (a.terms)
-			agent_terms<T>(a, i);
-		v[0] = agent_place(a, i);
-	}
-	count_rank<1>(a, i, v);
+	if (i >= a.A)
+		return;
+	if (a.terms)
+		agent_terms<T>(a, i);
+	agent_place(a, i);
 }
 
-constexpr unsigned kClassifyBlock = 1024;
-constexpr unsigned kClassifyChunks = 4; // 32-agent chunks per warp
-
-// classify: roles from count and rank (cell_solver.cpp:102-127: every agent but
-// the winner of a shared voxel is a conflict); the agents of shared voxels listed
-// in agent order (flags[2]); each winner reserves its voxel's group of slots
-// (owner[v] = first slot, flags[3] counts slots) and clears its reduced row; with
-// a writer list, the agents that write a voxel (alone or winner) listed in agent
-// order (flags[4]).  A warp takes kClassifyChunks consecutive chunks of 32 agents
-// (their loads in flight together).  A block scans its counts and reserves its
-// ranges with one 64-bit atomic on the adjacent, 8-byte aligned words flags[2..3]
-// (list entries low, slots high; neither total reaches 2^32, so no carry crosses)
-// and one on flags[4]: same-address atomics that return a value serialise, so
-// there is one per 4096 agents and word.
+// ballot: rank of every agent in its voxel; the winner of a voxel that may prove to
+// be alone there is marked a winner for now.  Apart from locate, whose FP64
+// conversions and loads it would wait for: its atomics (one per agent, 45 us for the
+// 4M of the dense workload) are all it does.
 template <typename T>
-__global__ void __launch_bounds__(kClassifyBlock, 2) cells_classify_kernel(CellArgs a)
-{
-	dev::pdl_wait();
-	constexpr int K = kClassifyChunks;
-	__shared__ uint32_t part[3][kClassifyBlock / 32];
-	__shared__ uint32_t base[3];
-	const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-	const uint64_t i0 = ((uint64_t)blockIdx.x * nw + warp) * (K * 32) + lane;
-	uint32_t v[K], cnt[K];
-	uint8_t role[K];
-#pragma unroll
-	for (int k = 0; k < K; k++)
-	{
-		const uint64_t i = i0 + k * 32;
-		v[k] = i < a.A ? a.vox[i] : kNoAgent;
-		cnt[k] = v[k] != kNoAgent ? a.rank[i] : 0u; // the rank, for now
-	}
-	// an agent of rank > 0 shares its voxel: only rank 0 needs the count (a
-	// scattered read that the block's scans would wait for)
-#pragma unroll
-	for (int k = 0; k < K; k++)
-	{
-		const bool first = v[k] != kNoAgent && cnt[k] == 0;
-		role[k] = v[k] == kNoAgent ? kRoleNone : (first ? kRoleWinner : kRoleLoser);
-		cnt[k] = first ? a.counts[v[k]] : 0u;
-	}
-	bool loser = false;
-	uint32_t bsh[K], bwr[K], seg_inc[K], tsh = 0, twr = 0, tseg = 0;
-	const uint32_t below = (1u << lane) - 1u;
-#pragma unroll
-	for (int k = 0; k < K; k++)
-	{
-		const uint64_t i = i0 + k * 32;
-		if (role[k] == kRoleWinner && cnt[k] == 1)
-			role[k] = kRoleAlone;
-		if (i < a.A)
-			a.role[i] = role[k];
-		loser |= role[k] == kRoleLoser;
-		bsh[k] = __ballot_sync(0xffffffffu, role[k] == kRoleWinner || role[k] == kRoleLoser);
-		bwr[k] = __ballot_sync(0xffffffffu, a.writers && (role[k] == kRoleAlone || role[k] == kRoleWinner));
-		// slots before this lane's in the warp's agent order (chunk-major)
-		uint32_t x = role[k] == kRoleWinner ? cnt[k] : 0u;
-		for (uint32_t o = 1; o < 32; o <<= 1)
-		{
-			const uint32_t t = __shfl_up_sync(0xffffffffu, x, o);
-			if (lane >= o)
-				x += t;
-		}
-		seg_inc[k] = tseg + x;
-		tseg += __shfl_sync(0xffffffffu, x, 31);
-		tsh += __popc(bsh[k]);
-		twr += __popc(bwr[k]);
-	}
-	if (__any_sync(0xffffffffu, loser) && lane == 0)
-		atomicOr(a.flags, 1u);
-	if (lane == 0)
-		part[0][warp] = tsh, part[1][warp] = tseg, part[2][warp] = twr;
-	__syncthreads();
-	if (warp == 0)
-	{
-		uint32_t p[3];
-#pragma unroll
-		for (int q = 0; q < 3; q++)
-			p[q] = lane < nw ? part[q][lane] : 0u;
-		for (uint32_t o = 1; o < 32; o <<= 1)
-#pragma unroll
-			for (int q = 0; q < 3; q++)
-			{
-				const uint32_t t = __shfl_up_sync(0xffffffffu, p[q], o);
-				if (lane >= o)
-					p[q] += t;
-			}
-		if (lane == 31)
-		{
-			unsigned long long old = 0ull;
-			if (p[0] | p[1])
-				old = atomicAdd(reinterpret_cast<unsigned long long*>(a.flags + 2),
-								((unsigned long long)p[1] << 32) | (unsigned long long)p[0]);
-			base[0] = (uint32_t)old;
-			base[1] = (uint32_t)(old >> 32);
-			base[2] = p[2] ? atomicAdd(a.flags + 4, p[2]) : 0u;
-		}
-#pragma unroll
-		for (int q = 0; q < 3; q++)
-		{
-			const uint32_t e = __shfl_up_sync(0xffffffffu, p[q], 1);
-			if (lane < nw)
-				part[q][lane] = lane == 0 ? 0u : e;
-		}
-	}
-	__syncthreads();
-	uint32_t osh = base[0] + part[0][warp], owr = base[2] + part[2][warp];
-	const uint32_t oseg = base[1] + part[1][warp];
-#pragma unroll
-	for (int k = 0; k < K; k++)
-	{
-		const uint64_t i = i0 + k * 32;
-		if ((bsh[k] >> lane) & 1u)
-			a.shared[osh + __popc(bsh[k] & below)] = (uint32_t)i;
-		if ((bwr[k] >> lane) & 1u)
-			a.writers[owr + __popc(bwr[k] & below)] = (uint32_t)i;
-		osh += __popc(bsh[k]);
-		owr += __popc(bwr[k]);
-		if (role[k] == kRoleWinner)
-		{
-			a.owner[v[k]] = oseg + seg_inc[k] - cnt[k];
-			T* rn = static_cast<T*>(a.rnum) + i * a.ts;
-			T* rd = static_cast<T*>(a.rden) + i * a.ts;
-			T* rf = static_cast<T*>(a.rfac) + i * a.ts;
-			for (uint64_t s = 0; s < a.S; s++)
-				rn[s] = rd[s] = rf[s] = T(0);
-		}
-	}
-}
-
-// group: every agent of a shared voxel (role from classify) writes (its index,
-// its voxel) into its voxel's group of slots.  One thread per agent: with many
-// agents per voxel nearly all of them write, and the loads of one agent (role,
-// voxel, rank, then its voxel's first slot) form a chain that only more threads in
-// flight hide.
-__global__ void cells_group_kernel(CellArgs a)
+__global__ void cells_ballot_kernel(CellArgs a)
 {
 	dev::pdl_wait();
 	const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+	const uint32_t v = i < a.A ? a.vox[i] : kNoAgent;
+	const uint32_t rank = count_rank(a, v);
 	if (i >= a.A)
 		return;
-	const uint8_t role = a.role[i];
-	if (role != kRoleWinner && role != kRoleLoser)
-		return;
-	const uint32_t v = a.vox[i];
-	a.sorted[(uint64_t)__ldg(a.owner + v) + a.rank[i]] = make_uint2((uint32_t)i, v);
+	a.role[i] = v == kNoAgent ? kRoleNone : (rank == 0 ? kRoleWinner : kRoleLoser);
+	if (v != kNoAgent && rank == 1)
+	{
+		// this agent's row takes the voxel's sums (FP64 builds: 1 + sum den; FP32 rows
+		// hold the bare sum, see fp32_update)
+		a.owner[v] = (uint32_t)i;
+		T* rn = static_cast<T*>(a.rnum) + i * a.ts;
+		T* rd = static_cast<T*>(a.rden) + i * a.ts;
+		T* rf = static_cast<T*>(a.rfac) + i * a.ts;
+		if (a.joined)
+			for (uint64_t k = 0; k < a.ts; k++)
+				rn[k] = T(0);
+		for (uint64_t s = 0; s < a.S; s++)
+		{
+			rn[s] = rf[s] = T(0);
+			rd[s] = sizeof(T) == 8 ? T(1) : T(0);
+		}
+	}
 }
 
-// group sum: a warp takes 32 consecutive slots and sums each voxel's terms with a
-// segmented scan (lanes of one voxel are consecutive); the last lane of each
-// voxel's run writes the winner's row: sum num, sum den (plus 1 in FP64 builds),
-// sum fac -- stored when the run is the voxel's whole group, else added with
-// atomics (the part holding the group's first slot adds the 1).  SC is S when
-// the launch fixes it at compile time (1-8: the per-substrate guards fold away),
-// else 0.
+constexpr unsigned kGroupBlock = 256;
+
+// Consecutive agents of a thread: 8 keep blocks and their atomics few; up to 2^20
+// agents 4, for more threads in flight (200,000 agents: 13.5 us with 16, 9.6 with 4).
+constexpr uint64_t kGroupWide = 1ull << 20;
+
+// group: final roles (cell_solver.cpp:102-127: every agent but the winner of a shared
+// voxel is a conflict); the agents of shared voxels listed in agent order (flags[2])
+// and, with a writer list, those that write a voxel (alone or winner; flags[3]).  A
+// thread takes Q consecutive agents, of which only the winners need their voxel's
+// count.  A block scans its counts and reserves its ranges with one atomic: atomics on
+// one address serialise.
+template <int Q>
+__global__ void __launch_bounds__(kGroupBlock, 6) cells_group_kernel(CellArgs a)
+{
+	__shared__ uint32_t part[2][kGroupBlock / 32];
+	__shared__ uint32_t base[2], total[2];
+	__shared__ uint32_t stage[kGroupBlock * Q];
+	dev::pdl_wait();
+	const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+	const uint64_t i0 = (blockIdx.x * (uint64_t)kGroupBlock + threadIdx.x) * Q;
+	const uint32_t n = i0 < a.A ? (uint32_t)min((uint64_t)Q, a.A - i0) : 0u;
+	struct alignas(Q) Roles
+	{
+		uint8_t r[Q];
+	} roles {};
+	if (n == Q)
+		roles = *reinterpret_cast<const Roles*>(a.role + i0);
+	else
+		for (uint32_t q = 0; q < n; q++)
+			roles.r[q] = a.role[i0 + q];
+	uint32_t shared = 0, writes = 0; // bit q: agent i0 + q
+	uint32_t cnt[Q]; // the winners' voxels, then their counts, all loads of a kind in flight together
+#pragma unroll
+	for (uint32_t q = 0; q < Q; q++)
+		cnt[q] = roles.r[q] == kRoleWinner ? a.vox[i0 + q] : 0u;
+#pragma unroll
+	for (uint32_t q = 0; q < Q; q++)
+		cnt[q] = roles.r[q] == kRoleWinner ? a.counts[cnt[q]] : 0u;
+#pragma unroll
+	for (uint32_t q = 0; q < Q; q++)
+	{
+		if (roles.r[q] == kRoleWinner)
+		{
+			if (cnt[q] == 1)
+				roles.r[q] = kRoleAlone;
+			else
+				a.sums[i0 + q] = a.owner[a.vox[i0 + q]];
+			writes |= 1u << q;
+		}
+		if (roles.r[q] >= kRoleWinner)
+			shared |= 1u << q;
+	}
+	if (n == Q)
+		*reinterpret_cast<Roles*>(a.role + i0) = roles;
+	else
+		for (uint32_t q = 0; q < n; q++)
+			a.role[i0 + q] = roles.r[q];
+	uint32_t psh = __popc(shared), pwr = a.writers ? __popc(writes) : 0u;
+#pragma unroll
+	for (uint32_t o = 1; o < 32; o <<= 1)
+	{
+		const uint32_t t0 = __shfl_up_sync(0xffffffffu, psh, o), t1 = __shfl_up_sync(0xffffffffu, pwr, o);
+		if (lane >= o)
+			psh += t0, pwr += t1;
+	}
+	if (lane == 31)
+		part[0][warp] = psh, part[1][warp] = pwr;
+	__syncthreads();
+	if (threadIdx.x == 0)
+	{
+		uint32_t sum[2] = { 0, 0 };
+		for (uint32_t w = 0; w < kGroupBlock / 32; w++)
+#pragma unroll
+			for (int l = 0; l < 2; l++)
+			{
+				const uint32_t t = part[l][w];
+				part[l][w] = sum[l];
+				sum[l] += t;
+			}
+		// both lists' ranges with one 64-bit atomic on their adjacent words (neither
+		// total reaches 2^32, so no carry crosses)
+		unsigned long long old = 0ull;
+		if (sum[0] | sum[1])
+			old = atomicAdd(reinterpret_cast<unsigned long long*>(a.flags + 2),
+							((unsigned long long)sum[1] << 32) | (unsigned long long)sum[0]);
+		if (sum[0]) // a shared voxel has a loser
+			a.flags[0] = 1;
+		total[0] = sum[0], total[1] = sum[1];
+		base[0] = (uint32_t)old, base[1] = (uint32_t)(old >> 32);
+	}
+	__syncthreads();
+	// the entries, in agent order, through shared memory: a thread's are side by side,
+	// so written directly each store of a warp would touch 32 sectors
+	for (int list = 0; list < (a.writers ? 2 : 1); list++)
+	{
+		uint32_t at = list ? part[1][warp] + pwr - __popc(writes) : part[0][warp] + psh - __popc(shared);
+		const uint32_t bits = list ? writes : shared;
+		uint32_t* to = (list ? a.writers : a.shared) + base[list];
+#pragma unroll
+		for (uint32_t q = 0; q < Q; q++)
+			if ((bits >> q) & 1u)
+				stage[at++] = (uint32_t)(i0 + q);
+		__syncthreads();
+		for (uint32_t k = threadIdx.x; k < total[list]; k += kGroupBlock)
+			to[k] = stage[k];
+		__syncthreads();
+	}
+}
+
+// reduce: every agent of a shared voxel adds its terms to its voxel's row.  Four-value atomics run at four times the values per
+// second of single ones (4M agents x 12 values on 182,253 voxels: 76 us against 241;
+// grouping the agents by voxel and summing each group with warp scans took 128).  A
+// warp whose agents all share one voxel (a crowd in one place) sums its terms first
+// and adds them once.
 template <typename T, int SC>
-__global__ void cells_group_sum_kernel(CellArgs a)
+__global__ void cells_reduce_kernel(CellArgs a)
 {
 	dev::pdl_wait();
 	const uint32_t count = __ldg(a.flags + a.list_word);
-	const uint32_t lane = threadIdx.x & 31;
-	const uint64_t gw = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-	const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
 	const uint32_t S = SC ? (uint32_t)SC : (uint32_t)a.S;
-	const bool vec = a.vec;
 	T* rnum = static_cast<T*>(a.rnum);
 	T* rden = static_cast<T*>(a.rden);
 	T* rfac = static_cast<T*>(a.rfac);
-	for (uint64_t j0 = gw * 32; j0 < count; j0 += nwarps * 32)
+	for (uint64_t j0 = blockIdx.x * (uint64_t)blockDim.x + (threadIdx.x & ~31u); j0 < count;
+		 j0 += (uint64_t)gridDim.x * blockDim.x)
 	{
-		const uint64_t j = j0 + lane;
-		uint32_t v = kNoAgent;
-		const T *pn = nullptr, *pd = nullptr, *pf = nullptr;
+		const uint64_t j = j0 + (threadIdx.x & 31);
+		uint64_t i = 0;
+		uint32_t v = kNoAgent, o = 0;
 		if (j < count)
 		{
-			// the agent's three rows lie side by side in a context's term rows
-			const uint2 iv = __ldg(a.sorted + j);
-			v = iv.y;
-			pn = static_cast<const T*>(a.num) + (uint64_t)iv.x * a.ts;
-			pd = static_cast<const T*>(a.den) + (uint64_t)iv.x * a.ts;
-			pf = static_cast<const T*>(a.fac) + (uint64_t)iv.x * a.ts;
+			i = __ldg(a.shared + j);
+			v = a.vox[i];
+			o = __ldg(a.owner + v);
 		}
-		uint32_t first, end;
-		key_run(v, first, end);
-		const uint32_t last = end - 1;
-		const bool writer = v != kNoAgent && lane == last;
-		uint32_t w = 0;
-		bool head = false, whole = false;
-		if (writer)
+		const T* num = static_cast<const T*>(a.num) + i * a.ts;
+		const T* den = static_cast<const T*>(a.den) + i * a.ts;
+		const T* fac = static_cast<const T*>(a.fac) + i * a.ts;
+		if (__all_sync(0xffffffffu, v == __shfl_sync(0xffffffffu, v, 0)))
 		{
-			const uint32_t seg0 = __ldg(a.owner + v), cnt = __ldg(a.counts + v);
-			w = __ldg(&a.sorted[seg0].x);
-			head = j0 + first == seg0;
-			whole = head && j0 + last == (uint64_t)seg0 + cnt - 1;
-		}
-		uint32_t kup[5];
-#pragma unroll
-		for (int k = 0; k < 5; k++)
-			kup[k] = __shfl_up_sync(0xffffffffu, v, 1u << k);
-		for (uint32_t s0 = 0; s0 < S; s0 += kSubBatch)
-		{
-			T n_[kSubBatch], d_[kSubBatch], f_[kSubBatch];
-#pragma unroll
-			for (int q = 0; q < kSubBatch; q++)
-				n_[q] = d_[q] = f_[q] = T(0);
-			if (v != kNoAgent)
+			for (uint32_t s = 0; s < S; s++)
 			{
-				row_load(pn, s0, S, vec, n_);
-				row_load(pd, s0, S, vec, d_);
-				row_load(pf, s0, S, vec, f_);
-			}
+				T x[3] = { num[s], den[s], fac[s] };
 #pragma unroll
-			for (int k = 0; k < 5; k++)
-			{
-				const uint32_t o = 1u << k;
-				const bool take = lane >= o && kup[k] == v;
-#pragma unroll
-				for (int q = 0; q < kSubBatch; q++)
-					if (s0 + q < S) // uniform across the warp
-					{
-						const T tn = __shfl_up_sync(0xffffffffu, n_[q], o);
-						const T td = __shfl_up_sync(0xffffffffu, d_[q], o);
-						const T tf = __shfl_up_sync(0xffffffffu, f_[q], o);
-						if (take)
-							n_[q] += tn, d_[q] += td, f_[q] += tf;
-					}
-			}
-			if (writer)
-			{
-				if (head && sizeof(T) == 8) // FP64 rows hold 1 + sum den; FP32 rows the bare sum (fp32_update)
-#pragma unroll
-					for (int q = 0; q < kSubBatch; q++)
-						d_[q] += T(1);
-				const uint64_t r = (uint64_t)w * a.ts;
-				if (whole)
+				for (int k = 0; k < 3; k++)
 				{
-					row_store(rnum + r, s0, S, vec, n_);
-					row_store(rden + r, s0, S, vec, d_);
-					row_store(rfac + r, s0, S, vec, f_);
+					for (int d = 16; d > 0; d >>= 1)
+						x[k] += __shfl_xor_sync(0xffffffffu, x[k], d);
+					if ((threadIdx.x & 31) == 0)
+						atomicAdd((k == 0 ? rnum : k == 1 ? rden : rfac) + (uint64_t)o * a.ts + s, x[k]);
 				}
-				else
-#pragma unroll
-					for (int q = 0; q < kSubBatch; q++)
-						if (s0 + q < S)
-						{
-							atomicAdd(rnum + r + s0 + q, n_[q]);
-							atomicAdd(rden + r + s0 + q, d_[q]);
-							atomicAdd(rfac + r + s0 + q, f_[q]);
-						}
 			}
+			continue;
+		}
+		if (v == kNoAgent)
+			continue;
+		const uint64_t row = (uint64_t)o * a.ts;
+		if (a.joined) // FP32 rows are padded to whole quads
+			add_values(rnum + row, num, sizeof(T) == 4 ? (3 * S + 3) / 4 * 4 : 3 * S, true);
+		else
+		{
+			add_values(rnum + row, num, S, a.vec);
+			add_values(rden + row, den, S, a.vec);
+			add_values(rfac + row, fac, S, a.vec);
 		}
 	}
 }
@@ -326,7 +293,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 1) cells_apply_kerne
 		agent_apply<T>(a, i);
 }
 
-// Over the agents that write a voxel (alone or winner; flags[4] of them, listed
+// Over the agents that write a voxel (alone or winner; flags[3] of them, listed
 // by classify) when they are fewer than half the agents, else over every agent
 // (agent_apply returns at once for the others): with many agents per voxel most
 // agents only lose their ballot, and a thread per agent would mostly wait on its
@@ -336,7 +303,7 @@ template <typename T, int SC>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 1) cells_apply_writers_kernel(CellArgs a)
 {
 	dev::pdl_wait();
-	const uint32_t count = __ldg(a.flags + 4);
+	const uint32_t count = __ldg(a.flags + 3);
 	const bool list = 2ull * count < a.A;
 	const uint64_t n = list ? count : a.A;
 	for (uint64_t j = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; j < n; j += (uint64_t)gridDim.x * blockDim.x)
@@ -369,13 +336,13 @@ __global__ void cells_release_kernel(CellArgs a, uint64_t agent)
 	const uint64_t s = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
 	if (s >= a.S)
 		return;
-	uint64_t idx[3];
+	uint32_t idx[3];
 	if (!locate(a, agent, idx))
 	{
 		atomicOr(a.err, DEV_ERR_AGENT_OUTSIDE);
 		return;
 	}
-	T* D = static_cast<T*>(a.field) + (idx[2] * a.n[1] + idx[1]) * a.pitch + idx[0] * a.S + s;
+	T* D = static_cast<T*>(a.field) + ((uint64_t)idx[2] * a.n[1] + idx[1]) * a.pitch + idx[0] * a.S + s;
 	const uint64_t k = agent * a.S + s;
 	const double I = a.pairs ? pair_value(a.internal[k]) : a.internal[k];
 	*D = (T)((double)*D + I * a.frac[k] / a.Vv);
@@ -432,65 +399,77 @@ CellArgs make_cell_args(const Context* c)
 	a.vec = rows_vectorizable(a, c->wsize);
 	a.terms = 1;
 	a.pairs = c->wsize == 4 ? 1 : 0; // FP32 contexts store internalized amounts as float pairs
-	a.rank = static_cast<uint32_t*>(c->a_rank.ptr);
-	a.sorted = static_cast<uint2*>(c->a_sorted.ptr);
+	a.sums = static_cast<uint32_t*>(c->a_sums.ptr);
+	a.joined = 1;
 	a.writers = static_cast<uint32_t*>(c->a_writers.ptr);
-	a.list_word = 2; // the grouped ballot (a batch sets 1 for its per-warp ballot)
+	a.list_word = 2; // (a batch sets 1 for its per-warp ballot)
 	set_fast_locate(a);
 	return a;
 }
 
 } // namespace cellsdev
 
-// The voxel-grouped ballot (cells_device.cuh) on `stream`; launch bookkeeping
-// through `c` when given.
+// The ballot of a single domain (cells_device.cuh) on `stream`; launch bookkeeping
+// through `c` when given.  The counts hold zeros already.
 template <typename T>
 static int run_ballot(Context* c, const CellArgs& a, cudaStream_t stream, int sm_count)
 {
 	const unsigned block = 256;
 	const unsigned grid = (unsigned)((a.A + block - 1) / block);
-	const uint64_t per_block = (uint64_t)kClassifyBlock * kClassifyChunks;
-	const unsigned cgrid = (unsigned)((a.A + per_block - 1) / per_block);
+	const bool wide = a.A > kGroupWide;
+	const uint64_t per_block = (uint64_t)kGroupBlock * (wide ? 8 : 4);
+	const unsigned ggrid = (unsigned)((a.A + per_block - 1) / per_block);
 	// the list of shared-voxel agents is only known on the device: grid-stride
-	const unsigned lgrid = std::min<unsigned>(grid, 16 * std::max(sm_count, 1));
+	const unsigned lgrid = std::min<unsigned>(grid, 24 * std::max(sm_count, 1));
 	const double S = (double)a.S, A = (double)a.A, w = (double)sizeof(T);
 	cudaEvent_t ev = nullptr;
 	if (c)
-		launch_begin(c, K_CELLS_LOCATE,
-					 A * (8.0 * a.dims + 1 + 4 + 4 + 4 + 4) + (a.terms ? A * (5 * S * 8 + 8 + 3 * S * w) : 0), &ev);
-	PCG_CUDA_TRY(launch_chained(cells_place_kernel<T>, grid, block, 0, stream, a));
+		launch_begin(c, K_CELLS_LOCATE, A * (8.0 * a.dims + 1 + 4 + 4) + (a.terms ? A * (5 * S * 8 + 8 + 3 * S * w) : 0),
+					 &ev);
+	PCG_CUDA_TRY(launch_chained(cells_locate_kernel<T>, grid, block, 0, stream, a));
 	if (c)
 		launch_end(c, K_CELLS_LOCATE, ev);
-	PCG_CUDA_TRY(cudaGetLastError());
+	// voxel in, role out, one count updated
 	if (c)
-		launch_begin(c, K_CELLS_BALLOT, A * (4 + 4 + 4 + 1), &ev);
-	PCG_CUDA_TRY(launch_chained(cells_classify_kernel<T>, cgrid, kClassifyBlock, 0, stream, a));
+		launch_begin(c, K_CELLS_BALLOT, A * (4 + 1 + 8), &ev);
+	PCG_CUDA_TRY(launch_chained(cells_ballot_kernel<T>, grid, block, 0, stream, a));
+	if (c)
+		launch_end(c, K_CELLS_BALLOT, ev);
+	// per agent its role in and out; shared-voxel agents and writers: list entry;
+	// writers: voxel and count
+	if (c)
+		launch_begin(c, K_CELLS_GROUP, 2 * A, &ev);
+	PCG_CUDA_TRY(launch_chained(wide ? cells_group_kernel<8> : cells_group_kernel<4>, ggrid, kGroupBlock, 0, stream, a));
 	if (c && c->timing && c->h_words) // list lengths for the per-agent byte counts
 	{
 		PCG_CUDA_TRY(
 			cudaMemcpyAsync(c->h_words + 2, a.flags + a.list_word, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
-		PCG_CUDA_TRY(cudaMemcpyAsync(c->h_words + 3, a.flags + 4, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
+		PCG_CUDA_TRY(cudaMemcpyAsync(c->h_words + 3, a.flags + 3, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
 	}
-	// shared-voxel agents: list entry, winner's row cleared; writers: list entry
 	if (c)
-		launch_end(c, K_CELLS_BALLOT, ev, 4.0 + 3 * S * w, 4.0);
-	PCG_CUDA_TRY(cudaGetLastError());
-	// per agent its role; per shared-voxel agent its voxel, rank and voxel's first
-	// slot, and the pair written
-	if (c)
-		launch_begin(c, K_CELLS_GROUP, A, &ev);
-	PCG_CUDA_TRY(launch_chained(cells_group_kernel, grid, block, 0, stream, a));
-	if (c)
-		launch_end(c, K_CELLS_GROUP, ev, 20.0);
-	PCG_CUDA_TRY(cudaGetLastError());
-	// per slot: the pair and the agent's three rows (one gathered term row in a
-	// context)
+		launch_end(c, K_CELLS_GROUP, ev, 4.0, 12.0);
+	// per shared-voxel agent: list entry, voxel, its row's index, role and terms
 	if (c)
 		launch_begin(c, K_CELLS_REDUCE, 0.0, &ev);
-	PCG_LAUNCH_BY_S(cells_group_sum_kernel, T, a.S, lgrid, block, stream, a);
+	PCG_LAUNCH_BY_S(cells_reduce_kernel, T, a.S, lgrid, block, stream, a);
 	if (c)
-		launch_end(c, K_CELLS_REDUCE, ev, 8.0 + 3 * S * w);
-	PCG_CUDA_TRY(cudaGetLastError());
+		launch_end(c, K_CELLS_REDUCE, ev, 13.0 + 3 * S * w);
+	return PCG_OK;
+}
+
+// Zeroes the counts: over the voxels that the last ballot counted agents in, or the
+// whole array.
+static int clear_counts(Context* c)
+{
+	const bool by_agent = c->counts_follow_vox && c->A * 16 < c->V;
+	const uint64_t threads = by_agent ? c->A : (c->V + 3) / 4;
+	uint32_t* counts = static_cast<uint32_t*>(c->counts.ptr);
+	cudaEvent_t ev;
+	launch_begin(c, K_CELLS_CLEAR, by_agent ? 8.0 * (double)c->A : 4.0 * (double)c->V, &ev);
+	PCG_CUDA_TRY(launch_chained(by_agent ? cells_clear_kernel<true> : cells_clear_kernel<false>,
+								(unsigned)((threads + 255) / 256), 256, 0, c->stream, counts,
+								static_cast<const uint32_t*>(c->a_vox.ptr), by_agent ? c->A : c->V));
+	launch_end(c, K_CELLS_CLEAR, ev);
 	return PCG_OK;
 }
 
@@ -510,12 +489,15 @@ static int run_cells(Context* c, bool recompute)
 		recompute = true;
 	if (recompute)
 	{
-		PCG_CUDA_TRY(cudaMemsetAsync(c->counts.ptr, 0, c->V * sizeof(uint32_t), c->stream));
+		int rc = clear_counts(c);
+		if (rc)
+			return rc;
+		c->counts_follow_vox = true; // from the ballot below on
 		// the terms (rates, volume in; three rows out) only after new agent data
 		a.terms = c->terms_dirty ? 1 : 0;
 		if (c->timing && !c->h_words && !(c->h_words = pinned_words_get()))
 			return fail(PCG_ERR_NOMEM, "pinned host memory for the device words");
-		const int rc = run_ballot<T>(c, a, c->stream, c->sm_count);
+		rc = run_ballot<T>(c, a, c->stream, c->sm_count);
 		if (rc)
 			return rc;
 		c->terms_dirty = false;
@@ -594,8 +576,8 @@ int launch_cells_fp32_buffers(const CellStepBuffers& b, cudaStream_t stream)
 	a.vec = rows_vectorizable(a, sizeof(float));
 	a.terms = 1;
 	a.pairs = 0; // the caller's FP64 amounts
-	a.rank = b.rank;
-	a.sorted = b.sorted;
+	a.sums = b.sums;
+	a.joined = 0;
 	a.list_word = 2;
 	set_fast_locate(a);
 	const uint64_t V = b.n[0] * b.n[1] * b.n[2];

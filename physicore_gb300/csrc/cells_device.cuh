@@ -50,9 +50,8 @@ struct CellArgs
 	uint32_t* counts;
 	uint8_t* role;    // [A] ballot role
 	uint32_t* shared; // [A] agents of voxels that hold several, flags[list_word] of them
-	uint32_t* flags;  // [0] conflict; entries of `shared` in word list_word; grouped ballot: [2..4]
-	uint32_t list_word; // 1 (batches: per-warp ballot) or 2 (grouped ballot: words 2, 3 = list, slots;
-	                    // 4 = writers)
+	uint32_t* flags;  // [0] conflict; entries of `shared` in word list_word; [3] writers
+	uint32_t list_word; // 1 (batches: per-warp ballot) or 2 (single domain; word 3 = writers)
 	uint32_t* err;
 	void* field;
 	int internalized;
@@ -61,15 +60,12 @@ struct CellArgs
 	int terms; // recompute the agent terms (their rates or volumes changed), not only positions
 	// fast voxel location (locate): bbmin and 1/voxel as floats; fast == 0 when the
 	// mesh's bounds or voxel edges are not exactly representable in FP32
-	float mf[3], rf[3];
+	float mf[3], rf[3], nf[3]; // nf: grid sides
 	int fast;
-	// voxel-grouped ballot (cells.cu): rank of each agent in its voxel, and the
-	// agents of shared voxels grouped by voxel (slot order)
-	uint32_t* rank;   // [A]
-	uint2* sorted;    // [A] (agent, voxel) pairs
-	// a context's grouped ballot (null for caller-owned buffers): the agents that
-	// write a voxel, flags[4] of them, in agent order (apply walks them instead of
-	// every agent)
+	uint32_t* sums; // [A], single domain: the row that holds a shared voxel's sums, at its winner
+	int joined;     // num, den and fac of an agent are one row of ts values (so are the sums)
+	// a context's own (null for caller-owned buffers): the agents that write a voxel,
+	// flags[3] of them, in agent order (apply walks them instead of every agent)
 	uint32_t* writers;
 };
 
@@ -86,6 +82,7 @@ inline void set_fast_locate(CellArgs& a)
 			a.fast = 0;
 		a.mf[d] = (float)m;
 		a.rf[d] = (float)(1.0 / h);
+		a.nf[d] = (float)a.n[d];
 	}
 }
 
@@ -102,47 +99,66 @@ inline int rows_vectorizable(const CellArgs& a, size_t wsize)
 		   al(a.den) && al(a.fac) && al(a.rnum) && al(a.rden) && al(a.rfac);
 }
 
+// float(p) by truncation, with integer operations: a conversion from FP64 takes the
+// FP64 pipe, which 4M agents' coordinates kept busy for longer than their loads take
+// (dense workload: 70 -> 30 us).  Values below the normal FP32 range become 0; false
+// above it and for NaN.
+__device__ __forceinline__ bool float_trunc(double p, float& f)
+{
+	const uint32_t hi = (uint32_t)__double2hiint(p), lo = (uint32_t)__double2loint(p);
+	const uint32_t mag = hi & 0x7fffffffu;
+	const uint32_t m = mag < (897u << 20) ? 0u : ((mag - (896u << 20)) << 3) | (lo >> 29);
+	f = __uint_as_float((hi & 0x80000000u) | m);
+	return mag < (1151u << 20);
+}
+
 // cartesian_mesh::voxel_position (mesh.cpp:37-61): idx = trunc(q) with the FP64
 // quotient q = (p - bbmin) / voxel, outside the grid when !(q >= 0) or q >= n;
 // false when outside.  The result is exactly the FP64 expression's, but the
 // division (a long sequence on this GPU's slow FP64 pipe) runs only near a voxel
-// boundary: qf = (float(p) - float(bbmin)) * float(1/voxel) is within
-// 2^-24 (3|q| + |p|/voxel) of q (one rounding each of p, the difference, the
-// reciprocal and the product; bbmin and voxel are exact as floats), so when qf
-// lies more than 2^-21 (|qf| + |p|/voxel) + 2^-40 from every integer, q lies
-// strictly inside the same unit interval and trunc(q), and the bounds test, are
+// boundary: qf = (pf - float(bbmin)) * float(1/voxel), pf = p truncated to FP32, is
+// within 2^-24 (3|q| + 2|p|/voxel) of q (2^-23 for p, one rounding each of the
+// difference, the reciprocal and the product; bbmin and voxel are exact as floats),
+// so when qf lies more than 2^-21 (|qf| + |pf|/voxel) + 2^-40 from every integer, q
+// lies strictly inside the same unit interval and trunc(q), and the bounds test, are
 // decided by qf.  Otherwise (and for NaN or huge positions) the FP64 division
-// decides.
-__device__ __forceinline__ bool locate_exact_axis(const CellArgs& a, double p, int d, uint64_t& idx)
+// decides.  fast: grids of at most 2^22 voxels a side.
+__device__ __forceinline__ bool locate_exact_axis(const CellArgs& a, double p, int d, uint32_t& idx)
 {
 	const double q = (p - a.bbmin[d]) / a.voxel[d];
 	if (!(q >= 0.0) || q >= (double)a.n[d])
 		return false;
-	idx = (uint64_t)q;
+	idx = (uint32_t)q;
 	return true;
 }
 
-__device__ __forceinline__ bool locate(const CellArgs& a, uint64_t i, uint64_t idx[3])
+__device__ __forceinline__ bool locate(const CellArgs& a, uint64_t i, uint32_t idx[3])
 {
 	idx[0] = idx[1] = idx[2] = 0;
-	for (int d = 0; d < a.dims; d++)
+	double p[3];
+#pragma unroll
+	for (int d = 0; d < 3; d++)
+		p[d] = d < a.dims ? a.pos[i * a.dims + d] : 0.0;
+#pragma unroll
+	for (int d = 0; d < 3; d++)
 	{
-		const double p = a.pos[i * a.dims + d];
-		if (a.fast)
+		if (d >= a.dims)
+			break;
+		float pf;
+		if (a.fast && float_trunc(p[d], pf))
 		{
-			const float pf = (float)p;
 			const float qf = __fmul_rn(__fsub_rn(pf, a.mf[d]), a.rf[d]);
 			const float fl = floorf(qf);
 			const float tol = fmaf(fabsf(qf) + fabsf(pf) * a.rf[d], 4.76837158e-7f, 9.09494702e-13f); // 2^-21, 2^-40
 			if (qf - fl > tol && (fl + 1.0f) - qf > tol)
 			{
-				if (fl < 0.0f || fl >= (float)a.n[d])
+				if (fl < 0.0f || fl >= a.nf[d])
 					return false;
-				idx[d] = (uint64_t)fl;
+				idx[d] = (uint32_t)fl;
 				continue;
 			}
 		}
-		if (!locate_exact_axis(a, p, d, idx[d]))
+		if (!locate_exact_axis(a, p[d], d, idx[d]))
 			return false;
 	}
 	return true;
@@ -190,7 +206,7 @@ __device__ __forceinline__ void agent_terms(const CellArgs& a, uint64_t i)
 // the grid (a device error then); returns it.
 __device__ __forceinline__ uint32_t agent_place(const CellArgs& a, uint64_t i)
 {
-	uint64_t idx[3];
+	uint32_t idx[3];
 	if (!a.active[i])
 	{
 		a.vox[i] = kNoAgent;
@@ -202,9 +218,11 @@ __device__ __forceinline__ uint32_t agent_place(const CellArgs& a, uint64_t i)
 		a.vox[i] = kNoAgent;
 		return kNoAgent;
 	}
-	const uint32_t v = (uint32_t)(idx[0] + a.n[0] * (idx[1] + a.n[1] * idx[2]));
+	// meshes have fewer than 2^32 voxels, fields fewer than 2^32 elements
+	const uint32_t row = idx[2] * (uint32_t)a.n[1] + idx[1];
+	const uint32_t v = row * (uint32_t)a.n[0] + idx[0];
 	a.vox[i] = v;
-	a.foff[i] = (uint32_t)((idx[2] * a.n[1] + idx[1]) * a.pitch + idx[0] * a.S);
+	a.foff[i] = row * (uint32_t)a.pitch + idx[0] * (uint32_t)a.S;
 	return v;
 }
 
@@ -300,25 +318,21 @@ __device__ __forceinline__ void list_shared(const CellArgs& a, uint64_t i, bool 
 	a.shared[base + __popc(group & ((1u << lane) - 1))] = (uint32_t)i;
 }
 
-// ---- voxel-grouped ballot (single-domain contexts)
+// ---- ballot of a single domain
 //
-// The reference sums every agent's terms into its voxel's winner with atomics
-// (cell_solver.cpp:79-129).  When tens of agents share a voxel those atomics
-// serialise on the winner's row, so here the ballot groups the agents of shared
-// voxels by voxel instead and sums each group with a segmented warp reduction:
-//   place:     voxel of each agent; a count per voxel (one atomic per run of
-//              lanes in the voxel) whose returned offset gives the agent's rank
-//              in its voxel (rank 0, the agent whose atomic landed first, is the
-//              winner, as the first compare-and-swap wins in the reference)
-//   classify:  roles from count and rank; the agents of shared voxels are listed
-//              in agent order (for the internalized pass), so are the agents that
-//              write a voxel (for apply), and each winner reserves its voxel's
-//              group of slots
-//   group:     every agent of a shared voxel writes (index, voxel) into its
-//              voxel's group
-//   group sum: warps reduce consecutive slots by voxel; a group that lies within
-//              one warp is stored once, a group split across warps adds its parts
-//              to the winner's row (cleared by classify) with atomics
+// The reference sums every agent's terms into its voxel's winner one value at a
+// time (cell_solver.cpp:79-129).  Here:
+//   locate:  voxel of each agent
+//   ballot:  a count per voxel (one atomic per run of lanes in the voxel) whose
+//            returned offset ranks the agent in its voxel.  Rank 0, the agent whose
+//            atomic landed first, wins (as the first compare-and-swap wins in the
+//            reference); rank 1, which only a shared voxel has, lends its row to the
+//            voxel's sums and clears it
+//   group:   roles (a winner alone in its voxel or not); the agents of shared voxels
+//            are listed in agent order (for reduce and the internalized pass), so are
+//            the agents that write a voxel (for apply)
+//   reduce:  every agent of a shared voxel adds its terms to the voxel's row, four
+//            FP32 values per atomic
 
 // Runs of equal keys among the lanes of a warp: the first lane of the caller's run
 // and the first lane after it (32 at the end of the warp).  All lanes call it.
@@ -332,29 +346,43 @@ __device__ __forceinline__ void key_run(uint32_t key, uint32_t& first, uint32_t&
 	end = later ? __ffs(later) - 1 : 32;
 }
 
-// Counts agents i0 + 32 k into voxels v[k] (k < K) and records their ranks in
-// their voxels: one atomic per run of lanes with the same voxel (agents given in
-// voxel order share one; in random order each lane has its own, which costs less
-// than grouping the lanes by voxel); the K chunks' atomics are in flight together.
-// All lanes of the warp call it (v[k] = kNoAgent for none).
-template <int K>
-__device__ __forceinline__ void count_rank(const CellArgs& a, uint64_t i0, const uint32_t (&v)[K])
+// Counts agent i into voxel v (kNoAgent for none) and returns its rank there: one
+// atomic per run of lanes with the same voxel (agents given in voxel order share one;
+// in random order each lane has its own, which costs less than grouping the lanes by
+// voxel).  All lanes of the warp call it.
+__device__ __forceinline__ uint32_t count_rank(const CellArgs& a, uint32_t v)
 {
 	const uint32_t lane = threadIdx.x & 31;
-	uint32_t first[K], end[K], base[K];
-#pragma unroll
-	for (int k = 0; k < K; k++)
-		key_run(v[k], first[k], end[k]);
-#pragma unroll
-	for (int k = 0; k < K; k++)
-		base[k] = v[k] != kNoAgent && lane == first[k] ? atomicAdd(a.counts + v[k], end[k] - first[k]) : 0u;
-#pragma unroll
-	for (int k = 0; k < K; k++)
+	uint32_t first, end;
+	key_run(v, first, end);
+	const uint32_t base = v != kNoAgent && lane == first ? atomicAdd(a.counts + v, end - first) : 0u;
+	return __shfl_sync(0xffffffffu, base, first) + (lane - first);
+}
+
+__device__ __forceinline__ void red_add4(float* p, float4 v)
+{
+	asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
+				 : "memory");
+}
+
+// Adds `count` values to p, four at a time where both start on 16-byte boundaries and
+// count is a multiple of four (quads).
+__device__ __forceinline__ void add_values(float* p, const float* q, uint32_t count, bool quads)
+{
+	if (quads)
 	{
-		const uint32_t b = __shfl_sync(0xffffffffu, base[k], first[k]);
-		if (v[k] != kNoAgent)
-			a.rank[i0 + 32 * k] = b + (lane - first[k]);
+#pragma unroll 6
+		for (uint32_t k = 0; k < count; k += 4)
+			red_add4(p + k, __ldg(reinterpret_cast<const float4*>(q + k)));
 	}
+	else
+		for (uint32_t k = 0; k < count; k++)
+			atomicAdd(p + k, q[k]);
+}
+__device__ __forceinline__ void add_values(double* p, const double* q, uint32_t count, bool)
+{
+	for (uint32_t k = 0; k < count; k++)
+		atomicAdd(p + k, q[k]);
 }
 
 // Change of an internalized amount.  The FP64 build evaluates the reference's
@@ -501,6 +529,8 @@ __device__ __forceinline__ void agent_apply(const CellArgs& a, uint64_t i)
 {
 	const uint8_t role = a.role[i];
 	const uint32_t off = a.foff[i];
+	// a winner's sums: in its own row (batches), or the one its voxel was lent
+	const uint64_t lent = a.list_word == 1 ? i : (uint64_t)a.sums[i];
 	if (role == kRoleNone || role == kRoleLoser)
 		return;
 	const bool alone = role == kRoleAlone;
@@ -509,9 +539,10 @@ __device__ __forceinline__ void agent_apply(const CellArgs& a, uint64_t i)
 	const bool vec = a.vec;
 	const uint32_t S = SC ? (uint32_t)SC : (uint32_t)a.S; // SC: S fixed at compile time (1-8), else 0
 	T* __restrict__ D = static_cast<T*>(a.field) + off;
-	const T* __restrict__ rn = static_cast<const T*>(alone ? a.num : a.rnum) + i * a.ts;
-	const T* __restrict__ rd = static_cast<const T*>(alone ? a.den : a.rden) + i * a.ts;
-	const T* __restrict__ rf = static_cast<const T*>(alone ? a.fac : a.rfac) + i * a.ts;
+	const uint64_t row = (alone ? i : lent) * a.ts;
+	const T* __restrict__ rn = static_cast<const T*>(alone ? a.num : a.rnum) + row;
+	const T* __restrict__ rd = static_cast<const T*>(alone ? a.den : a.rden) + row;
+	const T* __restrict__ rf = static_cast<const T*>(alone ? a.fac : a.rfac) + row;
 	double* __restrict__ I = a.internal + i * S;
 	for (uint32_t s0 = 0; s0 < S; s0 += kSubBatch)
 	{

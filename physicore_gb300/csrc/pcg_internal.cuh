@@ -242,7 +242,7 @@ struct Context
 	uint32_t xy_nseg = 0, xy_total = 0, xy_nslab = 0;
 	DeviceBuffer xy_segs, xy_done;
 	DeviceBuffer flags;    // uint32 [8]: [0] ballot conflict, [1] agents in shared voxels (batches),
-	                       // [2..3] and [4] the grouped ballot's counts (cells_device.cuh)
+	                       // [2] and [3] a single domain's list lengths (cells_device.cuh)
 	DeviceBuffer mass;     // double [S]
 	// per-step mass check (pcg_set_mass_check): FP64 totals [2 * S] before the
 	// first sweep and after the last one, added by the sweeps themselves, and
@@ -298,18 +298,18 @@ struct Context
 	DeviceBuffer a_foff;                  // uint32 [A]: field offset of the voxel's first substrate
 	DeviceBuffer a_role;                  // uint8 [A]: ballot role (cells_device.cuh)
 	DeviceBuffer a_shared;                // uint32 [A]: agents of voxels that hold several
-	DeviceBuffer a_rank;                  // uint32 [A]: rank of the agent in its voxel
-	DeviceBuffer a_sorted;                // uint2 [A]: (agent, voxel) of shared voxels grouped by voxel
+	DeviceBuffer a_sums;                  // uint32 [A]: at the winner of a shared voxel, the row of its sums
 	DeviceBuffer a_writers;               // uint32 [A]: agents that write a voxel (alone or winner)
-	// the ballot behind the cached roles, lists and reduced rows: 0 none, 1 the
-	// grouped ballot of a single-domain step, 2 a batch's per-warp ballot (their
-	// lists and counts differ, so a step of the other kind rebuilds)
+	// the ballot behind the cached roles, lists and reduced rows: 0 none, 1 a
+	// single-domain step's, 2 a batch's per-warp ballot (their lists differ, so a step
+	// of the other kind rebuilds)
 	uint8_t ballot_kind = 0;
+	bool counts_follow_vox = false;       // counts are zero but for the voxels in a_vox
 	uint64_t term_stride = 0;             // values per agent row of a_terms and a_reduced
 	DeviceBuffer a_terms;                 // real [A][term_stride]: num, den, fac of the agent (S each)
-	DeviceBuffer a_reduced;               // real [A][term_stride]: a winner's sums over its voxel
-	DeviceBuffer owner;                   // uint32 [V]: winning agent per voxel (batches), or the first
-										  // slot of the voxel's group in a_sorted (single domain)
+	DeviceBuffer a_reduced;               // real [A][term_stride]: sums over a shared voxel
+	DeviceBuffer owner;                   // uint32 [V]: winning agent per voxel (batches), or the agent
+										  // whose row holds a shared voxel's sums (single domain)
 	DeviceBuffer counts;                  // uint32 [V]: active agents per voxel
 
 	// measurement
@@ -379,10 +379,8 @@ struct CellStepBuffers
 	double* internal;
 	int internalized;
 	float* field;
-	// scratch: vox/foff/shared/rank/role [A], sorted [A] pairs, owner/counts [V], flags/err [4] each,
-	// terms [A*S] each
-	uint32_t *vox, *foff, *shared, *rank, *owner, *counts, *flags, *err;
-	uint2* sorted;
+	// scratch: vox/foff/shared/sums/role [A], owner/counts [V], flags/err [4] each, terms [A*S] each
+	uint32_t *vox, *foff, *shared, *sums, *owner, *counts, *flags, *err;
 	uint8_t* role;
 	float *num, *den, *fac, *rnum, *rden, *rfac;
 };

@@ -53,4 +53,5 @@ def test_truncated_rule_agrees_with_fp64_division():
         assert np.array_equal(inside[decided], ref_inside[decided]), (bbmin, voxel, n)
         both = decided & ref_inside
         assert np.array_equal(fl.astype(np.float64)[both], ref_idx[both]), (bbmin, voxel, n)
-        assert decided[-200_007:-7].mean() > (0.99 if abs(bbmin) < 1e6 else 0.0), (bbmin, voxel, n)
+        if abs(bbmin) < 1e6:  # with |p| / voxel near 2^20 the error bound reaches 1/2: nothing is decided
+            assert decided[-200_007:-7].mean() > 0.99, (bbmin, voxel, n)

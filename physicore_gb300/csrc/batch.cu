@@ -113,7 +113,7 @@ struct BatchArgs
 	const BatchDomain* doms;
 	const CUtensorMap* tmaps; // [domain][2]: y, z
 	WorkList list;
-	uint32_t* counter;        // tile counter of this launch (zeroed at the start of every step)
+	uint32_t* counter;        // tile counter of this launch (two words, dev::leave)
 	uint32_t* err;            // [0] DEV_ERR_* bits, [1] lowest failing domain
 	const uint8_t* recompute; // per domain: rebuild the ballot this step
 	uint32_t* steps_left;     // per domain: steps still to run in this call (0: the domain sits out)
@@ -216,6 +216,7 @@ __global__ void __launch_bounds__(sweep_threads<T>(), sizeof(T) == 4 ? 16 : 5) b
 		dev::fence_mbar_init();
 	}
 	__syncthreads();
+	dev::pdl_wait();
 	uint32_t phase = 0;
 	Unit cur = resolve_unit(b.list, blockIdx.x);
 	while (cur.t < b.list.total)
@@ -310,6 +311,7 @@ __global__ void __launch_bounds__(sweep_threads<T>(), sizeof(T) == 4 ? 16 : 5) b
 	}
 	if (half == 0)
 		dev::bulk_wait_all();
+	dev::leave(b.counter);
 }
 
 struct FaceRef
@@ -341,6 +343,7 @@ __global__ void __launch_bounds__(sweep_threads<T>()) batch_sweep_yz_kernel(Batc
 		dev::fence_mbar_init();
 	}
 	__syncthreads();
+	dev::pdl_wait();
 	uint32_t phase = 0, prev = 0xffffffffu, bad = 0;
 	bool ok = true;
 	Unit cur = resolve_unit(b.list, blockIdx.x);
@@ -493,6 +496,7 @@ __global__ void __launch_bounds__(sweep_threads<T>()) batch_sweep_yz_kernel(Batc
 		report(b, DEV_ERR_WAIT_TIMEOUT, bad);
 	if (threadIdx.x == 0)
 		dev::bulk_wait_all();
+	dev::leave(b.counter);
 }
 
 // ------------------------------------------------------------------ Dirichlet, bulk
@@ -502,6 +506,7 @@ __global__ void __launch_bounds__(sweep_threads<T>()) batch_sweep_yz_kernel(Batc
 template <typename T>
 __global__ void batch_faces_kernel(BatchArgs b)
 {
+	dev::pdl_wait();
 	const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
 	const uint64_t w0 = blockIdx.x * (uint64_t)blockDim.x + (threadIdx.x & ~31u);
 	for (uint64_t wu = w0; wu < b.list.total; wu += stride)
@@ -516,6 +521,7 @@ __global__ void batch_faces_kernel(BatchArgs b)
 template <typename T>
 __global__ void batch_interior_kernel(BatchArgs b)
 {
+	dev::pdl_wait();
 	const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
 	const uint64_t w0 = blockIdx.x * (uint64_t)blockDim.x + (threadIdx.x & ~31u);
 	for (uint64_t wu = w0; wu < b.list.total; wu += stride)
@@ -535,6 +541,7 @@ __global__ void batch_interior_kernel(BatchArgs b)
 template <typename T>
 __global__ void batch_bulk_kernel(BatchArgs b)
 {
+	dev::pdl_wait();
 	const int lane = threadIdx.x & 31;
 	const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
 	const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
@@ -564,6 +571,7 @@ __global__ void batch_bulk_kernel(BatchArgs b)
 // kClearChunk voxels.
 __global__ void batch_clear_counts_kernel(BatchArgs b)
 {
+	dev::pdl_wait();
 	const int lane = threadIdx.x & 31;
 	const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
 	const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
@@ -585,6 +593,7 @@ __global__ void batch_clear_counts_kernel(BatchArgs b)
 template <typename T>
 __global__ void batch_cells_locate_kernel(BatchArgs b)
 {
+	dev::pdl_wait();
 	const uint64_t u = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
 	const uint32_t k = warp_entry(b.list, u);
 	if (u >= b.list.total)
@@ -602,6 +611,7 @@ __global__ void batch_cells_locate_kernel(BatchArgs b)
 // Lanes of a warp may hold agents of two domains: the match key carries the domain.
 __global__ void batch_cells_ballot_kernel(BatchArgs b)
 {
+	dev::pdl_wait();
 	const uint64_t u = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
 	uint64_t key = ~0ull;
 	uint32_t v = kNoAgent, di = 0;
@@ -633,6 +643,7 @@ __global__ void batch_cells_ballot_kernel(BatchArgs b)
 template <typename T>
 __global__ void batch_cells_reduce_kernel(BatchArgs b)
 {
+	dev::pdl_wait();
 	const uint64_t u = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
 	uint8_t role = kRoleNone;
 	uint32_t di = 0;
@@ -659,6 +670,7 @@ __global__ void batch_cells_reduce_kernel(BatchArgs b)
 template <typename T>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 1) batch_cells_apply_kernel(BatchArgs b)
 {
+	dev::pdl_wait();
 	const uint64_t u = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
 	const uint32_t k = warp_entry(b.list, u);
 	if (u >= b.list.total || !b.steps_left[__ldg(b.list.dom + k)])
@@ -669,6 +681,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 1) batch_cells_apply
 template <typename T>
 __global__ void batch_cells_internalize_kernel(BatchArgs b, const uint32_t* __restrict__ block0, uint32_t ndom)
 {
+	dev::pdl_wait();
 	// Work is the domains' lists of agents in shared voxels, whose lengths are on
 	// the device.  Domain d owns blocks [block0[d], block0[d+1]) (in proportion to
 	// its agents, set when the batch is built) and splits its list among them.
@@ -696,6 +709,7 @@ __global__ void batch_cells_internalize_kernel(BatchArgs b, const uint32_t* __re
 // after * factor = before, and its totals cleared for the next step.
 __global__ void batch_mass_finish_kernel(const BatchDomain* doms, const uint32_t* steps_left, uint32_t count)
 {
+	dev::pdl_wait();
 	for (uint32_t d = blockIdx.x; d < count; d += gridDim.x)
 	{
 		const BatchDomain& D = doms[d];
@@ -721,6 +735,7 @@ __global__ void batch_mass_finish_kernel(const BatchDomain* doms, const uint32_t
 __global__ void batch_shared_bytes_kernel(const BatchDomain* doms, const uint32_t* steps_left, uint32_t count,
 										  uint32_t wsize, double* out)
 {
+	dev::pdl_wait();
 	double acc = 0.0;
 	for (uint32_t d = threadIdx.x; d < count; d += blockDim.x)
 	{
@@ -746,6 +761,7 @@ __global__ void batch_shared_bytes_kernel(const BatchDomain* doms, const uint32_
 // End of a step: one step fewer for every domain still running.
 __global__ void batch_count_step_kernel(uint32_t* steps_left, uint32_t count)
 {
+	dev::pdl_wait();
 	for (uint32_t d = blockIdx.x * blockDim.x + threadIdx.x; d < count; d += gridDim.x * blockDim.x)
 		if (steps_left[d])
 			steps_left[d]--;
@@ -1422,7 +1438,7 @@ BatchArgs args_for(pcg_batch* b, int list, int counter)
 	a.doms = static_cast<const BatchDomain*>(b->d_doms.ptr);
 	a.tmaps = static_cast<const CUtensorMap*>(b->d_tmaps.ptr);
 	a.list = b->lists[list];
-	a.counter = static_cast<uint32_t*>(b->d_counters.ptr) + counter;
+	a.counter = static_cast<uint32_t*>(b->d_counters.ptr) + 2 * counter;
 	a.err = static_cast<uint32_t*>(b->d_err.ptr);
 	a.recompute = static_cast<const uint8_t*>(b->d_recompute.ptr);
 	a.steps_left = static_cast<uint32_t*>(b->d_steps_left.ptr);
@@ -1441,7 +1457,7 @@ template <typename T>
 int launch_sweep(pcg_batch* b, int axis, const BatchArgs& a, unsigned grid, uint64_t smem, double bytes)
 {
 	LaunchScope s(b, axis == 0 ? K_SWEEP_X : axis == 1 ? K_SWEEP_Y : K_SWEEP_Z, bytes);
-	sweep_kernel<T>(b, axis, b->any_mass_check)<<<grid, sweep_threads<T>(), smem, b->stream>>>(a);
+	PCG_CUDA_TRY(launch_chained(sweep_kernel<T>(b, axis, b->any_mass_check), grid, sweep_threads<T>(), smem, b->stream, a));
 	PCG_CUDA_TRY(cudaGetLastError());
 	return PCG_OK;
 }
@@ -1451,7 +1467,6 @@ template <typename T>
 int launch_step(pcg_batch* b)
 {
 	const double* sb = b->step_bytes;
-	PCG_CUDA_TRY(cudaMemsetAsync(b->d_counters.ptr, 0, 4 * sizeof(uint32_t), b->stream));
 	int rc;
 	for (int axis = 0; axis < 3; axis++)
 		if (b->lists[axis].total && (rc = launch_sweep<T>(b, axis, args_for(b, axis, axis), b->grid[axis],
@@ -1461,29 +1476,30 @@ int launch_step(pcg_batch* b)
 	{
 		LaunchScope s(b, K_MASS_CHECK, sb[K_MASS_CHECK]);
 		const uint32_t N = (uint32_t)b->ctx.size();
-		batch_mass_finish_kernel<<<std::min<uint32_t>(N, 1024), 32, 0, b->stream>>>(
-			static_cast<const BatchDomain*>(b->d_doms.ptr), static_cast<const uint32_t*>(b->d_steps_left.ptr), N);
+		PCG_CUDA_TRY(launch_chained(batch_mass_finish_kernel, std::min<uint32_t>(N, 1024), 32, 0, b->stream,
+									static_cast<const BatchDomain*>(b->d_doms.ptr),
+									static_cast<const uint32_t*>(b->d_steps_left.ptr), N));
 		PCG_CUDA_TRY(cudaGetLastError());
 	}
 	if (b->lists[L_FACES].total)
 	{
 		LaunchScope s(b, K_DIRICHLET_FACES, sb[K_DIRICHLET_FACES]);
-		batch_faces_kernel<T><<<flat_grid(b, b->lists[L_FACES].total, 256), 256, 0, b->stream>>>(
-			args_for(b, L_FACES, 3));
+		PCG_CUDA_TRY(launch_chained(batch_faces_kernel<T>, flat_grid(b, b->lists[L_FACES].total, 256), 256, 0, b->stream,
+									args_for(b, L_FACES, 3)));
 		PCG_CUDA_TRY(cudaGetLastError());
 	}
 	if (b->lists[L_INTERIOR].total)
 	{
 		LaunchScope s(b, K_DIRICHLET_INTERIOR, sb[K_DIRICHLET_INTERIOR]);
-		batch_interior_kernel<T><<<flat_grid(b, b->lists[L_INTERIOR].total, 256), 256, 0, b->stream>>>(
-			args_for(b, L_INTERIOR, 3));
+		PCG_CUDA_TRY(launch_chained(batch_interior_kernel<T>, flat_grid(b, b->lists[L_INTERIOR].total, 256), 256, 0, b->stream,
+									args_for(b, L_INTERIOR, 3)));
 		PCG_CUDA_TRY(cudaGetLastError());
 	}
 	if (b->lists[L_BULK].total)
 	{
 		LaunchScope s(b, K_BULK, sb[K_BULK]);
-		batch_bulk_kernel<T><<<flat_grid(b, b->lists[L_BULK].total * 32, 256), 256, 0, b->stream>>>(
-			args_for(b, L_BULK, 3));
+		PCG_CUDA_TRY(launch_chained(batch_bulk_kernel<T>, flat_grid(b, b->lists[L_BULK].total * 32, 256), 256, 0, b->stream,
+									args_for(b, L_BULK, 3)));
 		PCG_CUDA_TRY(cudaGetLastError());
 	}
 	const uint64_t A = b->lists[L_AGENTS].total;
@@ -1494,36 +1510,40 @@ int launch_step(pcg_batch* b)
 		{
 			{
 				LaunchScope s(b, K_CELLS_CLEAR, sb[K_CELLS_CLEAR]);
-				batch_clear_counts_kernel<<<flat_grid(b, b->lists[L_CLEAR].total * 32, 256), 256, 0, b->stream>>>(
-					args_for(b, L_CLEAR, 3));
+				PCG_CUDA_TRY(launch_chained(batch_clear_counts_kernel, flat_grid(b, b->lists[L_CLEAR].total * 32, 256),
+											256, 0, b->stream, args_for(b, L_CLEAR, 3)));
 				PCG_CUDA_TRY(cudaGetLastError());
 			}
 			{
 				LaunchScope s(b, K_CELLS_LOCATE, sb[K_CELLS_LOCATE]);
-				batch_cells_locate_kernel<T><<<g, 256, 0, b->stream>>>(args_for(b, L_AGENTS, 3));
+				PCG_CUDA_TRY(launch_chained(batch_cells_locate_kernel<T>, g, 256, 0, b->stream, args_for(b,
+											L_AGENTS, 3)));
 				PCG_CUDA_TRY(cudaGetLastError());
 			}
 			{
 				LaunchScope s(b, K_CELLS_BALLOT, sb[K_CELLS_BALLOT]);
-				batch_cells_ballot_kernel<<<g, 256, 0, b->stream>>>(args_for(b, L_AGENTS, 3));
+				PCG_CUDA_TRY(launch_chained(batch_cells_ballot_kernel, g, 256, 0, b->stream, args_for(b, L_AGENTS,
+											3)));
 				PCG_CUDA_TRY(cudaGetLastError());
 			}
 			{
 				LaunchScope s(b, K_CELLS_REDUCE, sb[K_CELLS_REDUCE]);
-				batch_cells_reduce_kernel<T><<<g, 256, 0, b->stream>>>(args_for(b, L_AGENTS, 3));
+				PCG_CUDA_TRY(launch_chained(batch_cells_reduce_kernel<T>, g, 256, 0, b->stream, args_for(b,
+											L_AGENTS, 3)));
 				PCG_CUDA_TRY(cudaGetLastError());
 			}
 		}
 		{
 			LaunchScope s(b, K_CELLS_APPLY, sb[K_CELLS_APPLY]);
-			batch_cells_apply_kernel<T><<<g, 256, 0, b->stream>>>(args_for(b, L_AGENTS, 3));
+			PCG_CUDA_TRY(launch_chained(batch_cells_apply_kernel<T>, g, 256, 0, b->stream, args_for(b, L_AGENTS, 3)));
 			PCG_CUDA_TRY(cudaGetLastError());
 		}
 		{
 			LaunchScope s(b, K_CELLS_INTERNALIZE, sb[K_CELLS_INTERNALIZE]);
 			const uint32_t ndom = (uint32_t)b->ctx.size();
-			batch_cells_internalize_kernel<T><<<std::max(b->internalize_blocks, 1u), 256, 0, b->stream>>>(
-				args_for(b, L_AGENTS, 3), static_cast<const uint32_t*>(b->d_iblocks.ptr), ndom);
+			PCG_CUDA_TRY(launch_chained(batch_cells_internalize_kernel<T>, std::max(b->internalize_blocks, 1u), 256, 0,
+										b->stream, args_for(b, L_AGENTS, 3),
+										static_cast<const uint32_t*>(b->d_iblocks.ptr), ndom));
 			PCG_CUDA_TRY(cudaGetLastError());
 		}
 		if (b->timing) // the internalize pass's bytes, once the lists' lengths are known
@@ -1535,15 +1555,17 @@ int launch_step(pcg_batch* b)
 			const int rc2 = balloc(b->d_shared_bytes, sizeof(double), b->stream, b->device);
 			if (rc2)
 				return rc2;
-			batch_shared_bytes_kernel<<<1, 256, 0, b->stream>>>(
-				static_cast<const BatchDomain*>(b->d_doms.ptr), static_cast<const uint32_t*>(b->d_steps_left.ptr),
-				(uint32_t)b->ctx.size(), (uint32_t)sizeof(T), static_cast<double*>(b->d_shared_bytes.ptr));
+			PCG_CUDA_TRY(launch_chained(batch_shared_bytes_kernel, 1, 256, 0, b->stream,
+										static_cast<const BatchDomain*>(b->d_doms.ptr),
+										static_cast<const uint32_t*>(b->d_steps_left.ptr), (uint32_t)b->ctx.size(),
+										(uint32_t)sizeof(T), static_cast<double*>(b->d_shared_bytes.ptr)));
 			PCG_CUDA_TRY(cudaMemcpyAsync(b->h_shared_bytes, b->d_shared_bytes.ptr, sizeof(double),
 										 cudaMemcpyDeviceToHost, b->stream));
 		}
 	}
 	const uint32_t N = (uint32_t)b->ctx.size();
-	batch_count_step_kernel<<<(N + 255) / 256, 256, 0, b->stream>>>(static_cast<uint32_t*>(b->d_steps_left.ptr), N);
+	PCG_CUDA_TRY(launch_chained(batch_count_step_kernel, (N + 255) / 256, 256, 0,
+								b->stream, static_cast<uint32_t*>(b->d_steps_left.ptr), N));
 	PCG_CUDA_TRY(cudaGetLastError());
 	return PCG_OK;
 }
@@ -1748,7 +1770,6 @@ int time_axis(pcg_batch* b, int axis, const std::vector<size_t>& subset, double*
 	{
 		if (r == warm)
 			cudaEventRecord(e0, b->stream);
-		cudaMemsetAsync(a.counter, 0, sizeof(uint32_t), b->stream);
 		rc = launch_sweep<T>(b, axis, a, grid, smem, 0);
 	}
 	b->timing = timing;
@@ -2024,6 +2045,7 @@ int pcg_batch_create(pcg_batch** out, pcg_context* const* contexts, uint64_t cou
 	b->h_steps_left.assign(count, 0);
 	const uint32_t reset[2] = { 0, 0xffffffffu };
 	if (cudaMemcpyAsync(b->d_err.ptr, reset, sizeof(reset), cudaMemcpyHostToDevice, b->stream) != cudaSuccess ||
+		cudaMemsetAsync(b->d_counters.ptr, 0, 16 * sizeof(uint32_t), b->stream) != cudaSuccess ||
 		pcg::batch_wait(b) != cudaSuccess)
 		return bail(fail(PCG_ERR_CUDA, "could not clear the batch error word"));
 	if ((rc = pcg::refresh(b)))

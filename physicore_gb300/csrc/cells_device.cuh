@@ -262,6 +262,32 @@ __device__ __forceinline__ void warp_ballot(const CellArgs* a, uint64_t i, uint3
 	}
 }
 
+__device__ __forceinline__ void red_add4(float* p, float4 v)
+{
+	asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
+				 : "memory");
+}
+
+// Adds `count` values to p, four at a time where both start on 16-byte boundaries and
+// count is a multiple of four (quads).
+__device__ __forceinline__ void add_values(float* p, const float* q, uint32_t count, bool quads)
+{
+	if (quads)
+	{
+#pragma unroll 6
+		for (uint32_t k = 0; k < count; k += 4)
+			red_add4(p + k, __ldg(reinterpret_cast<const float4*>(q + k)));
+	}
+	else
+		for (uint32_t k = 0; k < count; k++)
+			atomicAdd(p + k, q[k]);
+}
+__device__ __forceinline__ void add_values(double* p, const double* q, uint32_t count, bool)
+{
+	for (uint32_t k = 0; k < count; k++)
+		atomicAdd(p + k, q[k]);
+}
+
 // Sums into the winner's row (cell_solver.cpp:102-127) and records agent i's
 // role, which it returns (kRoleLoser: a ballot conflict).  An agent alone in its
 // voxel adds nothing: its sums would be its own terms (0 + x, exactly), which
@@ -290,6 +316,11 @@ __device__ __forceinline__ uint8_t agent_reduce(const CellArgs& a, uint64_t i)
 	T* rnum = static_cast<T*>(a.rnum);
 	T* rden = static_cast<T*>(a.rden);
 	T* rfac = static_cast<T*>(a.rfac);
+	if (sizeof(T) == 4 && a.joined)
+	{
+		add_values(rnum + (uint64_t)w * a.ts, num + i * a.ts, (uint32_t)a.ts, true);
+		return role;
+	}
 	for (uint64_t s = 0; s < a.S; s++)
 	{
 		const uint64_t k = i * a.ts + s;
@@ -357,32 +388,6 @@ __device__ __forceinline__ uint32_t count_rank(const CellArgs& a, uint32_t v)
 	key_run(v, first, end);
 	const uint32_t base = v != kNoAgent && lane == first ? atomicAdd(a.counts + v, end - first) : 0u;
 	return __shfl_sync(0xffffffffu, base, first) + (lane - first);
-}
-
-__device__ __forceinline__ void red_add4(float* p, float4 v)
-{
-	asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
-				 : "memory");
-}
-
-// Adds `count` values to p, four at a time where both start on 16-byte boundaries and
-// count is a multiple of four (quads).
-__device__ __forceinline__ void add_values(float* p, const float* q, uint32_t count, bool quads)
-{
-	if (quads)
-	{
-#pragma unroll 6
-		for (uint32_t k = 0; k < count; k += 4)
-			red_add4(p + k, __ldg(reinterpret_cast<const float4*>(q + k)));
-	}
-	else
-		for (uint32_t k = 0; k < count; k++)
-			atomicAdd(p + k, q[k]);
-}
-__device__ __forceinline__ void add_values(double* p, const double* q, uint32_t count, bool)
-{
-	for (uint32_t k = 0; k < count; k++)
-		atomicAdd(p + k, q[k]);
 }
 
 // Change of an internalized amount.  The FP64 build evaluates the reference's

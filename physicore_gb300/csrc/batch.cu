@@ -857,7 +857,7 @@ using pcg::DeviceBuffer;
 struct pcg_batch
 {
 	int device = 0;
-	uint32_t* h_words = nullptr; // pinned host words for reading the error words
+	uint32_t* h_words = nullptr; // pinned host words that kernels set: error bits, lowest failing domain
 	pcg::DeviceBuffer d_iblocks;   // internalize: first block of each domain [N + 1]
 	uint32_t internalize_blocks = 0;
 	cudaEvent_t ev_block = nullptr; // blocking-sync event for host waits on the stream
@@ -871,7 +871,7 @@ struct pcg_batch
 	std::vector<pcg::BatchDomain> h_doms;
 	std::vector<CUtensorMap> h_tmaps;
 	std::vector<pcg::AxisConfig> cfg[3];
-	DeviceBuffer d_doms, d_tmaps, d_lists, d_counters, d_err, d_recompute, d_steps_left;
+	DeviceBuffer d_doms, d_tmaps, d_lists, d_counters, d_recompute, d_steps_left;
 	std::vector<uint32_t> h_steps_left;
 	pcg::WorkList lists[pcg::L_COUNT] {};
 	uint64_t smem[3] = { 0, 0, 0 };
@@ -947,6 +947,9 @@ Context* C(pcg_batch* b, size_t d) { return static_cast<Context*>(b->ctx[d]); }
 // Host wait for the batch stream, asleep (see stream_wait in capi.cu).
 cudaError_t batch_wait(pcg_batch* b)
 {
+	const cudaError_t q = cudaStreamQuery(b->stream);
+	if (q != cudaErrorNotReady)
+		return q;
 	if (!b->ev_block)
 	{
 		cudaError_t e = cudaEventCreateWithFlags(&b->ev_block, cudaEventBlockingSync | cudaEventDisableTiming);
@@ -1013,7 +1016,7 @@ BatchDomain describe_domain(pcg_batch* b, size_t d)
 		D.bulk[k] = c->bulk[k].ptr;
 	D.dt = c->dt;
 	D.cells = make_cell_args(c);
-	D.cells.err = static_cast<uint32_t*>(b->d_err.ptr);
+	D.cells.err = b->h_words;
 	D.cells.list_word = 1; // the batch's per-warp ballot lists shared-voxel agents in word 1
 	if (c->mass_check && c->mc_tot.ptr && c->mc_out.ptr)
 	{
@@ -1439,7 +1442,7 @@ BatchArgs args_for(pcg_batch* b, int list, int counter)
 	a.tmaps = static_cast<const CUtensorMap*>(b->d_tmaps.ptr);
 	a.list = b->lists[list];
 	a.counter = static_cast<uint32_t*>(b->d_counters.ptr) + 2 * counter;
-	a.err = static_cast<uint32_t*>(b->d_err.ptr);
+	a.err = b->h_words;
 	a.recompute = static_cast<const uint8_t*>(b->d_recompute.ptr);
 	a.steps_left = static_cast<uint32_t*>(b->d_steps_left.ptr);
 	return a;
@@ -1720,16 +1723,12 @@ int check_batch(pcg_batch* b)
 	if (e != cudaSuccess)
 		return fail(PCG_ERR_CUDA, std::string("batch stream synchronise: ") + cudaGetErrorString(e));
 	collect(b);
-	if (!b->h_words && !(b->h_words = pinned_words_get()))
-		return fail(PCG_ERR_NOMEM, "pinned host memory for the batch error words");
-	PCG_CUDA_TRY(cudaMemcpyAsync(b->h_words, b->d_err.ptr, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, b->stream));
-	PCG_CUDA_TRY(pcg::batch_wait(b));
-	const uint32_t word[2] = { b->h_words[0], b->h_words[1] };
+	volatile uint32_t* err = b->h_words;
+	const uint32_t word[2] = { err[0], err[1] };
 	if (word[0])
 	{
-		uint32_t* d = static_cast<uint32_t*>(b->d_err.ptr);
-		PCG_CUDA_TRY(cudaMemsetAsync(d, 0, sizeof(uint32_t), b->stream));
-		PCG_CUDA_TRY(cudaMemsetAsync(d + 1, 0xff, sizeof(uint32_t), b->stream));
+		err[0] = 0;
+		err[1] = 0xffffffffu;
 		std::string msg = device_error_text(word[0]);
 		if (word[1] != 0xffffffffu)
 			msg += " (batch domain " + std::to_string(word[1]) + ")";
@@ -2038,16 +2037,17 @@ int pcg_batch_create(pcg_batch** out, pcg_context* const* contexts, uint64_t cou
 	b->h_recompute.assign(count, 0);
 	int rc;
 	if ((rc = pcg::balloc(b->d_counters, 16 * sizeof(uint32_t), b->stream, b->device)) ||
-		(rc = pcg::balloc(b->d_err, 2 * sizeof(uint32_t), b->stream, b->device)) ||
 		(rc = pcg::balloc(b->d_recompute, count, b->stream, b->device)) ||
 		(rc = pcg::balloc(b->d_steps_left, count * sizeof(uint32_t), b->stream, b->device)))
 		return bail(rc);
 	b->h_steps_left.assign(count, 0);
-	const uint32_t reset[2] = { 0, 0xffffffffu };
-	if (cudaMemcpyAsync(b->d_err.ptr, reset, sizeof(reset), cudaMemcpyHostToDevice, b->stream) != cudaSuccess ||
-		cudaMemsetAsync(b->d_counters.ptr, 0, 16 * sizeof(uint32_t), b->stream) != cudaSuccess ||
+	if (!(b->h_words = pcg::pinned_words_get()))
+		return bail(fail(PCG_ERR_NOMEM, "pinned host memory for the batch error words"));
+	b->h_words[0] = 0;
+	b->h_words[1] = 0xffffffffu;
+	if (cudaMemsetAsync(b->d_counters.ptr, 0, 16 * sizeof(uint32_t), b->stream) != cudaSuccess ||
 		pcg::batch_wait(b) != cudaSuccess)
-		return bail(fail(PCG_ERR_CUDA, "could not clear the batch error word"));
+		return bail(fail(PCG_ERR_CUDA, "could not clear the batch's tile counters"));
 	if ((rc = pcg::refresh(b)))
 		return bail(rc);
 	*out = b;
@@ -2066,7 +2066,7 @@ int pcg_batch_destroy(pcg_batch* b)
 	for (cudaEvent_t e : b->event_pool)
 		cudaEventDestroy(e);
 	DeviceBuffer* bufs[] = { &b->d_doms,	 &b->d_tmaps,	  &b->d_lists,		&b->d_counters,
-							 &b->d_err, &b->d_recompute, &b->d_steps_left, &b->d_iblocks, &b->d_shared_bytes };
+							 &b->d_recompute, &b->d_steps_left, &b->d_iblocks, &b->d_shared_bytes };
 	for (DeviceBuffer* x : bufs)
 		pcg::free_buf(*x);
 	if (b->ev_sync)

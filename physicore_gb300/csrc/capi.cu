@@ -140,8 +140,14 @@ void pinned_words_put(uint32_t* w)
 // the CUDA calls of other threads in the process -- a server's admissions and
 // steps -- while it waits, which can be milliseconds when the stream's kernels
 // queue behind other work on the SMs.
+//
+// An idle stream is recognised by a query: recording an event on it and sleeping until
+// it completes takes 20-40 us, several times in a call that reads results back.
 cudaError_t stream_wait(Context* c)
 {
+	const cudaError_t q = cudaStreamQuery(c->stream);
+	if (q != cudaErrorNotReady)
+		return q;
 	if (!c->ev_block)
 	{
 		cudaError_t e = cudaEventCreateWithFlags(&c->ev_block, cudaEventBlockingSync | cudaEventDisableTiming);
@@ -290,7 +296,6 @@ void collect_timings(Context* c)
 
 // ------------------------------------------------------------------ helpers
 
-// Reads and clears the device error word after synchronising the stream.
 std::string device_error_text(uint32_t word)
 {
 	std::string msg = "device fault:";
@@ -305,25 +310,22 @@ std::string device_error_text(uint32_t word)
 	return msg;
 }
 
+// Waits for the stream, then reads and clears the error word.  Kernels set its bits in
+// pinned host memory (an atomic over the link, only when something is wrong), so
+// reading it takes no copy and no second wait.
 static int check_device(Context* c)
 {
-	if (!c->err.ptr)
+	if (!c->h_words)
 		return PCG_OK; // nothing has run on the device yet
-	if (!c->h_words && !(c->h_words = pinned_words_get()))
-		return fail(PCG_ERR_NOMEM, "pinned host memory for the device error word");
-	// The copy is queued only once the stream is idle: a copy waiting in a copy
-	// engine's queue for kernels (which may wait for other work to leave the SMs)
-	// holds up the copies other threads queue behind it.
 	cudaError_t e = stream_wait(c);
 	if (e != cudaSuccess)
 		return fail(PCG_ERR_CUDA, std::string("stream synchronise: ") + cudaGetErrorString(e));
-	PCG_CUDA_TRY(cudaMemcpyAsync(c->h_words, c->err.ptr, sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream));
-	PCG_CUDA_TRY(stream_wait(c));
 	collect_timings(c);
-	const uint32_t word = c->h_words[0];
+	volatile uint32_t* err = c->h_words;
+	const uint32_t word = *err;
 	if (word)
 	{
-		PCG_CUDA_TRY(cudaMemsetAsync(c->err.ptr, 0, sizeof(uint32_t), c->stream));
+		*err = 0;
 		return fail(PCG_ERR_DEVICE, device_error_text(word));
 	}
 	return PCG_OK;
@@ -748,11 +750,15 @@ int ensure_device_state(Context* c, bool defer_clear = false)
 		if (!c->stream)
 			c->stream = c->own_stream;
 	}
-	if (!c->err.ptr)
+	if (!c->h_words)
 	{
-		int rc = dalloc(c, c->err, sizeof(uint32_t) * 4);
-		if (!rc)
-			rc = dalloc(c, c->flags, sizeof(uint32_t) * 8);
+		if (!(c->h_words = pinned_words_get()))
+			return fail(PCG_ERR_NOMEM, "pinned host memory for the device error word");
+		c->h_words[0] = 0;
+	}
+	if (!c->flags.ptr)
+	{
+		int rc = dalloc(c, c->flags, sizeof(uint32_t) * 8);
 		if (!rc)
 			rc = dalloc(c, c->tickets, sizeof(uint32_t) * 8);
 		if (rc)
@@ -761,7 +767,6 @@ int ensure_device_state(Context* c, bool defer_clear = false)
 	}
 	if (!c->words_cleared && !defer_clear)
 	{
-		PCG_CUDA_TRY(cudaMemsetAsync(c->err.ptr, 0, sizeof(uint32_t) * 4, c->stream));
 		PCG_CUDA_TRY(cudaMemsetAsync(c->flags.ptr, 0, sizeof(uint32_t) * 8, c->stream));
 		PCG_CUDA_TRY(cudaMemsetAsync(c->tickets.ptr, 0, sizeof(uint32_t) * 8, c->stream));
 		c->words_cleared = true;
@@ -1063,7 +1068,7 @@ int pcg_destroy(pcg_context* c)
 		cudaStreamSynchronize(c->rb_stream);
 	pcg::collect_timings(c);
 	pcg::DeviceBuffer* all[] = { &c->field,		 &c->coef[0],	&c->coef[1],	&c->coef[2],	 &c->a_vox,
-								 &c->err,		&c->flags,		 &c->mass,		&c->tickets,
+								 &c->flags,		 &c->mass,		&c->tickets,
 								 &c->staging,	 &c->dir_offsets, &c->dir_values, &c->dir_conds, &c->face_values,
 								 &c->face_conds, &c->bulk[0],	&c->bulk[1],	&c->bulk[2],	 &c->a_pos,
 								 &c->a_sec,		 &c->a_sat,		&c->a_upt,		&c->a_net,		 &c->a_vol,
@@ -1761,8 +1766,6 @@ int pcg_set_kernel_timing(pcg_context* c, int enable)
 	if (c->timing && c->initialized && c->A && c->ballot_kind == 1 && c->flags.ptr)
 	{
 		pcg::DeviceGuard g(c->device);
-		if (!c->h_words && !(c->h_words = pcg::pinned_words_get()))
-			return fail(PCG_ERR_NOMEM, "pinned host memory for the device words");
 		PCG_CUDA_TRY(stream_wait(c));
 		PCG_CUDA_TRY(cudaMemcpy(c->h_words + 2, static_cast<uint32_t*>(c->flags.ptr) + 2, sizeof(uint32_t),
 								cudaMemcpyDeviceToHost));

@@ -409,7 +409,7 @@ CellArgs make_cell_args(const Context* c)
 	a.role = static_cast<uint8_t*>(c->a_role.ptr);
 	a.shared = static_cast<uint32_t*>(c->a_shared.ptr);
 	a.flags = static_cast<uint32_t*>(c->flags.ptr);
-	a.err = static_cast<uint32_t*>(c->err.ptr);
+	a.err = c->h_words;
 	a.field = c->field.ptr;
 	a.internalized = c->compute_internalized ? 1 : 0;
 	a.vec = rows_vectorizable(a, c->wsize);
@@ -456,7 +456,7 @@ static int run_ballot(Context* c, const CellArgs& a, cudaStream_t stream, int sm
 	if (c)
 		launch_begin(c, K_CELLS_GROUP, 2 * A, &ev);
 	PCG_CUDA_TRY(launch_chained(wide ? cells_group_kernel<8> : cells_group_kernel<4>, ggrid, kGroupBlock, 0, stream, a));
-	if (c && c->timing && c->h_words) // list lengths for the per-agent byte counts
+	if (c && c->timing) // list lengths for the per-agent byte counts
 	{
 		PCG_CUDA_TRY(
 			cudaMemcpyAsync(c->h_words + 2, a.flags + a.list_word, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
@@ -511,8 +511,6 @@ static int run_cells(Context* c, bool recompute)
 		c->counts_follow_vox = true; // from the ballot below on
 		// the terms (rates, volume in; three rows out) only after new agent data
 		a.terms = c->terms_dirty ? 1 : 0;
-		if (c->timing && !c->h_words && !(c->h_words = pinned_words_get()))
-			return fail(PCG_ERR_NOMEM, "pinned host memory for the device words");
 		rc = run_ballot<T>(c, a, c->stream, c->sm_count);
 		if (rc)
 			return rc;

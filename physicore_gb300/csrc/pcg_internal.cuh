@@ -150,11 +150,8 @@ int dalloc(Context* c, DeviceBuffer& b, size_t bytes);
 // bytes that pool holds free for reuse.
 cudaError_t pool_alloc(void** ptr, size_t bytes, cudaStream_t stream, int device);
 uint64_t pool_idle_bytes(int device);
-// Four pinned host words (capi.cu) for small device-to-host reads (error words):
-// a copy into pinned memory is a plain DMA, whereas a synchronous copy into
-// pageable memory goes through driver staging shared by every thread and, queued
-// behind other copies, stalls the transfers of all of them.  Null when pinned
-// memory cannot be had.
+// Four pinned host words (capi.cu) that kernels and small copies write: error words,
+// counts.  Null when pinned memory cannot be had.
 uint32_t* pinned_words_get();
 void pinned_words_put(uint32_t* w);
 // Host wait for the context's stream, asleep rather than spinning (capi.cu).
@@ -202,7 +199,7 @@ struct Context
 	bool initialized = false;
 	bool recompute_cells = true;
 	bool terms_dirty = true; // agent rates or volumes uploaded since the agent terms were computed
-	bool words_cleared = false; // err/flags words zeroed on the device
+	bool words_cleared = false; // flags and tile counters zeroed on the device
 	// bumped by every call that may reallocate a device buffer or change a
 	// parameter; batches compare it with the value they captured
 	uint64_t generation = 0;
@@ -222,8 +219,7 @@ struct Context
 	// context cost milliseconds once many contexts come and go, as under a server)
 	DeviceBuffer slab;
 	size_t slab_used = 0;
-	DeviceBuffer err;      // uint32 device error word
-	uint32_t* h_words = nullptr; // pinned host words for reading it
+	uint32_t* h_words = nullptr; // pinned host words: [0] the error word that kernels set, [2..3] timing counts
 	cudaEvent_t ev_block = nullptr; // blocking-sync event for host waits on the stream
 	DeviceBuffer tickets;  // uint32 [8]: tile counters of the persistent sweeps, two words each ([6]: fused x/y)
 	// CTAs per SM of the sweep kernels last launched on each axis ([3]: fused x/y)

@@ -545,7 +545,7 @@ SweepArgs base_args(const Context* c, int axis)
 	a.row_len = c->row_len;
 	a.pitch = c->pitch;
 	a.rows = c->rows;
-	a.err = static_cast<uint32_t*>(c->err.ptr);
+	a.err = c->h_words;
 	a.ticket = static_cast<uint32_t*>(c->tickets.ptr) + 2 * axis;
 	a.nx = (uint32_t)c->n[0], a.ny = (uint32_t)c->n[1], a.nz = (uint32_t)c->n[2];
 	if (c->wsize == 8)

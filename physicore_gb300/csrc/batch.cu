@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(sweep_threads<T>(), sizeof(T) == 4 ? 16 : 5) b
 	{
 		uint32_t drawn = 0;
 		if (threadIdx.x == 0)
-			drawn = gridDim.x + atomicAdd(b.counter, 1u); // the following tile's ticket, in flight meanwhile
+			drawn = dev::next_ticket(b.counter); // the following tile's ticket, in flight meanwhile
 		const uint32_t di = unit_domain(b.list, cur);
 		if (b.steps_left[di] == 0)
 		{
@@ -351,7 +351,7 @@ __global__ void __launch_bounds__(sweep_threads<T>()) batch_sweep_yz_kernel(Batc
 	{
 		uint32_t drawn = 0;
 		if (threadIdx.x == 0)
-			drawn = gridDim.x + atomicAdd(b.counter, 1u); // the following unit's ticket, in flight meanwhile
+			drawn = dev::next_ticket(b.counter); // the following unit's ticket, in flight meanwhile
 		const uint32_t di = unit_domain(b.list, cur);
 		if (b.steps_left[di] == 0)
 		{

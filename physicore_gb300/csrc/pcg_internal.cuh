@@ -111,7 +111,7 @@ struct SweepArgs
 	uint64_t smem_pitch;  // shared-memory row pitch (elements)
 	uint32_t rows_per_tile;
 	uint32_t* err;
-	uint32_t* ticket; // tile counter of the launch (two words, dev::leave), tiles handed out in order
+	uint32_t* ticket; // tile counter of the launch (two words, dev::leave), tiles handed out in order; null: a CTA per tile
 	// FP64 sweeps that scale their results: this axis's factors ([S] converged, then
 	// per point: axis 0 at [x*S + s], the others at [s*n + i]) and, at the last sweep
 	// of a step, the per-point factors of axis 0 and axis 1 (null when there are none)
@@ -550,13 +550,20 @@ __device__ __forceinline__ void fence_proxy_async_smem()
 // without, 90 with a trigger at each kernel's start, 72 at its end).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// The next tile of a persistent CTA (its first is blockIdx.x; one thread draws), or
+// none in a launch with a CTA per tile (no counter).
+__device__ __forceinline__ uint32_t next_ticket(uint32_t* counter)
+{
+	return counter ? gridDim.x + atomicAdd(counter, 1u) : 0xffffffffu;
+}
+
 // The end of a persistent launch: the last CTA to leave clears the tile counter
 // (counter[0]; counter[1] counts the CTAs that left and wraps to 0 by itself), so
 // that launches need no clearing operation before them.  Every CTA has drawn its
 // last ticket by then.
 __device__ __forceinline__ void leave(uint32_t* counter)
 {
-	if (threadIdx.x == 0 && atomicInc(counter + 1, gridDim.x - 1) == gridDim.x - 1)
+	if (counter && threadIdx.x == 0 && atomicInc(counter + 1, gridDim.x - 1) == gridDim.x - 1)
 		counter[0] = 0;
 }
 

@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(sweep_threads<T>()) sweep_yz_kernel(SweepArgs 
 				else
 					dev::tma_load_3d(base + c * chunk_elems, &tmap, (int)x0, (int)o, (int)(c * R), full);
 			}
-			drawn = gridDim.x + atomicAdd(a.ticket, 1u);
+			drawn = dev::next_ticket(a.ticket);
 		}
 		// lanes past the row hold zero-filled columns that are never stored
 		const uint32_t col = x0 + lane;
@@ -211,7 +211,7 @@ __global__ void __launch_bounds__(sweep_threads<T>()) sweep_x_kernel(SweepArgs a
 			if (lane < nrows)
 				dev::bulk_g2s(tile + lane * pitch, g + lane * a.pitch, row_bytes, bar);
 			if (lane == 0)
-				drawn = gridDim.x + atomicAdd(a.ticket, 1u);
+				drawn = dev::next_ticket(a.ticket);
 		}
 		ok = __syncthreads_and(dev::mbar_wait(bar, phase));
 		if (!ok)
@@ -514,9 +514,8 @@ Plan plan(const Context* c, int axis)
 	return p;
 }
 
-// CTAs of a persistent sweep launch: every one the device holds at once, at most
-// one per tile.
-int persistent_grid(Context* c, int slot, const void* kernel, int threads, uint64_t smem, uint64_t tiles, uint64_t* grid)
+// CTAs of a kernel that an SM holds at once.
+int resident_ctas(Context* c, int slot, const void* kernel, int threads, uint64_t smem, uint64_t* per_sm)
 {
 	Context::Resident& r = c->resident[slot];
 	if (r.kernel != kernel || r.smem != smem)
@@ -524,13 +523,34 @@ int persistent_grid(Context* c, int slot, const void* kernel, int threads, uint6
 		const int rc = allow_smem(kernel, c->device);
 		if (rc)
 			return rc;
-		int per_sm = 0;
-		PCG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
-		if (per_sm < 1)
+		int n = 0;
+		PCG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, smem));
+		if (n < 1)
 			return fail(PCG_ERR_UNSUPPORTED, "sweep tile does not fit in shared memory");
-		r = { kernel, smem, per_sm };
+		r = { kernel, smem, n };
 	}
-	*grid = std::min<uint64_t>((uint64_t)r.per_sm * (uint64_t)c->sm_count, tiles);
+	*per_sm = (uint64_t)r.per_sm;
+	return PCG_OK;
+}
+
+// The grid of a sweep.  Up to two tiles per resident CTA and 16 per SM: a CTA for each
+// tile and no counter, whose atomics on one address (two per CTA) take longer than
+// the hardware's hand-over of CTAs (steps of sweeps alone, 64^3 x 4: 17.1 -> 15.0 us;
+// 240x230x152 x 1, 1.1 waves: 48.3 -> 39.5; but 160x160x320 x 2, 2.1 waves: 69.6 ->
+// 73.7, and 40x40x200 x 20, 33 small tiles per SM: 39.0 -> 40.5).  Beyond that
+// persistent CTAs draw their tiles, so that a tile's load starts as soon as the last
+// one's stores have read shared memory.
+int sweep_grid(Context* c, int axis, const void* kernel, int threads, uint64_t smem, SweepArgs& a, uint64_t* grid)
+{
+	uint64_t per_sm = 0;
+	const int rc = resident_ctas(c, axis, kernel, threads, smem, &per_sm);
+	if (rc)
+		return rc;
+	const uint64_t sms = (uint64_t)c->sm_count, resident = per_sm * sms;
+	const bool direct = a.tiles <= 2 * resident && a.tiles <= 16 * sms;
+	if (direct)
+		a.ticket = nullptr;
+	*grid = direct ? a.tiles : std::min(resident, a.tiles);
 	return PCG_OK;
 }
 
@@ -614,7 +634,7 @@ int run_sweep_x(Context* c, bool mass_check)
 	const XKernel kernel = x_kernel<T>(c, mass_check);
 	uint64_t grid;
 	int rc;
-	if ((rc = persistent_grid(c, 0, reinterpret_cast<const void*>(kernel), sweep_threads<T>(), p.smem, a.tiles, &grid)))
+	if ((rc = sweep_grid(c, 0, reinterpret_cast<const void*>(kernel), sweep_threads<T>(), p.smem, a, &grid)))
 		return rc;
 	cudaEvent_t ev;
 	launch_begin(c, K_SWEEP_X, 2.0 * (double)(c->V * c->S) * (double)sizeof(T), &ev);
@@ -663,10 +683,11 @@ int run_sweep_xy(Context* c, bool mass_check)
 		default: return mc ? sweep_xy_kernel<T, 0, kMcIn> : sweep_xy_kernel<T, 0, 0>;
 		}
 	}();
-	uint64_t resident;
+	uint64_t per_sm = 0;
 	int rc;
-	if ((rc = persistent_grid(c, 3, reinterpret_cast<const void*>(kernel), sweep_threads<T>(), smem, ~0ull, &resident)))
+	if ((rc = resident_ctas(c, 3, reinterpret_cast<const void*>(kernel), sweep_threads<T>(), smem, &per_sm)))
 		return rc;
+	const uint64_t resident = per_sm * (uint64_t)c->sm_count;
 	// the lag must exceed the tiles in flight (about one per resident CTA), else y
 	// tiles are handed out while their slab's x tiles are still being solved
 	const uint64_t slab_tiles = (P * ny + R - 1) / R + P * ay.xblocks;
@@ -767,7 +788,7 @@ int run_sweep_yz(Context* c, int axis, bool fuse_faces, bool mass_check)
 	auto kernel = axis == 1 ? yz_kernel<T, 1>(scale, mass_check) : yz_kernel<T, 2>(scale, mass_check);
 	uint64_t grid;
 	int rc;
-	if ((rc = persistent_grid(c, axis, reinterpret_cast<const void*>(kernel), sweep_threads<T>(), p.smem, a.tiles, &grid)))
+	if ((rc = sweep_grid(c, axis, reinterpret_cast<const void*>(kernel), sweep_threads<T>(), p.smem, a, &grid)))
 		return rc;
 	cudaEvent_t ev;
 	launch_begin(c, kid, bytes, &ev);

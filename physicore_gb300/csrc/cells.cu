@@ -35,46 +35,43 @@ namespace {
 
 using namespace cellsdev;
 
-// clear: the counts of the last ballot, before the voxels that it recorded are
-// overwritten.  With BY_AGENT only the voxels that held an agent are written: the
-// counts are zero everywhere else.  One scattered word per agent (a 32-byte sector
-// each) against the whole array: the launcher takes the agents when they are fewer
-// than one per 16 voxels (320x320x256, 200,000 agents: 5.9 us, against 16 for the
-// array's 105 MB at the copy bandwidth; 200^3, 4M agents: the array, 7 us).
-template <bool BY_AGENT>
-__global__ void cells_clear_kernel(uint32_t* counts, const uint32_t* vox, uint64_t n)
+// How locate clears the counts for the ballot after it.
+enum : int
 {
-	dev::pdl_wait();
-	const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-	if constexpr (BY_AGENT)
-	{
-		if (i < n && vox[i] != kNoAgent)
-			counts[vox[i]] = 0;
-	}
-	else // n counts, four to a thread (the array starts on a 16-byte boundary)
-	{
-		const uint64_t k = 4 * i;
-		if (k + 4 <= n)
-			*reinterpret_cast<uint4*>(counts + k) = make_uint4(0, 0, 0, 0);
-		else
-			for (uint64_t q = k; q < n; q++)
-				counts[q] = 0;
-	}
-}
+	kClearNone = 0,    // they hold zeros already
+	kClearByAgent = 1, // over the voxels that the last ballot recorded: zero everywhere else
+	kClearArray = 2,   // every count, four to a thread (threads beyond the agents too)
+};
 
-// locate: terms (after new agent data) and voxel; the step's words (conflict flag,
-// list lengths) start at zero.
+// locate: terms (after new agent data) and voxel of each agent; the step's words
+// (conflict flag, list lengths) and the counts start at zero.  Clearing by agent
+// writes one scattered word per agent (a 32-byte sector each); the launcher takes it
+// when agents are fewer than one per 16 voxels (320x320x256, 200,000 agents: 6 us as a
+// kernel of its own, against 16 for the array's 105 MB at the copy bandwidth).
 template <typename T>
-__global__ void cells_locate_kernel(CellArgs a)
+__global__ void cells_locate_kernel(CellArgs a, int clear, uint64_t V)
 {
 	dev::pdl_wait();
 	const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
 	if (i == 0)
-	{
 		a.flags[0] = a.flags[1] = a.flags[2] = a.flags[3] = 0;
+	if (clear == kClearArray)
+	{
+		const uint64_t k = 4 * i; // the array starts on a 16-byte boundary
+		if (k + 4 <= V)
+			*reinterpret_cast<uint4*>(a.counts + k) = make_uint4(0, 0, 0, 0);
+		else
+			for (uint64_t q = k; q < V; q++)
+				a.counts[q] = 0;
 	}
 	if (i >= a.A)
 		return;
+	if (clear == kClearByAgent)
+	{
+		const uint32_t old = a.vox[i];
+		if (old != kNoAgent)
+			a.counts[old] = 0;
+	}
 	if (a.terms)
 		agent_terms<T>(a, i);
 	agent_place(a, i);
@@ -426,9 +423,9 @@ CellArgs make_cell_args(const Context* c)
 } // namespace cellsdev
 
 // The ballot of a single domain (cells_device.cuh) on `stream`; launch bookkeeping
-// through `c` when given.  The counts hold zeros already.
+// through `c` when given.  `clear` (kClear*): what is left of the counts of V voxels.
 template <typename T>
-static int run_ballot(Context* c, const CellArgs& a, cudaStream_t stream, int sm_count)
+static int run_ballot(Context* c, const CellArgs& a, int clear, uint64_t V, cudaStream_t stream, int sm_count)
 {
 	const unsigned block = 256;
 	const unsigned grid = (unsigned)((a.A + block - 1) / block);
@@ -439,10 +436,14 @@ static int run_ballot(Context* c, const CellArgs& a, cudaStream_t stream, int sm
 	const unsigned lgrid = std::min<unsigned>(grid, 24 * std::max(sm_count, 1));
 	const double S = (double)a.S, A = (double)a.A, w = (double)sizeof(T);
 	cudaEvent_t ev = nullptr;
+	const uint64_t threads = clear == kClearArray ? std::max<uint64_t>(a.A, (V + 3) / 4) : a.A;
 	if (c)
-		launch_begin(c, K_CELLS_LOCATE, A * (8.0 * a.dims + 1 + 4 + 4) + (a.terms ? A * (5 * S * 8 + 8 + 3 * S * w) : 0),
+		launch_begin(c, K_CELLS_LOCATE,
+					 A * (8.0 * a.dims + 1 + 4 + 4) + (a.terms ? A * (5 * S * 8 + 8 + 3 * S * w) : 0) +
+						 (clear == kClearByAgent ? 8 * A : clear == kClearArray ? 4.0 * (double)V : 0.0),
 					 &ev);
-	PCG_CUDA_TRY(launch_chained(cells_locate_kernel<T>, grid, block, 0, stream, a));
+	PCG_CUDA_TRY(launch_chained(cells_locate_kernel<T>, (unsigned)((threads + block - 1) / block), block, 0, stream, a, clear,
+								V));
 	if (c)
 		launch_end(c, K_CELLS_LOCATE, ev);
 	// voxel in, role out, one count updated
@@ -473,22 +474,6 @@ static int run_ballot(Context* c, const CellArgs& a, cudaStream_t stream, int sm
 	return PCG_OK;
 }
 
-// Zeroes the counts: over the voxels that the last ballot counted agents in, or the
-// whole array.
-static int clear_counts(Context* c)
-{
-	const bool by_agent = c->counts_follow_vox && c->A * 16 < c->V;
-	const uint64_t threads = by_agent ? c->A : (c->V + 3) / 4;
-	uint32_t* counts = static_cast<uint32_t*>(c->counts.ptr);
-	cudaEvent_t ev;
-	launch_begin(c, K_CELLS_CLEAR, by_agent ? 8.0 * (double)c->A : 4.0 * (double)c->V, &ev);
-	PCG_CUDA_TRY(launch_chained(by_agent ? cells_clear_kernel<true> : cells_clear_kernel<false>,
-								(unsigned)((threads + 255) / 256), 256, 0, c->stream, counts,
-								static_cast<const uint32_t*>(c->a_vox.ptr), by_agent ? c->A : c->V));
-	launch_end(c, K_CELLS_CLEAR, ev);
-	return PCG_OK;
-}
-
 template <typename T>
 static int run_cells(Context* c, bool recompute)
 {
@@ -505,13 +490,11 @@ static int run_cells(Context* c, bool recompute)
 		recompute = true;
 	if (recompute)
 	{
-		int rc = clear_counts(c);
-		if (rc)
-			return rc;
+		const int clear = c->counts_follow_vox && c->A * 16 < c->V ? kClearByAgent : kClearArray;
 		c->counts_follow_vox = true; // from the ballot below on
 		// the terms (rates, volume in; three rows out) only after new agent data
 		a.terms = c->terms_dirty ? 1 : 0;
-		rc = run_ballot<T>(c, a, c->stream, c->sm_count);
+		const int rc = run_ballot<T>(c, a, clear, c->V, c->stream, c->sm_count);
 		if (rc)
 			return rc;
 		c->terms_dirty = false;
@@ -549,8 +532,7 @@ int launch_cells(Context* c, bool recompute)
 	return c->wsize == 4 ? run_cells<float>(c, recompute) : run_cells<double>(c, recompute);
 }
 
-// The same kernels over caller-owned buffers: the counts are cleared here, the
-// conflict flag, ballot slots and reduced terms by the locate kernel.
+// The same kernels over caller-owned buffers.
 int launch_cells_fp32_buffers(const CellStepBuffers& b, cudaStream_t stream)
 {
 	if (b.A == 0)
@@ -608,8 +590,7 @@ int launch_cells_fp32_buffers(const CellStepBuffers& b, cudaStream_t stream)
 	if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev) !=
 												   cudaSuccess)
 		sm_count = 0;
-	PCG_CUDA_TRY(cudaMemsetAsync(b.counts, 0, V * sizeof(uint32_t), stream));
-	int rc = run_ballot<float>(nullptr, a, stream, sm_count);
+	int rc = run_ballot<float>(nullptr, a, kClearArray, V, stream, sm_count);
 	if (rc)
 		return rc;
 	PCG_CUDA_TRY(launch_chained(cells_apply_kernel<float>, grid, block, 0, stream, a));

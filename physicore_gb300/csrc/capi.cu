@@ -689,6 +689,8 @@ static int run_phases(Context* c, uint32_t phases, bool recompute)
 	// outputs (before writing any face), so the check reads no extra field pass.
 	const bool check = c->mass_check && (phases & PCG_PHASE_DIFFUSION);
 	const bool fuse = (phases & PCG_PHASE_DIFFUSION) && (phases & PCG_PHASE_DIRICHLET) && faces_fusable(c);
+	// and with bulk in the call too, it may apply the bulk update after the faces
+	const bool bulk = fuse && (phases & PCG_PHASE_BULK) && bulk_fusable(c);
 	if (phases & PCG_PHASE_DIFFUSION)
 	{
 		if (xy_fusable(c))
@@ -700,18 +702,18 @@ static int run_phases(Context* c, uint32_t phases, bool recompute)
 		{
 			if ((rc = launch_sweep_x(c, check)))
 				return rc;
-			if (c->dims >= 2 && (rc = launch_sweep_yz(c, 1, fuse && c->dims == 2, check && c->dims == 2)))
+			if (c->dims >= 2 && (rc = launch_sweep_yz(c, 1, fuse && c->dims == 2, bulk && c->dims == 2, check && c->dims == 2)))
 				return rc;
 		}
-		if (c->dims >= 3 && (rc = launch_sweep_yz(c, 2, fuse, check)))
+		if (c->dims >= 3 && (rc = launch_sweep_yz(c, 2, fuse, bulk, check)))
 			return rc;
 		if (check && (rc = launch_mass_check_finish(c)))
 			return rc;
 		c->mass_checked_steps += check;
 	}
-	if ((phases & PCG_PHASE_DIRICHLET) && (rc = launch_dirichlet(c, fuse)))
+	if ((phases & PCG_PHASE_DIRICHLET) && (rc = launch_dirichlet(c, fuse, bulk)))
 		return rc;
-	if ((phases & PCG_PHASE_BULK) && (rc = launch_bulk(c)))
+	if ((phases & PCG_PHASE_BULK) && !bulk && (rc = launch_bulk(c)))
 		return rc;
 	if ((phases & PCG_PHASE_CELLS) && (rc = launch_cells(c, recompute)))
 		return rc;

@@ -113,7 +113,8 @@ __device__ __forceinline__ T bulk_value(T D, T Sr, T U, T Tt, T dt)
 		return D + fmaf(-D, b, a) / (T(1) + b);
 	}
 	else
-		return (D + dt * Sr * Tt) / (T(1) + dt * (U + Sr));
+		// fused by name: where the products are hoisted out of a loop the compiler would not
+		return fma(dt * Sr, Tt, D) / fma(dt, U + Sr, T(1));
 }
 
 // The 16-byte chunk c of row r (fields and per-voxel tables have the same layout, and
@@ -205,6 +206,19 @@ __device__ __forceinline__ void faces_on_half(const ARGS& f, uint32_t x, uint32_
 		col[0] = vals[f_swept * S + s];
 	if (last && ((f.face_mask >> (f_swept + 1)) & 1u) && f.face_conds[(f_swept + 1) * S + s])
 		col[(len - 1) * stride] = vals[(f_swept + 1) * S + s];
+}
+
+// The bulk update, with uniform rates, of `len` points of substrate s of a column in
+// shared memory, `stride` apart.
+template <typename T>
+__device__ __forceinline__ void bulk_on_half(const void* const* tables, T dt, uint32_t s, T* col, uint32_t len,
+											 uint32_t stride)
+{
+	const T Sr = __ldg(static_cast<const T*>(tables[0]) + s), U = __ldg(static_cast<const T*>(tables[1]) + s),
+			Tt = __ldg(static_cast<const T*>(tables[2]) + s);
+#pragma unroll 4
+	for (uint32_t j = 0; j < len; j++)
+		col[j * stride] = bulk_value(col[j * stride], Sr, U, Tt, dt);
 }
 
 } // namespace fielddev

@@ -18,16 +18,24 @@ __global__ void dirichlet_faces_kernel(FaceArgs a)
 		fielddev::face_item<T>(a, idx);
 }
 
+// With bulk rates (the last sweep applied the bulk update to the field already) a node
+// gets its value's update, as the bulk pass after it would leave it.
 template <typename T>
 __global__ void dirichlet_interior_kernel(T* field, const uint64_t* offsets, const T* values, const uint8_t* conds,
-										  uint64_t K, uint64_t S)
+										  uint64_t K, uint64_t S, const T* supply, const T* uptake,
+										  const T* target, T dt)
 {
 	dev::pdl_wait();
 	for (uint64_t idx = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; idx < K * S;
 		 idx += (uint64_t)gridDim.x * blockDim.x)
 	{
-		if (conds[idx])
-			field[offsets[idx / S] + idx % S] = values[idx];
+		if (!conds[idx])
+			continue;
+		const uint64_t s = idx % S;
+		T v = values[idx];
+		if (supply)
+			v = fielddev::bulk_value(v, supply[s], uptake[s], target[s], dt);
+		field[offsets[idx / S] + s] = v;
 	}
 }
 
@@ -162,7 +170,7 @@ unsigned grid_for(const Context* c, uint64_t work, unsigned block)
 } // namespace
 
 template <typename T>
-static int run_dirichlet(Context* c, bool faces_done)
+static int run_dirichlet(Context* c, bool faces_done, bool bulk_done)
 {
 	const FaceArgs a = make_face_args(c);
 	if (a.face_mask && !faces_done)
@@ -180,16 +188,19 @@ static int run_dirichlet(Context* c, bool faces_done)
 		PCG_CUDA_TRY(launch_chained(dirichlet_interior_kernel<T>, grid_for(c, c->K * c->S, 256), 256, 0, c->stream,
 									static_cast<T*>(c->field.ptr), static_cast<const uint64_t*>(c->dir_offsets.ptr),
 									static_cast<const T*>(c->dir_values.ptr),
-									static_cast<const uint8_t*>(c->dir_conds.ptr), c->K, c->S));
+									static_cast<const uint8_t*>(c->dir_conds.ptr), c->K, c->S,
+									static_cast<const T*>(bulk_done ? c->bulk[0].ptr : nullptr),
+									static_cast<const T*>(c->bulk[1].ptr), static_cast<const T*>(c->bulk[2].ptr),
+									(T)c->dt));
 		launch_end(c, K_DIRICHLET_INTERIOR, ev);
 		PCG_CUDA_TRY(cudaGetLastError());
 	}
 	return PCG_OK;
 }
 
-int launch_dirichlet(Context* c, bool faces_done)
+int launch_dirichlet(Context* c, bool faces_done, bool bulk_done)
 {
-	return c->wsize == 4 ? run_dirichlet<float>(c, faces_done) : run_dirichlet<double>(c, faces_done);
+	return c->wsize == 4 ? run_dirichlet<float>(c, faces_done, bulk_done) : run_dirichlet<double>(c, faces_done, bulk_done);
 }
 
 template <typename T>

@@ -125,6 +125,10 @@ struct SweepArgs
 	const uint8_t* face_conds;
 	uint32_t face_mask;
 	uint32_t nx, ny, nz;
+	// y/z, last sweep of a step that also applies Dirichlet and uniform bulk rates: the
+	// bulk update of each solved tile after its faces (null tables when not fused)
+	const void* bulk[3];
+	double dt;
 	// mass check (kernels instantiated with it): FP64 totals [before S | after S];
 	// the x sweep adds its inputs, the last sweep its outputs (x as well when the
 	// mesh is 1-D)
@@ -341,11 +345,15 @@ int launch_sweep_x(Context* c, bool mass_check = false);
 // x and y sweeps of a 3-D mesh fused slab by slab (sweeps.cu), when xy_fusable
 bool xy_fusable(const Context* c);
 int launch_sweep_xy(Context* c, bool mass_check = false);
-int launch_sweep_yz(Context* c, int axis, bool fuse_faces = false, bool mass_check = false);
-// Dirichlet faces (unless the last sweep already wrote them) and interior nodes
-int launch_dirichlet(Context* c, bool faces_done = false);
+int launch_sweep_yz(Context* c, int axis, bool fuse_faces = false, bool fuse_bulk = false, bool mass_check = false);
+// Dirichlet faces (unless the last sweep already wrote them) and interior nodes; with
+// bulk_done the last sweep has applied the bulk update as well, and the nodes get
+// their values' bulk update
+int launch_dirichlet(Context* c, bool faces_done = false, bool bulk_done = false);
 // true when the last sweep of c can apply the boundary faces itself
 bool faces_fusable(const Context* c);
+// and, with it, the bulk update
+bool bulk_fusable(const Context* c);
 int launch_bulk(Context* c);
 int launch_cells(Context* c, bool recompute);
 int launch_release(Context* c, uint64_t agent);

@@ -42,8 +42,9 @@ using namespace solvers;
 // The y/z sweep.  A tile is 32 consecutive (x,s) elements at all n points of the
 // lines of one outer index; it arrives as nc TMA tensor boxes (32, R) of the field
 // described as the 3-D tensor (x*S+s, y, z), all completing on one mbarrier.  The
-// CTA solves its lines in place and one thread stores it back with nc box stores; the next tile's loads start once the stores have read
-// shared memory.  Loads and compute overlap across the CTAs an SM holds.
+// CTA solves its lines in place and one thread stores it back with nc box stores; the next
+// tile's loads start once the stores have read shared memory.  Loads and compute overlap
+// across the CTAs an SM holds.
 // Coefficients come from the axis's table (head rows, then per-substrate
 // constants), so most points need no coefficient load at all.
 //
@@ -53,7 +54,8 @@ using namespace solvers;
 // their solved values before the faces are written, into a.mc_tot[S + s].  A
 // lane's substrate is the same in every tile when S divides 32 (it then keeps one
 // running total and adds it once at the end), else it adds its total per tile.
-template <typename T, int AXIS, int MC, int SC>
+// BULK (the step's last sweep where bulk_fusable): the bulk update after the faces.
+template <typename T, int AXIS, int MC, int SC, bool BULK>
 __global__ void __launch_bounds__(sweep_threads<T>()) sweep_yz_kernel(SweepArgs a, const __grid_constant__ CUtensorMap tmap)
 {
 	extern __shared__ __align__(128) unsigned char smem[];
@@ -124,11 +126,14 @@ __global__ void __launch_bounds__(sweep_threads<T>()) sweep_yz_kernel(SweepArgs 
 				flush_classes(acc.value(), classes, kLanes, a.mc_tot + S + col % S);
 				acc.zero();
 			}
-		if (a.face_mask && in_row)
+		if ((BULK || a.face_mask) && in_row)
 		{
+			T* mine = half == 0 ? base + lane : base + m * kLanes + lane;
 			const uint32_t len = half == 0 ? m : n - m;
-			fielddev::faces_on_half<T, AXIS>(a, col / S, s, o, half == 0 ? base + lane : base + m * kLanes + lane, len,
-											 kLanes, half == 0, half == 0 ? n == m : n > m);
+			if (a.face_mask)
+				fielddev::faces_on_half<T, AXIS>(a, col / S, s, o, mine, len, kLanes, half == 0, half == 0 ? n == m : n > m);
+			if constexpr (BULK)
+				fielddev::bulk_on_half<T>(a.bulk, (T)a.dt, s, mine, len, kLanes);
 		}
 		if (threadIdx.x == 0)
 			next = drawn;
@@ -752,16 +757,18 @@ int run_sweep_xy(Context* c, bool mass_check)
 
 // FP64: `scale` when the sweep applies the scale factors (the last one always does).
 template <typename T, int AXIS>
-auto yz_kernel(bool scale, bool mass_check) -> void (*)(SweepArgs, const CUtensorMap)
+auto yz_kernel(bool scale, bool bulk, bool mass_check) -> void (*)(SweepArgs, const CUtensorMap)
 {
 	constexpr int SC = sizeof(T) == 8;
 	if (mass_check)
-		return sweep_yz_kernel<T, AXIS, kMcOut, SC>;
-	return scale ? sweep_yz_kernel<T, AXIS, 0, SC> : sweep_yz_kernel<T, AXIS, 0, 0>;
+		return bulk ? sweep_yz_kernel<T, AXIS, kMcOut, SC, true> : sweep_yz_kernel<T, AXIS, kMcOut, SC, false>;
+	if (bulk)
+		return sweep_yz_kernel<T, AXIS, 0, SC, true>;
+	return scale ? sweep_yz_kernel<T, AXIS, 0, SC, false> : sweep_yz_kernel<T, AXIS, 0, 0, false>;
 }
 
 template <typename T>
-int run_sweep_yz(Context* c, int axis, bool fuse_faces, bool mass_check)
+int run_sweep_yz(Context* c, int axis, bool fuse_faces, bool fuse_bulk, bool mass_check)
 {
 	SweepArgs a = base_args(c, axis);
 	if (mass_check)
@@ -772,6 +779,12 @@ int run_sweep_yz(Context* c, int axis, bool fuse_faces, bool mass_check)
 		a.face_values = f.values;
 		a.face_conds = f.conds;
 		a.face_mask = f.face_mask;
+	}
+	if (fuse_bulk)
+	{
+		for (int k = 0; k < 3; k++)
+			a.bulk[k] = c->bulk[k].ptr;
+		a.dt = c->dt;
 	}
 	a.xblocks = (c->row_len + kLanes - 1) / kLanes;
 	a.tiles = a.xblocks * (axis == 1 ? c->n[2] : c->n[1]);
@@ -785,7 +798,8 @@ int run_sweep_yz(Context* c, int axis, bool fuse_faces, bool mass_check)
 	const int kid = axis == 1 ? K_SWEEP_Y : K_SWEEP_Z;
 	const double bytes = 2.0 * (double)(c->V * c->S) * (double)sizeof(T);
 	const bool scale = axis == c->dims - 1 || !c->defer_scale;
-	auto kernel = axis == 1 ? yz_kernel<T, 1>(scale, mass_check) : yz_kernel<T, 2>(scale, mass_check);
+	auto kernel = axis == 1 ? yz_kernel<T, 1>(scale, fuse_bulk, mass_check)
+							: yz_kernel<T, 2>(scale, fuse_bulk, mass_check);
 	uint64_t grid;
 	int rc;
 	if ((rc = sweep_grid(c, axis, reinterpret_cast<const void*>(kernel), sweep_threads<T>(), p.smem, a, &grid)))
@@ -910,12 +924,25 @@ int launch_sweep_xy(Context* c, bool mass_check)
 	return c->wsize == 4 ? run_sweep_xy<float>(c, mass_check) : run_sweep_xy<double>(c, mass_check);
 }
 
-int launch_sweep_yz(Context* c, int axis, bool fuse_faces, bool mass_check)
+int launch_sweep_yz(Context* c, int axis, bool fuse_faces, bool fuse_bulk, bool mass_check)
 {
-	return c->wsize == 4 ? run_sweep_yz<float>(c, axis, fuse_faces, mass_check)
-						 : run_sweep_yz<double>(c, axis, fuse_faces, mass_check);
+	return c->wsize == 4 ? run_sweep_yz<float>(c, axis, fuse_faces, fuse_bulk, mass_check)
+						 : run_sweep_yz<double>(c, axis, fuse_faces, fuse_bulk, mass_check);
 }
 
 bool faces_fusable(const Context* c) { return c->dims >= 2; }
+
+// Uniform bulk rates in the last sweep's tiles save a pass over the field, but its
+// warps are few: with at least three tiles per SM they hide the work (97x131x61 x 5:
+// 30.3 -> 26.1 us a step of sweeps and bulk, 64^3 x 4, 512 tiles: 17.4 both, FP64 55 ->
+// 51), with fewer they do not (100^3 x 1, 400 tiles: 17.5 -> 19.1; 1000x800 x 3, 94:
+// 32 -> 60).  Per-voxel tables measured slower fused at every size (200x200x150 x 4:
+// 167 -> 213).  A kernel of its own: a test of the tables in one kernel for both cost
+// the sweeps without bulk 2 % (96x80x64 x 20: 68.1 -> 69.5).
+bool bulk_fusable(const Context* c)
+{
+	const uint64_t xblocks = (c->row_len + kLanes - 1) / kLanes, outer = c->dims == 2 ? 1 : c->n[1];
+	return c->bulk_mode == PCG_BULK_UNIFORM && faces_fusable(c) && xblocks * outer >= 3 * (uint64_t)c->sm_count;
+}
 
 } // namespace pcg

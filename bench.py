@@ -641,7 +641,7 @@ def run_fp64(args, w, local, det):
 
 
 def run_s1(args, local, det):
-    """One substrate at 320^3 in FP32 (x sweep on its row-per-thread path, y/z tiles
+    """One substrate at 320^3 in FP32 (x sweep with 16-byte row access, y/z tiles
     of 32 voxels): per-kernel device times and achieved bandwidth."""
     import physicore_gb300 as pcg
     from physicore_gb300 import workloads as W

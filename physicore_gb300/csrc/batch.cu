@@ -26,9 +26,8 @@
 // Autotuner: per sweep axis and size bucket (line length rounded up to 16, and
 // for x the substrate count) candidate mappings are timed on the batch's own
 // domains (fields saved and restored) and the fastest is kept for the process.
-//   x:   row-per-thread (a lane owns a row and solves its substrates one after
-//        another) or substrate-per-thread (S lanes share a row, one line each), times
-//        rows per tile;
+//   x:   rows per tile (S lanes share a row, one line each; a row per lane only by
+//        pcg_batch_force_config);
 //   y/z: points per TMA chunk (how early a line's solve can start vs. how many
 //        copies a tile takes).
 #include <algorithm>
@@ -177,17 +176,32 @@ __device__ __forceinline__ Unit resolve_unit(const WorkList& l, uint32_t t)
 // The domain of a unit inside the list.
 __device__ __forceinline__ uint32_t unit_domain(const WorkList& l, const Unit& u) { return __ldg(l.dom + u.k); }
 
-// Draws the next unit (warp 0; all its lanes call it) and leaves it in *slot; `di` is
-// the current unit's domain.
-__device__ __forceinline__ void draw_unit(const BatchArgs& b, uint32_t drawn, uint32_t di, Unit* slot)
+// Draws the next unit (warp 0; all its lanes call it) and returns it with its domain
+// *dom, leaving it in *slot for a second warp; `di` is the current unit's domain.  A
+// sweep of one warp (FP32) takes both from registers: through shared memory and with the
+// domain read again at the unit's start x took 749 instead of 731 us and z 775 instead of
+// 748 on 256 domains.
+template <typename T>
+__device__ __forceinline__ Unit draw_unit(const BatchArgs& b, uint32_t drawn, uint32_t di, Unit* slot, uint32_t* dom)
 {
 	const uint32_t lane = threadIdx.x & 31;
 	const Unit u = resolve_unit(b.list, __shfl_sync(0xffffffffu, drawn, 0));
-	const uint32_t dn = unit_domain(b.list, u);
+	const uint32_t dn = *dom = unit_domain(b.list, u);
 	if (dn != di && lane * 128 < sizeof(BatchDomain))
 		asm volatile("prefetch.global.L1 [%0];" ::"l"(reinterpret_cast<const char*>(b.doms + dn) + lane * 128));
-	if (lane == 0)
+	if (sweep_threads<T>() > 32 && lane == 0)
 		*slot = u;
+	return u;
+}
+
+// All threads' `ok`, a barrier of the sweep's CTA with it (one warp in FP32).
+template <typename T>
+__device__ __forceinline__ bool sweep_all(bool ok)
+{
+	if constexpr (sweep_threads<T>() == 32)
+		return __all_sync(0xffffffffu, ok);
+	else
+		return __syncthreads_and(ok);
 }
 
 // x: a tile is x_rows whole rows of one domain, bulk-copied into shared memory.
@@ -219,19 +233,23 @@ __global__ void __launch_bounds__(sweep_threads<T>(), sizeof(T) == 4 ? 16 : 5) b
 	dev::pdl_wait();
 	uint32_t phase = 0;
 	Unit cur = resolve_unit(b.list, blockIdx.x);
+	uint32_t dom = cur.t < b.list.total ? unit_domain(b.list, cur) : 0;
 	while (cur.t < b.list.total)
 	{
 		uint32_t drawn = 0;
 		if (threadIdx.x == 0)
 			drawn = dev::next_ticket(b.counter); // the following tile's ticket, in flight meanwhile
-		const uint32_t di = unit_domain(b.list, cur);
+		const uint32_t di = sweep_threads<T>() > 32 ? unit_domain(b.list, cur) : dom;
 		if (b.steps_left[di] == 0)
 		{
 			if (half == 0)
-				draw_unit(b, drawn, di, &next);
-			__syncthreads();
-			cur = next;
-			__syncthreads();
+				cur = draw_unit<T>(b, drawn, di, &next, &dom);
+			if (sweep_threads<T>() > 32)
+			{
+				__syncthreads();
+				cur = next;
+				__syncthreads();
+			}
 			continue;
 		}
 		const BatchDomain& D = b.doms[di];
@@ -241,6 +259,7 @@ __global__ void __launch_bounds__(sweep_threads<T>(), sizeof(T) == 4 ? 16 : 5) b
 		const uint32_t row_bytes = (uint32_t)round_up(D.row_len * sizeof(T), 16);
 		const uint32_t spitch = (uint32_t)D.x_smem_pitch;
 		T* g = static_cast<T*>(D.field) + r0 * D.pitch;
+		Unit drawn_unit {};
 		if (half == 0)
 		{
 			if (lane == 0)
@@ -248,7 +267,7 @@ __global__ void __launch_bounds__(sweep_threads<T>(), sizeof(T) == 4 ? 16 : 5) b
 			__syncwarp();
 			if (lane < nrows)
 				dev::bulk_g2s(tile + lane * spitch, g + lane * D.pitch, row_bytes, bar);
-			draw_unit(b, drawn, di, &next);
+			drawn_unit = draw_unit<T>(b, drawn, di, &next, &dom);
 		}
 		const T* tab = static_cast<const T*>(D.tab[0]);
 		const uint32_t head = D.head[0];
@@ -257,7 +276,7 @@ __global__ void __launch_bounds__(sweep_threads<T>(), sizeof(T) == 4 ? 16 : 5) b
 		const uint32_t s0 = by_row ? 0 : (wide ? lane : lane % S), s_step = by_row ? 1 : kLanes;
 		// the first lines' coefficient loads overlap the tile's arrival
 		LineCoef<T> L = line_coef(tab, S, head, n, MULTI ? min(s0, S - 1) : s0, half);
-		if (!__syncthreads_and(dev::mbar_wait(bar, phase)))
+		if (!sweep_all<T>(dev::mbar_wait(bar, phase)))
 		{
 			if (threadIdx.x == 0)
 				report(b, DEV_ERR_WAIT_TIMEOUT, di);
@@ -296,7 +315,7 @@ __global__ void __launch_bounds__(sweep_threads<T>(), sizeof(T) == 4 ? 16 : 5) b
 						flush_classes(ao.value(), stride, kLanes, mc + S + s);
 				}
 		}
-		cur = next;
+		cur = sweep_threads<T>() > 32 ? next : drawn_unit;
 		dev::fence_proxy_async_smem();
 		__syncthreads();
 		if (half == 0)
@@ -347,19 +366,23 @@ __global__ void __launch_bounds__(sweep_threads<T>()) batch_sweep_yz_kernel(Batc
 	uint32_t phase = 0, prev = 0xffffffffu, bad = 0;
 	bool ok = true;
 	Unit cur = resolve_unit(b.list, blockIdx.x);
+	uint32_t dom = cur.t < b.list.total ? unit_domain(b.list, cur) : 0;
 	while (cur.t < b.list.total)
 	{
 		uint32_t drawn = 0;
 		if (threadIdx.x == 0)
 			drawn = dev::next_ticket(b.counter); // the following unit's ticket, in flight meanwhile
-		const uint32_t di = unit_domain(b.list, cur);
+		const uint32_t di = sweep_threads<T>() > 32 ? unit_domain(b.list, cur) : dom;
 		if (b.steps_left[di] == 0)
 		{
 			if (half == 0)
-				draw_unit(b, drawn, di, &next);
-			__syncthreads();
-			cur = next;
-			__syncthreads();
+				cur = draw_unit<T>(b, drawn, di, &next, &dom);
+			if (sweep_threads<T>() > 32)
+			{
+				__syncthreads();
+				cur = next;
+				__syncthreads();
+			}
 			continue;
 		}
 		const BatchDomain& D = b.doms[di];
@@ -404,10 +427,11 @@ __global__ void __launch_bounds__(sweep_threads<T>()) batch_sweep_yz_kernel(Batc
 			}
 		}
 		prev = di;
+		Unit drawn_unit {};
 		if (half == 0)
 		{
 			__syncwarp();
-			draw_unit(b, drawn, di, &next);
+			drawn_unit = draw_unit<T>(b, drawn, di, &next, &dom);
 		}
 		const T* tab = static_cast<const T*>(D.tab[AXIS]);
 		const uint32_t head = D.head[AXIS], row_len = (uint32_t)D.row_len;
@@ -415,14 +439,14 @@ __global__ void __launch_bounds__(sweep_threads<T>()) batch_sweep_yz_kernel(Batc
 		uint32_t xb = xb0, o = ob0;
 		uint32_t col = xb * kLanes + lane;
 		LineCoef<T> L = line_coef(tab, S, head, n, col < row_len ? col % S : 0, half);
-		ok = __syncthreads_and(dev::mbar_wait(full, phase));
+		ok = sweep_all<T>(dev::mbar_wait(full, phase));
 		if (!ok)
 		{
 			bad = di;
 			break;
 		}
 		phase ^= 1;
-		cur = next;
+		cur = sweep_threads<T>() > 32 ? next : drawn_unit;
 		for (uint32_t j = 0; j < gcount; j++)
 		{
 			if (j)

@@ -69,7 +69,7 @@ __global__ void cells_locate_kernel(CellArgs a, int clear, uint64_t V)
 	if (clear == kClearByAgent)
 	{
 		const uint32_t old = a.vox[i];
-		if (old != kNoAgent)
+		if (old < V) // not kNoAgent
 			a.counts[old] = 0;
 	}
 	if (a.terms)
@@ -490,14 +490,22 @@ static int run_cells(Context* c, bool recompute)
 		recompute = true;
 	if (recompute)
 	{
-		const int clear = c->counts_follow_vox && c->A * 16 < c->V ? kClearByAgent : kClearArray;
-		c->counts_follow_vox = true; // from the ballot below on
+		// A captured ballot runs when its graph is replayed, any number of times or never,
+		// so it clears the whole array, and a later one relies on nothing it writes.
+		cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+		PCG_CUDA_TRY(cudaStreamIsCapturing(c->stream, &capture));
+		const bool runs = capture == cudaStreamCaptureStatusNone;
+		const int clear = runs && c->counts_follow_vox && c->A * 16 < c->V ? kClearByAgent : kClearArray;
 		// the terms (rates, volume in; three rows out) only after new agent data
 		a.terms = c->terms_dirty ? 1 : 0;
 		const int rc = run_ballot<T>(c, a, clear, c->V, c->stream, c->sm_count);
 		if (rc)
 			return rc;
-		c->terms_dirty = false;
+		if (runs)
+		{
+			c->counts_follow_vox = true;
+			c->terms_dirty = false;
+		}
 		c->ballot_kind = 1;
 	}
 	// per writer: list entry, role, offset, summed (or own) terms, density read and

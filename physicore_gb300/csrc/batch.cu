@@ -723,9 +723,9 @@ __global__ void batch_cells_internalize_kernel(BatchArgs b, const uint32_t* __re
 	const CellArgs& a = b.doms[d].cells;
 	if (!b.steps_left[d] || !a.internalized || !a.A || part >= parts)
 		return;
-	const uint32_t count = __ldg(a.flags + 1);
+	const uint32_t count = a.flags[1];
 	for (uint64_t j = (uint64_t)part * blockDim.x + threadIdx.x; j < count; j += (uint64_t)parts * blockDim.x)
-		agent_internalize<T>(a, __ldg(a.shared + j));
+		agent_internalize<T>(a, a.shared[j]);
 }
 
 // After the sweeps of a step: for every domain with the mass check on that runs
@@ -765,7 +765,7 @@ __global__ void batch_shared_bytes_kernel(const BatchDomain* doms, const uint32_
 	{
 		const CellArgs& a = doms[d].cells;
 		if (steps_left[d] && a.internalized && a.A)
-			acc += (double)__ldg(a.flags + 1) * (8.0 + 4.0 * a.S * wsize + 16.0 * a.S);
+			acc += (double)a.flags[1] * (8.0 + 4.0 * a.S * wsize + 16.0 * a.S);
 	}
 	for (int o = 16; o > 0; o >>= 1)
 		acc += __shfl_xor_sync(0xffffffffu, acc, o);

@@ -229,7 +229,7 @@ template <typename T, int SC>
 __global__ void cells_reduce_kernel(CellArgs a)
 {
 	dev::pdl_wait();
-	const uint32_t count = __ldg(a.flags + a.list_word);
+	const uint32_t count = a.flags[a.list_word];
 	const uint32_t S = SC ? (uint32_t)SC : (uint32_t)a.S;
 	T* rnum = static_cast<T*>(a.rnum);
 	T* rden = static_cast<T*>(a.rden);
@@ -242,9 +242,9 @@ __global__ void cells_reduce_kernel(CellArgs a)
 		uint32_t v = kNoAgent, o = 0;
 		if (j < count)
 		{
-			i = __ldg(a.shared + j);
+			i = a.shared[j];
 			v = a.vox[i];
-			o = __ldg(a.owner + v);
+			o = a.owner[v];
 		}
 		const T* num = static_cast<const T*>(a.num) + i * a.ts;
 		const T* den = static_cast<const T*>(a.den) + i * a.ts;
@@ -300,11 +300,11 @@ template <typename T, int SC>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 1) cells_apply_writers_kernel(CellArgs a)
 {
 	dev::pdl_wait();
-	const uint32_t count = __ldg(a.flags + 3);
+	const uint32_t count = a.flags[3];
 	const bool list = 2ull * count < a.A;
 	const uint64_t n = list ? count : a.A;
 	for (uint64_t j = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; j < n; j += (uint64_t)gridDim.x * blockDim.x)
-		agent_apply<T, SC>(a, list ? __ldg(a.writers + j) : j);
+		agent_apply<T, SC>(a, list ? a.writers[j] : j);
 }
 
 // Over the list of agents in shared voxels (empty when there was no conflict).
@@ -312,9 +312,9 @@ template <typename T, int SC>
 __global__ void cells_internalize_kernel(CellArgs a)
 {
 	dev::pdl_wait();
-	const uint32_t count = __ldg(a.flags + a.list_word);
+	const uint32_t count = a.flags[a.list_word];
 	for (uint64_t j = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; j < count; j += (uint64_t)gridDim.x * blockDim.x)
-		agent_internalize<T, SC>(a, __ldg(a.shared + j));
+		agent_internalize<T, SC>(a, a.shared[j]);
 }
 
 // Both passes of few agents, one to a thread of one block: the agents of shared voxels

@@ -273,11 +273,18 @@ __device__ __forceinline__ void red_add4(float* p, float4 v)
 __device__ __forceinline__ void add_values(float* p, const float* q, uint32_t count, bool quads)
 {
 	if (quads)
-	{
-#pragma unroll 6
-		for (uint32_t k = 0; k < count; k += 4)
-			red_add4(p + k, __ldg(reinterpret_cast<const float4*>(q + k)));
-	}
+		for (uint32_t k0 = 0; k0 < count; k0 += 24)
+		{
+			float4 v[6]; // loaded before the first atomic, which no later load may pass
+#pragma unroll
+			for (int k = 0; k < 6; k++)
+				if (k0 + 4 * k < count)
+					v[k] = *reinterpret_cast<const float4*>(q + k0 + 4 * k);
+#pragma unroll
+			for (int k = 0; k < 6; k++)
+				if (k0 + 4 * k < count)
+					red_add4(p + k0 + 4 * k, v[k]);
+		}
 	else
 		for (uint32_t k = 0; k < count; k++)
 			atomicAdd(p + k, q[k]);
@@ -540,7 +547,7 @@ __device__ __forceinline__ void agent_apply(const CellArgs& a, uint64_t i)
 		return;
 	const bool alone = role == kRoleAlone;
 	const bool track = alone && a.internalized;
-	const bool fused = track && __ldg(a.flags) == 0;
+	const bool fused = track && a.flags[0] == 0;
 	const bool vec = a.vec;
 	const uint32_t S = SC ? (uint32_t)SC : (uint32_t)a.S; // SC: S fixed at compile time (1-8), else 0
 	T* __restrict__ D = static_cast<T*>(a.field) + off;

@@ -553,7 +553,9 @@ __device__ __forceinline__ void fence_proxy_async_smem()
 // Programmatic dependent launch: a kernel launched with launch_chained may start
 // as its predecessor's last CTAs leave; pdl_wait blocks until the predecessor has
 // completed and its writes are visible, and comes before the kernel's first access to
-// global memory.  No kernel lets its successor start any earlier: CTAs that wait
+// global memory.  What earlier kernels of a step write is read by ordinary loads:
+// the read-only path (__ldg) takes data that is constant for the kernel's whole life,
+// which begins before the wait.  No kernel lets its successor start any earlier: CTAs that wait
 // beside a running kernel cost more than they save (96x80x64 x 20: 69 us a step
 // without, 90 with a trigger at each kernel's start, 72 at its end).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

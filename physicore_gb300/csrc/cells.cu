@@ -17,9 +17,9 @@
 //  * ballot: a run of lanes in one voxel counts with one atomic, whose returned
 //    offset ranks the agents of the voxel; rank 0 wins (the reference's first
 //    compare-and-swap wins, cell_solver.cpp:79-101).
-//  * group lists the agents of shared voxels and those that write a voxel; reduce
-//    adds the terms of the shared ones to a row per voxel with four-value atomics
-//    (cell_solver.cpp:102-127); the conflict flag stays on the device, so the step
+//  * group lists the agents of shared voxels and those that write a voxel; sort puts
+//    the shared ones side by side, voxel by voxel, and reduce sums their terms in
+//    registers (cell_solver.cpp:102-127); the conflict flag stays on the device, so the step
 //    never waits on the host (the Thrust backend copies it back every step,
 //    thrust_solver/src/cell_solver.cpp:251-252).
 //  * apply (over the agents that write a voxel) and internalize (over the agents
@@ -54,7 +54,8 @@ __global__ void cells_locate_kernel(CellArgs a, int clear, uint64_t V)
 	dev::pdl_wait();
 	const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
 	if (i == 0)
-		a.flags[0] = a.flags[1] = a.flags[2] = a.flags[3] = 0;
+		for (int k = 0; k < 6; k++)
+			a.flags[k] = 0;
 	if (clear == kClearArray)
 	{
 		const uint64_t k = 4 * i; // the array starts on a 16-byte boundary
@@ -81,7 +82,6 @@ __global__ void cells_locate_kernel(CellArgs a, int clear, uint64_t V)
 // be alone there is marked a winner for now.  Apart from locate, whose FP64
 // conversions and loads it would wait for: its atomics (one per agent, 45 us for the
 // 4M of the dense workload) are all it does.
-template <typename T>
 __global__ void cells_ballot_kernel(CellArgs a)
 {
 	dev::pdl_wait();
@@ -91,23 +91,7 @@ __global__ void cells_ballot_kernel(CellArgs a)
 	if (i >= a.A)
 		return;
 	a.role[i] = v == kNoAgent ? kRoleNone : (rank == 0 ? kRoleWinner : kRoleLoser);
-	if (v != kNoAgent && rank == 1)
-	{
-		// this agent's row takes the voxel's sums (FP64 builds: 1 + sum den; FP32 rows
-		// hold the bare sum, see fp32_update)
-		a.owner[v] = (uint32_t)i;
-		T* rn = static_cast<T*>(a.rnum) + i * a.ts;
-		T* rd = static_cast<T*>(a.rden) + i * a.ts;
-		T* rf = static_cast<T*>(a.rfac) + i * a.ts;
-		if (a.joined)
-			for (uint64_t k = 0; k < a.ts; k++)
-				rn[k] = T(0);
-		for (uint64_t s = 0; s < a.S; s++)
-		{
-			rn[s] = rf[s] = T(0);
-			rd[s] = sizeof(T) == 8 ? T(1) : T(0);
-		}
-	}
+	a.rank[i] = rank;
 }
 
 constexpr unsigned kGroupBlock = 256;
@@ -117,16 +101,19 @@ constexpr unsigned kGroupBlock = 256;
 constexpr uint64_t kGroupWide = 1ull << 20;
 
 // group: final roles (cell_solver.cpp:102-127: every agent but the winner of a shared
-// voxel is a conflict); the agents of shared voxels listed in agent order (flags[2])
-// and, with a writer list, those that write a voxel (alone or winner; flags[3]).  A
-// thread takes Q consecutive agents, of which only the winners need their voxel's
-// count.  A block scans its counts and reserves its ranges with one atomic: atomics on
-// one address serialise.
+// voxel is a conflict); the agents of shared voxels listed (flags[2]) and, with a
+// writer list, those that write a voxel (alone or winner; flags[3]), in agent order
+// within a block.  The winner of a shared voxel reserves a run of slots for its agents
+// (owner[v] = the first one, flags[4] counts slots) and lists the pieces of the run
+// (flags[5]).  A thread takes Q consecutive agents, of which only the winners need
+// their voxel's count.  A block scans its counts and reserves its ranges with two
+// atomics: atomics on one address serialise.
 template <int Q>
-__global__ void __launch_bounds__(kGroupBlock, 6) cells_group_kernel(CellArgs a)
+__global__ void __launch_bounds__(kGroupBlock, 5) cells_group_kernel(CellArgs a)
 {
-	__shared__ uint32_t part[2][kGroupBlock / 32];
-	__shared__ uint32_t base[2], total[2];
+	constexpr int kLists = 4; // shared agents, writers, slots, pieces
+	__shared__ uint32_t part[kLists][kGroupBlock / 32];
+	__shared__ uint32_t base[kLists], total[2];
 	__shared__ uint32_t stage[kGroupBlock * Q];
 	dev::pdl_wait();
 	const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -149,133 +136,262 @@ __global__ void __launch_bounds__(kGroupBlock, 6) cells_group_kernel(CellArgs a)
 #pragma unroll
 	for (uint32_t q = 0; q < Q; q++)
 		cnt[q] = roles.r[q] == kRoleWinner ? a.counts[cnt[q]] : 0u;
+	uint32_t own[kLists] = {};
 #pragma unroll
 	for (uint32_t q = 0; q < Q; q++)
 	{
 		if (roles.r[q] == kRoleWinner)
 		{
-			if (cnt[q] == 1)
-				roles.r[q] = kRoleAlone;
-			else
-				a.sums[i0 + q] = a.owner[a.vox[i0 + q]];
 			writes |= 1u << q;
+			if (cnt[q] == 1)
+			{
+				roles.r[q] = kRoleAlone;
+				cnt[q] = 0;
+			}
 		}
 		if (roles.r[q] >= kRoleWinner)
 			shared |= 1u << q;
+		own[2] += cnt[q]; // of shared voxels only
+		own[3] += pieces_of(cnt[q]);
 	}
 	if (n == Q)
 		*reinterpret_cast<Roles*>(a.role + i0) = roles;
 	else
 		for (uint32_t q = 0; q < n; q++)
 			a.role[i0 + q] = roles.r[q];
-	uint32_t psh = __popc(shared), pwr = a.writers ? __popc(writes) : 0u;
+	own[0] = __popc(shared);
+	own[1] = a.writers ? __popc(writes) : 0u;
+	uint32_t at[kLists];
 #pragma unroll
-	for (uint32_t o = 1; o < 32; o <<= 1)
+	for (int l = 0; l < kLists; l++)
 	{
-		const uint32_t t0 = __shfl_up_sync(0xffffffffu, psh, o), t1 = __shfl_up_sync(0xffffffffu, pwr, o);
-		if (lane >= o)
-			psh += t0, pwr += t1;
+		at[l] = own[l];
+#pragma unroll
+		for (uint32_t o = 1; o < 32; o <<= 1)
+		{
+			const uint32_t t = __shfl_up_sync(0xffffffffu, at[l], o);
+			if (lane >= o)
+				at[l] += t;
+		}
+		if (lane == 31)
+			part[l][warp] = at[l];
+		at[l] -= own[l];
 	}
-	if (lane == 31)
-		part[0][warp] = psh, part[1][warp] = pwr;
 	__syncthreads();
 	if (threadIdx.x == 0)
 	{
-		uint32_t sum[2] = { 0, 0 };
+		uint32_t sum[kLists] = {};
 		for (uint32_t w = 0; w < kGroupBlock / 32; w++)
 #pragma unroll
-			for (int l = 0; l < 2; l++)
+			for (int l = 0; l < kLists; l++)
 			{
 				const uint32_t t = part[l][w];
 				part[l][w] = sum[l];
 				sum[l] += t;
 			}
-		// both lists' ranges with one 64-bit atomic on their adjacent words (neither
-		// total reaches 2^32, so no carry crosses)
-		unsigned long long old = 0ull;
-		if (sum[0] | sum[1])
-			old = atomicAdd(reinterpret_cast<unsigned long long*>(a.flags + 2),
-							((unsigned long long)sum[1] << 32) | (unsigned long long)sum[0]);
+		// two ranges with each 64-bit atomic on adjacent words (no total reaches 2^32,
+		// so no carry crosses)
+#pragma unroll
+		for (int l = 0; l < kLists; l += 2)
+		{
+			unsigned long long old = 0ull;
+			if (sum[l] | sum[l + 1])
+				old = atomicAdd(reinterpret_cast<unsigned long long*>(a.flags + 2 + l),
+								((unsigned long long)sum[l + 1] << 32) | (unsigned long long)sum[l]);
+			base[l] = (uint32_t)old, base[l + 1] = (uint32_t)(old >> 32);
+		}
 		if (sum[0]) // a shared voxel has a loser
 			a.flags[0] = 1;
 		total[0] = sum[0], total[1] = sum[1];
-		base[0] = (uint32_t)old, base[1] = (uint32_t)(old >> 32);
 	}
 	__syncthreads();
 	// the entries, in agent order, through shared memory: a thread's are side by side,
 	// so written directly each store of a warp would touch 32 sectors
 	for (int list = 0; list < (a.writers ? 2 : 1); list++)
 	{
-		uint32_t at = list ? part[1][warp] + pwr - __popc(writes) : part[0][warp] + psh - __popc(shared);
+		uint32_t k = part[list][warp] + (list ? at[1] : at[0]);
 		const uint32_t bits = list ? writes : shared;
 		uint32_t* to = (list ? a.writers : a.shared) + base[list];
 #pragma unroll
 		for (uint32_t q = 0; q < Q; q++)
 			if ((bits >> q) & 1u)
-				stage[at++] = (uint32_t)(i0 + q);
+				stage[k++] = (uint32_t)(i0 + q);
 		__syncthreads();
 		for (uint32_t k = threadIdx.x; k < total[list]; k += kGroupBlock)
 			to[k] = stage[k];
 		__syncthreads();
 	}
+	uint32_t slot = base[2] + part[2][warp] + at[2], piece = base[3] + part[3][warp] + at[3];
+#pragma unroll
+	for (uint32_t q = 0; q < Q; q++)
+	{
+		const uint32_t np = pieces_of(cnt[q]);
+		if (np)
+		{
+			a.owner[a.vox[i0 + q]] = slot;
+			if (np <= 4)
+				for (uint32_t c = 0; c < np; c++)
+					a.pieces[piece + c] = make_piece(slot, cnt[q], c);
+		}
+		// a crowd's pieces by the whole warp
+		for (uint32_t crowds = __ballot_sync(0xffffffffu, np > 4); crowds; crowds &= crowds - 1)
+		{
+			const int l = __ffs(crowds) - 1;
+			const uint32_t s0 = __shfl_sync(0xffffffffu, slot, l), k0 = __shfl_sync(0xffffffffu, cnt[q], l),
+						   p0 = __shfl_sync(0xffffffffu, piece, l);
+			for (uint32_t c = lane; c < pieces_of(k0); c += 32)
+				a.pieces[p0 + c] = make_piece(s0, k0, c);
+		}
+		slot += cnt[q];
+		piece += np;
+	}
 }
 
-// reduce: every agent of a shared voxel adds its terms to its voxel's row.  Four-value atomics run at four times the values per
-// second of single ones (4M agents x 12 values on 182,253 voxels: 76 us against 241;
-// grouping the agents by voxel and summing each group with warp scans took 128).  A
-// warp whose agents all share one voxel (a crowd in one place) sums its terms first
-// and adds them once.
-template <typename T, int SC>
-__global__ void cells_reduce_kernel(CellArgs a)
+// sort: every agent of a shared voxel takes its slot of the voxel's run.  The rows of
+// voxels of several pieces, which add to them, start at zero.  Four consecutive agents
+// a thread, found by their roles: over the list, with an agent a turn, the chain from
+// entry to voxel to slot took 46 us for the 4M agents of the dense workload, 42
+// this way: two random words of L2 per agent.
+template <typename T>
+__global__ void cells_sort_kernel(CellArgs a)
 {
 	dev::pdl_wait();
-	const uint32_t count = a.flags[a.list_word];
-	const uint32_t S = SC ? (uint32_t)SC : (uint32_t)a.S;
-	T* rnum = static_cast<T*>(a.rnum);
-	T* rden = static_cast<T*>(a.rden);
-	T* rfac = static_cast<T*>(a.rfac);
-	for (uint64_t j0 = blockIdx.x * (uint64_t)blockDim.x + (threadIdx.x & ~31u); j0 < count;
-		 j0 += (uint64_t)gridDim.x * blockDim.x)
+	const uint64_t i0 = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) * 4;
+	if (i0 >= a.A)
+		return;
+	const uint32_t n = (uint32_t)min((uint64_t)4, a.A - i0);
+	Values<uint8_t, 4> role {};
+	Values<uint32_t, 4> vox {}, rank {};
+	if (n == 4)
 	{
-		const uint64_t j = j0 + (threadIdx.x & 31);
-		uint64_t i = 0;
-		uint32_t v = kNoAgent, o = 0;
-		if (j < count)
-		{
-			i = a.shared[j];
-			v = a.vox[i];
-			o = a.owner[v];
-		}
-		const T* num = static_cast<const T*>(a.num) + i * a.ts;
-		const T* den = static_cast<const T*>(a.den) + i * a.ts;
-		const T* fac = static_cast<const T*>(a.fac) + i * a.ts;
-		if (__all_sync(0xffffffffu, v == __shfl_sync(0xffffffffu, v, 0)))
-		{
-			for (uint32_t s = 0; s < S; s++)
-			{
-				T x[3] = { num[s], den[s], fac[s] };
+		role = *reinterpret_cast<const Values<uint8_t, 4>*>(a.role + i0);
+		if (max(max(role.t[0], role.t[1]), max(role.t[2], role.t[3])) < kRoleWinner)
+			return;
+		vox = *reinterpret_cast<const Values<uint32_t, 4>*>(a.vox + i0);
+		rank = *reinterpret_cast<const Values<uint32_t, 4>*>(a.rank + i0);
+	}
+	else
+		for (uint32_t q = 0; q < n; q++)
+			role.t[q] = a.role[i0 + q], vox.t[q] = a.vox[i0 + q], rank.t[q] = a.rank[i0 + q];
+	uint32_t first[4];
 #pragma unroll
-				for (int k = 0; k < 3; k++)
-				{
-					for (int d = 16; d > 0; d >>= 1)
-						x[k] += __shfl_xor_sync(0xffffffffu, x[k], d);
-					if ((threadIdx.x & 31) == 0)
-						atomicAdd((k == 0 ? rnum : k == 1 ? rden : rfac) + (uint64_t)o * a.ts + s, x[k]);
-				}
-			}
+	for (int q = 0; q < 4; q++)
+		first[q] = role.t[q] >= kRoleWinner ? a.owner[vox.t[q]] : 0u;
+#pragma unroll
+	for (int q = 0; q < 4; q++)
+	{
+		if (role.t[q] < kRoleWinner)
 			continue;
-		}
-		if (v == kNoAgent)
+		a.sorted[first[q] + rank.t[q]] = (uint32_t)(i0 + q);
+		if (rank.t[q] != 0 || a.counts[vox.t[q]] <= kPiece)
 			continue;
-		const uint64_t row = (uint64_t)o * a.ts;
-		if (a.joined) // FP32 rows are padded to whole quads
-			add_values(rnum + row, num, sizeof(T) == 4 ? (3 * S + 3) / 4 * 4 : 3 * S, true);
+		T* rows[3] = { static_cast<T*>(a.rnum), static_cast<T*>(a.rden), static_cast<T*>(a.rfac) };
+		for (int k = 0; k < (a.joined ? 1 : 3); k++)
+			for (uint64_t s = 0; s < (a.joined ? a.ts : a.S); s++)
+				rows[k][(i0 + q) * a.ts + s] = T(0);
+	}
+}
+
+// N values side by side of the rows of `count` agents of `list` (1 to 8), summed in pairs.
+template <typename T, int N>
+__device__ __forceinline__ void sum_rows(const T* rows, uint64_t ts, const uint32_t* list, uint32_t count, T (&s)[N])
+{
+	uint32_t i[8];
+	Values<T, N> x[8];
+#pragma unroll
+	for (uint32_t k = 0; k < 8; k++)
+		i[k] = k < count ? list[k] : 0u;
+#pragma unroll
+	for (uint32_t k = 0; k < 8; k++)
+		if (k < count)
+			x[k] = *reinterpret_cast<const Values<T, N>*>(rows + i[k] * ts);
 		else
+			x[k] = Values<T, N> {};
+#pragma unroll
+	for (int n = 0; n < N; n++)
+	{
+		s[n] = x[0].t[n] + x[1].t[n];
+		if (count > 2)
+			s[n] += x[2].t[n] + x[3].t[n];
+		if (count > 4)
 		{
-			add_values(rnum + row, num, S, a.vec);
-			add_values(rden + row, den, S, a.vec);
-			add_values(rfac + row, fac, S, a.vec);
+			T u = x[4].t[n] + x[5].t[n];
+			if (count > 6)
+				u += x[6].t[n] + x[7].t[n];
+			s[n] += u;
 		}
+	}
+}
+
+// Values [e, e + N) of a piece's rows: summed in pairs (at most five roundings for 32
+// agents) and stored to the winner's row, or added to it where the voxel has several
+// pieces.
+template <typename T, int N>
+__device__ __forceinline__ void reduce_piece(const CellArgs& a, uint2 piece, uint32_t e, uint32_t S)
+{
+	const uint32_t len = piece_len(piece), c = piece_number(piece);
+	const uint32_t* list = a.sorted + piece.x + c * kPiece;
+	const uint32_t arr = N == 1 ? e / S : 0, s0 = N == 1 ? e % S : e; // N == 1: three arrays
+	const T* rows = static_cast<const T*>(arr == 0 ? a.num : arr == 1 ? a.den : a.fac) + s0;
+	T* to = static_cast<T*>(arr == 0 ? a.rnum : arr == 1 ? a.rden : a.rfac) + s0 + a.sorted[piece.x] * a.ts;
+	Values<T, N> sum;
+	T u[N], w[N];
+	sum_rows<T, N>(rows, a.ts, list, min(len, 8u), sum.t);
+	if (len > 8)
+	{
+		sum_rows<T, N>(rows, a.ts, list + 8, min(len - 8, 8u), u);
+#pragma unroll
+		for (int n = 0; n < N; n++)
+			sum.t[n] += u[n];
+	}
+	if (len > 16)
+	{
+		sum_rows<T, N>(rows, a.ts, list + 16, min(len - 16, 8u), u);
+		if (len > 24)
+		{
+			sum_rows<T, N>(rows, a.ts, list + 24, len - 24, w);
+#pragma unroll
+			for (int n = 0; n < N; n++)
+				u[n] += w[n];
+		}
+#pragma unroll
+		for (int n = 0; n < N; n++)
+			sum.t[n] += u[n];
+	}
+	if (sizeof(T) == 8 && c == 0) // FP64 rows hold 1 + sum den, FP32 rows the bare sum (fp32_update)
+#pragma unroll
+		for (int n = 0; n < N; n++)
+			if (e + n >= S && e + n < 2 * S)
+				sum.t[n] += T(1);
+	if (piece_alone(piece))
+		*reinterpret_cast<Values<T, N>*>(to) = sum;
+	else
+		add_values(to, sum.t);
+}
+
+// reduce: the sums of every shared voxel (cell_solver.cpp:102-127), a thread for 16
+// bytes of the rows of a piece (a value of one of the three arrays where they are
+// apart).  Bound by the gather of rows in random order (4M agents, 182,253 voxels, S = 4:
+// 90 us, 6 blocks per SM with fewer registers 114).  One atomic per agent and quad takes
+// the same 90 us and no sort, but rounds the sum of k agents k times (1.3e-5 off at
+// 1,000 equal agents in FP32) and serialises on crowds (a ballot of 1M agents in 4 voxels, S = 4:
+// 1,231 us against 198; FP64 3,423 against 291).
+template <typename T, int SC>
+__global__ void __launch_bounds__(256) cells_reduce_kernel(CellArgs a)
+{
+	dev::pdl_wait();
+	constexpr int N = 16 / sizeof(T);
+	const uint32_t S = SC ? (uint32_t)SC : (uint32_t)a.S;
+	const uint32_t np = a.flags[5], parts = a.joined ? (3 * S + N - 1) / N : 3 * S;
+	const uint64_t items = (uint64_t)np * parts, stride = (uint64_t)gridDim.x * blockDim.x;
+	for (uint64_t w = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; w < items; w += stride)
+	{
+		const uint2 piece = a.pieces[w / parts];
+		const uint32_t q = (uint32_t)(w % parts);
+		if (a.joined)
+			reduce_piece<T, N>(a, piece, q * N, S);
+		else
+			reduce_piece<T, 1>(a, piece, q, S);
 	}
 }
 
@@ -291,7 +407,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 1) cells_apply_kerne
 }
 
 // Over the agents that write a voxel (alone or winner; flags[3] of them, listed
-// by classify) when they are fewer than half the agents, else over every agent
+// by group) when they are fewer than half the agents, else over every agent
 // (agent_apply returns at once for the others): with many agents per voxel most
 // agents only lose their ballot, and a thread per agent would mostly wait on its
 // role byte.  Grid-stride, so the grid need not match the device-side count.
@@ -412,7 +528,9 @@ CellArgs make_cell_args(const Context* c)
 	a.vec = rows_vectorizable(a, c->wsize);
 	a.terms = 1;
 	a.pairs = c->wsize == 4 ? 1 : 0; // FP32 contexts store internalized amounts as float pairs
-	a.sums = static_cast<uint32_t*>(c->a_sums.ptr);
+	a.rank = static_cast<uint32_t*>(c->a_rank.ptr);
+	a.sorted = static_cast<uint32_t*>(c->a_sorted.ptr);
+	a.pieces = static_cast<uint2*>(c->a_pieces.ptr);
 	a.joined = 1;
 	a.writers = static_cast<uint32_t*>(c->a_writers.ptr);
 	a.list_word = 2; // (a batch sets 1 for its per-warp ballot)
@@ -432,8 +550,11 @@ static int run_ballot(Context* c, const CellArgs& a, int clear, uint64_t V, cuda
 	const bool wide = a.A > kGroupWide;
 	const uint64_t per_block = (uint64_t)kGroupBlock * (wide ? 8 : 4);
 	const unsigned ggrid = (unsigned)((a.A + per_block - 1) / per_block);
-	// the list of shared-voxel agents is only known on the device: grid-stride
-	const unsigned lgrid = std::min<unsigned>(grid, 24 * std::max(sm_count, 1));
+	// the number of pieces, at most A / 2 (a shared voxel holds two agents or more), is
+	// only known on the device: grid-stride
+	const uint64_t parts = a.joined ? a.ts * sizeof(T) / 16 : 3 * a.S;
+	const unsigned rgrid =
+		(unsigned)std::min<uint64_t>((a.A / 2 * parts + block) / block, 24 * (uint64_t)std::max(sm_count, 1));
 	const double S = (double)a.S, A = (double)a.A, w = (double)sizeof(T);
 	cudaEvent_t ev = nullptr;
 	const uint64_t threads = clear == kClearArray ? std::max<uint64_t>(a.A, (V + 3) / 4) : a.A;
@@ -446,14 +567,14 @@ static int run_ballot(Context* c, const CellArgs& a, int clear, uint64_t V, cuda
 								V));
 	if (c)
 		launch_end(c, K_CELLS_LOCATE, ev);
-	// voxel in, role out, one count updated
+	// voxel in, role and rank out, one count updated
 	if (c)
-		launch_begin(c, K_CELLS_BALLOT, A * (4 + 1 + 8), &ev);
-	PCG_CUDA_TRY(launch_chained(cells_ballot_kernel<T>, grid, block, 0, stream, a));
+		launch_begin(c, K_CELLS_BALLOT, A * (4 + 1 + 4 + 8), &ev);
+	PCG_CUDA_TRY(launch_chained(cells_ballot_kernel, grid, block, 0, stream, a));
 	if (c)
 		launch_end(c, K_CELLS_BALLOT, ev);
 	// per agent its role in and out; shared-voxel agents and writers: list entry;
-	// writers: voxel and count
+	// writers: voxel and count (and, in shared voxels, first slot and pieces)
 	if (c)
 		launch_begin(c, K_CELLS_GROUP, 2 * A, &ev);
 	PCG_CUDA_TRY(launch_chained(wide ? cells_group_kernel<8> : cells_group_kernel<4>, ggrid, kGroupBlock, 0, stream, a));
@@ -465,12 +586,18 @@ static int run_ballot(Context* c, const CellArgs& a, int clear, uint64_t V, cuda
 	}
 	if (c)
 		launch_end(c, K_CELLS_GROUP, ev, 4.0, 12.0);
-	// per shared-voxel agent: list entry, voxel, its row's index, role and terms
+	// per agent its role; per shared-voxel agent: voxel, rank, its voxel's first slot; its slot
+	if (c)
+		launch_begin(c, K_CELLS_SORT, A, &ev);
+	PCG_CUDA_TRY(launch_chained(cells_sort_kernel<T>, (unsigned)((a.A + 4 * block - 1) / (4 * block)), block, 0, stream, a));
+	if (c)
+		launch_end(c, K_CELLS_SORT, ev, 16.0);
+	// per shared-voxel agent: slot and terms
 	if (c)
 		launch_begin(c, K_CELLS_REDUCE, 0.0, &ev);
-	PCG_LAUNCH_BY_S(cells_reduce_kernel, T, a.S, lgrid, block, stream, a);
+	PCG_LAUNCH_BY_S(cells_reduce_kernel, T, a.S, rgrid, block, stream, a);
 	if (c)
-		launch_end(c, K_CELLS_REDUCE, ev, 13.0 + 3 * S * w);
+		launch_end(c, K_CELLS_REDUCE, ev, 4.0 + 3 * S * w);
 	return PCG_OK;
 }
 
@@ -587,7 +714,9 @@ int launch_cells_fp32_buffers(const CellStepBuffers& b, cudaStream_t stream)
 	a.vec = rows_vectorizable(a, sizeof(float));
 	a.terms = 1;
 	a.pairs = 0; // the caller's FP64 amounts
-	a.sums = b.sums;
+	a.rank = b.rank;
+	a.sorted = b.sorted;
+	a.pieces = b.pieces;
 	a.joined = 0;
 	a.list_word = 2;
 	set_fast_locate(a);

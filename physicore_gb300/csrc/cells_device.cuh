@@ -50,8 +50,8 @@ struct CellArgs
 	uint32_t* counts;
 	uint8_t* role;    // [A] ballot role
 	uint32_t* shared; // [A] agents of voxels that hold several, flags[list_word] of them
-	uint32_t* flags;  // [0] conflict; entries of `shared` in word list_word; [3] writers
-	uint32_t list_word; // 1 (batches: per-warp ballot) or 2 (single domain; word 3 = writers)
+	uint32_t* flags;  // [0] conflict; entries of `shared` in word list_word
+	uint32_t list_word; // 1 (batches: per-warp ballot) or 2 (single domain; words 3, 4, 5 = writers, slots, pieces)
 	uint32_t* err;
 	void* field;
 	int internalized;
@@ -62,10 +62,14 @@ struct CellArgs
 	// mesh's bounds or voxel edges are not exactly representable in FP32
 	float mf[3], rf[3], nf[3]; // nf: grid sides
 	int fast;
-	uint32_t* sums; // [A], single domain: the row that holds a shared voxel's sums, at its winner
+	// single domain: ballot rank of each agent, and the agents of shared voxels side by
+	// side, voxel by voxel in the order of their ranks, in pieces of at most kPiece
+	uint32_t* rank;   // [A]
+	uint32_t* sorted; // [A]
+	uint2* pieces;    // [A / 2]
 	int joined;     // num, den and fac of an agent are one row of ts values (so are the sums)
 	// a context's own (null for caller-owned buffers): the agents that write a voxel,
-	// flags[3] of them, in agent order (apply walks them instead of every agent)
+	// flags[3] of them (apply walks them instead of every agent)
 	uint32_t* writers;
 };
 
@@ -268,31 +272,22 @@ __device__ __forceinline__ void red_add4(float* p, float4 v)
 				 : "memory");
 }
 
-// Adds `count` values to p, four at a time where both start on 16-byte boundaries and
-// count is a multiple of four (quads).
-__device__ __forceinline__ void add_values(float* p, const float* q, uint32_t count, bool quads)
+// Adds `count` values to p, four at a time: both start on 16-byte boundaries and count
+// is a multiple of four.
+__device__ __forceinline__ void add_quads(float* p, const float* q, uint32_t count)
 {
-	if (quads)
-		for (uint32_t k0 = 0; k0 < count; k0 += 24)
-		{
-			float4 v[6]; // loaded before the first atomic, which no later load may pass
+	for (uint32_t k0 = 0; k0 < count; k0 += 24)
+	{
+		float4 v[6]; // loaded before the first atomic, which no later load may pass
 #pragma unroll
-			for (int k = 0; k < 6; k++)
-				if (k0 + 4 * k < count)
-					v[k] = *reinterpret_cast<const float4*>(q + k0 + 4 * k);
+		for (int k = 0; k < 6; k++)
+			if (k0 + 4 * k < count)
+				v[k] = *reinterpret_cast<const float4*>(q + k0 + 4 * k);
 #pragma unroll
-			for (int k = 0; k < 6; k++)
-				if (k0 + 4 * k < count)
-					red_add4(p + k0 + 4 * k, v[k]);
-		}
-	else
-		for (uint32_t k = 0; k < count; k++)
-			atomicAdd(p + k, q[k]);
-}
-__device__ __forceinline__ void add_values(double* p, const double* q, uint32_t count, bool)
-{
-	for (uint32_t k = 0; k < count; k++)
-		atomicAdd(p + k, q[k]);
+		for (int k = 0; k < 6; k++)
+			if (k0 + 4 * k < count)
+				red_add4(p + k0 + 4 * k, v[k]);
+	}
 }
 
 // Sums into the winner's row (cell_solver.cpp:102-127) and records agent i's
@@ -323,11 +318,12 @@ __device__ __forceinline__ uint8_t agent_reduce(const CellArgs& a, uint64_t i)
 	T* rnum = static_cast<T*>(a.rnum);
 	T* rden = static_cast<T*>(a.rden);
 	T* rfac = static_cast<T*>(a.rfac);
-	if (sizeof(T) == 4 && a.joined)
-	{
-		add_values(rnum + (uint64_t)w * a.ts, num + i * a.ts, (uint32_t)a.ts, true);
-		return role;
-	}
+	if constexpr (sizeof(T) == 4)
+		if (a.joined)
+		{
+			add_quads(rnum + (uint64_t)w * a.ts, num + i * a.ts, (uint32_t)a.ts);
+			return role;
+		}
 	for (uint64_t s = 0; s < a.S; s++)
 	{
 		const uint64_t k = i * a.ts + s;
@@ -364,13 +360,42 @@ __device__ __forceinline__ void list_shared(const CellArgs& a, uint64_t i, bool 
 //   ballot:  a count per voxel (one atomic per run of lanes in the voxel) whose
 //            returned offset ranks the agent in its voxel.  Rank 0, the agent whose
 //            atomic landed first, wins (as the first compare-and-swap wins in the
-//            reference); rank 1, which only a shared voxel has, lends its row to the
-//            voxel's sums and clears it
+//            reference)
 //   group:   roles (a winner alone in its voxel or not); the agents of shared voxels
-//            are listed in agent order (for reduce and the internalized pass), so are
-//            the agents that write a voxel (for apply)
-//   reduce:  every agent of a shared voxel adds its terms to the voxel's row, four
-//            FP32 values per atomic
+//            are listed (for sort and the internalized pass), so are the agents that
+//            write a voxel (for apply); a run of slots per shared voxel, cut into
+//            pieces of at most kPiece agents
+//   sort:    every agent of a shared voxel into its slot: first slot + rank
+//   reduce:  the rows of a piece's agents summed in registers, in pairs
+
+constexpr uint32_t kPiece = 32;
+
+// A piece: x the voxel's first slot, y its number in the voxel (26 bits), whether it is
+// the only one, and its agents less one (5 bits).
+__device__ __forceinline__ uint2 make_piece(uint32_t slot, uint32_t count, uint32_t c)
+{
+	return make_uint2(slot, (c << 6) | (count <= kPiece ? 32u : 0u) | (min(count - c * kPiece, kPiece) - 1));
+}
+__device__ __forceinline__ uint32_t pieces_of(uint32_t count) { return count / kPiece + (count % kPiece != 0); }
+__device__ __forceinline__ uint32_t piece_len(uint2 p) { return (p.y & 31u) + 1; }
+__device__ __forceinline__ bool piece_alone(uint2 p) { return (p.y & 32u) != 0; }
+__device__ __forceinline__ uint32_t piece_number(uint2 p) { return p.y >> 6; }
+
+// N values that move together: 16 bytes, or one.
+template <typename T, int N>
+struct alignas(N * sizeof(T)) Values
+{
+	T t[N];
+};
+
+__device__ __forceinline__ void add_values(float* p, const float (&v)[4]) { red_add4(p, make_float4(v[0], v[1], v[2], v[3])); }
+template <typename T, int N>
+__device__ __forceinline__ void add_values(T* p, const T (&v)[N])
+{
+#pragma unroll
+	for (int n = 0; n < N; n++)
+		atomicAdd(p + n, v[n]);
+}
 
 // Runs of equal keys among the lanes of a warp: the first lane of the caller's run
 // and the first lane after it (32 at the end of the warp).  All lanes call it.
@@ -541,8 +566,6 @@ __device__ __forceinline__ void agent_apply(const CellArgs& a, uint64_t i)
 {
 	const uint8_t role = a.role[i];
 	const uint32_t off = a.foff[i];
-	// a winner's sums: in its own row (batches), or the one its voxel was lent
-	const uint64_t lent = a.list_word == 1 ? i : (uint64_t)a.sums[i];
 	if (role == kRoleNone || role == kRoleLoser)
 		return;
 	const bool alone = role == kRoleAlone;
@@ -551,7 +574,7 @@ __device__ __forceinline__ void agent_apply(const CellArgs& a, uint64_t i)
 	const bool vec = a.vec;
 	const uint32_t S = SC ? (uint32_t)SC : (uint32_t)a.S; // SC: S fixed at compile time (1-8), else 0
 	T* __restrict__ D = static_cast<T*>(a.field) + off;
-	const uint64_t row = (alone ? i : lent) * a.ts;
+	const uint64_t row = i * a.ts;
 	const T* __restrict__ rn = static_cast<const T*>(alone ? a.num : a.rnum) + row;
 	const T* __restrict__ rd = static_cast<const T*>(alone ? a.den : a.rden) + row;
 	const T* __restrict__ rf = static_cast<const T*>(alone ? a.fac : a.rfac) + row;

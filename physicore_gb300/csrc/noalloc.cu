@@ -14,9 +14,9 @@
 
 namespace {
 
-// 16 MiB of scratch: 8 bytes per voxel (row of its sums + count) plus 25 + 24*S bytes
-// per agent (voxel index, field offset, shared-voxel list entry, row of its voxel's
-// sums, 8 spare bytes, ballot role, six FP32 terms per substrate).
+// 16 MiB of scratch: 8 bytes per voxel (first slot + count) plus 25 + 24*S bytes per
+// agent (voxel index, field offset, shared-voxel list entry, rank in the voxel, slot,
+// half a piece, ballot role, six FP32 terms per substrate).
 constexpr size_t kScratchBytes = size_t(16) << 20;
 
 static __device__ __align__(256) unsigned char g_scratch[kScratchBytes];
@@ -96,8 +96,8 @@ extern "C" int pcg_cells_noalloc(float* field, uint64_t pitch, int dims, const i
 					"pcg_cells_noalloc: the mesh and agents need more than the fixed " + std::to_string(kScratchBytes) +
 						" bytes of scratch (about 8 bytes per voxel + (25 + 24*S) bytes per agent)");
 
-	// scratch layout: flags | err | owner[V] | counts[V] | vox[A] | foff[A] | shared[A] | sums[A] | 8 spare bytes per
-	// agent | role[A] | 6 x terms[A*S]
+	// scratch layout: flags | err | owner[V] | counts[V] | vox[A] | foff[A] | shared[A] | rank[A] | sorted[A], pieces[A/2]
+	// | role[A] | 6 x terms[A*S]
 	size_t off = 0;
 	const size_t o_flags = off;
 	off += 256;
@@ -113,9 +113,11 @@ extern "C" int pcg_cells_noalloc(float* field, uint64_t pitch, int dims, const i
 	off = align256(off + agents * 4);
 	const size_t o_shared = off;
 	off = align256(off + agents * 4);
-	const size_t o_sums = off;
+	const size_t o_rank = off;
 	off = align256(off + agents * 4);
-	off = align256(off + agents * 8); // spare: the problem sizes the entry point takes stay what they were
+	const size_t o_pieces = off; // 8-byte entries first
+	const size_t o_sorted = off + agents / 2 * 8;
+	off = align256(off + agents * 8);
 	const size_t o_role = off;
 	off = align256(off + agents);
 	size_t o_terms[6];
@@ -168,7 +170,9 @@ extern "C" int pcg_cells_noalloc(float* field, uint64_t pitch, int dims, const i
 	b.vox = reinterpret_cast<uint32_t*>(base + o_vox);
 	b.foff = reinterpret_cast<uint32_t*>(base + o_foff);
 	b.shared = reinterpret_cast<uint32_t*>(base + o_shared);
-	b.sums = reinterpret_cast<uint32_t*>(base + o_sums);
+	b.rank = reinterpret_cast<uint32_t*>(base + o_rank);
+	b.sorted = reinterpret_cast<uint32_t*>(base + o_sorted);
+	b.pieces = reinterpret_cast<uint2*>(base + o_pieces);
 	b.role = base + o_role;
 	float** t[6] = { &b.num, &b.den, &b.fac, &b.rnum, &b.rden, &b.rfac };
 	for (int k = 0; k < 6; k++)

@@ -64,6 +64,7 @@ enum KernelId : int
 	K_CELLS_CLEAR,
 	K_MASS_CHECK,
 	K_CELLS_GROUP,
+	K_CELLS_SORT,
 	K_SWEEP_XY,
 	K_COUNT
 };
@@ -242,7 +243,7 @@ struct Context
 	uint32_t xy_nseg = 0, xy_total = 0, xy_nslab = 0;
 	DeviceBuffer xy_segs, xy_done;
 	DeviceBuffer flags;    // uint32 [8]: [0] ballot conflict, [1] agents in shared voxels (batches),
-	                       // [2] and [3] a single domain's list lengths (cells_device.cuh)
+	                       // [2..5] a single domain's list lengths (cells_device.cuh)
 	DeviceBuffer mass;     // double [S]
 	// per-step mass check (pcg_set_mass_check): FP64 totals [2 * S] before the
 	// first sweep and after the last one, added by the sweeps themselves, and
@@ -298,7 +299,9 @@ struct Context
 	DeviceBuffer a_foff;                  // uint32 [A]: field offset of the voxel's first substrate
 	DeviceBuffer a_role;                  // uint8 [A]: ballot role (cells_device.cuh)
 	DeviceBuffer a_shared;                // uint32 [A]: agents of voxels that hold several
-	DeviceBuffer a_sums;                  // uint32 [A]: at the winner of a shared voxel, the row of its sums
+	DeviceBuffer a_rank;                  // uint32 [A]: rank of the agent in its voxel
+	DeviceBuffer a_sorted;                // uint32 [A]: agents of shared voxels, voxel by voxel
+	DeviceBuffer a_pieces;                // uint2 [A / 2]: their runs in pieces (cells_device.cuh)
 	DeviceBuffer a_writers;               // uint32 [A]: agents that write a voxel (alone or winner)
 	// the ballot behind the cached roles, lists and reduced rows: 0 none, 1 a
 	// single-domain step's, 2 a batch's per-warp ballot (their lists differ, so a step
@@ -308,8 +311,8 @@ struct Context
 	uint64_t term_stride = 0;             // values per agent row of a_terms and a_reduced
 	DeviceBuffer a_terms;                 // real [A][term_stride]: num, den, fac of the agent (S each)
 	DeviceBuffer a_reduced;               // real [A][term_stride]: sums over a shared voxel
-	DeviceBuffer owner;                   // uint32 [V]: winning agent per voxel (batches), or the agent
-										  // whose row holds a shared voxel's sums (single domain)
+	DeviceBuffer owner;                   // uint32 [V]: winning agent per voxel (batches), or the first
+										  // slot of a shared voxel (single domain)
 	DeviceBuffer counts;                  // uint32 [V]: active agents per voxel
 
 	// measurement
@@ -383,8 +386,10 @@ struct CellStepBuffers
 	double* internal;
 	int internalized;
 	float* field;
-	// scratch: vox/foff/shared/sums/role [A], owner/counts [V], flags/err [4] each, terms [A*S] each
-	uint32_t *vox, *foff, *shared, *sums, *owner, *counts, *flags, *err;
+	// scratch: vox/foff/shared/rank/sorted/role [A], pieces [A/2], owner/counts [V], flags [8], err [4], terms
+	// [A*S] each
+	uint32_t *vox, *foff, *shared, *rank, *sorted, *owner, *counts, *flags, *err;
+	uint2* pieces;
 	uint8_t* role;
 	float *num, *den, *fac, *rnum, *rden, *rfac;
 };

@@ -215,9 +215,11 @@ __device__ __forceinline__ bool sweep_all(bool ok)
 // its mc_tot.
 //
 // Registers are capped so that shared memory and not the register file sets how many
-// CTAs an SM holds (FP32 otherwise took 222 a thread: 149 -> 181 us on 48 domains).
+// CTAs an SM holds (FP32 otherwise took 222 a thread: 149 -> 181 us on 48 domains;
+// FP64 at 128 instead of 168 and 255, with one solver for scaled and unscaled domains:
+// x 230 -> 210, y 245 -> 220, z 428 -> 344 us on 48 domains of 1 to 6 substrates).
 template <typename T, int MC, bool SCALED, bool MULTI>
-__global__ void __launch_bounds__(sweep_threads<T>(), sizeof(T) == 4 ? 16 : 5) batch_sweep_x_kernel(BatchArgs b)
+__global__ void __launch_bounds__(sweep_threads<T>(), sizeof(T) == 4 ? 16 : 8) batch_sweep_x_kernel(BatchArgs b)
 {
 	extern __shared__ __align__(128) unsigned char smem[];
 	uint64_t* bar = reinterpret_cast<uint64_t*>(smem);
@@ -296,15 +298,11 @@ __global__ void __launch_bounds__(sweep_threads<T>(), sizeof(T) == 4 ? 16 : 5) b
 			ao.zero();
 			const Strided<T, 0, 1> left { row, S };
 			const Strided<T, 0, -1> right { row + (n - 1) * S, S };
-			if (SCALED && D.scaled[0])
-			{
-				const T* scale = static_cast<const T*>(D.sc[0]) + sc;
-				if constexpr (SCALED)
-					solve_tile<T, Strided<T, 0, 1>, Strided<T, 0, -1>, MC, 1>(
-						left, right, n, half, on, L, line_scale(T(1), __ldg(scale), scale + S, (int)S, n, half), &ai, &ao);
-			}
-			else
-				solve_tile<T, Strided<T, 0, 1>, Strided<T, 0, -1>, MC, 0>(left, right, n, half, on, L, {}, &ai, &ao);
+			LineScale<T> F { T(1), T(1), false };
+			if constexpr (SCALED)
+				if (D.scaled[0])
+					F = { T(1), __ldg(static_cast<const T*>(D.sc[0]) + sc), true };
+			solve_tile<T, Strided<T, 0, 1>, Strided<T, 0, -1>, MC, SCALED>(left, right, n, half, on, L, F, &ai, &ao);
 			if constexpr (MC != 0)
 				if (mc)
 				{
@@ -345,11 +343,11 @@ struct FaceRef
 // mbarrier, the warps solve their halves of it in place, and the boxes are stored
 // back before the next tile is requested (several CTAs per SM overlap these phases).
 // SCALED (FP64): some domain's sweep of this axis applies the scale factors (its last
-// sweep, or factors not deferred).  MC (mass check in this batch): on the domain's last
+// sweep, or factors not deferred); the others multiply by 1.  MC (mass check in this batch): on the domain's last
 // sweep, each tile's solved totals (before its faces are written) go to the domain's
 // mc_tot.
 template <typename T, int AXIS, int MC, bool SCALED>
-__global__ void __launch_bounds__(sweep_threads<T>()) batch_sweep_yz_kernel(BatchArgs b)
+__global__ void __launch_bounds__(sweep_threads<T>(), sizeof(T) == 8 ? 8 : 1) batch_sweep_yz_kernel(BatchArgs b)
 {
 	extern __shared__ __align__(128) unsigned char smem[];
 	uint64_t* full = reinterpret_cast<uint64_t*>(smem);
@@ -462,24 +460,19 @@ __global__ void __launch_bounds__(sweep_threads<T>()) batch_sweep_yz_kernel(Batc
 			acc.zero();
 			const Strided<T, kLanes, 1> left { tile + lane, 0 };
 			const Strided<T, kLanes, -1> right { tile + (n - 1) * kLanes + lane, 0 };
-			if (SCALED && D.scaled[AXIS])
-			{
-				if constexpr (SCALED)
+			LineScale<T> F { T(1), T(1), false };
+			if constexpr (SCALED)
+				if (D.scaled[AXIS])
 				{
 					T g = T(1);
 					if (D.gx && D.dims == AXIS + 1)
 						g = __ldg(static_cast<const T*>(D.gx) + (in_row ? col : 0));
 					if (AXIS == 2 && D.gy)
 						g *= __ldg(static_cast<const T*>(D.gy) + (uint64_t)s * D.n[1] + o);
-					const T* scale = static_cast<const T*>(D.sc[AXIS]);
-					solve_tile<T, Strided<T, kLanes, 1>, Strided<T, kLanes, -1>, MC, 1>(
-						left, right, n, half, true, L, line_scale(g, __ldg(scale + s), scale + S + (uint64_t)s * n, 1, n, half),
-						nullptr, &acc);
+					F = { g, g * __ldg(static_cast<const T*>(D.sc[AXIS]) + s), true };
 				}
-			}
-			else
-				solve_tile<T, Strided<T, kLanes, 1>, Strided<T, kLanes, -1>, MC, 0>(left, right, n, half, true, L, {}, nullptr,
-																					&acc);
+			solve_tile<T, Strided<T, kLanes, 1>, Strided<T, kLanes, -1>, MC, SCALED>(left, right, n, half, true, L, F, nullptr,
+																					 &acc);
 			if (D.dims == AXIS + 1)
 			{
 				if constexpr (MC != 0)

@@ -497,10 +497,10 @@ static uint64_t coefficient_table_fp32(const Context* c, int axis, std::vector<f
 }
 
 // FP64 table of one axis for the two-sided solve (sweep_solvers.cuh), in doubles:
-//   [E rows S x H | G rows S x H | e | ws | wl | wr, S each | converged factor S |
-//    factors: axis 0 at [i*S + s], the others at [s*n + i]]
-// E[j] = e_{j-1} (0 for j = 0) and G[j] = e_{j+1} for the H head points counted from a
-// line's end, e the value they converge to, b' the factors (mirrored about the
+//   [E rows S x H | G rows S x H | F rows S x H | e | ws | wl | wr, S each |
+//    converged factor S | factors: axis 0 at [i*S + s], the others at [s*n + i]]
+// E[j] = e_{j-1} (0 for j = 0), G[j] = e_{j+1} and F[j] = b'_j for the H head points
+// counted from a line's end, e the value e_j converges to, b' the factors (mirrored about the
 // meeting point), and at the meeting point, with tl = e and tr = e of the two halves'
 // last points, ws = 1 / (1 - tl tr), wl = ws tr, wr = ws tl.  *shrink: the smallest
 // factor.
@@ -533,7 +533,7 @@ static uint64_t coefficient_table_fp64(const Context* c, int axis, std::vector<d
 		H = std::max(H, h + 1);
 	}
 	H = round_up(H, kBlockPoints);
-	const uint64_t head = S * H, k = 2 * head;
+	const uint64_t head = S * H, k = 3 * head;
 	*scale_off = k + 4 * S;
 	tab.assign(*scale_off + S + n * S, 0.0);
 	double* sc = tab.data() + *scale_off;
@@ -543,6 +543,7 @@ static uint64_t coefficient_table_fp64(const Context* c, int axis, std::vector<d
 		{
 			tab[s * H + j] = j ? e[(j - 1) * S + s] : 0.0;
 			tab[head + s * H + j] = e[std::min(j + 1, L - 1) * S + s];
+			tab[2 * head + s * H + j] = b[j * S + s];
 		}
 		const double tl = e[(m - 1) * S + s], tr = lr ? e[(lr - 1) * S + s] : 0.0;
 		const double ws = lr ? 1 / (1 - tl * tr) : 1.0;

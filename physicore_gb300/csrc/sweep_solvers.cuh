@@ -34,6 +34,8 @@ namespace solvers {
 constexpr int kBlock = 8; // recurrence steps per pipelined block
 
 // Threads of a sweep CTA: a warp per tile (FP32), or one for each half of its lines.
+// FP64 kernels are compiled for 8 CTAs an SM (128 registers), 16 warps: with the 168 of
+// 6 CTAs, 64^3 x 8, 1024 tiles, took 24, 24 and 36 us for x, y and z instead of 19, 19 and 27.
 template <typename T>
 constexpr int sweep_threads()
 {
@@ -172,14 +174,13 @@ template <typename T>
 struct LineCoef;
 
 // The scale factors of one lane's half line at the last FP64 sweep: g the column's
-// factor from the other axes, mid = g times the converged factor, and the line's own
-// factors in memory (point j of the half at row[j * step]) for the head points.
+// factor from the other axes, mid = g times the line's converged factor (the head
+// points' are in LineCoef).
 template <typename T>
 struct LineScale
 {
 	double g, mid;
-	const double* row;
-	int step;
+	bool on; // false: g and mid are 1 and the line's own factors are left out
 };
 
 // ------------------------------------------------------------------ FP32
@@ -419,6 +420,7 @@ struct LineCoef<double>
 {
 	const double* hE; // inward coefficients of the head points
 	const double* hG; // outward
+	const double* hF; // scale factors
 	uint32_t H;
 	double e;
 	double ws, wo; // meeting point: weights of the half's own and the other half's value
@@ -427,24 +429,16 @@ struct LineCoef<double>
 __device__ __forceinline__ LineCoef<double> line_coef(const double* tab, uint32_t S, uint32_t H, uint32_t, uint32_t s,
 													  uint32_t half)
 {
-	const double* k = tab + 2 * S * H + s;
+	const double* k = tab + 3 * S * H + s;
 	LineCoef<double> L;
 	L.hE = tab + s * H;
 	L.hG = tab + (S + s) * H;
+	L.hF = tab + (2 * S + s) * H;
 	L.H = H;
 	L.e = __ldg(k);
 	L.ws = __ldg(k + S);
 	L.wo = __ldg(k + (2 + half) * S);
 	return L;
-}
-
-// The scale factors of a lane's half line from the axis's table: `sc` points at the
-// factor of the line's point 0, `step` separates its points', `mid` is the converged
-// one.
-__device__ __forceinline__ LineScale<double> line_scale(double g, double mid, const double* sc, int step, uint32_t n,
-														uint32_t half)
-{
-	return { g, g * mid, half == 0 ? sc : sc + (int64_t)(n - 1) * step, half == 0 ? step : -step };
 }
 
 // The 8 head coefficients from point j on.
@@ -482,6 +476,7 @@ __device__ __forceinline__ double solve_inward(const AC& ac, uint32_t len, const
 		double x[P], xn[P], c[P], cn[P];
 		ac.load(0, x);
 		head_block(L.hE, 0, c);
+#pragma unroll 1
 		for (uint32_t b = 0; b < hb; b++)
 		{
 			if (b + 1 < hb)
@@ -546,7 +541,6 @@ __device__ __forceinline__ void solve_outward(const AC& ac, uint32_t len, const 
 	const uint32_t nb = len / P, hb = min(L.H / P, nb);
 	ac.at(len - 1) = ymeet; // the recurrence then starts from a zero carry
 	double y = 0.0;
-	auto factor = [&](uint32_t j) { return F.g * __ldg(F.row + (int64_t)((int)j * F.step)); };
 	auto mid = [&](uint32_t b, double(&x)[P]) {
 #pragma unroll
 		for (int k = P - 1; k >= 0; k--)
@@ -561,7 +555,7 @@ __device__ __forceinline__ void solve_outward(const AC& ac, uint32_t len, const 
 	for (int j = (int)len - 1; j >= (int)(nb * P); j--)
 	{
 		y = dev::fmadd((uint32_t)j < L.H ? __ldg(L.hG + j) : L.e, y, ac.at(j));
-		const double o = SC ? y * ((uint32_t)j < L.H ? factor(j) : F.mid) : y;
+		const double o = SC ? y * ((uint32_t)j < L.H ? (F.on ? F.g * __ldg(L.hF + j) : 1.0) : F.mid) : y;
 		ac.at(j) = o;
 		if constexpr ((MC & kMcOut) != 0)
 			acc->add(o);
@@ -587,20 +581,19 @@ __device__ __forceinline__ void solve_outward(const AC& ac, uint32_t len, const 
 		else
 			mid(b, xa);
 	}
+#pragma unroll 1
 	for (int b = (int)hb - 1; b >= 0; b--)
 	{
 		double x[P], c[P], f[P];
 		ac.load((uint32_t)b * P, x);
 		head_block(L.hG, (uint32_t)b * P, c);
 		if constexpr (SC != 0)
-#pragma unroll
-			for (int k = 0; k < P; k++)
-				f[k] = factor((uint32_t)(b * P + k));
+			head_block(L.hF, (uint32_t)b * P, f);
 #pragma unroll
 		for (int k = P - 1; k >= 0; k--)
 		{
 			y = dev::fmadd(c[k], y, x[k]);
-			x[k] = SC ? y * f[k] : y;
+			x[k] = SC ? y * (F.on ? F.g * f[k] : 1.0) : y;
 		}
 		if constexpr ((MC & kMcOut) != 0)
 			acc->add_block(x);

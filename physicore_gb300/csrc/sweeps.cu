@@ -56,7 +56,7 @@ using namespace solvers;
 // running total and adds it once at the end), else it adds its total per tile.
 // BULK (the step's last sweep where bulk_fusable): the bulk update after the faces.
 template <typename T, int AXIS, int MC, int SC, bool BULK>
-__global__ void __launch_bounds__(sweep_threads<T>()) sweep_yz_kernel(SweepArgs a, const __grid_constant__ CUtensorMap tmap)
+__global__ void __launch_bounds__(sweep_threads<T>(), sizeof(T) == 8 ? 8 : 1) sweep_yz_kernel(SweepArgs a, const __grid_constant__ CUtensorMap tmap)
 {
 	extern __shared__ __align__(128) unsigned char smem[];
 	uint64_t* full = reinterpret_cast<uint64_t*>(smem);
@@ -112,8 +112,7 @@ __global__ void __launch_bounds__(sweep_threads<T>()) sweep_yz_kernel(SweepArgs 
 				g = __ldg(static_cast<const T*>(a.gx) + (in_row ? col : 0));
 			if (AXIS == 2 && a.gy)
 				g *= __ldg(static_cast<const T*>(a.gy) + (uint64_t)s * a.ny + o);
-			const T* sc = static_cast<const T*>(a.sc);
-			F = line_scale(g, __ldg(sc + s), sc + S + (uint64_t)s * n, 1, n, half);
+			F = { g, g * __ldg(static_cast<const T*>(a.sc) + s), true };
 		}
 		ok = __syncthreads_and(dev::mbar_wait(full, phase));
 		if (!ok)
@@ -175,7 +174,7 @@ __global__ void __launch_bounds__(sweep_threads<T>()) sweep_yz_kernel(SweepArgs 
 // and, on a 1-D mesh, outputs (kMcOut), added once at the end (per line when S is
 // above 32).
 template <typename T, int ST, int MC, int SC, bool VEC>
-__global__ void __launch_bounds__(sweep_threads<T>()) sweep_x_kernel(SweepArgs a)
+__global__ void __launch_bounds__(sweep_threads<T>(), sizeof(T) == 8 ? 8 : 1) sweep_x_kernel(SweepArgs a)
 {
 	constexpr bool kWide = ST < 0;
 	constexpr int STRIDE = ST > 0 ? ST : 0;
@@ -233,10 +232,7 @@ __global__ void __launch_bounds__(sweep_threads<T>()) sweep_x_kernel(SweepArgs a
 					L = line_coef(static_cast<const T*>(a.tab), S, a.head, n, min(s, S - 1), half);
 				LineScale<T> F {};
 				if constexpr (SC != 0)
-				{
-					const T* sc = static_cast<const T*>(a.sc) + min(s, S - 1);
-					F = line_scale(T(1), __ldg(sc), sc + S, (int)S, n, half);
-				}
+					F = { T(1), __ldg(static_cast<const T*>(a.sc) + min(s, S - 1)), true };
 				solve_tile<T, Strided<T, STRIDE, 1>, Strided<T, STRIDE, -1>, MC, SC>(
 					{ row + s, S }, { row + (n - 1) * S + s, S }, n, half, on, L, F, &ai, &ao);
 				if constexpr (MC != 0 && kWide)

@@ -883,9 +883,8 @@ static int alloc_agents(Context* c, uint64_t A)
 		return rc;
 	if ((rc = dalloc(c, c->a_shared, std::max<uint64_t>(A, 1) * sizeof(uint32_t))))
 		return rc;
-	for (DeviceBuffer* b : { &c->a_rank, &c->a_sorted, &c->a_pieces }) // a piece (8 bytes) per two agents
-		if ((rc = dalloc(c, *b, std::max<uint64_t>(A, 1) * sizeof(uint32_t))))
-			return rc;
+	if ((rc = dalloc(c, c->a_order, std::max<uint64_t>(round_up(A, 4), 4) * 3 * sizeof(uint32_t))))
+		return rc;
 	if ((rc = dalloc(c, c->a_writers, std::max<uint64_t>(A, 1) * sizeof(uint32_t))))
 		return rc;
 	c->term_stride = term_stride(S, w);
@@ -1079,7 +1078,7 @@ int pcg_destroy(pcg_context* c)
 								 &c->a_active,	 &c->a_internal, &c->a_frac,	&c->a_foff,		 &c->a_terms,
 								 &c->a_reduced,
 								 &c->owner,		 &c->counts,	&c->a_role,		&c->a_shared,	 &c->rb_staging[0],
-								 &c->rb_staging[1], &c->a_rank,	&c->a_sorted,	&c->a_pieces,	&c->a_writers,	 &c->xy_segs,
+								 &c->rb_staging[1], &c->a_order,	&c->a_writers,	 &c->xy_segs,
 								 &c->xy_done };
 	for (auto* b : all)
 		pcg::dfree(*b);

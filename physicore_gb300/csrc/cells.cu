@@ -528,9 +528,9 @@ CellArgs make_cell_args(const Context* c)
 	a.vec = rows_vectorizable(a, c->wsize);
 	a.terms = 1;
 	a.pairs = c->wsize == 4 ? 1 : 0; // FP32 contexts store internalized amounts as float pairs
-	a.rank = static_cast<uint32_t*>(c->a_rank.ptr);
-	a.sorted = static_cast<uint32_t*>(c->a_sorted.ptr);
-	a.pieces = static_cast<uint2*>(c->a_pieces.ptr);
+	a.rank = static_cast<uint32_t*>(c->a_order.ptr);
+	a.sorted = a.rank + round_up(c->A, 4); // each on a 16-byte boundary
+	a.pieces = reinterpret_cast<uint2*>(a.sorted + round_up(c->A, 4));
 	a.joined = 1;
 	a.writers = static_cast<uint32_t*>(c->a_writers.ptr);
 	a.list_word = 2; // (a batch sets 1 for its per-warp ballot)

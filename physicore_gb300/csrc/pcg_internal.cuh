@@ -299,9 +299,8 @@ struct Context
 	DeviceBuffer a_foff;                  // uint32 [A]: field offset of the voxel's first substrate
 	DeviceBuffer a_role;                  // uint8 [A]: ballot role (cells_device.cuh)
 	DeviceBuffer a_shared;                // uint32 [A]: agents of voxels that hold several
-	DeviceBuffer a_rank;                  // uint32 [A]: rank of the agent in its voxel
-	DeviceBuffer a_sorted;                // uint32 [A]: agents of shared voxels, voxel by voxel
-	DeviceBuffer a_pieces;                // uint2 [A / 2]: their runs in pieces (cells_device.cuh)
+	DeviceBuffer a_order;                 // single-domain ballot (cells_device.cuh): uint32 [A] ranks, uint32 [A] agents
+										  // of shared voxels by voxel, uint2 [A / 2] their pieces
 	DeviceBuffer a_writers;               // uint32 [A]: agents that write a voxel (alone or winner)
 	// the ballot behind the cached roles, lists and reduced rows: 0 none, 1 a
 	// single-domain step's, 2 a batch's per-warp ballot (their lists differ, so a step

@@ -981,8 +981,12 @@ uint64_t estimate_device_bytes(const Context* c)
 	const uint64_t row_len = c->n[0] * S, pitch = round_up(row_len, 32 / w), rows = c->n[1] * c->n[2];
 	uint64_t b = rows * pitch * w;               // field
 	b += V * S * w;                              // staging of pcg_get_field / pcg_set_field
-	for (int a = 0; a < c->dims; a++)            // coefficient tables (full and compressed; FP32: with lo parts)
-		b += (7 * c->n[a] * S + 96 * S + 64) * w;
+	for (int a = 0; a < c->dims; a++)            // coefficient tables with the longest heads
+	{
+		const uint64_t n = c->n[a];
+		b += w == 4 ? (3 * S * round_up(n, kBlockPoints) + 7 * round_up(S, 4)) * w
+					: (3 * S * round_up(n / 2 + 4, kBlockPoints) + (5 + n) * S) * w;
+	}
 	b += 3 * 256 + 2 * S * 8;                    // words, mass
 	b += c->K * (8 + S * (w + 1)) + 12 * S * (w + 1);
 	if (c->bulk_mode == PCG_BULK_UNIFORM)
@@ -990,7 +994,9 @@ uint64_t estimate_device_bytes(const Context* c)
 	else if (c->bulk_mode == PCG_BULK_PER_VOXEL)
 		b += 3 * rows * pitch * w;
 	if (A)
-		b += A * (c->dims * 8 + 6 * S * 8 + 8 + 1 + 8 + 5 + 16 + 2 * term_stride(S, w) * w) + V * 8;
+		// positions, six rates and amounts, volume, activity, offset and voxel, role and list
+		// entries, ballot order, terms and sums; counts and owners of the voxels
+		b += A * (c->dims * 8 + 6 * S * 8 + 8 + 1 + 8 + 1 + 8 + 2 * term_stride(S, w) * w) + 12 * round_up(A, 4) + V * 8;
 	return b;
 }
 

@@ -347,7 +347,7 @@ struct FaceRef
 // sweep, each tile's solved totals (before its faces are written) go to the domain's
 // mc_tot.
 template <typename T, int AXIS, int MC, bool SCALED>
-__global__ void __launch_bounds__(sweep_threads<T>(), sizeof(T) == 8 ? 8 : 1) batch_sweep_yz_kernel(BatchArgs b)
+__global__ void __launch_bounds__(sweep_threads<T>(), sizeof(T) == 8 ? 8 : 0) batch_sweep_yz_kernel(BatchArgs b)
 {
 	extern __shared__ __align__(128) unsigned char smem[];
 	uint64_t* full = reinterpret_cast<uint64_t*>(smem);

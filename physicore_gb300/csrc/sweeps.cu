@@ -56,7 +56,7 @@ using namespace solvers;
 // running total and adds it once at the end), else it adds its total per tile.
 // BULK (the step's last sweep where bulk_fusable): the bulk update after the faces.
 template <typename T, int AXIS, int MC, int SC, bool BULK>
-__global__ void __launch_bounds__(sweep_threads<T>(), sizeof(T) == 8 ? 8 : 1) sweep_yz_kernel(SweepArgs a, const __grid_constant__ CUtensorMap tmap)
+__global__ void __launch_bounds__(sweep_threads<T>(), sizeof(T) == 8 ? 8 : 0) sweep_yz_kernel(SweepArgs a, const __grid_constant__ CUtensorMap tmap)
 {
 	extern __shared__ __align__(128) unsigned char smem[];
 	uint64_t* full = reinterpret_cast<uint64_t*>(smem);
@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(sweep_threads<T>(), sizeof(T) == 8 ? 8 : 1) sw
 // and, on a 1-D mesh, outputs (kMcOut), added once at the end (per line when S is
 // above 32).
 template <typename T, int ST, int MC, int SC, bool VEC>
-__global__ void __launch_bounds__(sweep_threads<T>(), sizeof(T) == 8 ? 8 : 1) sweep_x_kernel(SweepArgs a)
+__global__ void __launch_bounds__(sweep_threads<T>(), sizeof(T) == 8 ? 8 : 0) sweep_x_kernel(SweepArgs a)
 {
 	constexpr bool kWide = ST < 0;
 	constexpr int STRIDE = ST > 0 ? ST : 0;

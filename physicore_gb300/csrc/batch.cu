@@ -302,7 +302,7 @@ __global__ void __launch_bounds__(sweep_threads<T>(), sizeof(T) == 4 ? 16 : 8) b
 			if constexpr (SCALED)
 				if (D.scaled[0])
 					F = { T(1), __ldg(static_cast<const T*>(D.sc[0]) + sc), true };
-			solve_tile<T, Strided<T, 0, 1>, Strided<T, 0, -1>, MC, SCALED>(left, right, n, half, on, L, F, &ai, &ao);
+			solve_tile<T, Strided<T, 0, 1>, Strided<T, 0, -1>, MC, SCALED, true>(left, right, n, half, on, L, F, &ai, &ao);
 			if constexpr (MC != 0)
 				if (mc)
 				{
@@ -471,7 +471,7 @@ __global__ void __launch_bounds__(sweep_threads<T>(), sizeof(T) == 8 ? 8 : 0) ba
 						g *= __ldg(static_cast<const T*>(D.gy) + (uint64_t)s * D.n[1] + o);
 					F = { g, g * __ldg(static_cast<const T*>(D.sc[AXIS]) + s), true };
 				}
-			solve_tile<T, Strided<T, kLanes, 1>, Strided<T, kLanes, -1>, MC, SCALED>(left, right, n, half, true, L, F, nullptr,
+			solve_tile<T, Strided<T, kLanes, 1>, Strided<T, kLanes, -1>, MC, SCALED, true>(left, right, n, half, true, L, F, nullptr,
 																					 &acc);
 			if (D.dims == AXIS + 1)
 			{

@@ -7,7 +7,7 @@
 // (both from a zero carry; b' as a pair hi + lo).  These sweeps move their bytes at
 // the copy bandwidth; what a shorter chain would save they do not wait for.
 //
-// FP64: the FP64 pipe sets the pace (one warp instruction per 16 cycles of an SM, with
+// FP64: the FP64 pipe sets the pace (one warp instruction per 20 cycles of an SM, with
 // a latency of several of those), so the line is solved with the fewest
 // operations and in two halves side by side.  It is eliminated from both ends
 // towards a meeting point and solved outwards from there (a twisted factorisation of
@@ -20,10 +20,11 @@
 // and the line's solution is b'_j y_j.  That factor depends on the substrate and the
 // position along the swept axis only, so it commutes with the sweeps of the other
 // axes: a step's sweeps leave it out and the last one multiplies by the product
-// (SC = 1): 7 FP64 operations per point and 3-D step instead of 9, and 1 in the
-// dependent chain of a point instead of 3.  A mesh whose factors would let the values
+// (SC = 1): 7 FP64 operations per point and 3-D step instead of 9 (8 at the head
+// points, whose factor is formed per point), and 1 in the dependent chain of a point
+// instead of 3.  A mesh whose factors would let the values
 // between the sweeps grow past 2^20 of the field's applies them in every sweep.
-// 160x144x128, 3 substrates: x 96.5 -> 56.3, y 84.5 -> 56.7, z 80.4 -> 79.7 us.
+// 160x144x128, 3 substrates: x 97 -> 58, y 86 -> 56, z 80 -> 75 us.
 #pragma once
 
 #include "pcg_internal.cuh"
@@ -253,9 +254,15 @@ __device__ __forceinline__ float coef_at(const float* head, uint32_t H, float mi
 // register sets, so that its blocks carry no copies or tests.  Which run a block
 // is in is the same for every lane of a warp (one n and H per launch).
 //
+// SMALL keeps the loops rolled: the batched y and z, with more code around the
+// solver, waited on instruction fetches with the compiler's own unrolling (990 served
+// requests: y 8.87 -> 8.52, z 9.09 -> 8.81 ms; 256 domains 2.29 -> 2.22 ms a step).  One
+// domain's kernels keep the unrolling, which long lines gain from (30,000 x 1: 340
+// instead of 364 us).
+//
 // MC (kMcIn / kMcOut bits) adds the line's input values to *acc_in and its
 // solved values to *acc_out.
-template <class AC, int MC>
+template <class AC, int MC, bool SMALL>
 __device__ __forceinline__ void solve_line(const AC& ac, uint32_t n, const LineCoef<float>& L, MassAcc<float>* acc_in,
 										   MassAcc<float>* acc_out)
 {
@@ -291,8 +298,7 @@ __device__ __forceinline__ void solve_line(const AC& ac, uint32_t n, const LineC
 		float e[P], en[P];
 		ac.load((0) * P, x);
 		fetch_head(L.hE, 0, e);
-		for (uint32_t b = 0; b < hb; b++)
-		{
+		auto fwd_head = [&](uint32_t b) {
 			if (b + 1 < hb)
 			{
 				ac.load((b + 1) * P, xn);
@@ -310,20 +316,37 @@ __device__ __forceinline__ void solve_line(const AC& ac, uint32_t n, const LineC
 				x[k] = xn[k];
 				e[k] = en[k];
 			}
+		};
+		if constexpr (SMALL)
+		{
+#pragma unroll 1
+			for (uint32_t b = 0; b < hb; b++)
+				fwd_head(b);
 		}
+		else
+			for (uint32_t b = 0; b < hb; b++)
+				fwd_head(b);
 	}
 	if (hb < q)
 	{
 		float xa[P], xb[P];
 		uint32_t b = hb;
 		ac.load((b) * P, xa);
-		for (; b + 2 < q; b += 2)
-		{
+		auto fwd_two = [&](uint32_t b) {
 			ac.load((b + 1) * P, xb);
 			fwd_mid(b, xa);
 			ac.load((b + 2) * P, xa);
 			fwd_mid(b + 1, xb);
+		};
+		if constexpr (SMALL)
+		{
+#pragma unroll 1
+			for (; b + 2 < q; b += 2)
+				fwd_two(b);
 		}
+		else
+			for (; b + 2 < q; b += 2)
+				fwd_two(b);
 		if (b + 1 < q)
 		{
 			ac.load((b + 1) * P, xb);
@@ -333,25 +356,41 @@ __device__ __forceinline__ void solve_line(const AC& ac, uint32_t n, const LineC
 		else
 			fwd_mid(b, xa);
 	}
-	for (uint32_t j = q * P; j < n; j++)
-	{
+	auto fwd_last = [&](uint32_t j) {
 		const float xj = ac.at(j);
 		if constexpr ((MC & kMcIn) != 0)
 			acc_in->add(xj);
 		d = dev::fmadd(coef_at(L.hE, L.H, L.mE, L.lE, n, j), d, xj);
 		ac.at(j) = d;
+	};
+	if constexpr (SMALL)
+	{
+#pragma unroll 1
+		for (uint32_t j = q * P; j < n; j++)
+			fwd_last(j);
 	}
+	else
+		for (uint32_t j = q * P; j < n; j++)
+			fwd_last(j);
 
 	// ---- back substitution
 	d = 0.f;
-	for (int j = (int)n - 1; j >= (int)(q * P); j--)
-	{
-		const float bl = coef_at(L.hBl, L.H, L.mBl, L.lBl, n, (uint32_t)j);
-		d = bwd_step(c, d, ac.at((uint32_t)j), coef_at(L.hB, L.H, L.mB, L.lB, n, (uint32_t)j), bl);
-		ac.at((uint32_t)j) = d;
+	auto bwd_last = [&](uint32_t j) {
+		const float bl = coef_at(L.hBl, L.H, L.mBl, L.lBl, n, j);
+		d = bwd_step(c, d, ac.at(j), coef_at(L.hB, L.H, L.mB, L.lB, n, j), bl);
+		ac.at(j) = d;
 		if constexpr ((MC & kMcOut) != 0)
 			acc_out->add(d);
+	};
+	if constexpr (SMALL)
+	{
+#pragma unroll 1
+		for (uint32_t j = n; j-- > q * P;)
+			bwd_last(j);
 	}
+	else
+		for (uint32_t j = n; j-- > q * P;)
+			bwd_last(j);
 	auto bwd_mid = [&](uint32_t b, float(&x)[P]) {
 #pragma unroll
 		for (int k = P - 1; k >= 0; k--)
@@ -365,13 +404,21 @@ __device__ __forceinline__ void solve_line(const AC& ac, uint32_t n, const LineC
 		float xa[P], xb[P];
 		uint32_t b = q - 1;
 		ac.load((b) * P, xa);
-		for (; b >= hb + 2; b -= 2)
-		{
+		auto bwd_two = [&](uint32_t b) {
 			ac.load((b - 1) * P, xb);
 			bwd_mid(b, xa);
 			ac.load((b - 2) * P, xa);
 			bwd_mid(b - 1, xb);
+		};
+		if constexpr (SMALL)
+		{
+#pragma unroll 1
+			for (; b >= hb + 2; b -= 2)
+				bwd_two(b);
 		}
+		else
+			for (; b >= hb + 2; b -= 2)
+				bwd_two(b);
 		if (b >= hb + 1)
 		{
 			ac.load((b - 1) * P, xb);
@@ -388,20 +435,19 @@ __device__ __forceinline__ void solve_line(const AC& ac, uint32_t n, const LineC
 		ac.load((hb - 1) * P, x);
 		fetch_head(L.hB, hb - 1, bb);
 		fetch_head(L.hBl, hb - 1, bl);
-		for (int b = (int)hb - 1; b >= 0; b--)
-		{
+		auto bwd_head = [&](uint32_t b) {
 			if (b > 0)
 			{
-				ac.load(((uint32_t)b - 1) * P, xn);
-				fetch_head(L.hB, (uint32_t)b - 1, bn);
-				fetch_head(L.hBl, (uint32_t)b - 1, bln);
+				ac.load((b - 1) * P, xn);
+				fetch_head(L.hB, b - 1, bn);
+				fetch_head(L.hBl, b - 1, bln);
 			}
 #pragma unroll
 			for (int k = P - 1; k >= 0; k--)
 				x[k] = d = bwd_step(c, d, x[k], bb[k], bl[k]);
 			if constexpr ((MC & kMcOut) != 0)
 				acc_out->add_block(x);
-			ac.store((uint32_t)b * P, x);
+			ac.store(b * P, x);
 #pragma unroll
 			for (int k = 0; k < P; k++)
 			{
@@ -409,7 +455,16 @@ __device__ __forceinline__ void solve_line(const AC& ac, uint32_t n, const LineC
 				bb[k] = bn[k];
 				bl[k] = bln[k];
 			}
+		};
+		if constexpr (SMALL)
+		{
+#pragma unroll 1
+			for (uint32_t b = hb; b-- > 0;)
+				bwd_head(b);
 		}
+		else
+			for (uint32_t b = hb; b-- > 0;)
+				bwd_head(b);
 	}
 }
 
@@ -610,7 +665,7 @@ __device__ __forceinline__ void solve_outward(const AC& ac, uint32_t len, const 
 // barriers.  FP32: the CTA's one warp solves whole lines.  FP64: warp `half` solves
 // its half of them; two barriers separate the reads of the other half's meeting
 // value from the writes around them (a line without a second half needs none).
-template <typename T, class ACL, class ACR, int MC, int SC>
+template <typename T, class ACL, class ACR, int MC, int SC, bool SMALL = false>
 __device__ __forceinline__ void solve_tile(const ACL& left, const ACR& right, uint32_t n, uint32_t half, bool on,
 										   const LineCoef<T>& L, const LineScale<T>& F, MassAcc<T>* acc_in = nullptr,
 										   MassAcc<T>* acc_out = nullptr)
@@ -618,7 +673,7 @@ __device__ __forceinline__ void solve_tile(const ACL& left, const ACR& right, ui
 	if constexpr (sizeof(T) == 4)
 	{
 		if (on)
-			solve_line<ACL, MC>(left, n, L, acc_in, acc_out);
+			solve_line<ACL, MC, SMALL>(left, n, L, acc_in, acc_out);
 	}
 	else
 	{

@@ -38,7 +38,6 @@ using namespace cellsdev;
 // How locate clears the counts for the ballot after it.
 enum : int
 {
-	kClearNone = 0,    // they hold zeros already
 	kClearByAgent = 1, // over the voxels that the last ballot recorded: zero everywhere else
 	kClearArray = 2,   // every count, four to a thread (threads beyond the agents too)
 };

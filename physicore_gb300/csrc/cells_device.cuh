@@ -251,21 +251,6 @@ __device__ __forceinline__ void agent_locate(const CellArgs& a, uint64_t i)
 	}
 }
 
-// Ballot of one warp (cell_solver.cpp:79-101 with a canonical winner).  `key`
-// must be unique per voxel across everything the warp holds (kNoAgent for none);
-// the lanes of a warp hold ascending agent indices of one domain per group.
-__device__ __forceinline__ void warp_ballot(const CellArgs* a, uint64_t i, uint32_t v, uint32_t key)
-{
-	const uint32_t group = __match_any_sync(0xffffffffu, key);
-	if (key == kNoAgent)
-		return;
-	if ((threadIdx.x & 31) == __ffs(group) - 1)
-	{
-		atomicMin(a->owner + v, (uint32_t)i); // the leader holds the group's lowest index
-		atomicAdd(a->counts + v, (uint32_t)__popc(group));
-	}
-}
-
 __device__ __forceinline__ void red_add4(float* p, float4 v)
 {
 	asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
